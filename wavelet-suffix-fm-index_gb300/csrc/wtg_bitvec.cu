@@ -29,145 +29,23 @@ WTG_WAIT_LIMIT_SETTER(bitvec)
 
 constexpr int BV_THREADS = 256;  // one 512-bit superblock per thread
 
-__device__ __forceinline__ uint64_t warp_max_u64(uint64_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    uint64_t t = __shfl_xor_sync(0xffffffffu, v, o);
-    v = t > v ? t : v;
-  }
-  return v;
-}
-
-// One pass over the bitvector: lane per 64-bit word, 8 lanes per 512-bit
-// superblock, a tile of 256 superblocks per CTA (coalesced 2 KB rows), one
-// decoupled look-back scan of the tile one-counts.
-constexpr int BVT_ITER = 8;                        // rows of 256 words per tile
-constexpr int BVT_SB = BVT_ITER * BV_THREADS / 8;  // superblocks per tile
-
-__global__ void __launch_bounds__(BV_THREADS)
-    bv_pass_kernel(const uint64_t* __restrict__ words, uint64_t size, uint64_t W, uint64_t NB, uint32_t flags,
-                   uint64_t* __restrict__ rank, uint32_t* __restrict__ samples, uint64_t samp_last,
-                   uint64_t* __restrict__ starts1, uint64_t* __restrict__ starts0, uint64_t* __restrict__ ends1,
-                   uint64_t* __restrict__ ends0, unsigned long long* info, uint64_t* status, uint32_t* counter,
-                   uint32_t* err) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_sb[BVT_SB];
-  __shared__ uint64_t s_prefix;
-  if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
-  __syncthreads();
-  const uint32_t tile = s_tile;
-  if (tile >= gridDim.x) return;  // only when the counter did not start at 0 (a stalled pass)
-  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane & 7;
-  const uint64_t wbase = (uint64_t)tile * (BVT_ITER * BV_THREADS);
-  const uint64_t tailmask = (size & 63) ? ((1ull << (size & 63)) - 1) : ~0ull;
-  uint64_t w[BVT_ITER];
-  uint32_t c[BVT_ITER], inc[BVT_ITER];
-#pragma unroll
-  for (int j = 0; j < BVT_ITER; ++j) {
-    const uint64_t wi = wbase + j * BV_THREADS + tid;
-    uint64_t x = wi < W ? __ldg(&words[wi]) : 0ull;
-    if (wi == W - 1) x &= tailmask;
-    w[j] = x;
-    c[j] = __popcll(x);
-    uint32_t v = c[j];
-#pragma unroll
-    for (int o = 1; o < 8; o <<= 1) {  // inclusive scan within the superblock's 8 lanes
-      const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-      if (g8 >= (uint32_t)o) v += t;
-    }
-    inc[j] = v;
-    if (g8 == 7) s_sb[j * (BV_THREADS / 8) + warp * 4 + (lane >> 3)] = v;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    constexpr int PER = BVT_SB / 32;
-    uint32_t loc[PER];
-    uint32_t sum = 0;
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      loc[q] = s_sb[lane * PER + q];
-      sum += loc[q];
-    }
-    uint32_t incw = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incw, o);
-      if (lane >= (uint32_t)o) incw += t;
-    }
-    uint32_t run = incw - sum;
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-      s_sb[lane * PER + q] = run;
-      run += loc[q];
-    }
-    const uint64_t total = __shfl_sync(0xffffffffu, incw, 31);
-    uint64_t prefix = 0;
-    if (tile == 0) {
-      if (lane == 0) lb_publish(status, tile, LB_FLAG_INC, total);
-    } else {
-      if (lane == 0) lb_publish(status, tile, LB_FLAG_AGG, total);
-      prefix = lb_lookback_warp(status, tile, err);
-      if (lane == 0) lb_publish(status, tile, LB_FLAG_INC, prefix + total);
-    }
-    if (lane == 0) s_prefix = prefix;
-  }
-  __syncthreads();
-  const uint64_t tprefix = s_prefix;
-  const uint64_t r_last = W - 8 * NB;  // words of the final superblock
-  uint64_t last1 = 0, last0 = 0;
-#pragma unroll
-  for (int j = 0; j < BVT_ITER; ++j) {
-    const uint32_t sbl = j * (BV_THREADS / 8) + warp * 4 + (lane >> 3);
-    const uint64_t b = (uint64_t)tile * BVT_SB + sbl;  // superblock
-    const uint64_t wi = wbase + j * BV_THREADS + tid;
-    const uint64_t sb_before = tprefix + s_sb[sbl];    // ones before the superblock
-    const uint32_t excl = inc[j] - c[j];               // ones before the word in its superblock
-    const uint32_t sbt = __shfl_sync(0xffffffffu, inc[j], (lane & ~7u) + 7);  // ones in the superblock
-    if (flags & WTG_RANK) {
-      // field k (1..7) = count before block k; the final superblock writes
-      // only fields 1..max(r,1), r = its words (rank_support_v_par.hpp:99-108)
-      const uint32_t kmax = (b < NB) ? 7u : (r_last > 1 ? (uint32_t)r_last : 1u);
-      uint64_t part = (g8 >= 1 && g8 <= kmax) ? ((uint64_t)excl << (63 - 9 * g8)) : 0ull;
-#pragma unroll
-      for (int o = 1; o < 8; o <<= 1) part |= __shfl_xor_sync(0xffffffffu, part, o);
-      if (g8 == 0 && b <= NB) {
-        rank[2 * b] = sb_before;
-        rank[2 * b + 1] = part;
-      }
-    }
-    if (b == NB && g8 == 0) {
-      info[INF_M1] = sb_before + sbt;
-      info[INF_M0] = size - (sb_before + sbt);
-    }
-    if (wi < W)
-      word_marks(w[j], c[j], sb_before + excl, wi, wi == W - 1 ? tailmask : ~0ull, flags & WTG_SELECT1,
-                 flags & WTG_SELECT0, samples, samp_last, starts1, starts0, ends1, ends0, last1, last0);
-  }
-  last1 = warp_max_u64(last_arg_end(words, last1, W, tailmask, 1));
-  last0 = warp_max_u64(last_arg_end(words, last0, W, tailmask, 0));
-  if (lane == 0) {
-    if (last1) atomicMax(&info[INF_LAST1], (unsigned long long)last1);
-    if (last0) atomicMax(&info[INF_LAST0], (unsigned long long)last0);
-  }
-}
-
-// position after the last one (t_b = 1) or zero (t_b = 0) of superblock sb
-// (eight words, all inside the bitvector); read through L2
-__device__ __forceinline__ uint64_t last_arg_end_sb(const uint64_t* __restrict__ words, uint64_t sb, int t_b) {
-  for (int j = 7; j >= 0; --j) {
-    uint64_t x = __ldcg(words + 8 * sb + j);
-    if (!t_b) x = ~x;
-    if (x) return ((8 * sb + j) << 6) + hi64(x) + 1;
-  }
-  return 0;
-}
-
-// Rank table and select samples of a wavelet tree's concatenated bitvector
-// when n % 512 == 0: superblock b is chunk c of level l (b = l * n/512 + c),
-// and the zeros before it are the zeros of the levels before l (lvl_zb) plus
-// the chunk's prefix within its level (the level passes' chunk counts,
-// scanned) -- no scan over the bits.  Levels l0..l1-1; thread per
-// superblock, grid-stride over each level's superblocks.
+// The pass over the bits.  A tile is SPT * 256 superblocks of 512 bits; the
+// tile's one-count is published, the ones before it come from a decoupled
+// look-back (word-count scan, no second pass over a count array), and every
+// superblock then gets its rank entry and select marks.  Thread per
+// superblock: its eight words in four 16-byte loads, popcount prefix and the
+// seven 9-bit fields in registers, one 16-byte rank entry.  A warp takes SPT
+// runs of 32 consecutive superblocks, so a run's counts are one warp scan.
+// With SPT = 4 the words are counted first and read again (from L2, the tile
+// is 64 KB) for the marks: a quarter of the look-backs, and few registers
+// held across the wait; SPT = 1 keeps a short bitvector on more SMs.
+// CTAs are resident and take tiles from a counter, in order.
+// One kernel serves every bitvector.  Bound by the integer ALU pipe.  Lanes
+// per word (8 to a superblock) with 64-bit arithmetic took 167 us for 842
+// Mbit and 226 us for 1.2 Gbit; this takes 83 us for the 842 Mbit (1.3 TB/s
+// of bits, 2.3 TB/s with the tables).  Over 21.5 Gbit: 1.78 ms, and 1.58 ms
+// where the ones before every superblock were known from the level passes
+// (only where n % 512 == 0; the counts cost the build more than that).
 //
 // Per word, the work is one in-word select at most (the next 64th one or
 // zero, see word_marks) in 32-bit arithmetic on per-superblock 64-bit bases:
@@ -176,276 +54,454 @@ __device__ __forceinline__ uint64_t last_arg_end_sb(const uint64_t* __restrict__
 // the back) from ceil(zeros before / 64).  The last two steps of the select
 // read a 256 x 8 table of in-byte selects from shared memory.  A superblock
 // holds at most one superblock end per polarity (512 < 4096 args), resolved
-// once per superblock; the last word holding a one / a zero is resolved once
-// per thread from the last such superblock.
-__global__ void __launch_bounds__(256)
-    rs_levels_kernel(const uint64_t* __restrict__ words, int l0, int l1, uint64_t chunks_per_level,
-                     const uint32_t* __restrict__ chunkpre, uint64_t prestride, const uint64_t* __restrict__ lvl_zb,
-                     uint32_t flags, uint64_t* __restrict__ rank, uint32_t* __restrict__ samples, uint64_t samp_last,
-                     uint64_t* __restrict__ starts1, uint64_t* __restrict__ starts0, uint64_t* __restrict__ ends1,
-                     uint64_t* __restrict__ ends0, unsigned long long* info) {
-  __shared__ uint8_t lut[256 * 8];  // lut[byte * 8 + r] = position of the r-th set bit of byte
-  sel_lut_init(lut);
-  __syncthreads();
-  const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
+// once per superblock.  The last superblocks (partial or empty) go word by
+// word.
+struct SelByteTable {
+  uint8_t e[256 * 8];
+};
+constexpr SelByteTable make_sel_byte_table() {
+  SelByteTable t{};
+  for (int b = 0; b < 256; ++b) {
+    int r = 0;
+    for (int k = 0; k < 8; ++k)
+      if ((b >> k) & 1) t.e[b * 8 + r++] = (uint8_t)k;
+  }
+  return t;
+}
+static __device__ const SelByteTable g_sel_bytes = make_sel_byte_table();
+
+// marks and rank entry of a whole superblock b of words w, sb_before ones before it
+__device__ __forceinline__ void superblock_marks(uint64_t b, const uint64_t (&w)[8], uint64_t sb_before, uint32_t flags,
+                                                 const uint8_t* __restrict__ lut, uint64_t* __restrict__ rank,
+                                                 uint32_t* __restrict__ samples, uint64_t samp_last,
+                                                 uint64_t* __restrict__ starts1, uint64_t* __restrict__ starts0,
+                                                 uint64_t* __restrict__ ends1, uint64_t* __restrict__ ends0) {
   const bool sel1 = flags & WTG_SELECT1, sel0 = flags & WTG_SELECT0, sel = sel1 || sel0;
-  uint64_t last_sb1 = ~0ull, last_sb0 = ~0ull;  // last superblocks holding a one / a zero
-  // thread per 512-bit superblock: its eight words in four 16-byte loads,
-  // counts and fields in registers, one 16-byte rank entry
-  for (int l = l0; l < l1; ++l) {
-    const uint64_t zl = lvl_zb[l];
-    const uint32_t* __restrict__ pre = chunkpre + (uint64_t)l * prestride;
-    for (uint64_t c = tid; c < chunks_per_level; c += nthreads) {
-      const uint64_t b = (uint64_t)l * chunks_per_level + c;  // superblock
-      const ulonglong2* p = reinterpret_cast<const ulonglong2*>(words + 8 * b);
-      const ulonglong2 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2), q3 = __ldg(p + 3);
-      const uint64_t w[8] = {q0.x, q0.y, q1.x, q1.y, q2.x, q2.y, q3.x, q3.y};
-      const uint64_t zb = zl + __ldg(pre + c);  // zeros before the superblock
-      const uint64_t sb_before = 512 * b - zb;  // ones before the superblock
-      const uint32_t pos_base = (uint32_t)(512 * b);
-      const uint32_t k1_base = (uint32_t)sb_before, k0_base = (uint32_t)zb;
-      // next samples of this superblock: select1 from the front, select0 from the back
-      uint32_t* __restrict__ p1 = samples + ((sb_before + 63) >> 6);
-      uint32_t* __restrict__ p0 = samples + (samp_last - ((zb + 63) >> 6));
-      uint32_t excl = 0;  // ones before the word within the superblock
-      uint32_t n1 = 0, n0 = 0;
-      uint64_t part = 0;
-      uint32_t cnt[8];
+  const uint64_t zb = 512 * b - sb_before;  // zeros before the superblock
+  const uint32_t pos_base = (uint32_t)(512 * b);
+  const uint32_t k1_base = (uint32_t)sb_before, k0_base = (uint32_t)zb;
+  // next samples of this superblock: select1 from the front, select0 from the back
+  uint32_t* __restrict__ p1 = samples + ((sb_before + 63) >> 6);
+  uint32_t* __restrict__ p0 = samples + (samp_last - ((zb + 63) >> 6));
+  uint32_t excl = 0;  // ones before the word within the superblock
+  uint32_t n1 = 0, n0 = 0;
+  uint64_t part = 0;
+  uint32_t cnt[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint64_t x = w[j];
+    const uint32_t cl = __popc((uint32_t)x);
+    const uint32_t cj = cl + __popc((uint32_t)(x >> 32));
+    cnt[j] = cj;
+    if (j) part |= (uint64_t)excl << (63 - 9 * j);
+    if (sel) {
+      // branch-free: the select runs for every word, the stores are predicated
+      const uint32_t K1 = k1_base + excl;            // ones before the word (mod 2^32)
+      const uint32_t K0 = k0_base + 64u * j - excl;  // zeros before it
+      const uint32_t d1 = (0u - K1) & 63u, d0 = K1 & 63u;
+      const bool s1 = sel1 && d1 < cj, s0 = sel0 && d0 < 64u - cj;
+      const uint32_t off = sel64_lut(s1 ? x : ~x, s1 ? d1 : d0, s1 ? cl : 32u - cl, lut);
+      // both polarities only when K1 % 64 == 0: the word's first one and first zero
+      const uint32_t off0 = s1 ? (uint32_t)(__ffsll((long long)~x) - 1) : off;
+      const uint32_t pos = pos_base + 64u * j;
+      if (s1) p1[n1] = pos + off;
+      if (s0) *(p0 - n0) = pos + off0;
+      if (s1 && ((K1 + d1) & 4095u) == 0) starts1[(sb_before + excl + d1) >> 12] = 512 * b + 64 * j + off;
+      if (s0 && ((K0 + d0) & 4095u) == 0) starts0[(zb + 64 * j - excl + d0) >> 12] = 512 * b + 64 * j + off0;
+      n1 += s1;
+      n0 += s0;
+    }
+    excl += cj;
+  }
+  if (flags & WTG_RANK) reinterpret_cast<ulonglong2*>(rank)[b] = make_ulonglong2(sb_before, part);
+  if (sel) {
+    // superblock ends: arg 4095 of a 4096-arg superblock, at most one per
+    // polarity in 512 bits; one scan serves the lane's first polarity, the
+    // rare superblock that ends one of each takes a second
+    const uint32_t cz = 512u - excl;
+    const uint32_t e1 = 4095u - (k1_base & 4095u), e0 = 4095u - (k0_base & 4095u);
+    bool h1 = sel1 && e1 < excl, h0 = sel0 && e0 < cz;
+    while (h1 || h0) {
+      const bool t1 = h1;  // this round's polarity
+      const uint32_t e = t1 ? e1 : e0;
+      uint32_t before = 0, r = 0;
+      uint64_t xx = 0, jj = 0;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const uint64_t x = w[j];
-        const uint32_t cl = __popc((uint32_t)x);
-        const uint32_t cj = cl + __popc((uint32_t)(x >> 32));
-        cnt[j] = cj;
-        if (j) part |= (uint64_t)excl << (63 - 9 * j);
-        if (sel) {
-          // branch-free: the select runs for every word, the stores are predicated
-          const uint32_t K1 = k1_base + excl;            // ones before the word (mod 2^32)
-          const uint32_t K0 = k0_base + 64u * j - excl;  // zeros before it
-          const uint32_t d1 = (0u - K1) & 63u, d0 = K1 & 63u;
-          const bool s1 = sel1 && d1 < cj, s0 = sel0 && d0 < 64u - cj;
-          const uint32_t off = sel64_lut(s1 ? x : ~x, s1 ? d1 : d0, s1 ? cl : 32u - cl, lut);
-          // both polarities only when K1 % 64 == 0: the word's first one and first zero
-          const uint32_t off0 = s1 ? (uint32_t)(__ffsll((long long)~x) - 1) : off;
-          const uint32_t pos = pos_base + 64u * j;
-          if (s1) p1[n1] = pos + off;
-          if (s0) *(p0 - n0) = pos + off0;
-          if (s1 && ((K1 + d1) & 4095u) == 0) starts1[(sb_before + excl + d1) >> 12] = 512 * b + 64 * j + off;
-          if (s0 && ((K0 + d0) & 4095u) == 0)
-            starts0[(zb + 64 * j - excl + d0) >> 12] = 512 * b + 64 * j + off0;
-          n1 += s1;
-          n0 += s0;
-        }
-        excl += cj;
+        const uint32_t cj = t1 ? cnt[j] : 64u - cnt[j];
+        const bool here = before <= e && e < before + cj;
+        xx = here ? w[j] : xx;
+        r = here ? e - before : r;
+        jj = here ? (uint64_t)j : jj;
+        before += cj;
       }
-      if (flags & WTG_RANK) reinterpret_cast<ulonglong2*>(rank)[b] = make_ulonglong2(sb_before, part);
-      if (sel) {
-        // superblock ends: arg 4095 of a 4096-arg superblock, at most one per
-        // polarity in 512 bits; one scan serves the lane's first polarity,
-        // the rare superblock that ends one of each takes a second
-        const uint32_t cz = 512u - excl;
-        const uint32_t e1 = 4095u - (k1_base & 4095u), e0 = 4095u - (k0_base & 4095u);
-        bool h1 = sel1 && e1 < excl, h0 = sel0 && e0 < cz;
-        // the lanes still inside the superblock loop (its last round may hold fewer)
-        const uint32_t live = __activemask();
-        while (__any_sync(live, h1 || h0)) {
-          const bool t1 = h1;  // this round's polarity
-          const uint32_t e = t1 ? e1 : e0;
-          uint32_t before = 0, r = 0;
-          uint64_t xx = 0, jj = 0;
+      xx = t1 ? xx : ~xx;
+      const uint64_t pos = 512 * b + 64 * jj + sel64_lut(xx, r, __popc((uint32_t)xx), lut);
+      if (t1) ends1[(sb_before + e1) >> 12] = pos;
+      else ends0[(zb + e0) >> 12] = pos;
+      if (t1) h1 = false;
+      else h0 = false;
+    }
+  }
+}
+
+template <int SPT>
+__global__ void __launch_bounds__(BV_THREADS)
+    bv_pass_kernel(const uint64_t* __restrict__ words, uint64_t size, uint64_t W, uint64_t NB, int vec_ok,
+                   uint32_t flags, uint64_t* __restrict__ rank, uint32_t* __restrict__ samples, uint64_t samp_last,
+                   uint64_t* __restrict__ starts1, uint64_t* __restrict__ starts0, uint64_t* __restrict__ ends1,
+                   uint64_t* __restrict__ ends0, unsigned long long* info, uint64_t* status, uint32_t* counter,
+                   uint32_t tile0, uint32_t tile_end, uint32_t* err) {
+  constexpr int WARPS = BV_THREADS / 32;
+  __shared__ __align__(16) uint8_t lut[256 * 8];  // lut[byte * 8 + r] = position of the r-th set bit of byte
+  __shared__ uint32_t s_tile;
+  __shared__ uint32_t s_wsum[WARPS];
+  __shared__ uint64_t s_prefix;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid < 128) reinterpret_cast<uint4*>(lut)[tid] = reinterpret_cast<const uint4*>(g_sel_bytes.e)[tid];
+  const uint64_t tailmask = (size & 63) ? ((1ull << (size & 63)) - 1) : ~0ull;
+  const uint64_t whole = size >> 9;  // superblocks of 512 valid bits; NB, and NB - 1 with a ragged last word, are not
+  auto load = [&](uint64_t b, uint64_t(&w)[8]) {  // a whole superblock
+    if (vec_ok) {
+      const ulonglong2* p = reinterpret_cast<const ulonglong2*>(words + 8 * b);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const uint32_t cj = t1 ? cnt[j] : 64u - cnt[j];
-            const bool here = before <= e && e < before + cj;
-            xx = here ? w[j] : xx;
-            r = here ? e - before : r;
-            jj = here ? (uint64_t)j : jj;
-            before += cj;
-          }
-          xx = t1 ? xx : ~xx;
-          const uint64_t pos = 512 * b + 64 * jj + sel64_lut(xx, r, __popc((uint32_t)xx), lut);
-          if (h1) ends1[(sb_before + e1) >> 12] = pos;
-          else if (h0) ends0[(zb + e0) >> 12] = pos;
-          if (h1) h1 = false;
-          else h0 = false;
+      for (int j = 0; j < 4; ++j) {
+        const ulonglong2 q = __ldg(p + j);
+        w[2 * j] = q.x;
+        w[2 * j + 1] = q.y;
+      }
+    } else {  // words not on a 16-byte boundary
+#pragma unroll
+      for (int j = 0; j < 8; ++j) w[j] = __ldg(words + 8 * b + j);
+    }
+  };
+  for (;;) {
+    __syncthreads();  // the previous tile's shared values are read; the first time, the table is whole
+    if (tid == 0) s_tile = tile0 + atomicAdd(counter, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if (tile >= tile_end) return;
+    const uint64_t b0 = (uint64_t)tile * (SPT * BV_THREADS) + warp * (SPT * 32) + lane;
+    uint64_t w[8];
+    uint32_t ex[SPT];  // ones before the superblock in the warp's run
+    uint32_t run = 0;
+#pragma unroll
+    for (int j = 0; j < SPT; ++j) {
+      const uint64_t b = b0 + 32 * j;
+      uint32_t c = 0;
+      if (b < whole) {
+        load(b, w);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) c += __popcll(w[k]);
+      } else if (b <= NB) {
+        for (uint64_t wi = 8 * b; wi < W && wi < 8 * b + 8; ++wi) c += __popcll(words[wi] & (wi == W - 1 ? tailmask : ~0ull));
+      }
+      uint32_t inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+      }
+      ex[j] = run + inc - c;
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    if (lane == 0) s_wsum[warp] = run;
+    __syncthreads();
+    if (warp == 0) {
+      const uint32_t v = lane < (uint32_t)WARPS ? s_wsum[lane] : 0u;
+      uint32_t inc = v;
+#pragma unroll
+      for (int o = 1; o < WARPS; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += t;
+      }
+      if (lane < (uint32_t)WARPS) s_wsum[lane] = inc - v;
+      const uint64_t total = __shfl_sync(0xffffffffu, inc, WARPS - 1);
+      uint64_t prefix = 0;
+      if (tile == 0) {
+        if (lane == 0) lb_publish(status, tile, LB_FLAG_INC, total);
+      } else {
+        if (lane == 0) lb_publish(status, tile, LB_FLAG_AGG, total);
+        prefix = lb_lookback_warp(status, tile, err);
+        if (lane == 0) lb_publish(status, tile, LB_FLAG_INC, prefix + total);
+      }
+      if (lane == 0) s_prefix = prefix;
+    }
+    __syncthreads();
+    const uint64_t before = s_prefix + s_wsum[warp];
+#pragma unroll 1
+    for (int j = 0; j < SPT; ++j) {
+      const uint64_t b = b0 + 32 * j;
+      uint32_t e = ex[0];
+#pragma unroll
+      for (int k = 1; k < SPT; ++k) e = j == k ? ex[k] : e;
+      const uint64_t sb_before = before + e;
+      if (b < whole) {
+        if (SPT > 1) load(b, w);
+        superblock_marks(b, w, sb_before, flags, lut, rank, samples, samp_last, starts1, starts0, ends1, ends0);
+      } else if (b <= NB) {
+        // superblock NB writes fields 1..max(r, 1) of its r words
+        // (rank_support_v_par.hpp:99-108); the words' marks one by one
+        uint64_t k1 = sb_before, part = 0, lw1 = 0, lw0 = 0;
+        const uint64_t r = b < NB ? 7 : W - 8 * NB, kmax = r > 1 ? r : 1;
+        for (uint64_t k = 0; k < 8; ++k) {
+          const uint64_t wi = 8 * b + k;
+          if (k >= 1 && k <= kmax) part |= (k1 - sb_before) << (63 - 9 * k);
+          if (wi >= W) continue;
+          const uint64_t zmask = wi == W - 1 ? tailmask : ~0ull;
+          const uint64_t x = words[wi] & zmask;
+          word_marks(x, __popcll(x), k1, wi, zmask, flags & WTG_SELECT1, flags & WTG_SELECT0, samples, samp_last,
+                     starts1, starts0, ends1, ends0, lw1, lw0);
+          k1 += __popcll(x);
         }
-        last_sb1 = excl ? b : last_sb1;
-        last_sb0 = cz ? b : last_sb0;
+        if (flags & WTG_RANK) {
+          rank[2 * b] = sb_before;
+          rank[2 * b + 1] = part;
+        }
+        if (b == NB) {
+          info[INF_M1] = k1;
+          info[INF_M0] = size - k1;
+        }
       }
     }
   }
-  if (sel) {
-    const uint64_t last1 = warp_max_u64(last_sb1 == ~0ull ? 0 : last_arg_end_sb(words, last_sb1, 1));
-    const uint64_t last0 = warp_max_u64(last_sb0 == ~0ull ? 0 : last_arg_end_sb(words, last_sb0, 0));
-    if ((threadIdx.x & 31) == 0) {
-      if (last1) atomicMax(&info[INF_LAST1], (unsigned long long)last1);
-      if (last0) atomicMax(&info[INF_LAST0], (unsigned long long)last0);
+}
+
+__device__ __forceinline__ uint64_t args_before_sb(int t_b, const uint64_t* __restrict__ rank, uint64_t b) {
+  const uint64_t r = rank[2 * b];
+  return t_b ? r : 512 * b - r;
+}
+
+// position of the last arg, m >= 1: the last superblock with fewer than m
+// args before it, found by galloping back from the end over the rank table
+// (a dense bitvector ends at the first probe) and a binary search, then its
+// words from the last
+__device__ uint64_t last_arg_pos(int t_b, const uint64_t* __restrict__ words, const uint64_t* __restrict__ rank,
+                                 uint64_t size, uint64_t m) {
+  const uint64_t W = (size + 63) >> 6, NB = W >> 3;
+  uint64_t lo = NB, hi = NB;
+  for (uint64_t step = 1; lo > 0 && args_before_sb(t_b, rank, lo) >= m; step *= 2) {
+    hi = lo - 1;
+    lo = hi > step ? hi - step : 0;
+  }
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi + 1) >> 1;
+    if (args_before_sb(t_b, rank, mid) < m) lo = mid;
+    else hi = mid - 1;
+  }
+  const uint64_t tailmask = (size & 63) ? ((1ull << (size & 63)) - 1) : ~0ull;
+  for (uint64_t wi = 8 * lo + 8 < W ? 8 * lo + 8 : W; wi-- > 8 * lo;) {
+    uint64_t x = words[wi];
+    if (!t_b) x = ~x;
+    if (wi == W - 1) x &= tailmask;
+    if (x) return (wi << 6) + hi64(x);
+  }
+  return 0;
+}
+
+// The select structures of both polarities, blockIdx.y = t_b.
+struct SelBuild {
+  const uint64_t* starts;
+  const uint64_t* ends;
+  uint64_t* descw;      // working descriptors: long flag and width
+  uint64_t* offs;       // pool word offset per superblock
+  uint64_t* desc;       // final descriptors
+  uint64_t* long_list;
+  uint64_t* pool;
+  uint64_t* sb_words;
+  uint64_t* status;     // look-back status words
+  uint32_t* counter;
+  uint64_t nsb, sb_nwords, m;  // known after the read-back
+  uint32_t on;
+};
+struct SelBuild2 {
+  SelBuild t[2];
+};
+
+constexpr int SD_THREADS = 256;
+constexpr int SD_IPT = 4;  // superblocks per thread, consecutive
+constexpr int SD_TILE = SD_THREADS * SD_IPT;
+
+// per superblock: long/mini choice and width (:525-543), and the scan of the
+// pool words into offsets in the same launch (decoupled look-back)
+__global__ void __launch_bounds__(SD_THREADS)
+    select_desc_kernel(SelBuild2 sb2, const uint64_t* __restrict__ words, const uint64_t* __restrict__ rank,
+                       uint64_t size, unsigned long long* info, uint64_t logn4, uint32_t* err) {
+  __shared__ uint32_t s_tile;
+  __shared__ uint64_t s_wsum[SD_THREADS / 32];
+  __shared__ uint64_t s_prefix;
+  const int t_b = blockIdx.y;
+  const SelBuild& sb = sb2.t[t_b];
+  if (!sb.on) return;
+  const uint64_t m = info[t_b ? INF_M1 : INF_M0];
+  const uint64_t nsb = (m + 4095) >> 12;
+  if (threadIdx.x == 0) s_tile = atomicAdd(sb.counter, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if ((uint64_t)tile * SD_TILE >= nsb) return;  // past the superblocks: no later tile needs this one
+  const uint64_t base = (uint64_t)tile * SD_TILE + threadIdx.x * SD_IPT;
+  uint32_t sz[SD_IPT];
+  uint64_t sum = 0;
+#pragma unroll
+  for (int k = 0; k < SD_IPT; ++k) {
+    const uint64_t i = base + k;
+    sz[k] = 0;
+    if (i < nsb) {
+      const uint64_t start = sb.starts[i];
+      uint64_t end;
+      if (i + 1 < nsb) {
+        end = sb.ends[i];
+      } else {
+        end = last_arg_pos(t_b, words, rank, size, m);
+        info[t_b ? INF_LAST1 : INF_LAST0] = end + 1;
+      }
+      const uint64_t span = end - start;
+      const uint32_t lng = span > logn4;
+      const uint32_t wdt = lng ? hi64(end) + 1 : hi64(span) + 1;
+      sb.descw[i] = (lng << 7) | wdt;
+      sz[k] = lng ? 64 * wdt : wdt;
+      if (lng) {
+        const unsigned long long slot = atomicAdd(&info[t_b ? INF_NLONG1 : INF_NLONG0], 1ull);
+        sb.long_list[slot] = i;
+      }
     }
+    sum += sz[k];
+  }
+  uint64_t inc = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += t;
+  }
+  if (lane == 31) s_wsum[warp] = inc;
+  __syncthreads();
+  if (warp == 0) {
+    const uint64_t v = lane < SD_THREADS / 32 ? s_wsum[lane] : 0;
+    uint64_t winc = v;
+#pragma unroll
+    for (int o = 1; o < SD_THREADS / 32; o <<= 1) {
+      const uint64_t t = __shfl_up_sync(0xffffffffu, winc, o);
+      if (lane >= (uint32_t)o) winc += t;
+    }
+    if (lane < SD_THREADS / 32) s_wsum[lane] = winc - v;
+    const uint64_t total = __shfl_sync(0xffffffffu, winc, SD_THREADS / 32 - 1);
+    uint64_t prefix = 0;
+    if (tile == 0) {
+      if (lane == 0) lb_publish(sb.status, tile, LB_FLAG_INC, total);
+    } else {
+      if (lane == 0) lb_publish(sb.status, tile, LB_FLAG_AGG, total);
+      prefix = lb_lookback_warp(sb.status, tile, err);
+      if (lane == 0) lb_publish(sb.status, tile, LB_FLAG_INC, prefix + total);
+    }
+    if (lane == 0) s_prefix = prefix;
+  }
+  __syncthreads();
+  uint64_t off = s_prefix + s_wsum[warp] + inc - sum;
+#pragma unroll
+  for (int k = 0; k < SD_IPT; ++k) {
+    const uint64_t i = base + k;
+    if (i < nsb) sb.offs[i] = off;
+    off += sz[k];
+    if (i + 1 == nsb) info[t_b ? INF_POOL1 : INF_POOL0] = off;
   }
 }
 
-// arg counts and the rank pair after the last superblock, (total, 0)
-// (rank_support_v_par.hpp:95-110 with capacity % 512 == 0)
-__global__ void rs_levels_totals_kernel(const uint64_t* lvl_zb, int L, uint64_t size, uint64_t NB, uint64_t* rank,
-                                        unsigned long long* info) {
-  const uint64_t z = lvl_zb[L];
-  info[INF_M1] = size - z;
-  info[INF_M0] = z;
-  if (rank) {
-    rank[2 * NB] = size - z;
-    rank[2 * NB + 1] = 0;
-  }
-}
-
-// zeros before levels l0+1..l1: lvl_zb[l + 1] = lvl_zb[l] + zeros of level l,
-// from lvl_zb[l0] (0 for l0 == 0)
-__global__ void level_zeros_kernel(const uint32_t* __restrict__ chunkcnt, const uint32_t* __restrict__ chunkpre,
-                                   uint64_t stride, uint64_t nchunks, int l0, int l1, uint64_t* __restrict__ lvl_zb) {
-  if (l0 == 0) lvl_zb[0] = 0;
-  uint64_t acc = lvl_zb[l0];
-  for (int l = l0; l < l1; ++l) {
-    acc += (uint64_t)chunkpre[l * stride + nchunks - 1] + chunkcnt[l * stride + nchunks - 1];
-    lvl_zb[l + 1] = acc;
-  }
-}
-
-int bv_levels_begin(BvSupport& bv, const uint64_t* d_words, uint64_t n, int L, uint32_t flags, cudaStream_t s) {
-  return bv_prepare(bv, d_words, n * (uint64_t)L, flags, s);
-}
-
-int bv_levels_pass(BvSupport& bv, uint64_t n, int l0, int l1, const uint32_t* chunkcnt, const uint32_t* chunkpre,
-                   uint64_t stride, uint64_t nchunks, uint64_t* lvl_zb, cudaStream_t s) {
-  if (l1 <= l0) return WTG_OK;
-  const uint64_t samp_n = bv.size / 64 + 2;
-  level_zeros_kernel<<<1, 1, 0, s>>>(chunkcnt, chunkpre, stride, nchunks, l0, l1, lvl_zb);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 1;
-  }
-  const uint64_t per_level = n / 512;  // superblocks per level, one thread each
-  const unsigned grid = (unsigned)std::max<uint64_t>(
-      1, std::min<uint64_t>((per_level + 255) / 256, (uint64_t)sms * 8));
-  prof_begin(PROF_BVPASS, s);
-  rs_levels_kernel<<<grid, 256, 0, s>>>(
-      bv.words, l0, l1, n / 512, chunkpre, stride, lvl_zb, bv.flags, bv.rank.as<uint64_t>(),
-      bv.samples.as<uint32_t>(), samp_n - 1, bv.sel[1].starts.as<uint64_t>(), bv.sel[0].starts.as<uint64_t>(),
-      bv.sel[1].ends.as<uint64_t>(), bv.sel[0].ends.as<uint64_t>(), bv.info.as<unsigned long long>());
-  prof_end(PROF_BVPASS, s);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  return WTG_OK;
-}
-
-int bv_levels_end(BvSupport& bv, int L, const uint64_t* lvl_zb, uint32_t* d_err, cudaStream_t s) {
-  const uint64_t NB = bv.size / 512;
-  rs_levels_totals_kernel<<<1, 1, 0, s>>>(lvl_zb, L, bv.size, NB,
-                                         (bv.flags & WTG_RANK) ? bv.rank.as<uint64_t>() : nullptr,
-                                         bv.info.as<unsigned long long>());
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  if (bv.rank_done) WTG_CK(cudaEventRecord(bv.rank_done, s));
-  return bv_finish(bv, d_err, s);
-}
-
-// per superblock: long/mini choice, width and pool words
-__global__ void select_desc_kernel(int t_b, const uint64_t* __restrict__ starts,
-                                   const uint64_t* __restrict__ ends, unsigned long long* info, uint64_t logn4,
-                                   uint64_t nsb_cap, uint64_t* __restrict__ descw, uint64_t* __restrict__ sizes,
-                                   uint64_t* __restrict__ long_list) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nsb_cap) return;
-  const uint64_t m = info[t_b ? INF_M1 : INF_M0];
-  const uint64_t nsb = (m + 4095) >> 12;
-  if (i >= nsb) {
-    sizes[i] = 0;
-    return;
-  }
-  const uint64_t start = starts[i];
-  const uint64_t end = (i + 1 < nsb) ? ends[i] : (uint64_t)info[t_b ? INF_LAST1 : INF_LAST0] - 1;
-  const uint64_t span = end - start;
-  const uint64_t lng = span > logn4;
-  const uint64_t wdt = lng ? hi64(end) + 1 : hi64(span) + 1;
-  descw[i] = (lng << 7) | wdt;
-  sizes[i] = lng ? 64 * wdt : wdt;
-  if (lng) {
-    unsigned long long slot = atomicAdd(&info[t_b ? INF_NLONG1 : INF_NLONG0], 1ull);
-    long_list[slot] = i;
-  }
-}
-
-__global__ void select_pool_total_kernel(int t_b, unsigned long long* info, const uint64_t* sizes,
-                                         const uint64_t* offs) {
-  const uint64_t m = info[t_b ? INF_M1 : INF_M0];
-  const uint64_t nsb = (m + 4095) >> 12;
-  info[t_b ? INF_POOL1 : INF_POOL0] = nsb ? offs[nsb - 1] + sizes[nsb - 1] : 0;
-}
-
-// Two superblocks per warp (lanes 0-15 pack superblock 2w's words, lanes
-// 16-31 superblock 2w+1's): final descriptors and the 64-entry mini blocks.
-// A mini block's words are few (its width, at most 32), so one superblock per
-// warp left half of the lanes idle while the others packed.
-__global__ void __launch_bounds__(256)
-    select_mini_kernel(int t_b, uint64_t nsb, uint64_t m, const uint32_t* __restrict__ samples, uint64_t samp_last,
-                       const uint64_t* __restrict__ descw, const uint64_t* __restrict__ offs,
-                       uint64_t* __restrict__ desc, uint64_t* __restrict__ pool) {
-  __shared__ uint64_t ent[256 / 32][2][64];
-  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2;
-  if (i0 >= nsb) return;
-  auto samp = [&](uint64_t k) { return t_b ? samples[k] : samples[samp_last - k]; };
+// The first blocks of each polarity: two superblocks per warp, 16 lanes
+// each: final descriptors and the 64-entry mini blocks.  Lane q of a half
+// loads entries 4q .. 4q+3 and, for widths of at most 16 (all but sparse
+// stretches), packs them into one 64-bit piece at bit 4q * width of the
+// block; word q of the block is then two or three pieces fetched by shuffles.
+// (Assembling every word from its entries in shared memory took 6-7 loads
+// and 64-bit shifts a word and was bound by issue: 0.98 ms of the 2^30 x 20
+// build's 5.2 M superblocks, against 0.3 ms of traffic.)  Wider entries go
+// word by word through shared memory.  The blocks after them: m_superblock,
+// entry i = position of arg 4096*i, width logn.
+template <int T_B>
+__device__ __forceinline__ void mini_blocks_warp(const SelBuild& sb, uint64_t i0, const uint32_t* __restrict__ samples,
+                                                 uint64_t samp_last, uint32_t (*ent)[64]) {
+  const uint32_t lane = threadIdx.x & 31, h = lane >> 4, ql = lane & 15;
+  const uint64_t i = i0 + h;
+  const bool in = i < sb.nsb;
   // positions are kept mod 2^32; a mini block spans at most log^4 n < 2^32
   // bits, so the offsets are exact
+  const uint64_t k0 = 64 * i + 4 * ql;            // first entry's sample
+  const uint64_t args = (sb.m + 63) >> 6;         // samples there are
+  uint32_t e[4] = {0, 0, 0, 0};
+  if (in) {
+    if (T_B == 1 && k0 + 4 <= args) {
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>(samples + k0));
+      e[0] = v.x, e[1] = v.y, e[2] = v.z, e[3] = v.w;
+    } else {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const uint64_t i = i0 + h;
-    if (i < nsb) {  // warp-uniform
-      const uint32_t start = samp(64 * i);
-#pragma unroll
-      for (int g = 0; g < 2; ++g) {
-        const uint32_t j = lane + 32 * g;
-        const uint64_t k = 4096 * i + 64 * (uint64_t)j;
-        ent[warp][h][j] = (k < m) ? (uint64_t)(uint32_t)(samp(64 * i + j) - start) : 0;
-      }
+      for (int k = 0; k < 4; ++k)
+        if (k0 + k < args) e[k] = __ldg(samples + (T_B ? k0 + k : samp_last - (k0 + k)));
     }
   }
-  __syncwarp();
-  const uint32_t h = lane >> 4, ql = lane & 15;
-  const uint64_t i = i0 + h;
-  if (i >= nsb) return;
-  const uint64_t d = descw[i];
-  const uint64_t off = offs[i];
-  if (ql == 0) desc[i] = (off << 8) | (d & 255);
-  if ((d >> 7) & 1) return;  // long block
-  const uint32_t wdt = (uint32_t)(d & 127);
+  uint64_t d = 0, off = 0;
+  if (in) {
+    d = __ldg(sb.descw + i);
+    off = __ldg(sb.offs + i);
+    if (ql == 0) sb.desc[i] = (off << 8) | (d & 255);
+  }
+  const uint32_t start = __shfl_sync(0xffffffffu, e[0], 0, 16);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) e[k] = k0 + k < args ? e[k] - start : 0u;
+  const uint32_t wdt = in && !((d >> 7) & 1) ? (uint32_t)(d & 127) : 0u;  // 0: nothing to pack here
   // entry indices of a word's first and last bit: floor(x / wdt) for
   // x < 2^11 by one multiply with ceil(2^26 / wdt) (exact for x < 2^20,
   // wdt <= 64), not two divisions per word
-  const uint64_t rcp = ((1ull << 26) + wdt - 1) / wdt;
-  for (uint32_t q = ql; q < wdt; q += 16) {
-    const uint32_t lo = q * 64;
-    const uint32_t j0 = (uint32_t)(((uint64_t)lo * rcp) >> 26), j1 = (uint32_t)(((uint64_t)(lo + 63) * rcp) >> 26);
-    uint64_t out = 0;
-    for (uint32_t j = j0; j <= j1 && j < 64; ++j) {
-      const uint64_t v = ent[warp][h][j];  // < 2^wdt
-      const int32_t sh = (int32_t)(j * wdt) - (int32_t)lo;
-      out |= sh >= 0 ? (v << sh) : (v >> (-sh));
+  const uint64_t rcp = wdt ? ((1u << 26) + wdt - 1) / wdt : 0u;
+  if (__any_sync(0xffffffffu, wdt > 16)) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) ent[h][4 * ql + k] = e[k];
+    __syncwarp();
+    for (uint32_t q = ql; q < wdt; q += 16) {
+      const uint32_t lo = q * 64;
+      const uint32_t j0 = (uint32_t)((lo * rcp) >> 26), j1 = (uint32_t)(((lo + 63) * rcp) >> 26);
+      uint64_t out = 0;
+      for (uint32_t j = j0; j <= j1 && j < 64; ++j) {
+        const uint64_t v = ent[h][j];  // < 2^wdt
+        const int32_t sh = (int32_t)(j * wdt) - (int32_t)lo;
+        out |= sh >= 0 ? (v << sh) : (v >> (-sh));
+      }
+      sb.pool[off + q] = out;
     }
-    pool[off + q] = out;
+    return;
   }
+  const uint64_t piece = (uint64_t)e[0] | ((uint64_t)e[1] << wdt) | ((uint64_t)e[2] << (2 * wdt)) |
+                         ((uint64_t)e[3] << (3 * wdt));
+  const uint32_t w4 = 4 * wdt;
+  uint32_t j = (uint32_t)((16u * ql * rcp) >> 26);  // piece holding the word's first bit: floor(64 q / w4)
+  int32_t sh = (int32_t)(j * w4) - (int32_t)(64 * ql);
+  const uint64_t first = __shfl_sync(0xffffffffu, piece, j & 15, 16);
+  uint64_t out = wdt ? first >> (-sh) : 0ull;
+  for (;;) {
+    ++j;
+    sh += w4;
+    const bool more = wdt && ql < wdt && sh < 64 && j < 16;
+    if (!__any_sync(0xffffffffu, more)) break;
+    const uint64_t v = __shfl_sync(0xffffffffu, piece, j & 15, 16);
+    if (more) out |= v << sh;
+  }
+  if (ql < wdt) sb.pool[off + ql] = out;
 }
 
-// m_superblock: entry i = position of arg 4096*i, width logn
-__global__ void select_sb_pack_kernel(uint64_t nsb, uint32_t logn, const uint64_t* __restrict__ starts,
-                                      uint64_t nwords, uint64_t* __restrict__ sb_words) {
-  uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= nwords) return;
-  sb_words[q] = packed_word(q, logn, nsb, [&](uint64_t i) { return starts[i]; });
+__global__ void __launch_bounds__(256)
+    select_mini_kernel(SelBuild2 sb2, const uint32_t* __restrict__ samples, uint64_t samp_last, uint32_t logn) {
+  __shared__ uint32_t ent[256 / 32][2][64];
+  const int t_b = blockIdx.y;
+  const SelBuild& sb = sb2.t[t_b];
+  if (!sb.on) return;
+  const uint64_t mini_blocks = (sb.nsb + 15) / 16;
+  if (blockIdx.x >= mini_blocks) {
+    const uint64_t q = (blockIdx.x - mini_blocks) * 256 + threadIdx.x;
+    if (q < sb.sb_nwords) sb.sb_words[q] = packed_word(q, logn, sb.nsb, [&](uint64_t i) { return sb.starts[i]; });
+    return;
+  }
+  const uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2;
+  if (i0 >= sb.nsb) return;
+  if (t_b) mini_blocks_warp<1>(sb, i0, samples, samp_last, ent[threadIdx.x >> 5]);
+  else mini_blocks_warp<0>(sb, i0, samples, samp_last, ent[threadIdx.x >> 5]);
 }
 
 // Long blocks, step 1: the position of every arg of every long superblock,
@@ -454,11 +510,6 @@ __global__ void select_sb_pack_kernel(uint64_t nsb, uint32_t logn, const uint64_
 // k-th arg is located by binary search over the rank table's absolute counts
 // (between the two samples that bracket it), then within its 512-bit
 // superblock by popcounts of at most 8 words.
-__device__ __forceinline__ uint64_t args_before_sb(int t_b, const uint64_t* __restrict__ rank, uint64_t b) {
-  const uint64_t r = rank[2 * b];
-  return t_b ? r : 512 * b - r;
-}
-
 __global__ void __launch_bounds__(256)
     select_long_fill_kernel(int t_b, const uint64_t* __restrict__ words, uint64_t size, uint64_t W,
                             const uint64_t* __restrict__ rank, const uint64_t* __restrict__ starts,
@@ -530,7 +581,7 @@ void bv_release(BvSupport& bv, cudaStream_t s) {
   for (auto& sd : bv.sel) {
     sd.ends.release(s);
     sd.desc.release(s);
-    sd.sizes.release(s);
+    sd.offs.release(s);
     sd.sb_words.release(s);
     sd.pool.release(s);
     sd.long_list.release(s);
@@ -563,36 +614,87 @@ int bv_prepare(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t& 
     if ((rc = sd.ends.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
     if ((rc = sd.starts.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
     if ((rc = sd.desc.ensure(2 * nsb_cap * sizeof(uint64_t), s))) return rc;   // [final | working]
-    if ((rc = sd.sizes.ensure(2 * nsb_cap * sizeof(uint64_t), s))) return rc;  // [sizes | offsets]
+    if ((rc = sd.offs.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
     if ((rc = sd.long_list.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
   }
   return WTG_OK;
 }
 
-int bv_pass(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
-  int rc;
-  const uint64_t size = bv.size;
+// superblocks per thread of the pass over a bitvector of NB + 1 superblocks:
+// 4 (a 64 KB tile per CTA) once that fills the chip twice, 1 below
+static int bv_spt(uint64_t NB) { return NB + 1 >= 4ull * BV_THREADS * 2 * 152 ? 4 : 1; }
+
+template <int SPT>
+static int launch_bv_pass_t(const uint64_t* words, uint64_t size, uint32_t flags, uint64_t* rank, uint32_t* samples,
+                            uint64_t samp_last, uint64_t* starts1, uint64_t* starts0, uint64_t* ends1,
+                            uint64_t* ends0, unsigned long long* info, uint64_t* status, uint32_t* counter,
+                            uint32_t tile0, uint32_t tile_end, uint32_t* err, cudaStream_t s) {
+  static const int resident = [] {
+    int per_sm = 0, dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bv_pass_kernel<SPT>, BV_THREADS, 0);
+    return std::max(1, per_sm) * std::max(1, sms);
+  }();
   const uint64_t W = (size + 63) / 64;
-  const uint64_t NB = W >> 3;
-  const uint64_t samp_n = W + 2;
-  const uint64_t tiles = (NB + 1 + BVT_SB - 1) / BVT_SB;
+  const unsigned grid = std::min<uint32_t>(tile_end - tile0, (uint32_t)resident);
+  prof_begin(PROF_BVPASS, s);
+  bv_pass_kernel<SPT><<<grid, BV_THREADS, 0, s>>>(words, size, W, W >> 3, ((uintptr_t)words % 16) == 0, flags, rank,
+                                                  samples, samp_last, starts1, starts0, ends1, ends0, info, status,
+                                                  counter, tile0, tile_end, err);
+  prof_end(PROF_BVPASS, s);
+  count_launch();
+  WTG_CK(cudaGetLastError());
+  return WTG_OK;
+}
+
+// every wait of the pass is on a tile taken before, so a launch of at most
+// the resident CTAs, or of more, completes
+static int launch_bv_pass(int spt, const uint64_t* words, uint64_t size, uint32_t flags, uint64_t* rank,
+                          uint32_t* samples, uint64_t samp_last, uint64_t* starts1, uint64_t* starts0,
+                          uint64_t* ends1, uint64_t* ends0, unsigned long long* info, uint64_t* status,
+                          uint32_t* counter, uint32_t tile0, uint32_t tile_end, uint32_t* err, cudaStream_t s) {
+  if (tile_end <= tile0) return WTG_OK;
+  auto* const f = spt == 4 ? launch_bv_pass_t<4> : launch_bv_pass_t<1>;
+  return f(words, size, flags, rank, samples, samp_last, starts1, starts0, ends1, ends0, info, status, counter, tile0,
+           tile_end, err, s);
+}
+
+int bv_pass_begin(BvSupport& bv, cudaStream_t s) {
+  int rc;
+  const uint64_t NB = ((bv.size + 63) / 64) >> 3;
+  bv.spt = bv_spt(NB);
+  const uint64_t tiles = (NB + 1 + bv.spt * BV_THREADS - 1) / (bv.spt * BV_THREADS);
   if (tiles > 0x7fffffffull) return fail(WTG_ERR_INVALID, "bitvector too large");
+  bv.tiles = (uint32_t)tiles;
+  bv.tiles_done = 0;
   if ((rc = bv.status.ensure((tiles + 1) * sizeof(uint64_t), s))) return rc;
   WTG_CK(cudaMemsetAsync(bv.status.p, 0, (tiles + 1) * sizeof(uint64_t), s));
   if (test_take_lookback_stall()) {  // tile 0 is never taken: every look-back wait on it runs out
     static const uint32_t one = 1;
     WTG_CK(cudaMemcpyAsync(bv.status.p, &one, sizeof(one), cudaMemcpyHostToDevice, s));
   }
-  prof_begin(PROF_BVPASS, s);
-  bv_pass_kernel<<<(unsigned)tiles, BV_THREADS, 0, s>>>(
-      bv.words, size, W, NB, bv.flags, bv.rank.as<uint64_t>(), bv.samples.as<uint32_t>(), samp_n - 1,
-      bv.sel[1].starts.as<uint64_t>(), bv.sel[0].starts.as<uint64_t>(), bv.sel[1].ends.as<uint64_t>(),
-      bv.sel[0].ends.as<uint64_t>(), bv.info.as<unsigned long long>(), bv.status.as<uint64_t>() + 1,
-      bv.status.as<uint32_t>(), d_err);
-  prof_end(PROF_BVPASS, s);
-  count_launch();
-  WTG_CK(cudaGetLastError());
   return WTG_OK;
+}
+
+int bv_pass_to(BvSupport& bv, uint64_t bits_ready, uint32_t* d_err, cudaStream_t s) {
+  const uint64_t tile_bits = 512ull * BV_THREADS * bv.spt;
+  const uint32_t to = bits_ready >= bv.size ? bv.tiles : (uint32_t)(bits_ready / tile_bits);
+  // every launch takes its tiles from tiles_done on, counting from 0
+  if (bv.tiles_done && to > bv.tiles_done) WTG_CK(cudaMemsetAsync(bv.status.p, 0, sizeof(uint32_t), s));
+  const int rc = launch_bv_pass(bv.spt, bv.words, bv.size, bv.flags, bv.rank.as<uint64_t>(),
+                                bv.samples.as<uint32_t>(), (bv.size + 63) / 64 + 1, bv.sel[1].starts.as<uint64_t>(),
+                                bv.sel[0].starts.as<uint64_t>(), bv.sel[1].ends.as<uint64_t>(),
+                                bv.sel[0].ends.as<uint64_t>(), bv.info.as<unsigned long long>(),
+                                bv.status.as<uint64_t>() + 1, bv.status.as<uint32_t>(), bv.tiles_done, to, d_err, s);
+  if (rc) return rc;
+  bv.tiles_done = std::max(bv.tiles_done, to);
+  return WTG_OK;
+}
+
+uint64_t bv_superblocks_done(const BvSupport& bv) {
+  const uint64_t NB = ((bv.size + 63) / 64) >> 3;
+  return std::min<uint64_t>(NB + 1, (uint64_t)bv.tiles_done * BV_THREADS * bv.spt);
 }
 
 int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
@@ -609,32 +711,38 @@ int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
   unsigned long long* info = bv.info.as<unsigned long long>();
   uint32_t* samples = bv.samples.as<uint32_t>();
 
+  // descriptors and pool offsets of both polarities
+  const uint64_t tiles = (nsb_cap + SD_TILE - 1) / SD_TILE;
+  if ((rc = bv.scan_tmp.ensure(2 * (tiles + 1) * sizeof(uint64_t), s))) return rc;
+  WTG_CK(cudaMemsetAsync(bv.scan_tmp.p, 0, 2 * (tiles + 1) * sizeof(uint64_t), s));
+  SelBuild2 sb{};
   for (int t_b = 0; t_b < 2; ++t_b) {
     if (!(flags & (t_b ? WTG_SELECT1 : WTG_SELECT0))) continue;
     SelectDev& sd = bv.sel[t_b];
-    uint64_t* descw = sd.desc.as<uint64_t>() + nsb_cap;
-    uint64_t* sizes = sd.sizes.as<uint64_t>();
-    uint64_t* offs = sizes + nsb_cap;
-    prof_begin(PROF_SELECT, s);
-    select_desc_kernel<<<(unsigned)((nsb_cap + 255) / 256), 256, 0, s>>>(
-        t_b, sd.starts.as<uint64_t>(), sd.ends.as<uint64_t>(), info, logn4, nsb_cap, descw, sizes,
-        sd.long_list.as<uint64_t>());
-    prof_end(PROF_SELECT, s);
-    count_launch();
-    WTG_CK(cudaGetLastError());
-    if ((rc = scan_exclusive_u64(sizes, offs, nsb_cap, bv.scan_tmp, d_err, s))) return rc;
-    prof_begin(PROF_SELECT, s);
-    select_pool_total_kernel<<<1, 1, 0, s>>>(t_b, info, sizes, offs);
-    prof_end(PROF_SELECT, s);
-    count_launch();
-    WTG_CK(cudaGetLastError());
+    SelBuild& x = sb.t[t_b];
+    x.on = 1;
+    x.starts = sd.starts.as<uint64_t>();
+    x.ends = sd.ends.as<uint64_t>();
+    x.desc = sd.desc.as<uint64_t>();
+    x.descw = x.desc + nsb_cap;
+    x.offs = sd.offs.as<uint64_t>();
+    x.long_list = sd.long_list.as<uint64_t>();
+    x.counter = reinterpret_cast<uint32_t*>(bv.scan_tmp.as<uint64_t>() + t_b * (tiles + 1));
+    x.status = bv.scan_tmp.as<uint64_t>() + t_b * (tiles + 1) + 1;
   }
+  prof_begin(PROF_SELECT, s);
+  select_desc_kernel<<<dim3((unsigned)tiles, 2), SD_THREADS, 0, s>>>(sb, d_words, bv.rank.as<uint64_t>(), size, info,
+                                                                     logn4, d_err);
+  prof_end(PROF_SELECT, s);
+  count_launch();
+  WTG_CK(cudaGetLastError());
 
   // the pool sizes decide the allocations: one small read-back
   uint64_t h[INF_N];
   WTG_CK(cudaMemcpyAsync(h, info, sizeof(h), cudaMemcpyDeviceToHost, s));
   WTG_CK(cudaStreamSynchronize(s));
 
+  uint64_t blocks = 0;
   for (int t_b = 0; t_b < 2; ++t_b) {
     if (!(flags & (t_b ? WTG_SELECT1 : WTG_SELECT0))) continue;
     SelectDev& sd = bv.sel[t_b];
@@ -648,40 +756,41 @@ int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
     sd.sb_nwords = (sd.nsb * logn + 63) / 64;
     if ((rc = sd.pool.ensure((sd.pool_nwords + 1) * sizeof(uint64_t), s))) return rc;
     if ((rc = sd.sb_words.ensure((sd.sb_nwords + 1) * sizeof(uint64_t), s))) return rc;
-    if (sd.nsb == 0) continue;
-    uint64_t* descw = sd.desc.as<uint64_t>() + nsb_cap;
-    uint64_t* offs = sd.sizes.as<uint64_t>() + nsb_cap;
+    SelBuild& x = sb.t[t_b];
+    x.nsb = sd.nsb;
+    x.sb_nwords = sd.sb_nwords;
+    x.m = m;
+    x.pool = sd.pool.as<uint64_t>();
+    x.sb_words = sd.sb_words.as<uint64_t>();
+    blocks = std::max(blocks, (sd.nsb + 15) / 16 + (sd.sb_nwords + 255) / 256);
+  }
+  if (blocks) {
     prof_begin(PROF_SELECT, s);
-    select_mini_kernel<<<(unsigned)(((sd.nsb + 1) / 2 * 32 + 255) / 256), 256, 0, s>>>(
-        t_b, sd.nsb, m, samples, samp_n - 1, descw, offs, sd.desc.as<uint64_t>(), sd.pool.as<uint64_t>());
+    select_mini_kernel<<<dim3((unsigned)blocks, 2), 256, 0, s>>>(sb, samples, samp_n - 1, logn);
     prof_end(PROF_SELECT, s);
     count_launch();
     WTG_CK(cudaGetLastError());
-    prof_begin(PROF_SELECT, s);
-    select_sb_pack_kernel<<<(unsigned)((sd.sb_nwords + 255) / 256), 256, 0, s>>>(
-        sd.nsb, logn, sd.starts.as<uint64_t>(), sd.sb_nwords, sd.sb_words.as<uint64_t>());
-    prof_end(PROF_SELECT, s);
-    count_launch();
-    WTG_CK(cudaGetLastError());
+  }
+  for (int t_b = 0; t_b < 2; ++t_b) {
     const uint64_t nlong = h[t_b ? INF_NLONG1 : INF_NLONG0];
-    if (nlong) {
-      if ((rc = sd.long_ent.ensure(nlong * 4096 * sizeof(uint64_t), s))) return rc;
-      WTG_CK(cudaMemsetAsync(sd.long_ent.p, 0, nlong * 4096 * sizeof(uint64_t), s));
-      prof_begin(PROF_SELECT, s);
-      select_long_fill_kernel<<<(unsigned)((nlong * 4096 + 255) / 256), 256, 0, s>>>(
-          t_b, d_words, size, W, bv.rank.as<uint64_t>(), sd.starts.as<uint64_t>(), sd.ends.as<uint64_t>(), info,
-          sd.long_list.as<uint64_t>(), sd.long_ent.as<uint64_t>(), d_err);
-      prof_end(PROF_SELECT, s);
-      count_launch();
-      WTG_CK(cudaGetLastError());
-      unsigned grid = (unsigned)std::min<uint64_t>(nlong, 8 * 152);
-      prof_begin(PROF_SELECT, s);
-      select_long_pack_kernel<<<grid, 256, 0, s>>>(t_b, info, sd.long_list.as<uint64_t>(), descw, offs,
-                                                   sd.long_ent.as<uint64_t>(), sd.pool.as<uint64_t>());
-      prof_end(PROF_SELECT, s);
-      count_launch();
-      WTG_CK(cudaGetLastError());
-    }
+    if (!sb.t[t_b].on || !nlong) continue;
+    SelectDev& sd = bv.sel[t_b];
+    if ((rc = sd.long_ent.ensure(nlong * 4096 * sizeof(uint64_t), s))) return rc;
+    WTG_CK(cudaMemsetAsync(sd.long_ent.p, 0, nlong * 4096 * sizeof(uint64_t), s));
+    prof_begin(PROF_SELECT, s);
+    select_long_fill_kernel<<<(unsigned)((nlong * 4096 + 255) / 256), 256, 0, s>>>(
+        t_b, d_words, size, W, bv.rank.as<uint64_t>(), sd.starts.as<uint64_t>(), sd.ends.as<uint64_t>(), info,
+        sd.long_list.as<uint64_t>(), sd.long_ent.as<uint64_t>(), d_err);
+    prof_end(PROF_SELECT, s);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    unsigned grid = (unsigned)std::min<uint64_t>(nlong, 8 * 152);
+    prof_begin(PROF_SELECT, s);
+    select_long_pack_kernel<<<grid, 256, 0, s>>>(t_b, info, sd.long_list.as<uint64_t>(), sb.t[t_b].descw,
+                                                 sb.t[t_b].offs, sd.long_ent.as<uint64_t>(), sd.pool.as<uint64_t>());
+    prof_end(PROF_SELECT, s);
+    count_launch();
+    WTG_CK(cudaGetLastError());
   }
   return WTG_OK;
 }
@@ -690,8 +799,8 @@ int bv_build(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t fla
              cudaStream_t s) {
   int rc;
   if ((rc = bv_prepare(bv, d_words, size, flags, s))) return rc;
-  if ((rc = bv_pass(bv, d_err, s))) return rc;
-  if (bv.rank_done) WTG_CK(cudaEventRecord(bv.rank_done, s));
+  if ((rc = bv_pass_begin(bv, s))) return rc;
+  if ((rc = bv_pass_to(bv, size, d_err, s))) return rc;
   return bv_finish(bv, d_err, s);
 }
 
@@ -706,7 +815,7 @@ int bv_build(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t fla
 // array of fixed size, so the call allocates nothing.  Every GPU that loads
 // the library holds this array until the process exits.
 constexpr uint64_t NOALLOC_MAX_BITS = 1ull << 34;  // 16 Gbit (2 GiB of bits)
-constexpr uint64_t NOALLOC_TILES = ((NOALLOC_MAX_BITS >> 9) + 1 + BVT_SB - 1) / BVT_SB;
+constexpr uint64_t NOALLOC_TILES = ((NOALLOC_MAX_BITS >> 9) + 1 + BV_THREADS - 1) / BV_THREADS;
 constexpr uint64_t NOALLOC_WORDS = 1 + NOALLOC_TILES + INF_N + 1;  // counter, status, info, error
 static __device__ __align__(256) uint64_t g_noalloc_scratch[NOALLOC_WORDS];
 
@@ -747,8 +856,9 @@ extern "C" int wtg_rank_build_noalloc(const uint64_t* d_words, uint64_t size_bit
   uint64_t* scratch = noalloc_scratch_ptr(dev, &rc);
   if (!scratch) return rc;
   cudaStream_t s = (cudaStream_t)stream;
-  const uint64_t W = (size_bits + 63) / 64, NB = W >> 3;
-  const uint64_t tiles = (NB + 1 + BVT_SB - 1) / BVT_SB;
+  const uint64_t NB = ((size_bits + 63) / 64) >> 3;
+  const int spt = bv_spt(NB);
+  const uint64_t tiles = (NB + 1 + spt * BV_THREADS - 1) / (spt * BV_THREADS);
   uint32_t* counter = (uint32_t*)scratch;
   uint64_t* status = scratch + 1;
   unsigned long long* info = (unsigned long long*)(scratch + 1 + NOALLOC_TILES);
@@ -756,10 +866,9 @@ extern "C" int wtg_rank_build_noalloc(const uint64_t* d_words, uint64_t size_bit
   // the array keeps the previous call's contents: clear what must start at 0
   WTG_CK(cudaMemsetAsync(scratch, 0, (1 + tiles) * sizeof(uint64_t), s));
   WTG_CK(cudaMemsetAsync(info, 0, (INF_N + 1) * sizeof(uint64_t), s));
-  bv_pass_kernel<<<(unsigned)tiles, BV_THREADS, 0, s>>>(d_words, size_bits, W, NB, WTG_RANK, d_rank, nullptr, 0,
-                                                       nullptr, nullptr, nullptr, nullptr, info, status, counter, err);
-  count_launch();
-  WTG_CK(cudaGetLastError());
+  if ((rc = launch_bv_pass(spt, d_words, size_bits, WTG_RANK, d_rank, nullptr, 0, nullptr, nullptr, nullptr, nullptr,
+                           info, status, counter, 0, (uint32_t)tiles, err, s)))
+    return rc;
   // read the error word on the caller's stream only: no device-wide wait
   uint32_t e = 0;
   WTG_CK(cudaMemcpyAsync(&e, err, sizeof(e), cudaMemcpyDeviceToHost, s));

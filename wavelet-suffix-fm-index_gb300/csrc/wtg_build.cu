@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(LV_THREADS, 3)
                  const uint2* __restrict__ base_lvl, uint32_t* __restrict__ bits32, uint64_t bit_off,
                  const uint32_t* __restrict__ chunkpre, uint32_t* __restrict__ chunkcnt_next,
                  uint32_t* __restrict__ nc0, uint32_t* __restrict__ nc1,
-                 uint32_t* __restrict__ znext, uint32_t* err, int bulk_ok, uint32_t* __restrict__ chunkcnt_self) {
+                 uint32_t* __restrict__ znext, uint32_t* err, int bulk_ok) {
   constexpr uint32_t CBYTES = CHUNK * sizeof(T);
   constexpr uint32_t CPB = LvShape<T>::CPB;
   constexpr uint32_t GBYTES = CBYTES * CPB;  // one bulk copy: CPB consecutive chunks
@@ -427,17 +427,14 @@ __global__ void __launch_bounds__(LV_THREADS, 3)
     }
 
     if (!SCATTER) {
-      // last level: bits only (and, when asked, the chunk's zero count)
-      uint32_t zc = 0;
+      // last level: bits only
 #pragma unroll 4
       for (int r = 0; r < WROWS; ++r) {
         const uint32_t k = r * 32 + lane;
         const bool valid = k < cvalid;
         const uint32_t om = __ballot_sync(0xffffffffu, valid && ((uint32_t)wt[k] & m1));
         myrow[r].x = om;  // every lane stores the same word: no branch
-        zc += __popc(__ballot_sync(0xffffffffu, valid) & ~om);
       }
-      if (chunkcnt_self && lane == 0) chunkcnt_self[c] = zc;
     } else if (uniform && cvalid == CHUNK) {
       // ---- fast path: full chunk inside one node
       if (p0 != cache_p) {
@@ -776,7 +773,6 @@ struct LevelArgs {
   uint32_t *nc0, *nc1;  // per chunk: counts of the next level's two nodes (emit_nodes)
   uint32_t* znext;
   uint32_t* err;
-  uint32_t* chunkcnt_self;
   bool scatter, emit_nodes, emit_tiles;
 };
 
@@ -786,7 +782,7 @@ static void launch_level_v(const LevelArgs& a, cudaStream_t st) {
   const size_t shm = LvShape<T>::template smem<SC>();
   level_kernel<T, SC, EN, ET><<<level_grid<T, SC, EN, ET>(a.n), LV_THREADS, shm, st>>>(
       (const T*)a.src, (T*)a.dst, a.n, a.L, a.level, a.base_lvl, a.bits32, a.bit_off, a.chunkpre,
-      a.chunkcnt_next, a.nc0, a.nc1, a.znext, a.err, bulk_ok, a.chunkcnt_self);
+      a.chunkcnt_next, a.nc0, a.nc1, a.znext, a.err, bulk_ok);
 }
 
 template <typename T>
@@ -943,28 +939,26 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   }
 
   // level passes; each scattering pass feeds the next level's chunk counts
-  // and (from level K on) its node tables.  With n % 512 == 0 the chunk
-  // counts of every level also give the rank/select pass its prefixes.
-  const bool rs_from_levels = flags && n > 0 && (n % CHUNK) == 0;
+  // and (from level K on) its node tables.
   // When the rank table goes to page-locked host memory during the build,
-  // the rank/select pass runs level by level after each level pass, and each
-  // level's rank entries are copied while the later levels are built (a copy
-  // to pageable memory would hold the host until it ends); otherwise it is
-  // one launch over all levels after the last pass.
-  const bool rs_by_level = rs_from_levels && t.host_rank && (flags & WTG_RANK) && host_page_locked(t.host_rank);
-  uint64_t* lvl_zb = nullptr;
-  if (rs_from_levels) {
-    if ((rc = t.scratch.ensure(((uint64_t)L + 1) * sizeof(uint64_t), s))) return rc;
-    lvl_zb = t.scratch.as<uint64_t>();
-    if ((rc = bv_levels_begin(t.bv, t.bits.as<uint64_t>(), n, L, flags, s))) return rc;
+  // the rank/select pass follows the levels, and the rank entries whose bits
+  // are final are copied while the later levels are built (a copy to pageable
+  // memory would hold the host until it ends); otherwise it is one launch
+  // after the last pass.
+  const bool rs_by_level = t.host_rank && (flags & WTG_RANK) && n && host_page_locked(t.host_rank);
+  if (flags) {
+    if ((rc = bv_prepare(t.bv, t.bits.as<uint64_t>(), n * (uint64_t)L, flags, s))) return rc;
+    if ((rc = bv_pass_begin(t.bv, s))) return rc;
   }
-  const uint64_t rank_words_per_level = 2 * (n / CHUNK);  // rank entries of one level when n % 512 == 0
-  auto copy_rank_level = [&](int l) -> int {
-    const uint64_t off = (uint64_t)l * rank_words_per_level;
+  uint64_t rank_copied = 0;  // superblocks whose rank entries were sent
+  auto copy_rank = [&]() -> int {
+    const uint64_t to = bv_superblocks_done(t.bv);
+    if (to <= rank_copied) return WTG_OK;
     WTG_CK(cudaEventRecord(t.copy_ev, s));
     WTG_CK(cudaStreamWaitEvent(t.copy_stream, t.copy_ev, 0));
-    WTG_CK(cudaMemcpyAsync(t.host_rank + off, t.bv.rank.as<uint64_t>() + off, rank_words_per_level * 8,
-                           cudaMemcpyDeviceToHost, t.copy_stream));
+    WTG_CK(cudaMemcpyAsync(t.host_rank + 2 * rank_copied, t.bv.rank.as<uint64_t>() + 2 * rank_copied,
+                           (to - rank_copied) * 16, cudaMemcpyDeviceToHost, t.copy_stream));
+    rank_copied = to;
     return WTG_OK;
   };
   if (n) {
@@ -990,7 +984,6 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
       uint32_t* tilepre = tilepre_all + (uint64_t)l * tst;
       a.chunkpre = tilepre;
       a.chunkcnt_next = tilecnt + (uint64_t)(l + 1) * tst;
-      a.chunkcnt_self = (!a.scatter && rs_from_levels) ? tilecnt + (uint64_t)l * tst : nullptr;
       a.znext = Z + ((1ull << (l + 1)) - 1);
       a.nc0 = a.emit_nodes ? t.nodecnt.as<uint32_t>() : nullptr;
       a.nc1 = a.emit_nodes ? a.nc0 + tst : nullptr;
@@ -1047,38 +1040,19 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
         count_launch();
         WTG_CK(cudaGetLastError());
       }
-      // a scattering level's chunk prefixes were scanned before its pass
       if (rs_by_level && l < L - 1) {
-        if ((rc = bv_levels_pass(t.bv, n, l, l + 1, tilecnt, tilepre_all, tst, tiles, lvl_zb, s))) return rc;
-        if ((rc = copy_rank_level(l))) return rc;
+        if ((rc = bv_pass_to(t.bv, ((uint64_t)l + 1) * n, d_err, s))) return rc;
+        if ((rc = copy_rank())) return rc;
       }
     }
   }
 
   // rank / select over the concatenated bitvector
-  t.bv.rank_done = (t.host_rank && (flags & WTG_RANK)) ? t.rank_ev : nullptr;
-  if (rs_from_levels) {
-    uint32_t* last_cnt = tilecnt + (uint64_t)(L - 1) * tst;
-    uint32_t* last_pre = tilepre_all + (uint64_t)(L - 1) * tst;
-    if ((rc = scan_exclusive_u32(last_cnt, last_pre, tiles, t.scan_tmp, d_err, s))) return rc;
-    if ((rc = bv_levels_pass(t.bv, n, rs_by_level ? L - 1 : 0, L, tilecnt, tilepre_all, tst, tiles, lvl_zb, s)))
-      return rc;
-    if (rs_by_level && (rc = copy_rank_level(L - 1))) return rc;
-    if ((rc = bv_levels_end(t.bv, L, lvl_zb, d_err, s))) return rc;
-  } else if (flags) {
-    if ((rc = bv_build(t.bv, t.bits.as<uint64_t>(), n * (uint64_t)L, flags, d_err, s))) return rc;
-  }
-  if (t.bv.rank_done) {
-    // the rank table (level by level: the rest, its final pair) was complete
-    // before the select finishing kernels started; its copy runs beside them
-    const uint64_t size = n * (uint64_t)L;
-    const uint64_t cap = (size + 63) / 64 * 64;
-    const uint64_t rank_words = size ? ((cap >> 9) + 1) * 2 : 2;
-    const uint64_t from = rs_by_level ? rank_words - 2 : 0;
-    WTG_CK(cudaStreamWaitEvent(t.copy_stream, t.bv.rank_done, 0));
-    WTG_CK(cudaMemcpyAsync(t.host_rank + from, t.bv.rank.as<uint64_t>() + from, (rank_words - from) * 8,
-                           cudaMemcpyDeviceToHost, t.copy_stream));
-    t.bv.rank_done = nullptr;
+  if (flags) {
+    if ((rc = bv_pass_to(t.bv, n * (uint64_t)L, d_err, s))) return rc;
+    // the select finishing kernels run beside the copy of the (last) rank entries
+    if (t.host_rank && (flags & WTG_RANK) && (rc = copy_rank())) return rc;
+    if ((rc = bv_finish(t.bv, d_err, s))) return rc;
   }
   return WTG_OK;
 }
@@ -1103,8 +1077,7 @@ void tree_release(TreeImpl& t) {
     t.copy_stream = nullptr;
   }
   if (t.copy_ev) cudaEventDestroy(t.copy_ev);
-  if (t.rank_ev) cudaEventDestroy(t.rank_ev);
-  t.copy_ev = t.rank_ev = nullptr;
+  t.copy_ev = nullptr;
   if (t.in_stream) {
     cudaStreamSynchronize(t.in_stream);
     cudaStreamDestroy(t.in_stream);

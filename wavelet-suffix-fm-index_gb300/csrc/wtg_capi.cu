@@ -228,7 +228,6 @@ int wtg_tree_build_out(const void* seq, uint64_t n, int elem_bytes, int levels, 
   }
   if (e == cudaSuccess && !t.copy_stream) e = cudaStreamCreateWithFlags(&t.copy_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess && !t.copy_ev) e = cudaEventCreateWithFlags(&t.copy_ev, cudaEventDisableTiming);
-  if (e == cudaSuccess && !t.rank_ev) e = cudaEventCreateWithFlags(&t.rank_ev, cudaEventDisableTiming);
   if (e != cudaSuccess) {
     if (fresh) wtg_tree_free(T);
     return cuda_fail(e, "stream/event create");

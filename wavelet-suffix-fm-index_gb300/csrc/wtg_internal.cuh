@@ -362,7 +362,7 @@ struct SelectDev {
   DevBuf ends;      // superblock end positions (upper-bound sized)
   DevBuf starts;    // superblock start positions (upper-bound sized)
   DevBuf desc;      // per superblock descriptor
-  DevBuf sizes;     // per superblock pool words (scan input)
+  DevBuf offs;      // per superblock pool word offset
   DevBuf sb_words;  // packed m_superblock
   DevBuf pool;      // packed mini/long blocks
   DevBuf long_list; // superblock ids of long blocks
@@ -380,26 +380,23 @@ struct BvSupport {
   DevBuf status;     // look-back status words + tile counter
   DevBuf scan_tmp;
   SelectDev sel[2];  // [t_b]
-  cudaEvent_t rank_done = nullptr;  // when set, recorded once the rank table is complete
+  // the pass over the bits: superblocks per thread, tiles, tiles launched so far
+  int spt = 1;
+  uint32_t tiles = 0, tiles_done = 0;
 };
 
 int bv_build(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t flags, uint32_t* d_err,
              cudaStream_t s);
-// the same in three steps: allocate and clear, the pass over the bits, and
+// the same in steps: allocate and clear; start the pass over the bits; run it
+// over the tiles that lie within the first bits_ready bits (in one call, or in
+// several as the bits become final: the whole vector with bits_ready >= size);
 // the select structures' finishing kernels
 int bv_prepare(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t& flags, cudaStream_t s);
-int bv_pass(BvSupport& bv, uint32_t* d_err, cudaStream_t s);
+int bv_pass_begin(BvSupport& bv, cudaStream_t s);
+int bv_pass_to(BvSupport& bv, uint64_t bits_ready, uint32_t* d_err, cudaStream_t s);
 int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s);
-// for a wavelet tree's bits with n % 512 == 0: the same structures from the
-// level passes' per-chunk zero counts (chunkcnt) and their scans (chunkpre),
-// both [L][stride], in three steps: allocate and clear; the pass over levels
-// l0..l1-1 (once over all levels, or level by level in order as each level's
-// bits and chunk prefixes are final), which extends lvl_zb (L + 1 words, the
-// zeros before each level) to l1; the totals and the select finishing kernels
-int bv_levels_begin(BvSupport& bv, const uint64_t* d_words, uint64_t n, int L, uint32_t flags, cudaStream_t s);
-int bv_levels_pass(BvSupport& bv, uint64_t n, int l0, int l1, const uint32_t* chunkcnt, const uint32_t* chunkpre,
-                   uint64_t stride, uint64_t nchunks, uint64_t* lvl_zb, cudaStream_t s);
-int bv_levels_end(BvSupport& bv, int L, const uint64_t* lvl_zb, uint32_t* d_err, cudaStream_t s);
+// superblocks whose rank entries the launched passes write
+uint64_t bv_superblocks_done(const BvSupport& bv);
 void bv_release(BvSupport& bv, cudaStream_t s);
 
 }  // namespace wtg

@@ -41,7 +41,7 @@ struct TreeImpl {
   uint64_t* host_bits = nullptr;
   uint64_t* host_rank = nullptr;
   cudaStream_t copy_stream = nullptr;
-  cudaEvent_t copy_ev = nullptr, rank_ev = nullptr;
+  cudaEvent_t copy_ev = nullptr;
   // input arriving in pieces (wtg_tree_build_out from page-locked memory):
   // piece i holds chunks [i * in_piece_chunks, (i + 1) * in_piece_chunks) of
   // 512 symbols and is on the device once in_ev[i] has fired; the pre-pass
