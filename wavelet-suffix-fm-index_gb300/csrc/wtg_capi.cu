@@ -248,20 +248,19 @@ int wtg_tree_build_out(const void* seq, uint64_t n, int elem_bytes, int levels, 
     if (pieces) {
       // the pieces start after everything queued on the build stream (the
       // buffer's allocation, a previous build's reads of it)
-      const uint64_t nchunks = (n + 511) / 512;
-      const uint64_t per = (nchunks + pieces - 1) / pieces;
+      const uint64_t per = ((n + pieces - 1) / pieces + 65535) / 65536 * 65536;  // whole count tiles
       ce = cudaEventRecord(t.in_ev[0], t.stream);
       if (ce == cudaSuccess) ce = cudaStreamWaitEvent(t.in_stream, t.in_ev[0], 0);
       for (int i = 0; ce == cudaSuccess && i < pieces; ++i) {
-        const uint64_t lo = std::min<uint64_t>(n, (uint64_t)i * per * 512);
-        const uint64_t hi = std::min<uint64_t>(n, ((uint64_t)i + 1) * per * 512);
+        const uint64_t lo = std::min<uint64_t>(n, (uint64_t)i * per);
+        const uint64_t hi = std::min<uint64_t>(n, ((uint64_t)i + 1) * per);
         if (hi > lo)
           ce = cudaMemcpyAsync((char*)t.seq.p + lo * elem_bytes, (const char*)seq + lo * elem_bytes,
                                (hi - lo) * elem_bytes, cudaMemcpyHostToDevice, t.in_stream);
         if (ce == cudaSuccess) ce = cudaEventRecord(t.in_ev[i], t.in_stream);
       }
       t.in_pieces = pieces;
-      t.in_piece_chunks = per;
+      t.in_piece_symbols = per;
     } else if (n) {
       ce = cudaMemcpyAsync(t.seq.p, seq, n * elem_bytes, cudaMemcpyHostToDevice, t.stream);
     }

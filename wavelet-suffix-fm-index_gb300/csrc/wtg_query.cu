@@ -189,7 +189,7 @@ int tree_node_table(TreeImpl& t, cudaStream_t s) {
   if ((rc = t.node_tab.ensure(nodes * sizeof(ulonglong2), s))) return rc;
   const uint64_t heap = 1ull << t.levels;
   node_table_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(
-      t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>() + 2 * heap, t.n, nodes,
+      t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>() + heap, t.n, nodes,
       t.node_tab.as<ulonglong2>());
   count_launch();
   WTG_CK(cudaGetLastError());

@@ -147,7 +147,7 @@ int tree_leaf_count(TreeImpl& t, uint64_t* sigma, cudaStream_t s) {
   const unsigned grid = (unsigned)std::min<uint64_t>((m + 255) / 256, 1024);
   const uint64_t heap = 1ull << t.levels;
   leaf_count_kernel<<<grid, 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                         t.zeros.as<uint32_t>() + 2 * heap, t.n, t.levels,
+                                         t.zeros.as<uint32_t>() + heap, t.n, t.levels,
                                          t.qout.as<unsigned long long>());
   count_launch();
   WTG_CK(cudaGetLastError());

@@ -12,10 +12,11 @@ struct LselImpl;
 //   seq        the input copied from the host (host-input builds only)
 //   lvl[0..1]  ping-pong buffers of the level orders, n symbols each
 //   bits       ceil(n*L/64) words of level bits + 2 zero words
-//   hist       S: exclusive scan of the 2^L key histogram (2^L + 1 x u32)
-//   zeros      [Z | ZS]: zeros per heap node and its exclusive scan (2 x 2^L x u32)
-//   base       per heap node (C - Zb, zeros + Zb) (2^L x uint2)
-//   status     per level: tile counter + look-back status words
+//   zeros      [Z | C]: left-child size and start per heap node (2 x 2^L x u32)
+//   chunkpre   per 1024-symbol chunk the digit counts before it (16 x u32)
+//   cnode      per chunk the node of its first symbol
+//   rec        per node of a group's first level its bases (32 x u32)
+//   status     per group of levels: tile counter + look-back status words
 //   bv         rank/select supports over `bits`
 //   lvl_args   ones before each level start, L + 1 words (filled on first use
 //              after a build by tree_level_args)
@@ -27,8 +28,7 @@ struct TreeImpl {
   uint64_t bit_words = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  DevBuf seq, lvl[2], bits, hist, zeros, base, status, scan_tmp, err, scratch, nodes, qbuf, qout;
-  DevBuf nodecnt;  // per chunk: the node counts of a level pass, then their scans
+  DevBuf seq, lvl[2], bits, zeros, chunkpre, cnode, rec, status, scan_tmp, err, scratch, nodes, qbuf, qout;
   BvSupport bv;
   DevBuf lvl_args;
   bool lvl_args_ok = false;
@@ -43,14 +43,14 @@ struct TreeImpl {
   cudaStream_t copy_stream = nullptr;
   cudaEvent_t copy_ev = nullptr;
   // input arriving in pieces (wtg_tree_build_out from page-locked memory):
-  // piece i holds chunks [i * in_piece_chunks, (i + 1) * in_piece_chunks) of
-  // 512 symbols and is on the device once in_ev[i] has fired; the pre-pass
-  // counts each piece as it lands.  in_pieces = 0: the input is resident.
+  // piece i holds symbols [i * in_piece_symbols, (i + 1) * in_piece_symbols)
+  // and is on the device once in_ev[i] has fired; the first count pass counts
+  // each piece as it lands.  in_pieces = 0: the input is resident.
   static constexpr int IN_PIECES_MAX = 8;
   cudaStream_t in_stream = nullptr;
   cudaEvent_t in_ev[IN_PIECES_MAX] = {};
   int in_pieces = 0;
-  uint64_t in_piece_chunks = 0;
+  uint64_t in_piece_symbols = 0;
   std::vector<LselImpl*> deps;  // learned select indexes reading this tree
 };
 
