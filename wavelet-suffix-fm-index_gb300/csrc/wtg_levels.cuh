@@ -15,13 +15,13 @@
 // order, all nodes) the second is base(p, d) + Z_d(i), base(p, d) =
 // C_{l+TAU}(p 2^TAU + d) - Z_d(C_l(p)), and the first base_j(p, q) + the sum
 // of Z_d(i) over the digits d that start with q.  So a group is three passes:
-//   count_kernel  per 1024-symbol chunk its digit counts, scanned over the
-//                 chunks in the same launch (decoupled look-back), and the
-//                 node of its first symbol;
-//   node_kernel   per node the digit counts before its two ends, from which
-//                 the starts and left-child sizes of the next TAU levels and
-//                 the record of its bases;
-//   pass_kernel   the bits of the TAU levels and the scatter.
+//   count_kernel       per 1024-symbol chunk its digit counts, scanned over
+//                      the chunks in the same launch (decoupled look-back);
+//   node_pass_kernel   per node the digit counts before its two ends, from
+//                      which the starts and left-child sizes of the next TAU
+//                      levels and the record of its bases; and the node of
+//                      each chunk's first symbol;
+//   level_pass_kernel  the bits of the TAU levels and the scatter.
 //
 // Symbols lose the bits already used: the order is stored in the narrowest
 // of 4, 2 and 1 bytes that holds the remaining bits.  2^30 32-bit symbols
@@ -30,9 +30,16 @@
 //
 // All passes work on 32 symbols per lane (a row): a lane reads its row with
 // 32-byte loads, gathers the digit's bit planes (one 32-bit word per bit, bit
-// i = symbol i), and digit counts are popcounts of masks.  That leaves a
-// pass bound by instruction issue: about 45 warp instructions per 32 symbols
-// and four levels, where a ballot per level and 32 symbols took 36 for each.
+// i = symbol i), and digit counts are popcounts of masks.  A scattering pass
+// takes about 72 warp instructions per 32 symbols for its four levels, where
+// a ballot per level and 32 symbols took 36 for each level; it is bound by the
+// integer ALU pipe (65 %) and shared-memory latency at 21-24 warps per SM.
+// At 2^30 symbols a pass takes 3.5 ms (4 to 2 bytes), 3.0 ms (2 bytes), 2.9
+// ms (1 byte), the last one 2.1 ms, the count passes 0.32-0.75 ms; a level
+// pass took 1.43 ms before, 19 of them.  Measured and not kept: 32 warps per
+// SM (64 registers: spills, 3-5 % slower), the scan of the row counts by
+// columns through shared memory (110 instructions fewer a chunk, 4 % slower),
+// a swizzled sorted chunk (two instructions a symbol, 5 % slower).
 #pragma once
 #include <type_traits>
 
@@ -158,24 +165,7 @@ __device__ __forceinline__ uint32_t row_mask(uint32_t row, uint32_t lo, uint32_t
 
 // ------------------------------------------------------------ node search
 
-// the last p in [0, cnt) with C[p] <= pos (C[0] = 0, not decreasing): a warp
-// tries 32 evenly spaced entries at a time
-__device__ __forceinline__ uint32_t find_node_warp(const uint32_t* __restrict__ C, uint32_t cnt, uint32_t pos) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t lo = 0, len = cnt;  // the answer lies in [lo, lo + len)
-  while (len > 1) {
-    const uint32_t step = (len + 31) / 32;
-    const uint32_t at = lane * step;
-    const bool le = at < len && __ldg(C + lo + at) <= pos;
-    const uint32_t hit = __popc(__ballot_sync(0xffffffffu, le));  // >= 1: C[lo] <= pos
-    const uint32_t first = (hit - 1) * step;
-    lo += first;
-    len = min(step, len - first);
-  }
-  return lo;
-}
-
-// the same over [lo, hi] by one thread
+// the last p in [lo, hi] with C[p] <= pos (C[lo] <= pos, not decreasing)
 __device__ __forceinline__ uint32_t find_node(const uint32_t* __restrict__ C, uint32_t lo, uint32_t hi, uint32_t pos) {
   while (lo < hi) {
     const uint32_t mid = (lo + hi + 1) >> 1;
@@ -190,14 +180,12 @@ __device__ __forceinline__ uint32_t find_node(const uint32_t* __restrict__ C, ui
 // Digit counts of every chunk and their exclusive scan over the chunks:
 // chunkpre[c * 16 + d] = symbols before chunk c with digit d, and the totals
 // at c = nchunks.  A CTA takes tiles of 8 * cpw chunks from a counter (so the
-// look-back always waits on tiles that have started).  cnode (levels below
-// the root only): the node of each chunk's first symbol.  Bound by the read
+// look-back always waits on tiles that have started).  Bound by the read
 // of the sequence for 4-byte symbols, by issue for narrower ones.
 template <typename T, int TB>
 __global__ void __launch_bounds__(LV_THREADS)
     count_kernel(const T* __restrict__ src, uint64_t n, int ds, uint32_t nchunks, int cpw,
-                 const uint32_t* __restrict__ Cl, uint32_t nodes, uint32_t* __restrict__ chunkpre,
-                 uint32_t* __restrict__ cnode, uint64_t* __restrict__ status, uint32_t sstride,
+                 uint32_t* __restrict__ chunkpre, uint64_t* __restrict__ status, uint32_t sstride,
                  uint32_t* __restrict__ counter, uint32_t tile0, uint32_t tile_end, uint32_t* __restrict__ err) {
   constexpr int MAX_TC = 64;  // chunks per tile
   constexpr int ND = 1 << TB;
@@ -215,32 +203,30 @@ __global__ void __launch_bounds__(LV_THREADS)
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= tile_end) return;
-    for (int k = 0; k < cpw; ++k) {
+    // narrow symbols two chunks at a time (cpw is 1 or even): both rows are on
+    // their way before the first is counted
+    constexpr int AHEAD = sizeof(T) == 4 ? 1 : 2;
+    for (int k = 0; k < cpw; k += AHEAD) {
       const uint32_t lc = warp * cpw + k;
       const uint32_t c = tile * tc + lc;
-      uint32_t pk[NP];
+      const uint64_t base = (uint64_t)c << LOG_CHUNK;
+      uint32_t w[AHEAD][8 * sizeof(T)];
 #pragma unroll
-      for (int i = 0; i < NP; ++i) pk[i] = 0;
-      if (c < nchunks) {
-        const uint64_t base = (uint64_t)c << LOG_CHUNK;
-        uint32_t w[8 * sizeof(T)], B[TB];
-        load_row<T>(src, base + 32 * lane, n, w);
-        planes<T, TB>(w, ds, B);
-        const uint32_t valid = (uint32_t)min((uint64_t)CHUNK, n - base);
-        digit_counts<TB>(B, row_mask(lane, 0, valid), pk);
-        if (nodes > 1) {
-          const uint32_t p = find_node_warp(Cl, nodes, (uint32_t)base);
-          if (lane == 0) {
-            cnode[c] = p;
-            if (c + 1 == nchunks) cnode[nchunks] = nodes - 1;
-          }
+      for (int h = 0; h < AHEAD; ++h)
+        if (k + h < cpw) load_row<T>(src, base + h * CHUNK + 32 * lane, n, w[h]);  // zeros past the end
+#pragma unroll
+      for (int h = 0; h < AHEAD; ++h) {
+        if (k + h >= cpw) break;
+        uint32_t pk[NP], B[TB];
+        planes<T, TB>(w[h], ds, B);
+        const uint64_t cb = base + h * CHUNK;
+        digit_counts<TB>(B, row_mask(lane, 0, cb < n ? (uint32_t)min((uint64_t)CHUNK, n - cb) : 0u), pk);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) pk[i] = __reduce_add_sync(0xffffffffu, pk[i]);  // halves stay below 2^16
+        if (lane == 0) {
+#pragma unroll
+          for (int i = 0; i < NP; ++i) s_pk[lc + h][i] = pk[i];
         }
-      }
-#pragma unroll
-      for (int i = 0; i < NP; ++i) pk[i] = __reduce_add_sync(0xffffffffu, pk[i]);  // halves stay below 2^16
-      if (lane == 0) {
-#pragma unroll
-        for (int i = 0; i < NP; ++i) s_pk[lc][i] = pk[i];
       }
     }
     __syncthreads();
@@ -301,12 +287,14 @@ __global__ void __launch_bounds__(LV_THREADS)
 // prefixes plus the counts of the end chunks' heads), then the starts C and
 // left-child sizes Z of its descendants on the next TB levels and its record
 // (see REC).  Node tables are in heap order: node p of level m at
-// 2^m - 1 + p.  Work is a handful of kilobytes a node, latency bound.
+// 2^m - 1 + p.  Work is a handful of kilobytes a node, latency bound.  Below
+// the root, then thread per chunk: the node of its first symbol (neighbours
+// search the same way, so their loads coincide).
 template <typename T, int TB>
 __global__ void __launch_bounds__(LV_THREADS)
     node_pass_kernel(const T* __restrict__ src, uint64_t n, int ds, int l, uint32_t* __restrict__ C,
                      uint32_t* __restrict__ Z, const uint32_t* __restrict__ chunkpre, uint32_t nchunks, int scatter,
-                     uint32_t* __restrict__ rec) {
+                     uint32_t* __restrict__ rec, uint32_t* __restrict__ cnode) {
   constexpr uint32_t ND = 1u << TB;
   const uint32_t lane = threadIdx.x & 31;
   const uint64_t nodes = 1ull << l;
@@ -355,7 +343,7 @@ __global__ void __launch_bounds__(LV_THREADS)
     const uint32_t za = __shfl_sync(0xffffffffu, pz, a), zb = __shfl_sync(0xffffffffu, pz, b & 31);
     const uint64_t h = (nodes << j) - 1 + (p << j) + q;
     if (in) {
-      C[h] = ca;
+      if (j) C[h] = ca;  // (the node's own start is there)
       if (j < TB) Z[h] = mid - ca;
     }
     // digit d's scatter base goes to lane 16 + d
@@ -367,6 +355,13 @@ __global__ void __launch_bounds__(LV_THREADS)
         rec[p * REC + lane] = ca - (zb - za);
       }
     }
+  }
+  if (l) {
+    const uint32_t* __restrict__ Cl = C + nodes - 1;
+    const uint32_t threads = gridDim.x * blockDim.x;
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += threads)
+      cnode[c] = find_node(Cl, 0, (uint32_t)nodes - 1, c << LOG_CHUNK);
+    if (blockIdx.x == 0 && threadIdx.x == 0) cnode[nchunks] = (uint32_t)nodes - 1;
   }
 }
 
@@ -407,8 +402,17 @@ __device__ __forceinline__ void sts32(uint32_t a, uint32_t v) {
 __device__ __forceinline__ void sts64(uint32_t a, uint32_t x, uint32_t y) {
   asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
 }
+// ORs v in when it has a bit (lanes with nothing to add would all meet on one word)
 __device__ __forceinline__ void ors32(uint32_t a, uint32_t v) {
-  asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %1, 0;\n @p red.shared.or.b32 [%0], %1;\n}\n" ::"r"(a), "r"(v)
+               : "memory");
+}
+// appends the low bit of p at the top of `one` when sel has a bit, else of `zero`
+__device__ __forceinline__ void append_to(uint32_t sel, uint32_t p, uint32_t& one, uint32_t& zero) {
+  asm("{\n .reg .pred q;\n setp.ne.u32 q, %2, 0;\n @q shf.r.wrap.b32 %0, %0, %3, 1;\n"
+      " @!q shf.r.wrap.b32 %1, %1, %3, 1;\n}\n"
+      : "+r"(one), "+r"(zero)
+      : "r"(sel), "r"(p));
 }
 template <typename T>
 __device__ __forceinline__ void sts_sym(uint32_t a, uint32_t v) {
@@ -471,8 +475,7 @@ struct LevelPass {
     const uint32_t v = __funnelshift_rc(acc, 0u, 32u - len);
     const uint32_t a = buf + ((off >> 5) << 2), sh = off & 31;
     ors32(a, v << sh);
-    const uint32_t hi = __funnelshift_l(v, 0u, sh);
-    if (hi) ors32(a + 4, hi);
+    ors32(a + 4, __funnelshift_l(v, 0u, sh));
   }
 
   // The symbols V of the rows, all of one node with record word rv (lane r
@@ -570,8 +573,7 @@ struct LevelPass {
             sts32(a2, __funnelshift_r(lds32(a2), P2, 1));
           }
           if constexpr (TAU > 2) {
-            if ((B[0] >> i) & 1u) a11 = __funnelshift_r(a11, P1, 1);
-            else a10 = __funnelshift_r(a10, P1, 1);
+            append_to(B[0] & (1u << i), P1, a11, a10);
           }
         }
         PL >>= 1;
@@ -633,7 +635,9 @@ struct LevelPass {
     }
     pz -= z0;
     bool bad = false;
-    uint32_t gp = 0, ls = 0, len = 0;
+    // (its words of the bitvector, one lane each over all strings of the
+    // segment: a string of many words takes no longer than many short ones)
+    uint32_t info = 0, glo = 0, ghi = 0, nw = 0;  // info: local start | bits << 11 | level << 22
     {
       const int j = 31 - __clz(lane + 1);
       const uint32_t q = lane + 1 - (1u << j);
@@ -641,31 +645,48 @@ struct LevelPass {
       const uint32_t da = in ? q << (TB - j) : 0u, db = in ? (q + 1) << (TB - j) : 0u;
       const uint32_t za = __shfl_sync(0xffffffffu, pz, da), zb = __shfl_sync(0xffffffffu, pz, db);
       if (in) {
-        ls = lds16(S + 2 * da);
-        len = lds16(S + 2 * db) - ls;
-        gp = rv + (zb - za);
-        if ((uint64_t)gp + len > a.n) bad = true, len = 0;
+        const uint32_t ls = lds16(S + 2 * da);
+        const uint32_t len = lds16(S + 2 * db) - ls;
+        const uint32_t gp = rv + (zb - za);
+        if ((uint64_t)gp + len > a.n) {
+          bad = true;
+        } else if (len) {
+          const uint64_t g = (uint64_t)(a.level + j) * a.n + gp;
+          glo = (uint32_t)g;
+          ghi = (uint32_t)(g >> 32);
+          nw = ((glo & 31) + len + 31) >> 5;
+          info = ls | (len << 11) | ((uint32_t)j << 22);
+        }
       }
     }
+    uint32_t wx = nw;  // words of the strings before
 #pragma unroll
-    for (int j = 1; j < TAU; ++j) {
-      const int per = 32 >> j;  // lanes per string
-      const uint32_t r = (1u << j) - 1 + lane / per;
-      const uint32_t g32 = __shfl_sync(0xffffffffu, gp, r), l0 = __shfl_sync(0xffffffffu, ls, r),
-                     ln = __shfl_sync(0xffffffffu, len, r);
-      const uint64_t g = (uint64_t)(a.level + j) * a.n + g32;
-      const uint32_t head = (uint32_t)g & 31;  // bits of the first word before the string
-      const uint32_t nw = ln ? (head + ln + 31) >> 5 : 0u;
-      const uint32_t buf = levelbuf(base, j);
-      for (uint32_t k = lane % per; k < nw; k += per) {
-        const int32_t lo = (int32_t)(l0 + 32 * k) - (int32_t)head;  // local bit of the word's bit 0
-        const uint32_t wa = buf + (uint32_t)((lo >> 5) * 4);
+    for (int o = 1; o < 16; o <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, wx, o);
+      if (lane >= (uint32_t)o) wx += x;
+    }
+    const uint32_t words = __shfl_sync(0xffffffffu, wx, (1 << TAU) - 2);
+    wx -= nw;
+    for (uint32_t at = 0; at < words; at += 32) {
+      const uint32_t i = at + lane;
+      uint32_t r = 0;  // the last string with at most i words before it (lane 0 has none: wx = 0)
+#pragma unroll
+      for (int o = 1 << (TAU - 1); o > 0; o >>= 1) {
+        const uint32_t x = __shfl_sync(0xffffffffu, wx, r + o);
+        if (r + o < (1u << TAU) - 1 && x <= i) r += o;
+      }
+      const uint32_t k = i - __shfl_sync(0xffffffffu, wx, r);
+      const uint32_t inf = __shfl_sync(0xffffffffu, info, r);
+      const uint32_t g0 = __shfl_sync(0xffffffffu, glo, r), g1 = __shfl_sync(0xffffffffu, ghi, r);
+      if (i < words) {
+        const uint32_t head = g0 & 31, ln = (inf >> 11) & 0x7FFu;
+        const int32_t lo = (int32_t)((inf & 0x7FFu) + 32 * k) - (int32_t)head;  // local bit of the word's bit 0
+        const uint32_t wa = levelbuf(base, 0) + (inf >> 22) * 512 + (uint32_t)((lo >> 5) * 4);
         const uint32_t val = __funnelshift_r(lds32(wa), lds32(wa + 4), lo & 31);
-        uint32_t mask = 0xFFFFFFFFu;
-        if (k == 0) mask <<= head;
+        uint32_t mask = k == 0 ? 0xFFFFFFFFu << head : 0xFFFFFFFFu;
         const uint32_t end = head + ln - 32 * k;  // valid bits end here
         if (end < 32) mask &= (1u << end) - 1;
-        put_bits(a.bits, (g >> 5) + k, val, mask);
+        put_bits(a.bits, (((uint64_t)g1 << 32 | g0) >> 5) + k, val, mask);
       }
     }
     if constexpr (SCATTER) {
@@ -682,14 +703,10 @@ struct LevelPass {
         const uint32_t total = FULL ? CHUNK : lds16(S + 2 * ND);
         const uint32_t stage = base + 4096;
         const int dsh = a.ds;
-        if (FULL) {
 #pragma unroll 8
-          for (uint32_t i = lane; i < CHUNK; i += 32) {
-            const uint32_t x = lds_sym<Tin>(stage + i * (uint32_t)sizeof(Tin));
-            dst[i + lds32(S + 64 + (((x >> dsh) & 15u) << 2))] = (Tout)x;
-          }
-        } else {
-          for (uint32_t i = lane; i < total; i += 32) {
+        for (uint32_t r = 0; r < 32; ++r) {
+          const uint32_t i = 32 * r + lane;
+          if (FULL || i < total) {
             const uint32_t x = lds_sym<Tin>(stage + i * (uint32_t)sizeof(Tin));
             dst[i + lds32(S + 64 + (((x >> dsh) & 15u) << 2))] = (Tout)x;
           }

@@ -1,5 +1,7 @@
 // wtg_pass_last.cu -- count and node passes, and the pass of a tree's last
 // group of levels (bits only).
+#include <algorithm>
+
 #include "wtg_pass.cuh"
 
 namespace wtg {
@@ -23,17 +25,17 @@ int count_t(const LevelGroup& a, uint32_t tile0, uint32_t tile1, cudaStream_t s)
   static int per_sm = 0;
   const PassArgs& p = a.pass;
   return launch_resident(count_kernel<T, TB>, per_sm, tile1 - tile0, 0, s, (const T*)p.src, p.n, p.ds + a.tau - TB,
-                         p.nchunks, a.cpw, p.Cl, p.nodes, a.chunkpre, a.cnode, a.status, a.sstride, a.counter, tile0,
-                         tile1, p.err);
+                         p.nchunks, a.cpw, a.chunkpre, a.status, a.sstride, a.counter, tile0, tile1, p.err);
 }
 
 template <typename T, int TB>
 int nodes_t(const LevelGroup& a, cudaStream_t s) {
   static int per_sm = 0;
   const PassArgs& p = a.pass;
-  return launch_resident(node_pass_kernel<T, TB>, per_sm, ((uint64_t)p.nodes + LV_WARPS - 1) / LV_WARPS, 0, s,
-                         (const T*)p.src, p.n, p.ds + a.tau - TB, p.level, a.C, a.Z, p.chunkpre, p.nchunks,
-                         (int)a.scatter, a.rec);
+  const uint64_t ctas = std::max(((uint64_t)p.nodes + LV_WARPS - 1) / LV_WARPS,
+                                 p.nodes > 1 ? ((uint64_t)p.nchunks + LV_THREADS - 1) / LV_THREADS : 1);
+  return launch_resident(node_pass_kernel<T, TB>, per_sm, ctas, 0, s, (const T*)p.src, p.n, p.ds + a.tau - TB, p.level,
+                         a.C, a.Z, p.chunkpre, p.nchunks, (int)a.scatter, a.rec, a.cnode);
 }
 
 template <typename T, int TAU>
