@@ -378,6 +378,7 @@ void tree_release(TreeImpl& t) {
   t.lvl_args_ok = false;
   t.fm_paths.release(s);
   t.node_tab.release(s);
+  t.node_step.release(s);
   t.node_tab_ok = false;
   t.scratch.release(s);
   t.nodes.release(s);

@@ -1,0 +1,88 @@
+// wtg_order.cuh -- large query batches taken in the order of their positions
+// (internal).
+//
+// A wavelet-tree query reads one rank entry and one word per level, at a
+// position that grows with the query's own position inside every node.  In
+// the caller's order each of these reads is a trip to DRAM once the tree is
+// larger than L2; sorted by the top bits of the position, the queries in
+// flight read a narrow window of every node, which stays in L2 and shares
+// sectors.  The sort is two 8-bit passes over (position, query number) pairs.
+#pragma once
+#include "wtg_radix.cuh"
+#include "wtg_tree.cuh"
+
+namespace wtg {
+
+struct QueryOrder {
+  const uint32_t* pos;  // positions, sorted by their top bits (n: outside the sequence)
+  const uint32_t* id;   // the query each belongs to
+};
+
+// Queries per sorted batch: bounds the scratch (16 bytes a query, 1 GB) and
+// the query numbers.
+constexpr uint64_t ORDER_BATCH = 1ull << 26;
+
+static __global__ void __launch_bounds__(256)
+    order_keys_kernel(const uint64_t* __restrict__ q, uint64_t nq, uint64_t n, uint32_t* __restrict__ pos) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nq; k += stride) {
+    const uint64_t i = q[k];
+    pos[k] = (uint32_t)(i < n ? i : n);
+  }
+}
+
+// When sorting pays: the tree is larger than what L2 keeps of it (its bits
+// from about 100 MB on, with the rank table 125 MB), has enough levels to
+// make up for the sort and for reading the other arguments by query number,
+// and the batch is large enough.  Measured (ms as they come / sorted):
+// access, 2^30 x 20 levels, 2^26 queries 47.0 / 14.3, 2^20 queries 0.81 / 0.50,
+// 2^19 0.40 / 0.34; rank, 2^27 x 8, 2^24 queries 1.94 / 1.36; but 2^26 x 8
+// 0.92 / 1.36 and 2^28 x 3 0.61 / 1.23.  Trees that L2 holds gain only by
+// the sectors that neighbours share, over many levels: 2^24 x 20, 2^22
+// queries 0.60 / 0.45, 2^20 queries 0.16 / 0.16; 2^25 x 12 0.35 / 0.39.
+inline bool order_pays(const TreeImpl& t, uint64_t nq) {
+  const uint64_t bytes = t.n * (uint64_t)t.levels / 8;
+  if (bytes >= (100ull << 20)) return t.levels >= 6 && nq >= (1ull << 20);
+  return bytes >= (20ull << 20) && t.levels >= 16 && nq >= (1ull << 21);
+}
+
+// Calls launch(sorted, order, first query, queries) over the batch: in sorted
+// batches where that pays and the scratch is to be had, otherwise once over
+// all queries as they come.
+template <typename F>
+int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch) {
+  if (!order_pays(t, nq)) return launch(false, QueryOrder{}, 0, nq);
+  const uint64_t most = nq < ORDER_BATCH ? nq : ORDER_BATCH;
+  const uint64_t pairs = (most + 63) / 64 * 64;
+  constexpr int passes = 2;
+  const uint64_t status = radix_status_bytes(most, passes);
+  const uint64_t bytes = 16 * pairs + passes * RS_RADIX * 4 + status + 16;
+  uint8_t* scratch = nullptr;
+  if (cudaMallocAsync(&scratch, bytes, s) != cudaSuccess) {
+    cudaGetLastError();  // no room: the queries as they come
+    return launch(false, QueryOrder{}, 0, nq);
+  }
+  uint32_t* const key[2] = {(uint32_t*)scratch, (uint32_t*)scratch + pairs};
+  uint32_t* const val[2] = {(uint32_t*)scratch + 2 * pairs, (uint32_t*)scratch + 3 * pairs};
+  uint32_t* hist = (uint32_t*)scratch + 4 * pairs;
+  uint8_t* st = (uint8_t*)(hist + passes * RS_RADIX);
+  const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
+  const int lo = bits > 8 * passes ? bits - 8 * passes : 0;
+  int rc = WTG_OK;
+  for (uint64_t at = 0; at < nq && rc == WTG_OK; at += most) {
+    const uint64_t m = nq - at < most ? nq - at : most;
+    order_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(pos + at, m, t.n, key[0]);
+    count_launch();
+    if (cudaGetLastError() != cudaSuccess) {
+      rc = fail(WTG_ERR_CUDA, "query order: launch failed");
+      break;
+    }
+    int cur = 0;
+    rc = radix_sort_pairs<uint32_t>(key, val, m, lo, passes, true, hist, st, t.err.as<uint32_t>(), cur, s);
+    if (rc == WTG_OK) rc = launch(true, QueryOrder{key[cur], val[cur]}, at, m);
+  }
+  cudaFreeAsync(scratch, s);
+  return rc;
+}
+
+}  // namespace wtg

@@ -3,6 +3,7 @@
 // select, one thread per query; plus the alphabet remap helper.
 #include <algorithm>
 
+#include "wtg_order.cuh"
 #include "wtg_select.cuh"
 #include "wtg_tree.cuh"
 
@@ -12,71 +13,74 @@ __device__ __forceinline__ int bit_at(const uint64_t* __restrict__ w, uint64_t p
   return (int)((w[p >> 6] >> (p & 63)) & 1);
 }
 
-// Node table: for every heap node h of levels 0..L-1 (root 0, children
-// 2h+1 / 2h+2), x = global bit offset of the node's start and y = ones before
-// it.  These are the `offset` and `o = m_tree_rank(offset)` that wt_int's
-// queries recompute at every level (wt_int_par.hpp:527-536, 561-572,
-// 596-606); with them tabulated, a query level costs one rank probe and one
-// bit word, fetched together with the next level's node entry.
+// Node tables: for every heap node h of levels 0..L-1 (root 0, children
+// 2h+1 / 2h+2)
+//   tab  : x = global bit offset of the node's start, y = ones before it --
+//          the `offset` and `o = m_tree_rank(offset)` that wt_int's queries
+//          recompute at every level (wt_int_par.hpp:527-536, 561-572,
+//          596-606);
+//   step : the two constants that take a position of the node to its child:
+//          with x the position inside the level and R the ones before it
+//          (rank1 of the concatenated bits), bit 0 goes on at step.x + x - R
+//          and bit 1 at step.y + R, positions inside the next level; after
+//          the last level the position inside the leaf.  All modulo 2^32.
+// With step, a query level costs one rank entry, one word and 8 bytes of a
+// table that is read beside them; tab took two 16-byte entries a level.
 __global__ void node_table_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                                  const uint32_t* __restrict__ C, uint64_t n, uint64_t nodes,
-                                  ulonglong2* __restrict__ tab) {
+                                  const uint32_t* __restrict__ Z, const uint32_t* __restrict__ C, uint64_t n, int L,
+                                  uint64_t nodes, ulonglong2* __restrict__ tab, uint2* __restrict__ step) {
   const uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= nodes) return;
   const uint64_t l = 63 - __clzll((long long)(h + 1));
-  const uint64_t off = l * n + C[h];
-  tab[h] = make_ulonglong2(off, rank1_dev(rt, tree, off));
+  const uint32_t c = C[h];
+  const uint64_t off = l * n + c;
+  const uint64_t y = rank1_dev(rt, tree, off);
+  tab[h] = make_ulonglong2(off, y);
+  const uint32_t Y = (uint32_t)y;
+  step[h] = (int)l + 1 < L ? make_uint2(Y, c + Z[h] - Y) : make_uint2(Y - c, 0u - Y);
 }
 
-// rank1(pos) with the word holding pos already loaded
-__device__ __forceinline__ uint64_t rank1_with_word(const uint64_t* __restrict__ rt, uint64_t pos, uint64_t word) {
+// ones before bit pos (mod 2^32), and the word holding pos
+__device__ __forceinline__ uint32_t rank_step(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                              uint64_t pos, uint64_t& word) {
   const ulonglong2 e = __ldg(reinterpret_cast<const ulonglong2*>(rt) + (pos >> 9));
-  uint64_t r = e.x + ((e.y >> (63 - 9 * ((pos & 0x1FF) >> 6))) & 0x1FF);
-  if (pos & 63) r += __popcll(word & ((1ull << (pos & 63)) - 1));
-  return r;
+  word = __ldg(tree + (pos >> 6));
+  const uint32_t in = (uint32_t)(e.y >> (63 - 9 * ((uint32_t)(pos >> 6) & 7))) & 0x1FFu;
+  return (uint32_t)e.x + in + __popcll(word & ((1ull << (pos & 63)) - 1));
 }
 
 // wt_int::operator[] (wt_int/wt_int_par.hpp:519-541) and inverse_select
 // (:588-611): descend by the bit at i; the symbol is the path, the rank the
 // final position
-template <bool INV>
+template <bool INV, bool ORD>
 __global__ void wt_descend_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                                  const ulonglong2* __restrict__ tab, uint64_t n, int L,
-                                  const uint64_t* __restrict__ q, uint64_t nq, uint64_t* __restrict__ out,
+                                  const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
+                                  QueryOrder ord, uint64_t nq, uint64_t* __restrict__ out,
                                   uint64_t* __restrict__ sym_out) {
-  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  uint64_t i = q[k];
+  const uint64_t i = ORD ? ord.pos[k] : q[k];
+  if (ORD) k = ord.id[k];
   if (i >= n) {
     out[k] = NONE64;
     if (INV) sym_out[k] = NONE64;
     return;
   }
-  uint64_t h = 0, c = 0;
-  ulonglong2 nd = __ldg(tab);
-  for (int lv = 0; lv < L; ++lv) {
-    const uint64_t pos = nd.x + i;
-    ulonglong2 c0 = nd, c1 = nd;
-    if (lv + 1 < L) {
-      c0 = __ldg(tab + 2 * h + 1);
-      c1 = __ldg(tab + 2 * h + 2);
-    }
-    const uint64_t word = __ldg(tree + (pos >> 6));
-    const uint64_t r = rank1_with_word(rt, pos, word) - nd.y;
-    const uint64_t bit = (word >> (pos & 63)) & 1;
-    c = (c << 1) | bit;
-    if (bit) {
-      i = r;
-      h = 2 * h + 2;
-      nd = c1;
-    } else {
-      i -= r;
-      h = 2 * h + 1;
-      nd = c0;
-    }
+  uint32_t x = (uint32_t)i, h = 1;  // h: heap id + 1, the path with a leading 1
+  uint64_t lbase = 0;
+  for (int lv = 0; lv < L; ++lv, lbase += n) {
+    const uint64_t pos = lbase + x;
+    uint2 st = make_uint2(0u, 0u);
+    if (INV || lv + 1 < L) st = __ldg(step + (h - 1));
+    uint64_t word;
+    const uint32_t R = rank_step(tree, rt, pos, word);
+    const uint32_t bit = (uint32_t)(word >> (pos & 63)) & 1u;
+    x = bit ? st.y + R : st.x + x - R;
+    h = 2 * h + bit;
   }
+  const uint64_t c = h - (1u << L);
   if (INV) {
-    out[k] = i;
+    out[k] = x;
     sym_out[k] = c;
   } else {
     out[k] = c;
@@ -84,13 +88,15 @@ __global__ void wt_descend_kernel(const uint64_t* __restrict__ tree, const uint6
 }
 
 // wt_int::rank (wt_int_par.hpp:553-577): descend along c's path
+template <bool ORD>
 __global__ void wt_rank_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                               const ulonglong2* __restrict__ tab, uint64_t n, int L,
-                               const uint64_t* __restrict__ q, const uint64_t* __restrict__ sym, uint64_t nq,
+                               const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
+                               QueryOrder ord, const uint64_t* __restrict__ sym, uint64_t nq,
                                uint64_t* __restrict__ out) {
-  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  uint64_t i = q[k];
+  if (ORD) k = ord.id[k];
+  const uint64_t i = q[k];
   const uint64_t c = sym[k];
   if (i > n) {
     out[k] = NONE64;
@@ -100,21 +106,16 @@ __global__ void wt_rank_kernel(const uint64_t* __restrict__ tree, const uint64_t
     out[k] = 0;
     return;
   }
-  uint64_t h = 0;
-  ulonglong2 nd = __ldg(tab);
-  for (int lv = 0; lv < L && i; ++lv) {
-    const uint64_t bit = (c >> (L - 1 - lv)) & 1;
-    const uint64_t child = 2 * h + 1 + bit;
-    ulonglong2 next = nd;
-    if (lv + 1 < L) next = __ldg(tab + child);
-    const uint64_t pos = nd.x + i;
-    const uint64_t word = __ldg(tree + (pos >> 6));
-    const uint64_t r = rank1_with_word(rt, pos, word) - nd.y;
-    i = bit ? r : i - r;
-    h = child;
-    nd = next;
+  const uint32_t path = (uint32_t)c | (1u << L);
+  uint32_t x = (uint32_t)i;
+  uint64_t lbase = 0;
+  for (int lv = 0; lv < L; ++lv, lbase += n) {
+    const uint2 st = __ldg(step + ((path >> (L - lv)) - 1));
+    uint64_t word;
+    const uint32_t R = rank_step(tree, rt, lbase + x, word);
+    x = (path >> (L - 1 - lv)) & 1u ? st.y + R : st.x + x - R;
   }
-  out[k] = i;
+  out[k] = x;
 }
 
 // wt_int::select (wt_int_par.hpp:622-660)
@@ -182,15 +183,18 @@ static int need(const TreeImpl& t, uint32_t f, const char* what) {
   return WTG_OK;
 }
 
+WTG_WAIT_LIMIT_SETTER(query)
+
 int tree_node_table(TreeImpl& t, cudaStream_t s) {
   int rc;
   if (t.node_tab_ok) return WTG_OK;
   const uint64_t nodes = (1ull << t.levels) - 1;
   if ((rc = t.node_tab.ensure(nodes * sizeof(ulonglong2), s))) return rc;
+  if ((rc = t.node_step.ensure(nodes * sizeof(uint2), s))) return rc;
   const uint64_t heap = 1ull << t.levels;
   node_table_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(
-      t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>() + heap, t.n, nodes,
-      t.node_tab.as<ulonglong2>());
+      t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>(), t.zeros.as<uint32_t>() + heap, t.n,
+      t.levels, nodes, t.node_tab.as<ulonglong2>(), t.node_step.as<uint2>());
   count_launch();
   WTG_CK(cudaGetLastError());
   t.node_tab_ok = true;
@@ -202,12 +206,14 @@ int launch_wt_access(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* ou
   if ((rc = need(t, WTG_RANK, "access"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  wt_descend_kernel<false><<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                    t.node_tab.as<ulonglong2>(), t.n, t.levels, idx, nq, out,
-                                                    nullptr);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  return WTG_OK;
+  return in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    auto* const f = sorted ? wt_descend_kernel<false, true> : wt_descend_kernel<false, false>;
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n,
+                               t.levels, idx + at, o, m, out + at, nullptr);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  });
 }
 
 int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64_t nq, uint64_t* out,
@@ -216,11 +222,14 @@ int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64
   if ((rc = need(t, WTG_RANK, "rank"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  wt_rank_kernel<<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                           t.node_tab.as<ulonglong2>(), t.n, t.levels, idx, sym, nq, out);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  return WTG_OK;
+  return in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    auto* const f = sorted ? wt_rank_kernel<true> : wt_rank_kernel<false>;
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n,
+                               t.levels, idx + at, o, sym + at, m, out + at);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  });
 }
 
 int launch_wt_inverse_select(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* rank_out,
@@ -229,12 +238,14 @@ int launch_wt_inverse_select(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint
   if ((rc = need(t, WTG_RANK, "inverse_select"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  wt_descend_kernel<true><<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                   t.node_tab.as<ulonglong2>(), t.n, t.levels, idx, nq, rank_out,
-                                                   sym_out);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  return WTG_OK;
+  return in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    auto* const f = sorted ? wt_descend_kernel<true, true> : wt_descend_kernel<true, false>;
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n,
+                               t.levels, idx + at, o, m, rank_out + at, sym_out + at);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  });
 }
 
 int launch_wt_select(const TreeImpl& t, const uint64_t* i, const uint64_t* sym, uint64_t nq, uint64_t* out,

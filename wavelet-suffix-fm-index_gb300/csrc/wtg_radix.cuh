@@ -93,11 +93,11 @@ struct RadixStatus {
   static constexpr S AGG = S(1) << SHIFT, INC = S(2) << SHIFT, MASK = AGG - 1;
 };
 
-// byte `b` of a key
-__device__ __forceinline__ uint32_t key_byte(uint64_t k, int b) {
-  return __byte_perm((uint32_t)k, (uint32_t)(k >> 32), 0x4440 + b) & 255u;
+// the 8-bit digit of a key at bit `shift` (a multiple of 8 for 8-byte keys)
+__device__ __forceinline__ uint32_t key_digit(uint64_t k, int shift) {
+  return __byte_perm((uint32_t)k, (uint32_t)(k >> 32), 0x4440 + (shift >> 3)) & 255u;
 }
-__device__ __forceinline__ uint32_t key_byte(uint32_t k, int b) { return (k >> (8 * b)) & 255u; }
+__device__ __forceinline__ uint32_t key_digit(uint32_t k, int shift) { return (k >> shift) & 255u; }
 
 // lanes of the warp with the same 8-bit digit (all 32 take part)
 __device__ __forceinline__ uint32_t same_digit(uint32_t d) {
@@ -111,11 +111,10 @@ __device__ __forceinline__ uint32_t same_digit(uint32_t d) {
   return m;
 }
 
-// One pass over key byte `byte`.  IOTA: the values are the indices (val is
-// not read).
+// One pass.  IOTA: the values are the indices (val is not read).
 template <typename K, typename S, bool IOTA>
 __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
-    radix_pass_kernel(const K* __restrict__ key, const uint32_t* __restrict__ val, uint64_t n, int byte,
+    radix_pass_kernel(const K* __restrict__ key, const uint32_t* __restrict__ val, uint64_t n, int shift,
                       const uint32_t* __restrict__ bases, S* status, uint32_t* counter, K* __restrict__ key_out,
                       uint32_t* __restrict__ val_out, uint32_t* err) {
   using RS = RadixStatus<S>;
@@ -140,7 +139,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
   for (int j = 0; j < RS_IPT; ++j) k[j] = off + 32 * j < tn ? kp[32 * j] : ~K(0);  // past the end: digit 255
 #pragma unroll
   for (int j = 0; j < RS_IPT; ++j) {
-    const uint32_t d = key_byte(k[j], byte);
+    const uint32_t d = key_digit(k[j], shift);
     const uint32_t m = same_digit(d);
     const uint32_t old = wc[w][d];
     rk[j] = old + __popc(m & lt);
@@ -218,7 +217,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
   // into digit order, keys first, then the values through the same room
 #pragma unroll
   for (int j = 0; j < RS_IPT; ++j) {
-    rk[j] += wc[w][key_byte(k[j], byte)];
+    rk[j] += wc[w][key_digit(k[j], shift)];
     s_key[rk[j]] = k[j];
   }
   __syncthreads();
@@ -227,7 +226,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
   for (int j = 0; j < RS_IPT; ++j) {
     const uint32_t i = tid + j * RS_THREADS;
     const K x = s_key[i];
-    g[j] = i + gdelta[key_byte(x, byte)];
+    g[j] = i + gdelta[key_digit(x, shift)];
     if (i >= tn) g[j] = 0xffffffffu;
     if (g[j] < n) key_out[g[j]] = x;  // (always, but for places past the end and a failed look-back)
   }
@@ -243,7 +242,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
     if (g[j] < n) val_out[g[j]] = s_val[tid + j * RS_THREADS];
 }
 
-// Sorts n pairs by key bits [lo, lo + 8 passes), lo a multiple of 8; the pairs are in key[cur] /
+// Sorts n pairs by key bits [lo, lo + 8 passes), lo a multiple of 8 for 8-byte keys; the pairs are in key[cur] /
 // val[cur] and end there (cur flips once per pass).  iota: the values of the
 // first pass are the indices.  hist: passes * 256 words, status: its bytes
 // from radix_status_bytes; both are scratch.  Asynchronous.
@@ -262,10 +261,10 @@ int radix_passes(K* const key[2], uint32_t* const val[2], uint64_t n, int lo, in
     uint32_t* counter = reinterpret_cast<uint32_t*>(st);
     S* words = reinterpret_cast<S*>(st + 16);
     if (iota && p == 0)
-      radix_pass_kernel<K, S, true><<<tiles, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo / 8, hist, words, counter,
+      radix_pass_kernel<K, S, true><<<tiles, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo, hist, words, counter,
                                                                  key[cur ^ 1], val[cur ^ 1], d_err);
     else
-      radix_pass_kernel<K, S, false><<<tiles, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo / 8 + p,
+      radix_pass_kernel<K, S, false><<<tiles, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo + 8 * p,
                                                                   hist + p * RS_RADIX, words, counter, key[cur ^ 1],
                                                                   val[cur ^ 1], d_err);
     count_launch();

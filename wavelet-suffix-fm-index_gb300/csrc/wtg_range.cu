@@ -8,6 +8,7 @@
 // per query bound.
 #include <algorithm>
 
+#include "wtg_order.cuh"
 #include "wtg_select.cuh"
 #include "wtg_tree.cuh"
 
@@ -19,55 +20,91 @@ constexpr int RQ_STACK = 32;  // DFS stack entries per query (at most L + 1 <= 2
 
 __device__ __forceinline__ int level_of(uint64_t h) { return 63 - __clzll((long long)(h + 1)); }
 
-// lex_count (wt_int_par.hpp:715-745) and, with SMALLER_ONLY,
-// lex_smaller_count (:758-782): descend along c's path carrying the
-// position bounds; symbols below / above c are counted where the path turns.
-template <bool SMALLER_ONLY>
+// lex_count (wt_int_par.hpp:715-745): descend along c's path carrying both
+// bounds (positions inside the level; the node's step constants take them to
+// its child, see node_table_kernel); symbols below / above c are counted
+// where the path turns.
+template <bool ORD>
 __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                              const ulonglong2* __restrict__ tab, uint64_t n, int L, const uint64_t* __restrict__ qi,
-                              const uint64_t* __restrict__ qj, const uint64_t* __restrict__ qc, uint64_t nq,
-                              uint64_t* __restrict__ out_rank, uint64_t* __restrict__ out_smaller,
-                              uint64_t* __restrict__ out_greater) {
-  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+                              const uint2* __restrict__ step, uint64_t n, int L, QueryOrder ord,
+                              const uint64_t* __restrict__ qi, const uint64_t* __restrict__ qj,
+                              const uint64_t* __restrict__ qc, uint64_t nq, uint64_t* __restrict__ out_rank,
+                              uint64_t* __restrict__ out_smaller, uint64_t* __restrict__ out_greater) {
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  uint64_t i = qi[k], j = SMALLER_ONLY ? 0 : qj[k];
-  const uint64_t c = qc[k];
-  const bool ok = SMALLER_ONLY ? i <= n : (i <= j && j <= n);
-  if (!ok) {
+  if (ORD) k = ord.id[k];
+  const uint64_t i = qi[k], j = qj[k], c = qc[k];
+  if (i > j || j > n) {
     out_rank[k] = NONE64;
     out_smaller[k] = NONE64;
-    if (!SMALLER_ONLY) out_greater[k] = NONE64;
+    out_greater[k] = NONE64;
     return;
   }
   if ((1ull << L) <= c) {  // c above every symbol of the tree
     out_rank[k] = 0;
-    out_smaller[k] = SMALLER_ONLY ? i : j - i;
-    if (!SMALLER_ONLY) out_greater[k] = 0;
+    out_smaller[k] = j - i;
+    out_greater[k] = 0;
     return;
   }
-  uint64_t smaller = 0, greater = 0, h = 0;
+  const uint32_t path = (uint32_t)c | (1u << L);
+  uint32_t x = (uint32_t)i, y = (uint32_t)j, smaller = 0, greater = 0;  // counts below 2^32
+  uint64_t lbase = 0;
+  for (int lv = 0; lv < L; ++lv, lbase += n) {
+    const uint2 st = __ldg(step + ((path >> (L - lv)) - 1));
+    const uint32_t rx = (uint32_t)rank1_dev(rt, tree, lbase + x);
+    const uint32_t ry = (uint32_t)rank1_dev(rt, tree, lbase + y);
+    if ((path >> (L - 1 - lv)) & 1u) {
+      smaller += (y - x) - (ry - rx);
+      x = st.y + rx;
+      y = st.y + ry;
+    } else {
+      greater += ry - rx;
+      x = st.x + x - rx;
+      y = st.x + y - ry;
+    }
+  }
+  out_rank[k] = x;
+  out_smaller[k] = smaller;
+  out_greater[k] = greater;
+}
+
+// lex_smaller_count (wt_int_par.hpp:758-782): the same with one bound
+__global__ void wt_lex_smaller_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                      const ulonglong2* __restrict__ tab, uint64_t n, int L,
+                                      const uint64_t* __restrict__ qi, const uint64_t* __restrict__ qc, uint64_t nq,
+                                      uint64_t* __restrict__ out_rank, uint64_t* __restrict__ out_smaller) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nq) return;
+  uint64_t i = qi[k];
+  const uint64_t c = qc[k];
+  if (i > n) {
+    out_rank[k] = NONE64;
+    out_smaller[k] = NONE64;
+    return;
+  }
+  if ((1ull << L) <= c) {  // c above every symbol of the tree
+    out_rank[k] = 0;
+    out_smaller[k] = i;
+    return;
+  }
+  uint64_t smaller = 0, h = 0;
   ulonglong2 nd = __ldg(tab);
-  for (int lv = 0; lv < L && (!SMALLER_ONLY || i); ++lv) {
+  for (int lv = 0; lv < L && i; ++lv) {
     const uint64_t bit = (c >> (L - 1 - lv)) & 1;
     const uint64_t child = 2 * h + 1 + bit;
     const ulonglong2 next = lv + 1 < L ? __ldg(tab + child) : nd;
     const uint64_t oi = rank1_dev(rt, tree, nd.x + i) - nd.y;
-    const uint64_t oj = SMALLER_ONLY ? 0 : rank1_dev(rt, tree, nd.x + j) - nd.y;
     if (bit) {
-      smaller += SMALLER_ONLY ? i - oi : (j - i) - (oj - oi);
+      smaller += i - oi;
       i = oi;
-      j = oj;
     } else {
-      if (!SMALLER_ONLY) greater += oj - oi;
       i -= oi;
-      j -= oj;
     }
     h = child;
     nd = next;
   }
   out_rank[k] = i;
   out_smaller[k] = smaller;
-  if (!SMALLER_ONLY) out_greater[k] = greater;
 }
 
 // Value bounds of range_search_2d (wt_int_par.hpp:805-809): vrb is clamped
@@ -91,13 +128,15 @@ struct RqEntry {
 // range lies inside [vlb, vrb] adds its whole range at once (the reference
 // descends to its leaves, which hold the same positions), so at most two
 // partially covered nodes per level are expanded.
+template <bool ORD>
 __global__ void wt_range_count_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                                      const ulonglong2* __restrict__ tab, uint64_t n, int L,
+                                      const ulonglong2* __restrict__ tab, uint64_t n, int L, QueryOrder ord,
                                       const uint64_t* __restrict__ qlb, const uint64_t* __restrict__ qrb,
                                       const uint64_t* __restrict__ qvlb, const uint64_t* __restrict__ qvrb,
                                       uint64_t nq, uint64_t* __restrict__ out) {
-  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
+  if (ORD) k = ord.id[k];
   const uint64_t lb0 = qlb[k], rb0 = qrb[k];
   uint64_t vlb = qvlb[k], vrb = qvrb[k];
   if (lb0 <= rb0 && rb0 >= n) {
@@ -336,12 +375,14 @@ int launch_wt_lex_count(TreeImpl& t, const uint64_t* i, const uint64_t* j, const
   if ((rc = need_rank(t, "lex_count"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  wt_lex_kernel<false><<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                t.node_tab.as<ulonglong2>(), t.n, t.levels, i, j, c, nq, rank_out,
-                                                smaller_out, greater_out);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  return WTG_OK;
+  return in_order(t, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    auto* const f = sorted ? wt_lex_kernel<true> : wt_lex_kernel<false>;
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n, t.levels,
+                               o, i + at, j + at, c + at, m, rank_out + at, smaller_out + at, greater_out + at);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  });
 }
 
 int launch_wt_lex_smaller_count(TreeImpl& t, const uint64_t* i, const uint64_t* c, uint64_t nq, uint64_t* rank_out,
@@ -350,9 +391,9 @@ int launch_wt_lex_smaller_count(TreeImpl& t, const uint64_t* i, const uint64_t* 
   if ((rc = need_rank(t, "lex_smaller_count"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  wt_lex_kernel<true><<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                               t.node_tab.as<ulonglong2>(), t.n, t.levels, i, nullptr, c, nq,
-                                               rank_out, smaller_out, nullptr);
+  wt_lex_smaller_kernel<<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
+                                                  t.node_tab.as<ulonglong2>(), t.n, t.levels, i, c, nq, rank_out,
+                                                  smaller_out);
   count_launch();
   WTG_CK(cudaGetLastError());
   return WTG_OK;
@@ -364,12 +405,14 @@ int launch_wt_range_count(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, c
   if ((rc = need_rank(t, "range_search_2d"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  wt_range_count_kernel<<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                  t.node_tab.as<ulonglong2>(), t.n, t.levels, lb, rb, vlb, vrb, nq,
-                                                  count_out);
-  count_launch();
-  WTG_CK(cudaGetLastError());
-  return WTG_OK;
+  return in_order(t, lb, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    auto* const f = sorted ? wt_range_count_kernel<true> : wt_range_count_kernel<false>;
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_tab.as<ulonglong2>(), t.n,
+                               t.levels, o, lb + at, rb + at, vlb + at, vrb + at, m, count_out + at);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  });
 }
 
 int launch_wt_range_report(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, const uint64_t* vlb,

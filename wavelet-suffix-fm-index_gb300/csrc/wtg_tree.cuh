@@ -33,7 +33,8 @@ struct TreeImpl {
   DevBuf lvl_args;
   bool lvl_args_ok = false;
   DevBuf fm_paths;  // per-symbol node paths for FM-index counting
-  DevBuf node_tab;  // per heap node: bit offset of its start, ones before it
+  DevBuf node_tab;   // per heap node: bit offset of its start, ones before it
+  DevBuf node_step;  // per heap node: the constants that take a position to its child
   bool node_tab_ok = false;
   uint64_t gen = 0;  // builds so far (indexes built on the tree record it)
   // host destinations filled while the build runs (wtg_tree_build_out): the
