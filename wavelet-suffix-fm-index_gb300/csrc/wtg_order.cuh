@@ -23,6 +23,15 @@ struct QueryOrder {
 constexpr uint64_t ORDER_BATCH = 1ull << 26;
 
 static __global__ void __launch_bounds__(256)
+    pattern_keys_kernel(const uint64_t* __restrict__ off, uint64_t npat, uint32_t* __restrict__ len) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < npat; k += stride) {
+    const uint64_t m = off[k + 1] - off[k];
+    len[k] = (uint32_t)(m < 255 ? m : 255);
+  }
+}
+
+static __global__ void __launch_bounds__(256)
     order_keys_kernel(const uint64_t* __restrict__ q, uint64_t nq, uint64_t n, uint32_t* __restrict__ pos) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nq; k += stride) {
@@ -46,17 +55,15 @@ inline bool order_pays(const TreeImpl& t, uint64_t nq) {
   return bytes >= (20ull << 20) && t.levels >= 16 && nq >= (1ull << 21);
 }
 
-// Calls launch(sorted, order, first query, queries) over the batch: in sorted
-// batches where that pays and the scratch is to be had, otherwise once over
-// all queries as they come.
-template <typename F>
-int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch) {
-  if (!order_pays(t, nq)) return launch(false, QueryOrder{}, 0, nq);
+// Sorts the queries of each batch of at most ORDER_BATCH by 8 * passes bits,
+// from bit lo on, of the 32-bit keys that make_keys(first, queries, keys)
+// writes, and calls launch(true, order, first, queries) for it; without room
+// for the scratch launch(false, {}, 0, nq).
+template <typename K, typename F>
+int sorted_batches(uint64_t nq, int lo, int passes, uint32_t* d_err, cudaStream_t s, K make_keys, F launch) {
   const uint64_t most = nq < ORDER_BATCH ? nq : ORDER_BATCH;
   const uint64_t pairs = (most + 63) / 64 * 64;
-  constexpr int passes = 2;
-  const uint64_t status = radix_status_bytes(most, passes);
-  const uint64_t bytes = 16 * pairs + passes * RS_RADIX * 4 + status + 16;
+  const uint64_t bytes = 16 * pairs + passes * RS_RADIX * 4 + radix_status_bytes(most, passes);
   uint8_t* scratch = nullptr;
   if (cudaMallocAsync(&scratch, bytes, s) != cudaSuccess) {
     cudaGetLastError();  // no room: the queries as they come
@@ -66,23 +73,50 @@ int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F la
   uint32_t* const val[2] = {(uint32_t*)scratch + 2 * pairs, (uint32_t*)scratch + 3 * pairs};
   uint32_t* hist = (uint32_t*)scratch + 4 * pairs;
   uint8_t* st = (uint8_t*)(hist + passes * RS_RADIX);
-  const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
-  const int lo = bits > 8 * passes ? bits - 8 * passes : 0;
   int rc = WTG_OK;
   for (uint64_t at = 0; at < nq && rc == WTG_OK; at += most) {
     const uint64_t m = nq - at < most ? nq - at : most;
-    order_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(pos + at, m, t.n, key[0]);
+    make_keys(at, m, key[0]);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) {
       rc = fail(WTG_ERR_CUDA, "query order: launch failed");
       break;
     }
     int cur = 0;
-    rc = radix_sort_pairs<uint32_t>(key, val, m, lo, passes, true, hist, st, t.err.as<uint32_t>(), cur, s);
+    rc = radix_sort_pairs<uint32_t>(key, val, m, lo, passes, true, hist, st, d_err, cur, s);
     if (rc == WTG_OK) rc = launch(true, QueryOrder{key[cur], val[cur]}, at, m);
   }
   cudaFreeAsync(scratch, s);
   return rc;
+}
+
+// Calls launch(sorted, order, first query, queries) over the batch: sorted by
+// position where that pays, otherwise once over all queries as they come.
+template <typename F>
+int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch) {
+  if (!order_pays(t, nq)) return launch(false, QueryOrder{}, 0, nq);
+  constexpr int passes = 2;
+  const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
+  return sorted_batches(
+      nq, bits > 8 * passes ? bits - 8 * passes : 0, passes, t.err.as<uint32_t>(), s,
+      [&](uint64_t at, uint64_t m, uint32_t* key) {
+        order_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(pos + at, m, t.n, key);
+      },
+      launch);
+}
+
+// Patterns by length (one sort pass), from 2^16 of them on: a warp runs as
+// long as its longest pattern, and lengths of 8 to 32 left 48 % of the lanes
+// without work.
+template <typename F>
+int by_length(const uint64_t* off, uint64_t npat, uint32_t* d_err, cudaStream_t s, F launch) {
+  if (npat < (1ull << 16)) return launch(false, QueryOrder{}, 0, npat);
+  return sorted_batches(
+      npat, 0, 1, d_err, s,
+      [&](uint64_t at, uint64_t m, uint32_t* key) {
+        pattern_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(off + at, m, key);
+      },
+      launch);
 }
 
 }  // namespace wtg
