@@ -23,6 +23,9 @@
 #include "wtg_tree.cuh"
 
 namespace wtg {
+
+WTG_WAIT_LIMIT_SETTER(fm)
+
 namespace {
 
 constexpr int FM_SMEM_STEPS = 2048;  // steps kept in shared memory (8 bytes each)

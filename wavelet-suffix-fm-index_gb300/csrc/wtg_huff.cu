@@ -35,10 +35,15 @@
 #include <queue>
 #include <vector>
 
+#include "wtg_blocks.cuh"
+#include "wtg_fm_table.cuh"
+#include "wtg_order.cuh"
 #include "wtg_select.cuh"
 #include "wtg_tree.cuh"
 
 namespace wtg {
+
+WTG_WAIT_LIMIT_SETTER(huff)
 
 constexpr int HUFF_MAX_NODES = 511;
 constexpr uint16_t HUFF_NONE = 0xFFFF;
@@ -65,7 +70,8 @@ struct HuffImpl {
   uint64_t path[256] = {0};
   int len[256] = {0};
   int leaf[256];
-  DevBuf text, seq[2], bits, chunkz, chunkpre, scan_tmp, err, hist, dnodes, dpath, dnode_at, nbase, ids, qbuf;
+  DevBuf text, seq[2], bits, chunkz, chunkpre, scan_tmp, err, hist, dnodes, dpath, dnode_at, nbase, ids, qbuf, fminfo, fmsteps;
+  uint32_t fm_steps = 0;  // steps of all codes (fm counting)
   BvSupport bv;
   HuffImpl() { std::fill(leaf, leaf + 256, -1); }
 };
@@ -315,6 +321,138 @@ __global__ void huff_fm_count_kernel(HuffView v, const uint64_t* __restrict__ C,
   out[q] = ep > sp ? ep - sp : 0;
 }
 
+// The same for texts below 2^32 bytes, as fm_count_kernel does it over the
+// balanced tree: step constants per symbol and depth, 192-bit blocks for large
+// batches, an interval table of short strings, patterns by length.
+constexpr int HF_SMEM_STEPS = 3072;  // steps kept in shared memory (8 bytes each)
+constexpr int HF_MAX_DEPTH = 64;     // a code of a text below 2^40 bytes is shorter
+
+// per byte: first step, code length, number among the text's bytes (0xFFFF: absent)
+struct HuffSymbol {
+  uint32_t first;
+  uint16_t len, dense;
+};
+
+struct HuffFmInfo {
+  HuffSymbol sym[256];
+  uint64_t path[256];   // code bits, the root's first
+  uint8_t byte_of[256]; // dense number -> byte
+  uint64_t depth[HF_MAX_DEPTH];  // first bit of each depth's run
+};
+
+// steps[first + d]: x = position of the node's bits in its depth's run, y =
+// ones before them (mod 2^32).  With r the ones before (depth + x + i), bit 1
+// goes on at i' = r - y, bit 0 at i' = i - (r - y).
+__global__ void huff_steps_kernel(const HuffNodeDev* __restrict__ nodes, const HuffFmInfo* __restrict__ info,
+                                  uint2* __restrict__ steps) {
+  const uint32_t c = threadIdx.x;
+  const HuffSymbol s = info->sym[c];
+  if (s.dense == 0xFFFF) return;
+  uint16_t u = 0;
+  for (uint32_t d = 0; d < s.len; ++d) {
+    steps[s.first + d] = make_uint2((uint32_t)(nodes[u].bv_pos - info->depth[d]), (uint32_t)nodes[u].rank);
+    u = (info->path[c] >> d) & 1 ? nodes[u].child1 : nodes[u].child0;
+  }
+}
+
+template <bool BLOCKS>
+struct HuffFm {
+  const uint64_t* bits;
+  const uint64_t* rt;
+  const uint4* blocks;
+  const HuffFmInfo* info;
+  const uint2* steps;
+  const uint64_t* C;
+  uint32_t n, sigma;
+  __device__ __forceinline__ void ranks(uint64_t px, uint64_t py, uint32_t& rx, uint32_t& ry) const {
+    if constexpr (BLOCKS) {
+      uint32_t ox, oy;
+      const uint64_t bx = block_of(px, ox), by = block_of(py, oy);
+      uint64_t v[4];
+      block_load(blocks, bx, v);
+      rx = block_at(v, ox).ones;
+      if (bx != by) block_load(blocks, by, v);
+      ry = block_at(v, oy).ones;
+    } else {
+      rx = (uint32_t)rank1_dev(rt, bits, px);
+      ry = (uint32_t)rank1_dev(rt, bits, py);
+    }
+  }
+  // prepends a symbol of the text to the interval [x, y)
+  __device__ __forceinline__ void step(const uint2* __restrict__ st, HuffSymbol s, uint64_t path, uint32_t base,
+                                       uint32_t& x, uint32_t& y) const {
+    for (uint32_t d = 0; d < s.len; ++d, path >>= 1) {
+      const uint2 c = st[s.first + d];
+      const uint64_t at = info->depth[d] + c.x;
+      uint32_t rx, ry;
+      ranks(at + x, at + y, rx, ry);
+      rx -= c.y;
+      ry -= c.y;
+      const bool one = path & 1;
+      x = one ? rx : x - rx;
+      y = one ? ry : y - ry;
+    }
+    x += base;
+    y += base;
+  }
+};
+
+template <bool BLOCKS>
+__global__ void huff_table_kernel(HuffFm<BLOCKS> t, uint64_t prev_count, const uint2* __restrict__ prev,
+                                  uint2* __restrict__ out) {
+  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= prev_count * t.sigma) return;
+  const uint32_t k = (uint32_t)(i / prev_count), c = t.info->byte_of[k];
+  const uint2 v = prev ? prev[i - k * prev_count] : make_uint2(0u, t.n);
+  uint32_t x = v.x, y = v.y;
+  if (x < y) t.step(t.steps, t.info->sym[c], t.info->path[c], (uint32_t)t.C[c], x, y);
+  out[i] = x < y ? make_uint2(x, y) : make_uint2(0u, 0u);
+}
+
+template <bool BLOCKS, bool ORD>
+__global__ void __launch_bounds__(256, 5)
+    huff_count_kernel(HuffFm<BLOCKS> t, uint32_t nsteps, int K, const uint2* __restrict__ table,
+                      const uint8_t* __restrict__ pat, const uint64_t* __restrict__ off,
+                      const uint64_t* __restrict__ total, QueryOrder ord, uint64_t m, uint64_t* __restrict__ out) {
+  extern __shared__ uint2 s_steps[];  // nsteps, or none
+  __shared__ HuffSymbol s_sym[256];
+  __shared__ uint32_t s_C[256];
+  for (uint32_t i = threadIdx.x; i < nsteps; i += blockDim.x) s_steps[i] = t.steps[i];
+  s_sym[threadIdx.x] = t.info->sym[threadIdx.x];
+  s_C[threadIdx.x] = (uint32_t)t.C[threadIdx.x];
+  __syncthreads();
+  const uint2* const st = nsteps ? s_steps : t.steps;
+  uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= m) return;
+  if (ORD) p = ord.id[p];
+  const uint64_t a = off[p], b = off[p + 1];
+  PatternReader rd(pat, *total);
+  uint32_t x = 0, y = t.n;
+  uint64_t i = b;
+  bool known = true;  // every symbol read so far is one of the text's
+  if (K && b - a >= (uint64_t)K) {
+    uint32_t at = 0, scale = 1;
+    for (int k = 0; k < K; ++k) {
+      const uint32_t d = s_sym[rd.at(--i)].dense;
+      known = known && d != 0xFFFF;
+      at += d * scale;
+      scale *= t.sigma;
+    }
+    if (known) {
+      const uint2 v = __ldg(table + at);
+      x = v.x;
+      y = v.y;
+    }
+  }
+  while (known && i > a && x < y) {
+    const uint32_t c = rd.at(--i);
+    const HuffSymbol s = s_sym[c];
+    known = s.dense != 0xFFFF;
+    if (known) t.step(st, s, __ldg(t.info->path + c), s_C[c], x, y);
+  }
+  out[p] = known && y > x ? y - x : 0;
+}
+
 unsigned hgrid(uint64_t items, unsigned per, unsigned cap) {
   return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((items + per - 1) / per, cap));
 }
@@ -327,7 +465,7 @@ void huff_delete(HuffImpl* h) {
   if (!h) return;
   cudaStream_t s = h->stream;
   DevBuf* bufs[] = {&h->text, &h->seq[0], &h->seq[1], &h->bits, &h->chunkz, &h->chunkpre, &h->scan_tmp, &h->err,
-                    &h->hist, &h->dnodes, &h->dpath, &h->dnode_at, &h->nbase, &h->ids, &h->qbuf};
+                    &h->hist, &h->dnodes, &h->dpath, &h->dnode_at, &h->nbase, &h->ids, &h->qbuf, &h->fminfo, &h->fmsteps};
   for (DevBuf* d : bufs) d->release(s);
   bv_release(h->bv, s);
   cudaStreamSynchronize(s);
@@ -480,6 +618,24 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
     }
   std::vector<uint16_t> ids;
   for (int d = 0; d <= depths; ++d) ids.insert(ids.end(), inner[d].begin(), inner[d].end());
+  {
+    static_assert(HF_MAX_DEPTH >= 64, "");
+    HuffFmInfo fi;
+    uint32_t first = 0, dense = 0;
+    for (int c = 0; c < 256; ++c) {
+      fi.sym[c] = {first, (uint16_t)h.len[c], 0xFFFF};
+      fi.path[c] = h.path[c];
+      fi.byte_of[c] = 0;
+      if (h.leaf[c] < 0) continue;
+      fi.byte_of[dense] = (uint8_t)c;
+      fi.sym[c].dense = (uint16_t)dense++;
+      first += (uint32_t)h.len[c];
+    }
+    for (int d = 0; d < HF_MAX_DEPTH; ++d) fi.depth[d] = d <= depths ? D[d] : h.size;
+    h.fm_steps = first;
+    if ((rc = h.fminfo.ensure(sizeof(HuffFmInfo), s))) return rc;
+    WTG_CK(cudaMemcpyAsync(h.fminfo.p, &fi, sizeof(fi), cudaMemcpyHostToDevice, s));
+  }
   DevBuf& dids = h.ids;
   if ((rc = dids.ensure(std::max<size_t>(ids.size(), 1) * sizeof(uint16_t), s))) return rc;
   if (!ids.empty())
@@ -604,14 +760,57 @@ int launch_huff_query(HuffImpl& h, int what, const uint64_t* a, const uint64_t* 
   return WTG_OK;
 }
 
+template <bool BLOCKS>
+static int huff_fm_run(HuffImpl& h, const uint4* blocks, const uint64_t* C, const uint8_t* pat, const uint64_t* off,
+                       uint64_t npat, uint64_t* out, cudaStream_t s) {
+  const HuffFm<BLOCKS> v{h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), blocks, h.fminfo.as<HuffFmInfo>(),
+                         h.fmsteps.as<uint2>(), C, (uint32_t)h.n, (uint32_t)h.sigma};
+  const uint32_t in_smem = h.fm_steps <= (uint32_t)HF_SMEM_STEPS ? h.fm_steps : 0u;
+  return with_fm_table<uint2>(
+      h.sigma, npat, s,
+      [&](uint64_t prev_count, const uint2* prev, uint2* next) -> int {
+        huff_table_kernel<BLOCKS><<<(unsigned)((prev_count * h.sigma + 127) / 128), 128, 0, s>>>(v, prev_count, prev,
+                                                                                                next);
+        count_launch();
+        WTG_CK(cudaGetLastError());
+        return WTG_OK;
+      },
+      [&](int K, const uint2* table) -> int {
+        return by_length(off, npat, h.err.as<uint32_t>(), s,
+                         [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+                           auto* const f = sorted ? huff_count_kernel<BLOCKS, true> : huff_count_kernel<BLOCKS, false>;
+                           f<<<(unsigned)((m + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(
+                               v, in_smem, K, table, pat, off + at, off + npat, o, m, out + at);
+                           count_launch();
+                           WTG_CK(cudaGetLastError());
+                           return WTG_OK;
+                         });
+      });
+}
+
 int launch_huff_fm_count(HuffImpl& h, const uint64_t* C, const uint8_t* pat, const uint64_t* off, uint64_t npat,
                          uint64_t* out, cudaStream_t s) {
   if (!npat) return WTG_OK;
   if (!(h.flags & WTG_RANK)) return fail(WTG_ERR_INVALID, "counting needs the rank support");
-  huff_fm_count_kernel<<<(unsigned)((npat + 255) / 256), 256, 0, s>>>(huff_view(h), C, pat, off, npat, out);
+  if (h.n >= (1ull << 32) || !h.n) {  // positions beyond 32 bits (and the empty text)
+    huff_fm_count_kernel<<<(unsigned)((npat + 255) / 256), 256, 0, s>>>(huff_view(h), C, pat, off, npat, out);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  }
+  int rc;
+  if ((rc = h.fmsteps.ensure(std::max<uint32_t>(h.fm_steps, 1) * sizeof(uint2), s))) return rc;
+  huff_steps_kernel<<<1, 256, 0, s>>>(h.dnodes.as<HuffNodeDev>(), h.fminfo.as<HuffFmInfo>(), h.fmsteps.as<uint2>());
   count_launch();
   WTG_CK(cudaGetLastError());
-  return WTG_OK;
+  // as for the balanced tree: blocks once the batch probes a good part of them
+  uint4* blocks = h.size && npat >= block_count(h.size) / 8
+                      ? make_blocks(h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), h.size, s)
+                      : nullptr;
+  rc = blocks ? huff_fm_run<true>(h, blocks, C, pat, off, npat, out, s)
+              : huff_fm_run<false>(h, blocks, C, pat, off, npat, out, s);
+  if (blocks) cudaFreeAsync(blocks, s);
+  return rc;
 }
 
 }  // namespace wtg

@@ -196,6 +196,9 @@ int set_wait_limits_bitvec(const uint32_t lim[2]);
 int set_wait_limits_core(const uint32_t lim[2]);
 int set_wait_limits_sa(const uint32_t lim[2]);
 int set_wait_limits_query(const uint32_t lim[2]);
+int set_wait_limits_huff(const uint32_t lim[2]);
+int set_wait_limits_fm(const uint32_t lim[2]);
+int set_wait_limits_range(const uint32_t lim[2]);
 
 // Host-side failure injection for the tests (no device fault is ever made):
 // test_take_alloc_failure() is true for the one device allocation the armed

@@ -14,6 +14,8 @@
 
 namespace wtg {
 
+WTG_WAIT_LIMIT_SETTER(range)
+
 namespace {
 
 constexpr int RQ_STACK = 32;  // DFS stack entries per query (at most L + 1 <= 25 live)
