@@ -143,14 +143,6 @@ int tree_levels_from_max(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int
   return WTG_OK;
 }
 
-
-// chunks per warp of a count tile: more per tile (fewer look-backs) once the
-// tiles still fill the chip eight times
-static int count_cpw(uint64_t nchunks) {
-  const uint64_t c = nchunks / ((uint64_t)LV_WARPS * sm_count() * 8);
-  return c >= 8 ? 8 : c >= 4 ? 4 : c >= 2 ? 2 : 1;
-}
-
 int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32_t flags) {
   cudaStream_t s = t.stream;
   int rc;

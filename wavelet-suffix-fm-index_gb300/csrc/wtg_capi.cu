@@ -1200,6 +1200,7 @@ int wtg_set_wait_limits(uint32_t lookback_spins, uint32_t mbarrier_tries) {
   if ((rc = set_wait_limits_sa(lim))) return rc;
   if ((rc = set_wait_limits_query(lim))) return rc;
   if ((rc = set_wait_limits_huff(lim))) return rc;
+  if ((rc = set_wait_limits_huff_pass(lim))) return rc;
   if ((rc = set_wait_limits_fm(lim))) return rc;
   if ((rc = set_wait_limits_range(lim))) return rc;
   return set_wait_limits_core(lim);

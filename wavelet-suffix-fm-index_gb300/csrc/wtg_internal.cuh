@@ -197,6 +197,7 @@ int set_wait_limits_core(const uint32_t lim[2]);
 int set_wait_limits_sa(const uint32_t lim[2]);
 int set_wait_limits_query(const uint32_t lim[2]);
 int set_wait_limits_huff(const uint32_t lim[2]);
+int set_wait_limits_huff_pass(const uint32_t lim[2]);
 int set_wait_limits_fm(const uint32_t lim[2]);
 int set_wait_limits_range(const uint32_t lim[2]);
 

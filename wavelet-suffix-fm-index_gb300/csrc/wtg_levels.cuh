@@ -51,6 +51,7 @@ constexpr int CHUNK = 1024;  // symbols per warp chunk: 32 rows of 32
 constexpr int LOG_CHUNK = 10;
 constexpr int LV_THREADS = 256;
 constexpr int LV_WARPS = LV_THREADS / 32;
+constexpr uint32_t HUFF_OUT = 0xFFFF0000u;  // a Huffman-shaped tree's group passes take up to this many symbols
 constexpr int REC = 32;  // words of a node record: bit bases (j, q) at 2^j - 1 + q, scatter bases at 16 + d
 
 // ------------------------------------------------------------------- rows
@@ -85,6 +86,31 @@ __device__ __forceinline__ void load_row(const T* __restrict__ src, uint64_t i0,
       w[k] = x;
     }
   }
+}
+
+// A Huffman-shaped tree's symbols stay bytes; a row of them is taken through
+// the group's digit table (shared memory) to 16-bit words, the next four code
+// bits above the byte (ds = 8), so that a pass sorts by the digit and stores
+// the byte.  3.5 instructions per 32 symbols.
+template <typename T, bool HUFF>
+__device__ __forceinline__ void load_symbols(const void* __restrict__ src, const uint16_t* s_lut, uint64_t i0,
+                                             uint64_t n, uint32_t (&w)[8 * sizeof(T)]) {
+  if constexpr (HUFF) {
+    uint32_t b[8];
+    load_row<uint8_t>(static_cast<const uint8_t*>(src), i0, n, b);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      w[2 * k] = __byte_perm(s_lut[b[k] & 0xFFu], s_lut[(b[k] >> 8) & 0xFFu], 0x5410);
+      w[2 * k + 1] = __byte_perm(s_lut[(b[k] >> 16) & 0xFFu], s_lut[b[k] >> 24], 0x5410);
+    }
+  } else {
+    load_row<T>(static_cast<const T*>(src), i0, n, w);
+  }
+}
+
+__device__ __forceinline__ void load_lut(const uint16_t* __restrict__ lut, uint16_t* s_lut) {
+  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_lut[i] = lut[i];
+  __syncthreads();
 }
 
 // bit planes of the rows' TB-bit digits at bit ds: B[0] the digit's top bit.
@@ -177,22 +203,40 @@ __device__ __forceinline__ uint32_t find_node(const uint32_t* __restrict__ C, ui
 
 // ------------------------------------------------------------------ count
 
+// A group of levels of a Huffman-shaped tree, whose node sizes are known from
+// the byte counts before the build: the records and starts of its first
+// level's inner nodes come from the host.  Codes that end inside the group are
+// padded with zeros; the strings and children that are not inner nodes are
+// left out (word 15 of a record: bit 2^j - 1 + q for string (j, q), bit 16 + d
+// for child d).
+struct HuffGroup {
+  const uint16_t* lut;     // per byte: the group's digit << 8 | byte
+  const uint64_t* lv;      // first bit of the group's levels (4), symbols in them (4), symbols of the next group
+  const uint32_t* starts;  // of the first level's nodes
+  uint32_t* cnode;
+  uint32_t nodes;
+};
+
 // Digit counts of every chunk and their exclusive scan over the chunks:
 // chunkpre[c * 16 + d] = symbols before chunk c with digit d, and the totals
 // at c = nchunks.  A CTA takes tiles of 8 * cpw chunks from a counter (so the
 // look-back always waits on tiles that have started).  Bound by the read
 // of the sequence for 4-byte symbols, by issue for narrower ones.
-template <typename T, int TB>
+// HUFF also finds the chunks' nodes (there is no node pass, see HuffGroup).
+template <typename T, int TB, bool HUFF = false>
 __global__ void __launch_bounds__(LV_THREADS)
-    count_kernel(const T* __restrict__ src, uint64_t n, int ds, uint32_t nchunks, int cpw,
+    count_kernel(const void* __restrict__ src, uint64_t n, int ds, uint32_t nchunks, int cpw,
                  uint32_t* __restrict__ chunkpre, uint64_t* __restrict__ status, uint32_t sstride,
-                 uint32_t* __restrict__ counter, uint32_t tile0, uint32_t tile_end, uint32_t* __restrict__ err) {
+                 uint32_t* __restrict__ counter, uint32_t tile0, uint32_t tile_end, uint32_t* __restrict__ err,
+                 HuffGroup hg) {
   constexpr int MAX_TC = 64;  // chunks per tile
   constexpr int ND = 1 << TB;
   constexpr int NP = 1 << (TB - 1);
   __shared__ __align__(16) uint32_t s_pk[MAX_TC][8];  // per chunk: packed digit counts
   __shared__ uint32_t s_part[16][17];                 // per part of the tile and digit: sums, then prefixes
   __shared__ uint32_t s_tile;
+  __shared__ uint16_t s_lut[HUFF ? 256 : 1];
+  if constexpr (HUFF) load_lut(hg.lut, s_lut);
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t tc = LV_WARPS * cpw;
   const uint32_t d = threadIdx.x & 15, part = threadIdx.x >> 4;
@@ -213,7 +257,7 @@ __global__ void __launch_bounds__(LV_THREADS)
       uint32_t w[AHEAD][8 * sizeof(T)];
 #pragma unroll
       for (int h = 0; h < AHEAD; ++h)
-        if (k + h < cpw) load_row<T>(src, base + h * CHUNK + 32 * lane, n, w[h]);  // zeros past the end
+        if (k + h < cpw) load_symbols<T, HUFF>(src, s_lut, base + h * CHUNK + 32 * lane, n, w[h]);  // zeros past the end
 #pragma unroll
       for (int h = 0; h < AHEAD; ++h) {
         if (k + h >= cpw) break;
@@ -276,6 +320,15 @@ __global__ void __launch_bounds__(LV_THREADS)
         chunkpre[(uint64_t)c * 16 + d] = run;
         run += count_of(lc);
         if (c + 1 == nchunks) chunkpre[(uint64_t)nchunks * 16 + d] = run;
+      }
+    }
+    if constexpr (HUFF) {
+      for (uint32_t lc = threadIdx.x; lc < tc; lc += LV_THREADS) {
+        const uint32_t c = tile * tc + lc;
+        if (c < nchunks) {
+          hg.cnode[c] = find_node(hg.starts, 0, hg.nodes - 1, c << LOG_CHUNK);
+          if (c + 1 == nchunks) hg.cnode[nchunks] = hg.nodes - 1;
+        }
       }
     }
   }
@@ -448,6 +501,7 @@ struct PassArgs {
   const uint32_t* rec;       // [nodes][REC]
   uint32_t* bits;
   uint32_t* err;
+  HuffGroup huff;  // HUFF passes only
 };
 
 // stores the low `take` bits of val, bits [at, at + take) of the bit array
@@ -457,7 +511,17 @@ __device__ __forceinline__ void put_bits(uint32_t* __restrict__ bits, uint64_t w
   else if (val & mask) atomicOr(bits + word, val & mask);
 }
 
-template <typename Tin, typename Tout, int TAU, bool SCATTER>
+// first bit and symbols of the group's level j
+template <bool HUFF>
+__device__ __forceinline__ uint64_t level_begin(const PassArgs& a, int j) {
+  return HUFF ? __ldg(a.huff.lv + j) : (uint64_t)(a.level + j) * a.n;
+}
+template <bool HUFF>
+__device__ __forceinline__ uint64_t level_size(const PassArgs& a, int j) {
+  return HUFF ? __ldg(a.huff.lv + 4 + j) : a.n;
+}
+
+template <typename Tin, typename Tout, int TAU, bool SCATTER, bool HUFF>
 struct LevelPass {
   static constexpr int NW = 8 * sizeof(Tin);
   static constexpr int TB = SCATTER ? TAU : TAU - 1;  // bits that order the strings
@@ -641,17 +705,21 @@ struct LevelPass {
     {
       const int j = 31 - __clz(lane + 1);
       const uint32_t q = lane + 1 - (1u << j);
-      const bool in = j >= 1 && j < TAU;
+      bool in = j >= 1 && j < TAU;
+      if constexpr (HUFF) {
+        const uint32_t inner = __shfl_sync(0xffffffffu, rv, 15);
+        in = in && (inner >> lane & 1u);
+      }
       const uint32_t da = in ? q << (TB - j) : 0u, db = in ? (q + 1) << (TB - j) : 0u;
       const uint32_t za = __shfl_sync(0xffffffffu, pz, da), zb = __shfl_sync(0xffffffffu, pz, db);
       if (in) {
         const uint32_t ls = lds16(S + 2 * da);
         const uint32_t len = lds16(S + 2 * db) - ls;
         const uint32_t gp = rv + (zb - za);
-        if ((uint64_t)gp + len > a.n) {
+        if ((uint64_t)gp + len > level_size<HUFF>(a, j)) {
           bad = true;
         } else if (len) {
-          const uint64_t g = (uint64_t)(a.level + j) * a.n + gp;
+          const uint64_t g = level_begin<HUFF>(a, j) + gp;
           glo = (uint32_t)g;
           ghi = (uint32_t)(g >> 32);
           nw = ((glo & 31) + len + 31) >> 5;
@@ -692,9 +760,13 @@ struct LevelPass {
     if constexpr (SCATTER) {
       const uint32_t s0 = lds16(S + 2 * (lane & 15)), s1 = lds16(S + 2 * ((lane & 15) + 1));
       const uint32_t gd = __shfl_sync(0xffffffffu, rv, 16 + (lane & 15)) + zc;
+      const uint64_t next = HUFF ? __ldg(a.huff.lv + 8) : a.n;  // symbols of the next order
+      bool goes_on = true;
+      if constexpr (HUFF) goes_on = __shfl_sync(0xffffffffu, rv, 15) >> (16 + (lane & 15)) & 1u;
       if (lane < 16) {
-        if (s1 > s0 && (uint64_t)gd + (s1 - s0) > a.n) bad = true;
-        sts32(S + 64 + 4 * lane, gd - s0);
+        if (goes_on && s1 > s0 && (uint64_t)gd + (s1 - s0) > next) bad = true;
+        // (the places of symbols that leave the order come out beyond it)
+        sts32(S + 64 + 4 * lane, goes_on ? gd - s0 : HUFF_OUT);
         zc += s1 - s0;
       }
       if (!__any_sync(0xffffffffu, bad)) {
@@ -708,7 +780,8 @@ struct LevelPass {
           const uint32_t i = 32 * r + lane;
           if (FULL || i < total) {
             const uint32_t x = lds_sym<Tin>(stage + i * (uint32_t)sizeof(Tin));
-            dst[i + lds32(S + 64 + (((x >> dsh) & 15u) << 2))] = (Tout)x;
+            const uint32_t at = i + lds32(S + 64 + (((x >> dsh) & 15u) << 2));
+            if (!HUFF || at < next) dst[at] = (Tout)x;
           }
         }
       }
@@ -724,7 +797,8 @@ struct LevelPass {
   static __device__ __noinline__ void scattered_chunk(const PassArgs& a, uint32_t c, uint32_t zc, uint32_t base) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
-    const Tin* __restrict__ src = static_cast<const Tin*>(a.src);
+    using Src = typename std::conditional<HUFF, uint8_t, Tin>::type;
+    const Src* __restrict__ src = static_cast<const Src*>(a.src);
     // running counts before the row: (j, q) at word 2^j - 1 + q, j = 1 .. TB
     uint32_t pz = lane < (uint32_t)ND ? zc : 0u;
     const uint32_t z0 = pz;
@@ -748,20 +822,22 @@ struct LevelPass {
     for (int r = 0; r < 32; ++r) {
       const uint64_t i = ((uint64_t)c << LOG_CHUNK) + 32 * r + lane;
       const bool valid = i < a.n;
-      const uint32_t x = valid ? (uint32_t)src[i] : 0u;
+      uint32_t x = valid ? (uint32_t)src[i] : 0u;
+      if constexpr (HUFF) x = __ldg(a.huff.lut + x);
       const uint32_t dg = (x >> a.ds) & ((1u << TAU) - 1);  // TAU bits
       const uint32_t p = valid ? find_node(a.Cl, p_lo, p_hi, (uint32_t)i) : p_lo;
       const uint32_t* __restrict__ rp = a.rec + (uint64_t)p * REC;
       uint32_t m = __ballot_sync(0xffffffffu, valid);
+      const uint32_t inner = HUFF ? __ldg(rp + 15) : 0u;
 #pragma unroll
       for (int j = 0; j < TAU; ++j) {
         const bool bit = (dg >> (TAU - 1 - j)) & 1u;
         const uint32_t q = dg >> (TAU - j);  // the j bits above
-        if (j >= 1 && valid) {
+        if (j >= 1 && valid && (!HUFF || (inner >> ((1 << j) - 1 + q) & 1u))) {
           const uint32_t pos = __ldg(rp + (1 << j) - 1 + q) + lds32(base + 4 * ((1 << j) - 1 + q)) + __popc(m & lt);
-          if (pos >= a.n) bad = true;
+          if (pos >= level_size<HUFF>(a, j)) bad = true;
           else if (bit) {
-            const uint64_t g = (uint64_t)(a.level + j) * a.n + pos;
+            const uint64_t g = level_begin<HUFF>(a, j) + pos;
             atomicOr(a.bits + (g >> 5), 1u << (g & 31));
           }
         }
@@ -775,9 +851,9 @@ struct LevelPass {
         m &= bit ? bm : ~bm;
       }
       if constexpr (SCATTER) {
-        if (valid) {
+        if (valid && (!HUFF || (inner >> (16 + dg) & 1u))) {
           const uint32_t pos = __ldg(rp + 16 + dg) + lds32(base + 4 * (15 + dg)) + __popc(m & lt);
-          if (pos >= a.n) bad = true;
+          if (pos >= (HUFF ? __ldg(a.huff.lv + 8) : a.n)) bad = true;
           else static_cast<Tout*>(a.dst)[pos] = (Tout)x;
         }
         __syncwarp();
@@ -817,13 +893,14 @@ __device__ __forceinline__ void first_level_bits(uint32_t* __restrict__ bits, ui
   if (lane == 0 && end > 1024) put_bits(bits, G + 32, last >> (32 - head), (1u << (end - 1024)) - 1);
 }
 
-template <typename Tin, typename Tout, int TAU, bool SCATTER, int CTAS>
+template <typename Tin, typename Tout, int TAU, bool SCATTER, int CTAS, bool HUFF = false>
 __global__ void __launch_bounds__(LV_THREADS, CTAS) level_pass_kernel(PassArgs a) {
-  using P = LevelPass<Tin, Tout, TAU, SCATTER>;
+  using P = LevelPass<Tin, Tout, TAU, SCATTER, HUFF>;
+  __shared__ uint16_t s_lut[HUFF ? 256 : 1];
+  if constexpr (HUFF) load_lut(a.huff.lut, s_lut);
   extern __shared__ __align__(16) unsigned char lv_smem_raw[];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t base = ((smem_addr(lv_smem_raw) + 2047u) & ~2047u) + warp * lv_warp_bytes<Tin, SCATTER>();
-  const Tin* __restrict__ src = static_cast<const Tin*>(a.src);
   const uint32_t stride = gridDim.x * LV_WARPS;
   for (uint32_t c = blockIdx.x * LV_WARPS + warp; c < a.nchunks; c += stride) {
     const uint64_t cbase = (uint64_t)c << LOG_CHUNK;
@@ -833,11 +910,11 @@ __global__ void __launch_bounds__(LV_THREADS, CTAS) level_pass_kernel(PassArgs a
     if (a.nodes > 1) p = __ldg(a.cnode + c);
     uint32_t zc = lane < (uint32_t)P::ND ? __ldg(a.chunkpre + (uint64_t)c * 16 + lane) : 0u;
     uint32_t w[P::NW], B[TAU];
-    load_row<Tin>(src, cbase + 32 * lane, a.n, w);
+    load_symbols<Tin, HUFF>(a.src, s_lut, cbase + 32 * lane, a.n, w);
     if (a.nodes > 1 && p + 1 < a.nodes) cend = __ldg(a.Cl + p + 1);
     uint32_t rv = __ldg(a.rec + (uint64_t)p * REC + lane);
     planes<Tin, TAU>(w, a.ds, B);
-    first_level_bits(a.bits, (uint64_t)a.level * a.n + cbase,
+    first_level_bits(a.bits, level_begin<HUFF>(a, 0) + cbase,
                      cvalid == CHUNK ? B[0] : B[0] & row_mask(lane, 0, cvalid), cvalid);
     if (cend >= cbase + CHUNK && cvalid == CHUNK) {
       P::template segment<true>(a, w, B, 0xFFFFFFFFu, zc, rv, base);

@@ -1,5 +1,6 @@
 // wtg_pass.cuh -- launchers of the level passes (internal; the kernels are in
-// wtg_levels.cuh, instantiated by wtg_pass_scatter.cu and wtg_pass_last.cu).
+// wtg_levels.cuh, instantiated by wtg_pass_scatter.cu, wtg_pass_last.cu and
+// wtg_pass_huff.cu).
 #pragma once
 #include "wtg_levels.cuh"
 
@@ -27,6 +28,13 @@ int launch_count(const LevelGroup& a, uint32_t tile0, uint32_t tile1, cudaStream
 int launch_nodes(const LevelGroup& a, cudaStream_t s);
 int launch_pass(const LevelGroup& a, cudaStream_t s);
 int launch_pass_scatter(const LevelGroup& a, cudaStream_t s);
+// the two passes of a Huffman-shaped tree's group (wtg_pass_huff.cu)
+int launch_huff_count(const LevelGroup& a, uint32_t tiles, cudaStream_t s);
+int launch_huff_pass(const LevelGroup& a, cudaStream_t s);
+
+// chunks per warp of a count tile: more per tile (fewer look-backs) once the
+// tiles still fill the chip eight times
+int count_cpw(uint64_t nchunks);
 
 int lv_sm_count();
 

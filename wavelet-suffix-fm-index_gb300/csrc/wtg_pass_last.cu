@@ -18,14 +18,19 @@ int lv_sm_count() {
   return n;
 }
 
+int count_cpw(uint64_t nchunks) {
+  const uint64_t c = nchunks / ((uint64_t)LV_WARPS * lv_sm_count() * 8);
+  return c >= 8 ? 8 : c >= 4 ? 4 : c >= 2 ? 2 : 1;
+}
+
 namespace {
 
 template <typename T, int TB>
 int count_t(const LevelGroup& a, uint32_t tile0, uint32_t tile1, cudaStream_t s) {
   static int per_sm = 0;
   const PassArgs& p = a.pass;
-  return launch_resident(count_kernel<T, TB>, per_sm, tile1 - tile0, 0, s, (const T*)p.src, p.n, p.ds + a.tau - TB,
-                         p.nchunks, a.cpw, a.chunkpre, a.status, a.sstride, a.counter, tile0, tile1, p.err);
+  return launch_resident(count_kernel<T, TB>, per_sm, tile1 - tile0, 0, s, p.src, p.n, p.ds + a.tau - TB,
+                         p.nchunks, a.cpw, a.chunkpre, a.status, a.sstride, a.counter, tile0, tile1, p.err, p.huff);
 }
 
 template <typename T, int TB>
