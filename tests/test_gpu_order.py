@@ -7,7 +7,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-N, L, NQ, SMALL = (1 << 26) + 3, 20, (1 << 21) + 5, 1 << 19  # 168 MB of bits; SMALL is never sorted
+N, L, NQ, SMALL = (1 << 26) + 3, 20, (5 << 19) + 5, 1 << 19  # 168 MB of bits; SMALL is never sorted
 
 
 @pytest.fixture(scope="module")
@@ -72,3 +72,19 @@ def test_inverse_select_from_host_arrays(setup):
     parts = [t.inverse_select(i[a:a + SMALL]) for a in range(0, NQ, SMALL)]
     assert np.array_equal(r, np.concatenate([p[0] for p in parts]))
     assert np.array_equal(c, np.concatenate([p[1] for p in parts]))
+
+
+@pytest.mark.parametrize("m", [(1 << 20) + 1, NQ])  # sorted over the two tables, and over the blocks
+def test_batches_with_and_without_blocks(setup, m):
+    torch, t, seq, idx, sym, end = setup
+    st = torch.cuda.current_stream().cuda_stream
+    i, c = idx[-m:], sym[-m:]
+    got = torch.empty((2, m), dtype=torch.int64, device="cuda")
+    exp = torch.empty((2, m), dtype=torch.int64, device="cuda")
+    for out, piece in ((got, m), (exp, SMALL)):
+        for at in range(0, m, piece):
+            k = min(piece, m - at)
+            t.access_device(i.data_ptr() + 8 * at, k, out[0].data_ptr() + 8 * at, st)
+            t.rank_device(i.data_ptr() + 8 * at, c.data_ptr() + 8 * at, k, out[1].data_ptr() + 8 * at, st)
+    torch.cuda.synchronize()
+    assert torch.equal(got, exp)

@@ -3,6 +3,7 @@
 // select, one thread per query; plus the alphabet remap helper.
 #include <algorithm>
 
+#include "wtg_blocks.cuh"
 #include "wtg_order.cuh"
 #include "wtg_select.cuh"
 #include "wtg_tree.cuh"
@@ -49,12 +50,37 @@ __device__ __forceinline__ uint32_t rank_step(const uint64_t* __restrict__ tree,
   return (uint32_t)e.x + in + __popcll(word & ((1ull << (pos & 63)) - 1));
 }
 
+// What the descents probe: the rank table and the bitvector, or for large
+// sorted batches the blocks made of them (one sector a level instead of two:
+// the sorted descent is bound by the lines its loads look up in L1).
+template <bool BLOCKS>
+struct LevelBits {
+  const uint64_t* tree;
+  const uint64_t* rt;
+  const uint4* blocks;
+  // ones before pos (mod 2^32), and the bit at it
+  __device__ __forceinline__ uint32_t rank(uint64_t pos, uint32_t& bit) const {
+    if constexpr (BLOCKS) {
+      uint32_t off;
+      uint64_t v[4];
+      block_load(blocks, block_of(pos, off), v);
+      const BlockProbe r = block_at(v, off);
+      bit = r.bit;
+      return r.ones;
+    } else {
+      uint64_t word;
+      const uint32_t R = rank_step(tree, rt, pos, word);
+      bit = (uint32_t)(word >> (pos & 63)) & 1u;
+      return R;
+    }
+  }
+};
+
 // wt_int::operator[] (wt_int/wt_int_par.hpp:519-541) and inverse_select
 // (:588-611): descend by the bit at i; the symbol is the path, the rank the
 // final position
-template <bool INV, bool ORD>
-__global__ void wt_descend_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                                  const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
+template <bool INV, bool ORD, bool BLOCKS>
+__global__ void wt_descend_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
                                   QueryOrder ord, uint64_t nq, uint64_t* __restrict__ out,
                                   uint64_t* __restrict__ sym_out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -69,12 +95,10 @@ __global__ void wt_descend_kernel(const uint64_t* __restrict__ tree, const uint6
   uint32_t x = (uint32_t)i, h = 1;  // h: heap id + 1, the path with a leading 1
   uint64_t lbase = 0;
   for (int lv = 0; lv < L; ++lv, lbase += n) {
-    const uint64_t pos = lbase + x;
     uint2 st = make_uint2(0u, 0u);
     if (INV || lv + 1 < L) st = __ldg(step + (h - 1));
-    uint64_t word;
-    const uint32_t R = rank_step(tree, rt, pos, word);
-    const uint32_t bit = (uint32_t)(word >> (pos & 63)) & 1u;
+    uint32_t bit;
+    const uint32_t R = bits.rank(lbase + x, bit);
     x = bit ? st.y + R : st.x + x - R;
     h = 2 * h + bit;
   }
@@ -88,9 +112,8 @@ __global__ void wt_descend_kernel(const uint64_t* __restrict__ tree, const uint6
 }
 
 // wt_int::rank (wt_int_par.hpp:553-577): descend along c's path
-template <bool ORD>
-__global__ void wt_rank_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                               const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
+template <bool ORD, bool BLOCKS>
+__global__ void wt_rank_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
                                QueryOrder ord, const uint64_t* __restrict__ sym, uint64_t nq,
                                uint64_t* __restrict__ out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -111,8 +134,8 @@ __global__ void wt_rank_kernel(const uint64_t* __restrict__ tree, const uint64_t
   uint64_t lbase = 0;
   for (int lv = 0; lv < L; ++lv, lbase += n) {
     const uint2 st = __ldg(step + ((path >> (L - lv)) - 1));
-    uint64_t word;
-    const uint32_t R = rank_step(tree, rt, lbase + x, word);
+    uint32_t bit;
+    const uint32_t R = bits.rank(lbase + x, bit);
     x = (path >> (L - 1 - lv)) & 1u ? st.y + R : st.x + x - R;
   }
   out[k] = x;
@@ -201,50 +224,61 @@ int tree_node_table(TreeImpl& t, cudaStream_t s) {
   return WTG_OK;
 }
 
-int launch_wt_access(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* out, cudaStream_t s) {
+// Blocks (built from the bitvector for the call: 1.1 ms for 2^30 x 20 levels,
+// 112 M blocks) pay once the batch probes a good part of them and there are
+// levels enough.  Access, sorted, ms without / with blocks: 2^30 x 20, 2^26
+// queries 14.2 / 11.3, 2^25 7.00 / 6.07, 2^24 3.42 / 3.39, 2^23 1.63 / 2.10;
+// 2^27 x 20 (14 M blocks), 2^26 6.52 / 5.98, 2^23 0.89 / 0.86, 2^22 0.48 /
+// 0.53; but 2^28 x 8 (11 M), 2^26 4.52 / 4.28, 2^25 2.19 / 2.17, 2^24 1.04 / 1.10.
+static bool blocks_pay(const TreeImpl& t, uint64_t nq) {
+  return order_pays(t, nq) && t.levels >= 12 && nq >= block_count(t.n * (uint64_t)t.levels) / 3;
+}
+
+// in_order, with the blocks where they pay and there is room for them:
+// launch(bits, ordered, order, first query, queries), ordered a bool constant
+template <typename F>
+static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t s, F launch) {
   int rc;
-  if ((rc = need(t, WTG_RANK, "access"))) return rc;
   if (!nq) return WTG_OK;
   if ((rc = tree_node_table(t, s))) return rc;
-  return in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
-    auto* const f = sorted ? wt_descend_kernel<false, true> : wt_descend_kernel<false, false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n,
-                               t.levels, idx + at, o, m, out + at, nullptr);
+  const uint64_t* const words = t.bits.as<uint64_t>();
+  const uint64_t* const rt = t.bv.rank.as<uint64_t>();
+  uint4* const blocks = blocks_pay(t, nq) ? make_blocks(words, rt, t.n * (uint64_t)t.levels, s) : nullptr;
+  rc = in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    if (sorted && blocks) launch(LevelBits<true>{words, rt, blocks}, std::true_type{}, o, at, m);
+    else if (sorted) launch(LevelBits<false>{words, rt, nullptr}, std::true_type{}, o, at, m);
+    else launch(LevelBits<false>{words, rt, nullptr}, std::false_type{}, o, at, m);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
+  });
+  if (blocks) cudaFreeAsync(blocks, s);
+  return rc;
+}
+
+int launch_wt_access(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* out, cudaStream_t s) {
+  if (int rc = need(t, WTG_RANK, "access")) return rc;
+  return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
+    wt_descend_kernel<false, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
+                                                             m, out + at, nullptr);
   });
 }
 
 int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64_t nq, uint64_t* out,
                    cudaStream_t s) {
-  int rc;
-  if ((rc = need(t, WTG_RANK, "rank"))) return rc;
-  if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
-  return in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
-    auto* const f = sorted ? wt_rank_kernel<true> : wt_rank_kernel<false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n,
-                               t.levels, idx + at, o, sym + at, m, out + at);
-    count_launch();
-    WTG_CK(cudaGetLastError());
-    return WTG_OK;
+  if (int rc = need(t, WTG_RANK, "rank")) return rc;
+  return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
+    wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o, sym + at,
+                                                   m, out + at);
   });
 }
 
 int launch_wt_inverse_select(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* rank_out,
                              uint64_t* sym_out, cudaStream_t s) {
-  int rc;
-  if ((rc = need(t, WTG_RANK, "inverse_select"))) return rc;
-  if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
-  return in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
-    auto* const f = sorted ? wt_descend_kernel<true, true> : wt_descend_kernel<true, false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n,
-                               t.levels, idx + at, o, m, rank_out + at, sym_out + at);
-    count_launch();
-    WTG_CK(cudaGetLastError());
-    return WTG_OK;
+  if (int rc = need(t, WTG_RANK, "inverse_select")) return rc;
+  return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
+    wt_descend_kernel<true, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
+                                                            m, rank_out + at, sym_out + at);
   });
 }
 
