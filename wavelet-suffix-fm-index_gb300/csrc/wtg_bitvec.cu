@@ -574,21 +574,17 @@ static uint32_t logn_of(uint64_t size) {
 
 void bv_release(BvSupport& bv, cudaStream_t s) {
   bv.rank.release(s);
-  bv.samples.release(s);
-  bv.info.release(s);
-  bv.status.release(s);
-  bv.scan_tmp.release(s);
+  bv.work.release(s);
   for (auto& sd : bv.sel) {
-    sd.ends.release(s);
-    sd.desc.release(s);
-    sd.offs.release(s);
     sd.sb_words.release(s);
     sd.pool.release(s);
-    sd.long_list.release(s);
     sd.long_ent.release(s);
-    sd.starts.release(s);
   }
 }
+
+// superblocks per thread of the pass over a bitvector of NB + 1 superblocks:
+// 4 (a 64 KB tile per CTA) once that fills the chip twice, 1 below
+static int bv_spt(uint64_t NB) { return NB + 1 >= 4ull * BV_THREADS * 2 * 152 ? 4 : 1; }
 
 int bv_prepare(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t& flags, cudaStream_t s) {
   int rc;
@@ -602,27 +598,48 @@ int bv_prepare(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t& 
   const uint64_t NB = W >> 3;
   const uint64_t nsb_cap = size / 4096 + 2;
   const uint64_t samp_n = W + 2;
-  if ((rc = bv.info.ensure(INF_N * sizeof(uint64_t), s))) return rc;
-  WTG_CK(cudaMemsetAsync(bv.info.p, 0, INF_N * sizeof(uint64_t), s));
+  bv.spt = bv_spt(NB);
+  const uint64_t tiles = (NB + 1 + bv.spt * BV_THREADS - 1) / (bv.spt * BV_THREADS);
+  if (tiles > 0x7fffffffull) return fail(WTG_ERR_INVALID, "bitvector too large");
+  bv.tiles = (uint32_t)tiles;
+  bv.tiles_done = 0;
   if (flags & WTG_RANK)
     if ((rc = bv.rank.ensure(2 * (NB + 1) * sizeof(uint64_t), s))) return rc;
-  if (flags & (WTG_SELECT1 | WTG_SELECT0))
-    if ((rc = bv.samples.ensure(samp_n * sizeof(uint32_t), s))) return rc;
+  DevLayout lay;
+  const uint64_t sd_tiles = (nsb_cap + SD_TILE - 1) / SD_TILE;
+  const size_t info = lay.add(INF_N * sizeof(uint64_t));
+  const size_t status = lay.add((tiles + 1) * sizeof(uint64_t));
+  const size_t scan = lay.add(2 * (sd_tiles + 1) * sizeof(uint64_t));
+  const size_t clear = lay.bytes;  // these start at 0
+  const size_t samples = lay.add(flags & (WTG_SELECT1 | WTG_SELECT0) ? samp_n * sizeof(uint32_t) : 0);
+  const size_t per = (nsb_cap * sizeof(uint64_t) + 255) / 256 * 256;
+  size_t sel[2] = {0, 0};
+  for (int t_b = 0; t_b < 2; ++t_b)
+    if (flags & (t_b ? WTG_SELECT1 : WTG_SELECT0)) sel[t_b] = lay.add(6 * per);
+  if ((rc = bv.work.ensure(lay.bytes, s))) return rc;
+  uint8_t* const w = bv.work.as<uint8_t>();
+  WTG_CK(cudaMemsetAsync(w, 0, clear, s));
+  bv.info.p = w + info;
+  bv.status.p = w + status;
+  bv.scan_tmp.p = w + scan;
+  bv.samples.p = w + samples;
   for (int t_b = 0; t_b < 2; ++t_b) {
-    if (!(flags & (t_b ? WTG_SELECT1 : WTG_SELECT0))) continue;
     SelectDev& sd = bv.sel[t_b];
-    if ((rc = sd.ends.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
-    if ((rc = sd.starts.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
-    if ((rc = sd.desc.ensure(2 * nsb_cap * sizeof(uint64_t), s))) return rc;   // [final | working]
-    if ((rc = sd.offs.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
-    if ((rc = sd.long_list.ensure(nsb_cap * sizeof(uint64_t), s))) return rc;
+    sd.ends = sd.starts = sd.offs = sd.long_list = sd.desc = DevPart{};
+    if (!(flags & (t_b ? WTG_SELECT1 : WTG_SELECT0))) continue;
+    uint8_t* const p = w + sel[t_b];
+    sd.ends.p = p;
+    sd.starts.p = p + per;
+    sd.offs.p = p + 2 * per;
+    sd.long_list.p = p + 3 * per;
+    sd.desc.p = p + 4 * per;  // 2 * nsb_cap entries
+  }
+  if (test_take_lookback_stall()) {  // tile 0 is never taken: every look-back wait on it runs out
+    static const uint32_t one = 1;
+    WTG_CK(cudaMemcpyAsync(bv.status.p, &one, sizeof(one), cudaMemcpyHostToDevice, s));
   }
   return WTG_OK;
 }
-
-// superblocks per thread of the pass over a bitvector of NB + 1 superblocks:
-// 4 (a 64 KB tile per CTA) once that fills the chip twice, 1 below
-static int bv_spt(uint64_t NB) { return NB + 1 >= 4ull * BV_THREADS * 2 * 152 ? 4 : 1; }
 
 template <int SPT>
 static int launch_bv_pass_t(const uint64_t* words, uint64_t size, uint32_t flags, uint64_t* rank, uint32_t* samples,
@@ -658,23 +675,6 @@ static int launch_bv_pass(int spt, const uint64_t* words, uint64_t size, uint32_
   auto* const f = spt == 4 ? launch_bv_pass_t<4> : launch_bv_pass_t<1>;
   return f(words, size, flags, rank, samples, samp_last, starts1, starts0, ends1, ends0, info, status, counter, tile0,
            tile_end, err, s);
-}
-
-int bv_pass_begin(BvSupport& bv, cudaStream_t s) {
-  int rc;
-  const uint64_t NB = ((bv.size + 63) / 64) >> 3;
-  bv.spt = bv_spt(NB);
-  const uint64_t tiles = (NB + 1 + bv.spt * BV_THREADS - 1) / (bv.spt * BV_THREADS);
-  if (tiles > 0x7fffffffull) return fail(WTG_ERR_INVALID, "bitvector too large");
-  bv.tiles = (uint32_t)tiles;
-  bv.tiles_done = 0;
-  if ((rc = bv.status.ensure((tiles + 1) * sizeof(uint64_t), s))) return rc;
-  WTG_CK(cudaMemsetAsync(bv.status.p, 0, (tiles + 1) * sizeof(uint64_t), s));
-  if (test_take_lookback_stall()) {  // tile 0 is never taken: every look-back wait on it runs out
-    static const uint32_t one = 1;
-    WTG_CK(cudaMemcpyAsync(bv.status.p, &one, sizeof(one), cudaMemcpyHostToDevice, s));
-  }
-  return WTG_OK;
 }
 
 int bv_pass_to(BvSupport& bv, uint64_t bits_ready, uint32_t* d_err, cudaStream_t s) {
@@ -713,8 +713,6 @@ int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
 
   // descriptors and pool offsets of both polarities
   const uint64_t tiles = (nsb_cap + SD_TILE - 1) / SD_TILE;
-  if ((rc = bv.scan_tmp.ensure(2 * (tiles + 1) * sizeof(uint64_t), s))) return rc;
-  WTG_CK(cudaMemsetAsync(bv.scan_tmp.p, 0, 2 * (tiles + 1) * sizeof(uint64_t), s));
   SelBuild2 sb{};
   for (int t_b = 0; t_b < 2; ++t_b) {
     if (!(flags & (t_b ? WTG_SELECT1 : WTG_SELECT0))) continue;
@@ -799,7 +797,6 @@ int bv_build(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t fla
              cudaStream_t s) {
   int rc;
   if ((rc = bv_prepare(bv, d_words, size, flags, s))) return rc;
-  if ((rc = bv_pass_begin(bv, s))) return rc;
   if ((rc = bv_pass_to(bv, size, d_err, s))) return rc;
   return bv_finish(bv, d_err, s);
 }

@@ -156,9 +156,18 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   ++t.gen;
   const uint64_t heap = 1ull << L;  // heap ids 0 .. 2^L - 2, plus one pad entry
 
-  if ((rc = t.err.ensure(sizeof(uint32_t), s))) return rc;
-  WTG_CK(cudaMemsetAsync(t.err.p, 0, sizeof(uint32_t), s));
-  uint32_t* d_err = t.err.as<uint32_t>();
+  const uint32_t nchunks = (uint32_t)((n + CHUNK - 1) / CHUNK);
+  const int cpw = count_cpw(nchunks);
+  const uint32_t tc = LV_WARPS * cpw, tiles = (nchunks + tc - 1) / tc;
+  const int groups = n ? (L + 3) / 4 : 0;  // all but the last of four levels
+  // the error word, and the look-back state per group: 16 arrays of tile words, a counter
+  const uint64_t group_words = 16ull * tiles + 1;
+  const size_t err_bytes = 16 + groups * group_words * sizeof(uint64_t);
+  if ((rc = t.err.ensure(err_bytes, s))) return rc;
+  WTG_CK(cudaMemsetAsync(t.err.p, 0, err_bytes, s));
+  t.err.elsewhere = false;
+  uint32_t* d_err = t.err.arm(s, s);
+  uint64_t* const group_status = t.err.as<uint64_t>() + 2;
 
   // every string's edge words are ORed in
   if ((rc = t.bits.ensure((t.bit_words + 2) * sizeof(uint64_t), s))) return rc;
@@ -168,7 +177,7 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   uint32_t* Z = t.zeros.as<uint32_t>();
   uint32_t* C = Z + heap;
   if (n == 0) WTG_CK(cudaMemsetAsync(Z, 0, 2 * heap * sizeof(uint32_t), s));
-  else WTG_CK(cudaMemsetAsync(C, 0, sizeof(uint32_t), s));  // the root starts at 0
+  else if (L == 1) WTG_CK(cudaMemsetAsync(C, 0, sizeof(uint32_t), s));  // the root (otherwise the first node pass)
 
   // When the rank table goes to page-locked host memory during the build,
   // the rank/select pass follows the levels, and the rank entries whose bits
@@ -178,7 +187,6 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   const bool rs_by_level = t.host_rank && (flags & WTG_RANK) && n && host_page_locked(t.host_rank);
   if (flags) {
     if ((rc = bv_prepare(t.bv, t.bits.as<uint64_t>(), n * (uint64_t)L, flags, s))) return rc;
-    if ((rc = bv_pass_begin(t.bv, s))) return rc;
   }
   uint64_t rank_copied = 0;  // superblocks whose rank entries were sent
   auto copy_rank = [&]() -> int {
@@ -192,20 +200,25 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
     return WTG_OK;
   };
   if (n) {
-    const uint32_t nchunks = (uint32_t)((n + CHUNK - 1) / CHUNK);
-    const int cpw = count_cpw(nchunks);
-    const uint32_t tc = LV_WARPS * cpw, tiles = (nchunks + tc - 1) / tc;
-    const int groups = (L + 3) / 4;  // all but the last of four levels
-    if ((rc = t.chunkpre.ensure(((uint64_t)nchunks + 1) * 16 * sizeof(uint32_t), s))) return rc;
-    if ((rc = t.cnode.ensure(((uint64_t)nchunks + 1) * sizeof(uint32_t), s))) return rc;
-    if ((rc = t.rec.ensure((1ull << (4 * (groups - 1))) * REC * sizeof(uint32_t), s))) return rc;
-    // look-back state per group: 16 arrays of tile words, a counter
-    const uint64_t group_words = 16ull * tiles + 1;
-    if ((rc = t.status.ensure(groups * group_words * sizeof(uint64_t), s))) return rc;
-    WTG_CK(cudaMemsetAsync(t.status.p, 0, groups * group_words * sizeof(uint64_t), s));
     // sequence buffers: what the groups after the first read
-    const uint64_t pad = 64;
     auto bytes_of = [&](int bits_left) { return bits_left > 16 ? 4 : bits_left > 8 ? 2 : 1; };
+    const bool repack = eb == 8 || (uintptr_t)d_seq % 32;
+    size_t lvl_bytes[2] = {0, repack ? n * std::min(eb, 4) : 0};
+    for (int g = 0, sb = std::min(eb, 4); g + 1 < groups; ++g) {
+      sb = std::min(sb, bytes_of(L - 4 * g - 4));
+      lvl_bytes[g & 1] = std::max<size_t>(lvl_bytes[g & 1], n * sb);
+    }
+    DevLayout lay;
+    const size_t at_pre = lay.add(((uint64_t)nchunks + 1) * 16 * sizeof(uint32_t));
+    const size_t at_cnode = lay.add(((uint64_t)nchunks + 1) * sizeof(uint32_t));
+    const size_t at_rec = lay.add((1ull << (4 * (groups - 1))) * REC * sizeof(uint32_t));
+    const size_t at_lvl[2] = {lay.add(lvl_bytes[0]), lay.add(lvl_bytes[1])};
+    if ((rc = t.work.ensure(lay.bytes, s))) return rc;
+    uint8_t* const work = t.work.as<uint8_t>();
+    uint32_t* const chunkpre = (uint32_t*)(work + at_pre);
+    uint32_t* const cnode = (uint32_t*)(work + at_cnode);
+    uint32_t* const rec = (uint32_t*)(work + at_rec);
+    void* const lvl[2] = {work + at_lvl[0], work + at_lvl[1]};
     const void* src = d_seq;
     int sb = eb;
     bool waited = t.in_pieces == 0;
@@ -214,19 +227,18 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
       waited = true;
       return WTG_OK;
     };
-    if (eb == 8 || (uintptr_t)d_seq % 32) {
+    if (repack) {
       sb = std::min(eb, 4);
       if ((rc = wait_pieces())) return rc;
-      if ((rc = t.lvl[1].ensure(n * sb + pad, s))) return rc;
       const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16);
       if (eb == 8) {
-        repack_kernel<uint64_t, uint32_t><<<grid, 256, 0, s>>>((const uint64_t*)d_seq, n, t.lvl[1].as<uint32_t>());
+        repack_kernel<uint64_t, uint32_t><<<grid, 256, 0, s>>>((const uint64_t*)d_seq, n, (uint32_t*)lvl[1]);
         count_launch();
         WTG_CK(cudaGetLastError());
       } else {
-        WTG_CK(cudaMemcpyAsync(t.lvl[1].p, d_seq, n * sb, cudaMemcpyDeviceToDevice, s));
+        WTG_CK(cudaMemcpyAsync(lvl[1], d_seq, n * sb, cudaMemcpyDeviceToDevice, s));
       }
-      src = t.lvl[1].p;
+      src = lvl[1];
     }
     for (int g = 0; g < groups; ++g) {
       const int l = 4 * g;
@@ -243,24 +255,20 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
       a.pass.nchunks = nchunks;
       a.pass.nodes = 1u << l;
       a.pass.Cl = C + ((1ull << l) - 1);
-      a.pass.chunkpre = t.chunkpre.as<uint32_t>();
-      a.pass.cnode = t.cnode.as<uint32_t>();
-      a.pass.rec = t.rec.as<uint32_t>();
+      a.pass.chunkpre = chunkpre;
+      a.pass.cnode = cnode;
+      a.pass.rec = rec;
       a.pass.bits = t.bits.as<uint32_t>();
       a.pass.err = d_err;
-      if (scatter) {
-        DevBuf& dst = t.lvl[g & 1];
-        if ((rc = dst.ensure(n * a.dst_bytes + pad, s))) return rc;
-        a.pass.dst = dst.p;
-      }
+      if (scatter) a.pass.dst = lvl[g & 1];
       a.C = C;
       a.Z = Z;
-      a.chunkpre = t.chunkpre.as<uint32_t>();
-      a.cnode = t.cnode.as<uint32_t>();
-      a.rec = t.rec.as<uint32_t>();
+      a.chunkpre = chunkpre;
+      a.cnode = cnode;
+      a.rec = rec;
       a.cpw = cpw;
-      a.counter = reinterpret_cast<uint32_t*>(t.status.as<uint64_t>() + g * group_words);
-      a.status = t.status.as<uint64_t>() + g * group_words + 1;
+      a.counter = reinterpret_cast<uint32_t*>(group_status + g * group_words);
+      a.status = group_status + g * group_words + 1;
       a.sstride = tiles;
       const int tb = scatter ? 4 : a.tau - 1;  // digit bits counted
       if (tb > 0) {
@@ -356,14 +364,9 @@ void tree_release(TreeImpl& t) {
   t.in_pieces = 0;
   lsel_detach_all(t);
   t.seq.release(s);
-  t.lvl[0].release(s);
-  t.lvl[1].release(s);
   t.bits.release(s);
   t.zeros.release(s);
-  t.status.release(s);
-  t.chunkpre.release(s);
-  t.cnode.release(s);
-  t.rec.release(s);
+  t.work.release(s);
   t.scan_tmp.release(s);
   t.err.release(s);
   t.lvl_args.release(s);

@@ -26,7 +26,7 @@ struct wtg_huff {
 struct wtg_bv {
   wtg::BvSupport bv;
   wtg::DevBuf words;  // device copy for host-input builds
-  wtg::DevBuf err;
+  wtg::ErrWord err;
   wtg::DevBuf qbuf;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
@@ -56,12 +56,13 @@ int check_seq_args(uint64_t n, int eb, int levels, uint32_t flags) {
   return WTG_OK;
 }
 
-int sync_and_check(cudaStream_t s, const uint32_t* d_err) {
-  WTG_CK(cudaStreamSynchronize(s));
+// waits for the stream; an error that a kernel reported stays until the next build
+int sync_and_check(cudaStream_t s, ErrWord& err) {
   uint32_t e = 0;
-  if (d_err) {
-    WTG_CK(cudaMemcpy(&e, d_err, sizeof(e), cudaMemcpyDeviceToHost));
-  }
+  const bool read = err.p && (err.pending || err.elsewhere);
+  if (read) WTG_CK(cudaMemcpyAsync(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost, s));
+  WTG_CK(cudaStreamSynchronize(s));
+  if (!e) err.pending = false;
   if (e == DERR_LOOKBACK_TIMEOUT) return fail(WTG_ERR_TIMEOUT, "a device-side wait timed out; results are invalid");
   if (e == DERR_BAD_INDEX) return fail(WTG_ERR_CUDA, "a computed index fell outside its buffer (inconsistent tables)");
   if (e) return fail(WTG_ERR_CUDA, "device reported error code " + std::to_string(e));
@@ -87,7 +88,7 @@ int build_tree_common(wtg_tree* T, const void* d_seq, uint64_t n, int eb, int le
 // runs `launch` on device copies of host query arrays
 template <typename F>
 int host_query(DevBuf& qbuf, cudaStream_t s, const uint64_t* const* ins, int nin, uint64_t nq,
-               uint64_t* const* outs, int nout, const uint32_t* d_err, F launch) {
+               uint64_t* const* outs, int nout, ErrWord& err, F launch) {
   int rc;
   if (nq == 0) return WTG_OK;
   if ((rc = qbuf.ensure((size_t)(nin + nout) * nq * sizeof(uint64_t), s))) return rc;
@@ -101,7 +102,7 @@ int host_query(DevBuf& qbuf, cudaStream_t s, const uint64_t* const* ins, int nin
   if ((rc = launch(din, dout))) return rc;
   for (int k = 0; k < nout; ++k)
     WTG_CK(cudaMemcpyAsync(outs[k], dout[k], nq * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  return sync_and_check(s, d_err);
+  return sync_and_check(s, err);
 }
 
 // Variable-size answers: the query arrays go to the device, `count` fills
@@ -125,11 +126,11 @@ int host_variable_query(TreeImpl& t, const uint64_t* const* ins, int nin, uint64
   uint64_t* d_off = d_cnt + nq;
   if ((rc = count(din, d_cnt))) return rc;
   WTG_CK(cudaMemcpyAsync(counts_out, d_cnt, nq * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  if (!nv || !cap) return sync_and_check(s, t.err.as<uint32_t>());
-  if ((rc = answer_offsets(d_cnt, nq, d_off, t.scan_tmp, t.err.as<uint32_t>(), s))) return rc;
+  if (!nv || !cap) return sync_and_check(s, t.err);
+  if ((rc = answer_offsets(d_cnt, nq, d_off, t.scan_tmp, t.err.arm(s, t.stream), s))) return rc;
   uint64_t total = 0;
   WTG_CK(cudaMemcpyAsync(&total, d_off + nq, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  if ((rc = sync_and_check(s, t.err.as<uint32_t>()))) return rc;
+  if ((rc = sync_and_check(s, t.err))) return rc;
   const uint64_t m = std::min(total, cap);
   if (!m) return WTG_OK;
   if ((rc = t.qout.ensure((size_t)nv * m * sizeof(uint64_t), s))) return rc;
@@ -138,7 +139,7 @@ int host_variable_query(TreeImpl& t, const uint64_t* const* ins, int nin, uint64
   if ((rc = fill(din, (const uint64_t*)d_off, m, dout))) return rc;
   for (int k = 0; k < nv; ++k)
     WTG_CK(cudaMemcpyAsync(outs[k], dout[k], m * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  return sync_and_check(s, t.err.as<uint32_t>());
+  return sync_and_check(s, t.err);
 }
 
 void fill_select_info(const BvSupport& bv, int t_b, uint64_t info[8]) {
@@ -196,7 +197,7 @@ int wtg_tree_build(const void* seq, uint64_t n, int elem_bytes, int levels, uint
     if (ce != cudaSuccess) rc = cuda_fail(ce, "cudaMemcpyAsync(seq)");
   }
   if (rc == WTG_OK) rc = build_tree_common(T, t.seq.p, n, elem_bytes, levels, flags);
-  if (rc == WTG_OK) rc = sync_and_check(t.stream, t.err.as<uint32_t>());
+  if (rc == WTG_OK) rc = sync_and_check(t.stream, t.err);
   if (rc != WTG_OK) {
     if (fresh) wtg_tree_free(T);
     return rc;
@@ -272,7 +273,7 @@ int wtg_tree_build_out(const void* seq, uint64_t n, int elem_bytes, int levels, 
   t.host_bits = nullptr;
   t.host_rank = nullptr;
   t.in_pieces = 0;
-  if (rc == WTG_OK) rc = sync_and_check(t.stream, t.err.as<uint32_t>());
+  if (rc == WTG_OK) rc = sync_and_check(t.stream, t.err);
   if (rc == WTG_OK) {
     const cudaError_t ce = cudaStreamSynchronize(t.copy_stream);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "copies of the outputs");
@@ -318,7 +319,7 @@ int wtg_tree_build_device(const void* d_seq, uint64_t n, int elem_bytes, int lev
 
 int wtg_tree_sync(wtg_tree* T) {
   if (!T) return fail(WTG_ERR_INVALID, "null tree");
-  return sync_and_check(T->t.stream, T->t.err.as<uint32_t>());
+  return sync_and_check(T->t.stream, T->t.err);
 }
 
 int wtg_tree_free(wtg_tree* T) {
@@ -351,7 +352,7 @@ int wtg_tree_get_bits(wtg_tree* T, uint64_t* dst, uint64_t nwords) {
   if (!T || (!dst && nwords)) return fail(WTG_ERR_INVALID, "null argument");
   if (nwords != T->t.bit_words) return fail(WTG_ERR_INVALID, "nwords does not match the tree");
   if (nwords) WTG_CK(cudaMemcpyAsync(dst, T->t.bits.p, nwords * 8, cudaMemcpyDeviceToHost, T->t.stream));
-  return sync_and_check(T->t.stream, T->t.err.as<uint32_t>());
+  return sync_and_check(T->t.stream, T->t.err);
 }
 
 int wtg_tree_get_nodes(wtg_tree* T, int index_bytes, uint64_t n_entries, void* dst) {
@@ -363,7 +364,7 @@ int wtg_tree_get_nodes(wtg_tree* T, int index_bytes, uint64_t n_entries, void* d
   if ((rc = t.nodes.ensure(bytes, t.stream))) return rc;
   if ((rc = tree_nodes(t, index_bytes, n_entries, t.nodes.p))) return rc;
   if (bytes) WTG_CK(cudaMemcpyAsync(dst, t.nodes.p, bytes, cudaMemcpyDeviceToHost, t.stream));
-  return sync_and_check(t.stream, t.err.as<uint32_t>());
+  return sync_and_check(t.stream, t.err);
 }
 
 int wtg_tree_get_rank(wtg_tree* T, uint64_t* dst, uint64_t nwords) {
@@ -371,14 +372,14 @@ int wtg_tree_get_rank(wtg_tree* T, uint64_t* dst, uint64_t nwords) {
   if (!(T->t.flags & WTG_RANK)) return fail(WTG_ERR_INVALID, "rank support not built");
   if (nwords != rank_words_of(T->t.n * (uint64_t)T->t.levels)) return fail(WTG_ERR_INVALID, "nwords mismatch");
   WTG_CK(cudaMemcpyAsync(dst, T->t.bv.rank.p, nwords * 8, cudaMemcpyDeviceToHost, T->t.stream));
-  return sync_and_check(T->t.stream, T->t.err.as<uint32_t>());
+  return sync_and_check(T->t.stream, T->t.err);
 }
 
 int wtg_tree_get_select(wtg_tree* T, int t_b, uint64_t* sb_words, uint64_t* desc, uint64_t* pool) {
   if (!T || (t_b != 0 && t_b != 1)) return fail(WTG_ERR_INVALID, "bad argument");
   int rc = copy_select(T->t.bv, t_b, sb_words, desc, pool, T->t.stream);
   if (rc) return rc;
-  return sync_and_check(T->t.stream, T->t.err.as<uint32_t>());
+  return sync_and_check(T->t.stream, T->t.err);
 }
 
 int wtg_tree_device_ptrs(wtg_tree* T, uint64_t ptrs[8]) {
@@ -402,7 +403,7 @@ int wtg_query_access(wtg_tree* T, const uint64_t* idx, uint64_t nq, uint64_t* ou
   TreeImpl& t = T->t;
   const uint64_t* ins[1] = {idx};
   uint64_t* outs[1] = {out};
-  return host_query(t.qbuf, t.stream, ins, 1, nq, outs, 1, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 1, nq, outs, 1, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_wt_access(t, din[0], nq, dout[0], t.stream);
                     });
@@ -413,7 +414,7 @@ int wtg_query_rank(wtg_tree* T, const uint64_t* idx, const uint64_t* sym, uint64
   TreeImpl& t = T->t;
   const uint64_t* ins[2] = {idx, sym};
   uint64_t* outs[1] = {out};
-  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 1, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 1, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_wt_rank(t, din[0], din[1], nq, dout[0], t.stream);
                     });
@@ -424,7 +425,7 @@ int wtg_query_inverse_select(wtg_tree* T, const uint64_t* idx, uint64_t nq, uint
   TreeImpl& t = T->t;
   const uint64_t* ins[1] = {idx};
   uint64_t* outs[2] = {rank_out, sym_out};
-  return host_query(t.qbuf, t.stream, ins, 1, nq, outs, 2, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 1, nq, outs, 2, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_wt_inverse_select(t, din[0], nq, dout[0], dout[1], t.stream);
                     });
@@ -435,7 +436,7 @@ int wtg_query_select(wtg_tree* T, const uint64_t* i, const uint64_t* sym, uint64
   TreeImpl& t = T->t;
   const uint64_t* ins[2] = {i, sym};
   uint64_t* outs[1] = {out};
-  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 1, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 1, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_wt_select(t, din[0], din[1], nq, dout[0], t.stream);
                     });
@@ -461,7 +462,7 @@ int wtg_query_lex_count(wtg_tree* T, const uint64_t* i, const uint64_t* j, const
   TreeImpl& t = T->t;
   const uint64_t* ins[3] = {i, j, c};
   uint64_t* outs[3] = {rank_out, smaller_out, greater_out};
-  return host_query(t.qbuf, t.stream, ins, 3, nq, outs, 3, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 3, nq, outs, 3, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_wt_lex_count(t, din[0], din[1], din[2], nq, dout[0], dout[1], dout[2],
                                                  t.stream);
@@ -474,7 +475,7 @@ int wtg_query_lex_smaller_count(wtg_tree* T, const uint64_t* i, const uint64_t* 
   TreeImpl& t = T->t;
   const uint64_t* ins[2] = {i, c};
   uint64_t* outs[2] = {rank_out, smaller_out};
-  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 2, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 2, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_wt_lex_smaller_count(t, din[0], din[1], nq, dout[0], dout[1], t.stream);
                     });
@@ -533,7 +534,7 @@ int wtg_query_expand(wtg_tree* T, const uint64_t* nodes, uint64_t nn, uint64_t* 
   if ((rc = launch_wt_expand(t, d, nn, d + 4 * nn, d + 8 * nn, s))) return rc;
   WTG_CK(cudaMemcpyAsync(left, d + 4 * nn, 4 * nn * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   WTG_CK(cudaMemcpyAsync(right, d + 8 * nn, 4 * nn * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  return sync_and_check(s, t.err.as<uint32_t>());
+  return sync_and_check(s, t.err);
 }
 
 int wtg_query_expand_ranges(wtg_tree* T, const uint64_t v[4], const uint64_t* ranges, uint64_t nr, uint64_t* left,
@@ -549,7 +550,7 @@ int wtg_query_expand_ranges(wtg_tree* T, const uint64_t v[4], const uint64_t* ra
   if ((rc = launch_wt_expand_ranges(t, v[0], d, nr, d + 2 * nr, d + 4 * nr, s))) return rc;
   WTG_CK(cudaMemcpyAsync(left, d + 2 * nr, 2 * nr * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   WTG_CK(cudaMemcpyAsync(right, d + 4 * nr, 2 * nr * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  return sync_and_check(s, t.err.as<uint32_t>());
+  return sync_and_check(s, t.err);
 }
 
 int wtg_query_lex_count_device(wtg_tree* T, const uint64_t* d_i, const uint64_t* d_j, const uint64_t* d_c,
@@ -571,7 +572,8 @@ static int bv_common(wtg_bv* B, const uint64_t* d_words, uint64_t size, uint32_t
   int rc;
   if ((rc = B->err.ensure(sizeof(uint32_t), B->stream))) return rc;
   WTG_CK(cudaMemsetAsync(B->err.p, 0, sizeof(uint32_t), B->stream));
-  return bv_build(B->bv, d_words, size, flags, B->err.as<uint32_t>(), B->stream);
+  B->err.elsewhere = false;
+  return bv_build(B->bv, d_words, size, flags, B->err.arm(B->stream, B->stream), B->stream);
 }
 
 int wtg_bv_build(const uint64_t* words, uint64_t size_bits, uint32_t flags, wtg_bv** out) {
@@ -597,7 +599,7 @@ int wtg_bv_build(const uint64_t* words, uint64_t size_bits, uint32_t flags, wtg_
     if (ce != cudaSuccess) rc = cuda_fail(ce, "copy bitvector");
   }
   if (rc == WTG_OK) rc = bv_common(B, B->words.as<uint64_t>(), size_bits, flags);
-  if (rc == WTG_OK) rc = sync_and_check(B->stream, B->err.as<uint32_t>());
+  if (rc == WTG_OK) rc = sync_and_check(B->stream, B->err);
   if (rc != WTG_OK) {
     wtg_bv_free(B);
     return rc;
@@ -631,7 +633,7 @@ int wtg_bv_build_device(const uint64_t* d_words, uint64_t size_bits, uint32_t fl
 
 int wtg_bv_sync(wtg_bv* B) {
   if (!B) return fail(WTG_ERR_INVALID, "null bitvector");
-  return sync_and_check(B->stream, B->err.as<uint32_t>());
+  return sync_and_check(B->stream, B->err);
 }
 
 int wtg_bv_free(wtg_bv* B) {
@@ -658,7 +660,7 @@ int wtg_bv_get_rank(wtg_bv* B, uint64_t* dst, uint64_t nwords) {
   if (!(B->bv.flags & WTG_RANK)) return fail(WTG_ERR_INVALID, "rank support not built");
   if (nwords != rank_words_of(B->bv.size)) return fail(WTG_ERR_INVALID, "nwords mismatch");
   WTG_CK(cudaMemcpyAsync(dst, B->bv.rank.p, nwords * 8, cudaMemcpyDeviceToHost, B->stream));
-  return sync_and_check(B->stream, B->err.as<uint32_t>());
+  return sync_and_check(B->stream, B->err);
 }
 
 int wtg_bv_select_info(wtg_bv* B, int t_b, uint64_t info[8]) {
@@ -672,14 +674,14 @@ int wtg_bv_get_select(wtg_bv* B, int t_b, uint64_t* sb_words, uint64_t* desc, ui
   if (!B || (t_b != 0 && t_b != 1)) return fail(WTG_ERR_INVALID, "bad argument");
   int rc = copy_select(B->bv, t_b, sb_words, desc, pool, B->stream);
   if (rc) return rc;
-  return sync_and_check(B->stream, B->err.as<uint32_t>());
+  return sync_and_check(B->stream, B->err);
 }
 
 int wtg_bv_rank(wtg_bv* B, const uint64_t* idx, uint64_t nq, uint64_t* out) {
   if (!B || (nq && (!idx || !out))) return fail(WTG_ERR_INVALID, "null argument");
   const uint64_t* ins[1] = {idx};
   uint64_t* outs[1] = {out};
-  return host_query(B->qbuf, B->stream, ins, 1, nq, outs, 1, B->err.as<uint32_t>(),
+  return host_query(B->qbuf, B->stream, ins, 1, nq, outs, 1, B->err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_bv_rank(B->bv, din[0], nq, dout[0], B->stream);
                     });
@@ -689,7 +691,7 @@ int wtg_bv_select(wtg_bv* B, int t_b, const uint64_t* i, uint64_t nq, uint64_t* 
   if (!B || (t_b != 0 && t_b != 1) || (nq && (!i || !out))) return fail(WTG_ERR_INVALID, "bad argument");
   const uint64_t* ins[1] = {i};
   uint64_t* outs[1] = {out};
-  return host_query(B->qbuf, B->stream, ins, 1, nq, outs, 1, B->err.as<uint32_t>(),
+  return host_query(B->qbuf, B->stream, ins, 1, nq, outs, 1, B->err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_bv_select(B->bv, t_b, din[0], nq, dout[0], B->stream);
                     });
@@ -778,7 +780,7 @@ int wtg_fm_count(wtg_tree* T, const uint64_t* C, uint64_t sigma, const uint8_t* 
   if (total) WTG_CK(cudaMemcpyAsync(dPat, pat, total, cudaMemcpyHostToDevice, s));
   if ((rc = launch_fm_count(t, dC, sigma, dPat, dOff, npat, dOut, s))) return rc;
   WTG_CK(cudaMemcpyAsync(out, dOut, npat * 8, cudaMemcpyDeviceToHost, s));
-  return sync_and_check(s, t.err.as<uint32_t>());
+  return sync_and_check(s, t.err);
 }
 
 int wtg_fm_count_device(wtg_tree* T, const uint64_t* d_C, uint64_t sigma, const uint8_t* d_pat,
@@ -795,7 +797,7 @@ int wtg_tree_level_select(wtg_tree* T, int t_b, const uint64_t* level, const uin
   TreeImpl& t = T->t;
   const uint64_t* ins[2] = {level, k};
   uint64_t* outs[1] = {out};
-  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 1, t.err.as<uint32_t>(),
+  return host_query(t.qbuf, t.stream, ins, 2, nq, outs, 1, t.err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_level_select(t, t_b, din[0], din[1], nq, dout[0], t.stream);
                     });
@@ -822,7 +824,7 @@ int wtg_lsel_build(wtg_tree* T, uint32_t segments, uint32_t samples, uint32_t ma
     fresh = true;
   }
   rc = lsel_build(*M->m, T->t, segments, samples, max_window, T->t.stream);
-  if (rc == WTG_OK) rc = sync_and_check(T->t.stream, T->t.err.as<uint32_t>());
+  if (rc == WTG_OK) rc = sync_and_check(T->t.stream, T->t.err);
   if (rc != WTG_OK) {
     if (fresh) wtg_lsel_free(M);
     return rc;
@@ -858,7 +860,7 @@ int wtg_lsel_query(wtg_lsel* M, int t_b, const uint64_t* level, const uint64_t* 
   if (!t) return fail(WTG_ERR_INVALID, "the index's tree was freed");
   const uint64_t* ins[2] = {level, k};
   uint64_t* outs[1] = {out};
-  return host_query(M->qbuf, t->stream, ins, 2, nq, outs, 1, t->err.as<uint32_t>(),
+  return host_query(M->qbuf, t->stream, ins, 2, nq, outs, 1, t->err,
                     [&](const uint64_t** din, uint64_t** dout) {
                       return launch_lsel_query(*M->m, t_b, din[0], din[1], nq, dout[0], t->stream);
                     });
@@ -1170,21 +1172,21 @@ int wtg_tree_serialize(wtg_tree* T, void* dst, uint64_t cap, uint64_t* len) {
   if (!T || !len) return fail(WTG_ERR_INVALID, "null argument");
   int rc = tree_serialize(T->t, (uint8_t*)dst, cap, len);
   if (rc) return rc;
-  return dst ? sync_and_check(T->t.stream, T->t.err.as<uint32_t>()) : WTG_OK;
+  return dst ? sync_and_check(T->t.stream, T->t.err) : WTG_OK;
 }
 
 int wtg_tree_sigma(wtg_tree* T, uint64_t* sigma) {
   if (!T || !sigma) return fail(WTG_ERR_INVALID, "null argument");
   int rc = tree_leaf_count(T->t, sigma, T->t.stream);
   if (rc) return rc;
-  return sync_and_check(T->t.stream, T->t.err.as<uint32_t>());
+  return sync_and_check(T->t.stream, T->t.err);
 }
 
 int wtg_bv_serialize(wtg_bv* B, uint32_t part, void* dst, uint64_t cap, uint64_t* len) {
   if (!B || !len) return fail(WTG_ERR_INVALID, "null argument");
   int rc = bv_serialize(B->bv, part, (uint8_t*)dst, cap, len, B->stream);
   if (rc) return rc;
-  return dst ? sync_and_check(B->stream, B->err.as<uint32_t>()) : WTG_OK;
+  return dst ? sync_and_check(B->stream, B->err) : WTG_OK;
 }
 
 // ------------------------------------------------ failure handling knobs
@@ -1227,7 +1229,8 @@ int wtg_remap_alphabet(void* seq, uint64_t n, int elem_bytes, uint64_t* sigma_ou
   if ((rc = check_device())) return rc;
   cudaStream_t s;
   WTG_CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  DevBuf d, tmp, scan_tmp, err;
+  DevBuf d, tmp, scan_tmp;
+  ErrWord err;
   rc = d.ensure(n * elem_bytes, s);
   if (!rc) rc = err.ensure(sizeof(uint32_t), s);
   if (!rc) {
@@ -1235,12 +1238,12 @@ int wtg_remap_alphabet(void* seq, uint64_t n, int elem_bytes, uint64_t* sigma_ou
     if (ce == cudaSuccess && n) ce = cudaMemcpyAsync(d.p, seq, n * elem_bytes, cudaMemcpyHostToDevice, s);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "copy sequence");
   }
-  if (!rc) rc = remap_alphabet_device(d.p, n, elem_bytes, sigma_out, tmp, scan_tmp, err.as<uint32_t>(), s);
+  if (!rc) rc = remap_alphabet_device(d.p, n, elem_bytes, sigma_out, tmp, scan_tmp, err.arm(s, s), s);
   if (!rc && n) {
     cudaError_t ce = cudaMemcpyAsync(seq, d.p, n * elem_bytes, cudaMemcpyDeviceToHost, s);
     if (ce != cudaSuccess) rc = cuda_fail(ce, "copy sequence back");
   }
-  if (!rc) rc = sync_and_check(s, err.as<uint32_t>());
+  if (!rc) rc = sync_and_check(s, err);
   d.release(s);
   tmp.release(s);
   scan_tmp.release(s);

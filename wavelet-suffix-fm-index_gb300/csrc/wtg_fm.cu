@@ -184,7 +184,7 @@ int fm_run(TreeImpl& t, const uint4* blocks, uint64_t sigma, const uint8_t* pat,
         return WTG_OK;
       },
       [&](int K, const uint2* table) -> int {
-        return by_length(off, npat, t.err.as<uint32_t>(), s,
+        return by_length(off, npat, t.err.arm(s, t.stream), s,
                          [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
                            auto* const f = sorted ? fm_count_kernel<BLOCKS, true> : fm_count_kernel<BLOCKS, false>;
                            f<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(v, K, table, pat, off + at, off + npat, o, m,

@@ -79,7 +79,8 @@ struct HuffImpl {
   uint64_t path[256] = {0};
   int len[256] = {0};
   int leaf[256];
-  DevBuf text, seq[2], bits, chunkz, chunkpre, scan_tmp, err, hist, dnodes, dpath, dnode_at, nbase, ids, qbuf, fminfo, fmsteps;
+  DevBuf text, seq[2], bits, chunkz, chunkpre, scan_tmp, hist, dnodes, dpath, dnode_at, nbase, ids, qbuf, fminfo, fmsteps;
+  ErrWord err;
   DevBuf groups, cnode, status;  // the groups' tables, the chunks' nodes, look-back words
   uint32_t fm_steps = 0;  // steps of all codes (fm counting)
   BvSupport bv;
@@ -718,7 +719,8 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
   h.flags = flags;
   if ((rc = h.err.ensure(sizeof(uint32_t), s))) return rc;
   WTG_CK(cudaMemsetAsync(h.err.p, 0, sizeof(uint32_t), s));
-  uint32_t* d_err = h.err.as<uint32_t>();
+  h.err.elsewhere = false;
+  uint32_t* d_err = h.err.arm(s, s);
   // histogram -> shape (host)
   if ((rc = h.hist.ensure(256 * sizeof(uint64_t), s))) return rc;
   WTG_CK(cudaMemsetAsync(h.hist.p, 0, 256 * sizeof(uint64_t), s));
@@ -885,7 +887,7 @@ BvSupport& huff_bv(HuffImpl& h) { return h.bv; }
 const uint64_t* huff_bits(const HuffImpl& h) { return h.bits.as<uint64_t>(); }
 DevBuf& huff_text(HuffImpl& h) { return h.text; }
 DevBuf& huff_qbuf(HuffImpl& h) { return h.qbuf; }
-const uint32_t* huff_err(const HuffImpl& h) { return h.err.as<uint32_t>(); }
+ErrWord& huff_err(HuffImpl& h) { return h.err; }
 void huff_set_stream(HuffImpl& h, cudaStream_t s, bool own) {
   h.stream = s;
   h.own_stream = own;
@@ -944,7 +946,7 @@ static int huff_fm_run(HuffImpl& h, const uint4* blocks, const uint64_t* C, cons
         return WTG_OK;
       },
       [&](int K, const uint2* table) -> int {
-        return by_length(off, npat, h.err.as<uint32_t>(), s,
+        return by_length(off, npat, h.err.arm(s, h.stream), s,
                          [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
                            auto* const f = sorted ? huff_count_kernel<BLOCKS, true> : huff_count_kernel<BLOCKS, false>;
                            f<<<(unsigned)((m + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(

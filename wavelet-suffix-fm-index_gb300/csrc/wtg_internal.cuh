@@ -353,6 +353,38 @@ struct DevBuf {
   T* as() const { return (T*)p; }
 };
 
+// A part of a DevBuf, which owns it.
+struct DevPart {
+  void* p = nullptr;
+  template <typename T>
+  T* as() const { return (T*)p; }
+};
+
+// Lays parts out one after the other, each on a 256-byte boundary: one
+// allocation for what a build needs (an allocation is 2.3-3.6 us of host time,
+// its release 0.7, and a small build is mostly host time).
+struct DevLayout {
+  size_t bytes = 0;
+  size_t add(size_t n) {
+    const size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  }
+};
+
+// A handle's device error word.  Reading it costs 13 us, so it is read only
+// when a kernel that can set it was launched since it was last found clear: on
+// the handle's own stream, the check after the next wait covers the launch;
+// on another stream nothing does, and every later check reads it.
+struct ErrWord : DevBuf {
+  bool pending = false, elsewhere = false;
+  uint32_t* arm(cudaStream_t s, cudaStream_t own) {
+    pending = true;
+    if (s != own) elsewhere = true;
+    return as<uint32_t>();
+  }
+};
+
 int scan_exclusive_u32(const uint32_t* in, uint32_t* out, uint64_t n, DevBuf& scratch, uint32_t* d_err,
                        cudaStream_t s);
 int scan_exclusive_u64(const uint64_t* in, uint64_t* out, uint64_t n, DevBuf& scratch, uint32_t* d_err,
@@ -367,13 +399,14 @@ int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8
 // Flat select_support_mcl on the device.
 struct SelectDev {
   uint64_t arg_cnt = 0, nsb = 0, logn = 0, logn4 = 0, has_long = 0, sb_nwords = 0, pool_nwords = 0;
-  DevBuf ends;      // superblock end positions (upper-bound sized)
-  DevBuf starts;    // superblock start positions (upper-bound sized)
-  DevBuf desc;      // per superblock descriptor
-  DevBuf offs;      // per superblock pool word offset
+  // parts of BvSupport::work
+  DevPart ends;      // superblock end positions (upper-bound sized)
+  DevPart starts;    // superblock start positions (upper-bound sized)
+  DevPart desc;      // per superblock descriptor [final | working]
+  DevPart offs;      // per superblock pool word offset
+  DevPart long_list; // superblock ids of long blocks
   DevBuf sb_words;  // packed m_superblock
   DevBuf pool;      // packed mini/long blocks
-  DevBuf long_list; // superblock ids of long blocks
   DevBuf long_ent;  // 4096 unpacked positions per long block
 };
 
@@ -383,10 +416,11 @@ struct BvSupport {
   const uint64_t* words = nullptr;  // device
   uint32_t flags = 0;
   DevBuf rank;       // rank_support_v table
-  DevBuf samples;    // every 64th arg, low 32 bits: select1 from the front, select0 from the back
-  DevBuf info;       // device scalars (see bitvec.cu)
-  DevBuf status;     // look-back status words + tile counter
-  DevBuf scan_tmp;
+  DevBuf work;       // what follows, and the per-superblock arrays of sel
+  DevPart info;      // device scalars (see bitvec.cu)
+  DevPart status;    // look-back status words + tile counter
+  DevPart scan_tmp;  // the same for the descriptors' scan
+  DevPart samples;   // every 64th arg, low 32 bits: select1 from the front, select0 from the back
   SelectDev sel[2];  // [t_b]
   // the pass over the bits: superblocks per thread, tiles, tiles launched so far
   int spt = 1;
@@ -395,12 +429,11 @@ struct BvSupport {
 
 int bv_build(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t flags, uint32_t* d_err,
              cudaStream_t s);
-// the same in steps: allocate and clear; start the pass over the bits; run it
+// the same in steps: allocate and clear; run the pass over the bits
 // over the tiles that lie within the first bits_ready bits (in one call, or in
 // several as the bits become final: the whole vector with bits_ready >= size);
 // the select structures' finishing kernels
 int bv_prepare(BvSupport& bv, const uint64_t* d_words, uint64_t size, uint32_t& flags, cudaStream_t s);
-int bv_pass_begin(BvSupport& bv, cudaStream_t s);
 int bv_pass_to(BvSupport& bv, uint64_t bits_ready, uint32_t* d_err, cudaStream_t s);
 int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s);
 // superblocks whose rank entries the launched passes write

@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(LV_THREADS)
     const uint32_t za = __shfl_sync(0xffffffffu, pz, a), zb = __shfl_sync(0xffffffffu, pz, b & 31);
     const uint64_t h = (nodes << j) - 1 + (p << j) + q;
     if (in) {
-      if (j) C[h] = ca;  // (the node's own start is there)
+      if (j || !l) C[h] = ca;  // (below the root the node's own start is there)
       if (j < TB) Z[h] = mid - ca;
     }
     // digit d's scatter base goes to lane 16 + d

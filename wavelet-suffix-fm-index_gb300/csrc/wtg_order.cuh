@@ -98,7 +98,7 @@ int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F la
   constexpr int passes = 2;
   const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
   return sorted_batches(
-      nq, bits > 8 * passes ? bits - 8 * passes : 0, passes, t.err.as<uint32_t>(), s,
+      nq, bits > 8 * passes ? bits - 8 * passes : 0, passes, t.err.arm(s, t.stream), s,
       [&](uint64_t at, uint64_t m, uint32_t* key) {
         order_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(pos + at, m, t.n, key);
       },

@@ -10,13 +10,14 @@ struct LselImpl;
 
 // Device memory layout of one tree (all stream-ordered, reused across rebuilds):
 //   seq        the input copied from the host (host-input builds only)
-//   lvl[0..1]  ping-pong buffers of the level orders, n symbols each
 //   bits       ceil(n*L/64) words of level bits + 2 zero words
 //   zeros      [Z | C]: left-child size and start per heap node (2 x 2^L x u32)
-//   chunkpre   per 1024-symbol chunk the digit counts before it (16 x u32)
-//   cnode      per chunk the node of its first symbol
-//   rec        per node of a group's first level its bases (32 x u32)
-//   status     per group of levels: tile counter + look-back status words
+//   work       of the build: per 1024-symbol chunk the digit counts before it
+//              (16 x u32) and the node of its first symbol; per node of a
+//              group's first level its bases (32 x u32); the level orders
+//              between the groups (two buffers)
+//   err        the error word, then per group of levels a tile counter and
+//              look-back status words
 //   bv         rank/select supports over `bits`
 //   lvl_args   ones before each level start, L + 1 words (filled on first use
 //              after a build by tree_level_args)
@@ -28,7 +29,8 @@ struct TreeImpl {
   uint64_t bit_words = 0;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
-  DevBuf seq, lvl[2], bits, zeros, chunkpre, cnode, rec, status, scan_tmp, err, scratch, nodes, qbuf, qout;
+  DevBuf seq, bits, zeros, work, scan_tmp, scratch, nodes, qbuf, qout;
+  ErrWord err;  // followed by the status words of the build
   BvSupport bv;
   DevBuf lvl_args;
   bool lvl_args_ok = false;
@@ -164,7 +166,7 @@ BvSupport& huff_bv(HuffImpl& h);
 const uint64_t* huff_bits(const HuffImpl& h);
 DevBuf& huff_text(HuffImpl& h);
 DevBuf& huff_qbuf(HuffImpl& h);
-const uint32_t* huff_err(const HuffImpl& h);
+ErrWord& huff_err(HuffImpl& h);
 // what: 0 access, 1 rank(a, b), 2 select(a, b), 3 inverse_select (out, out2)
 int launch_huff_query(HuffImpl& h, int what, const uint64_t* a, const uint64_t* b, uint64_t nq, uint64_t* out,
                       uint64_t* out2, cudaStream_t s);
