@@ -8,7 +8,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-NPAT, SMALL = (1 << 17) + 9, 1 << 12
+NPAT, SMALL = (1 << 19) + 9, 1 << 13
 
 
 def _setup(wtg, torch, sigma, n, seed):

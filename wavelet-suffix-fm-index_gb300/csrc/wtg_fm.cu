@@ -70,7 +70,10 @@ struct FmTree {
   const uint2* steps;
   uint64_t n, sigma;
   int L;
-  // ones before the positions px <= py; what they share is read once
+  // ones before the positions px <= py.  SHARE: what they share is read once,
+  // for batches bound by their reads; a small batch waits for its reads, and
+  // the second would wait for the first (2^14 patterns: 58 us against 67)
+  template <bool SHARE>
   __device__ __forceinline__ void ranks(uint64_t px, uint64_t py, uint32_t& rx, uint32_t& ry) const {
     if constexpr (BLOCKS) {
       uint32_t ox, oy;
@@ -84,21 +87,29 @@ struct FmTree {
       const ulonglong2* __restrict__ re = reinterpret_cast<const ulonglong2*>(rt);
       const ulonglong2 ex = __ldg(re + (px >> 9));
       const uint64_t wx = __ldg(tree + (px >> 6));
-      ulonglong2 ey = ex;
-      uint64_t wy = wx;
-      if ((px ^ py) >> 9) ey = __ldg(re + (py >> 9));
-      if ((px ^ py) >> 6) wy = __ldg(tree + (py >> 6));
+      ulonglong2 ey;
+      uint64_t wy;
+      if constexpr (SHARE) {
+        ey = ex;
+        wy = wx;
+        if ((px ^ py) >> 9) ey = __ldg(re + (py >> 9));
+        if ((px ^ py) >> 6) wy = __ldg(tree + (py >> 6));
+      } else {
+        ey = __ldg(re + (py >> 9));
+        wy = __ldg(tree + (py >> 6));
+      }
       rx = fm_rank(ex, wx, px);
       ry = fm_rank(ey, wy, py);
     }
   }
   // prepends symbol c (< sigma) to the interval [x, y)
+  template <bool SHARE>
   __device__ __forceinline__ void step(const uint2* __restrict__ st, uint32_t c, uint32_t& x, uint32_t& y) const {
     uint64_t lbase = 0;
     for (int l = 0; l < L; ++l, lbase += n) {
       const uint2 s = st[c * L + l];
       uint32_t rx, ry;
-      ranks(lbase + x, lbase + y, rx, ry);
+      ranks<SHARE>(lbase + x, lbase + y, rx, ry);
       const bool one = (c >> (L - 1 - l)) & 1;
       x = one ? s.y + rx : s.x + x - rx;
       y = one ? s.y + ry : s.x + y - ry;
@@ -116,7 +127,7 @@ __global__ void fm_table_kernel(FmTree<BLOCKS> t, uint64_t prev_count, const uin
   const uint32_t c = (uint32_t)(i / prev_count);
   const uint2 v = prev ? prev[i - c * prev_count] : make_uint2(0u, (uint32_t)t.n);
   uint32_t x = v.x, y = v.y;
-  if (x < y) t.step(t.steps, c, x, y);
+  if (x < y) t.template step<true>(t.steps, c, x, y);
   out[i] = x < y ? make_uint2(x, y) : make_uint2(0u, 0u);
 }
 
@@ -165,7 +176,7 @@ __global__ void __launch_bounds__(256, 6)
   while (known && i > a && x < y) {
     const uint32_t c = rd.at(--i);
     known = c < t.sigma;
-    if (known) t.step(st, c, x, y);
+    if (known) t.template step<ORD>(st, c, x, y);
   }
   out[p] = known && y > x ? y - x : 0;
 }
@@ -175,8 +186,9 @@ int fm_run(TreeImpl& t, const uint4* blocks, uint64_t sigma, const uint8_t* pat,
            uint64_t* out, cudaStream_t s) {
   const FmTree<BLOCKS> v{t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), blocks, t.fm_paths.as<uint2>(), t.n, sigma,
                          t.levels};
+  const bool pays = fm_batch_pays(npat, t.levels);
   return with_fm_table<uint2>(
-      sigma, npat, s,
+      pays, sigma, npat, s,
       [&](uint64_t prev_count, const uint2* prev, uint2* next) -> int {
         fm_table_kernel<BLOCKS><<<(unsigned)((prev_count * sigma + 127) / 128), 128, 0, s>>>(v, prev_count, prev, next);
         count_launch();
@@ -184,7 +196,7 @@ int fm_run(TreeImpl& t, const uint4* blocks, uint64_t sigma, const uint8_t* pat,
         return WTG_OK;
       },
       [&](int K, const uint2* table) -> int {
-        return by_length(off, npat, t.err.arm(s, t.stream), s,
+        return by_length(pays, off, npat, pays ? t.err.arm(s, t.stream) : nullptr, s,
                          [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
                            auto* const f = sorted ? fm_count_kernel<BLOCKS, true> : fm_count_kernel<BLOCKS, false>;
                            f<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(v, K, table, pat, off + at, off + npat, o, m,
@@ -213,8 +225,9 @@ int launch_fm_count(TreeImpl& t, const uint64_t* C, uint64_t sigma, const uint8_
   // blocks pay once the batch probes a good part of them: making them is a
   // read and write of the bits (35 us for 8e8 bits), a probe saves a sector
   const uint64_t size = t.n * (uint64_t)t.levels;
-  uint4* blocks = npat >= block_count(size) / 8 ? make_blocks(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), size, s)
-                                                : nullptr;
+  uint4* blocks = fm_batch_pays(npat, t.levels) && npat >= block_count(size) / 8
+                      ? make_blocks(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), size, s)
+                      : nullptr;
   rc = blocks ? fm_run<true>(t, blocks, sigma, pat, off, npat, out, s)
               : fm_run<false>(t, blocks, sigma, pat, off, npat, out, s);
   if (blocks) cudaFreeAsync(blocks, s);

@@ -26,12 +26,18 @@ struct PatternReader {
   }
 };
 
+// Whether a batch of npat patterns over `levels` levels a symbol is worth the
+// launches that prepare it (blocks, the table's K, the sort by length: 50 to 90
+// us).  Counts of 20 symbols over 2^20 to 2^26 symbols, us without / with: 3
+// levels, 2^17 patterns 101-117 / 134-150, 2^18 168-205 / 164-181; 8 levels,
+// 2^16 200-273 / 183-272, 2^17 338-416 / 210-333.
+inline bool fm_batch_pays(uint64_t npat, uint64_t levels) { return npat * levels >= (3ull << 18); }
+
 // Symbols K of the interval table for a batch: all strings of K symbols have
 // at most a quarter of the batch's patterns and 2^19 entries (4 MB of 8-byte
-// intervals, a few percent of L2), and the batch is large enough for the K
-// launches (2^24 patterns of 20 symbols over 6 symbols: K = 7, 0.1 ms).
+// intervals, a few percent of L2).
 inline int fm_table_symbols(uint64_t sigma, uint64_t npat) {
-  if (npat < (1ull << 16) || sigma < 2) return 0;
+  if (sigma < 2) return 0;
   int K = 0;
   for (uint64_t count = sigma; count <= npat / 4 && count <= (1ull << 19) && K < 19; count *= sigma) ++K;
   return K;
@@ -40,8 +46,8 @@ inline int fm_table_symbols(uint64_t sigma, uint64_t npat) {
 // Makes the table (V: an interval) and calls count(K, table); without room
 // for it, or where it does not pay, count(0, nullptr).
 template <typename V, typename MakeF, typename CountF>
-int with_fm_table(uint64_t sigma, uint64_t npat, cudaStream_t s, MakeF make, CountF count) {
-  const int K = fm_table_symbols(sigma, npat);
+int with_fm_table(bool pays, uint64_t sigma, uint64_t npat, cudaStream_t s, MakeF make, CountF count) {
+  const int K = pays ? fm_table_symbols(sigma, npat) : 0;
   if (!K) return count(0, (const V*)nullptr);
   uint64_t entries = 1;
   for (int k = 0; k < K; ++k) entries *= sigma;

@@ -930,14 +930,20 @@ int launch_huff_query(HuffImpl& h, int what, const uint64_t* a, const uint64_t* 
   return WTG_OK;
 }
 
+// (levels: the bits of a code on average)
+static bool huff_batch_pays(const HuffImpl& h, uint64_t npat) {
+  return fm_batch_pays(npat, (h.size + h.n - 1) / h.n);
+}
+
 template <bool BLOCKS>
 static int huff_fm_run(HuffImpl& h, const uint4* blocks, const uint64_t* C, const uint8_t* pat, const uint64_t* off,
                        uint64_t npat, uint64_t* out, cudaStream_t s) {
   const HuffFm<BLOCKS> v{h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), blocks, h.fminfo.as<HuffFmInfo>(),
                          h.fmsteps.as<uint2>(), C, (uint32_t)h.n, (uint32_t)h.sigma};
   const uint32_t in_smem = h.fm_steps <= (uint32_t)HF_SMEM_STEPS ? h.fm_steps : 0u;
+  const bool pays = huff_batch_pays(h, npat);
   return with_fm_table<uint2>(
-      h.sigma, npat, s,
+      pays, h.sigma, npat, s,
       [&](uint64_t prev_count, const uint2* prev, uint2* next) -> int {
         huff_table_kernel<BLOCKS><<<(unsigned)((prev_count * h.sigma + 127) / 128), 128, 0, s>>>(v, prev_count, prev,
                                                                                                 next);
@@ -946,7 +952,7 @@ static int huff_fm_run(HuffImpl& h, const uint4* blocks, const uint64_t* C, cons
         return WTG_OK;
       },
       [&](int K, const uint2* table) -> int {
-        return by_length(off, npat, h.err.arm(s, h.stream), s,
+        return by_length(pays, off, npat, pays ? h.err.arm(s, h.stream) : nullptr, s,
                          [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
                            auto* const f = sorted ? huff_count_kernel<BLOCKS, true> : huff_count_kernel<BLOCKS, false>;
                            f<<<(unsigned)((m + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(
@@ -974,7 +980,7 @@ int launch_huff_fm_count(HuffImpl& h, const uint64_t* C, const uint8_t* pat, con
   count_launch();
   WTG_CK(cudaGetLastError());
   // as for the balanced tree: blocks once the batch probes a good part of them
-  uint4* blocks = h.size && npat >= block_count(h.size) / 8
+  uint4* blocks = h.size && huff_batch_pays(h, npat) && npat >= block_count(h.size) / 8
                       ? make_blocks(h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), h.size, s)
                       : nullptr;
   rc = blocks ? huff_fm_run<true>(h, blocks, C, pat, off, npat, out, s)

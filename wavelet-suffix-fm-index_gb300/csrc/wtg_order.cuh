@@ -40,18 +40,26 @@ static __global__ void __launch_bounds__(256)
   }
 }
 
-// When sorting pays: the tree is larger than what L2 keeps of it (its bits
-// from about 100 MB on, with the rank table 125 MB), has enough levels to
-// make up for the sort and for reading the other arguments by query number,
-// and the batch is large enough.  Measured (ms as they come / sorted):
-// access, 2^30 x 20 levels, 2^26 queries 47.0 / 14.3, 2^20 queries 0.81 / 0.50,
-// 2^19 0.40 / 0.34; rank, 2^27 x 8, 2^24 queries 1.94 / 1.36; but 2^26 x 8
-// 0.92 / 1.36 and 2^28 x 3 0.61 / 1.23.  Trees that L2 holds gain only by
-// the sectors that neighbours share, over many levels: 2^24 x 20, 2^22
-// queries 0.60 / 0.45, 2^20 queries 0.16 / 0.16; 2^25 x 12 0.35 / 0.39.
-inline bool order_pays(const TreeImpl& t, uint64_t nq) {
+// what L2 keeps of a tree: its bits from about 100 MB on (with the rank table 125 MB)
+inline bool larger_than_l2(const TreeImpl& t) { return t.n * (uint64_t)t.levels / 8 >= (100ull << 20); }
+
+// When sorting pays: the tree is larger than what L2 keeps of it, has enough
+// levels to make up for the sort (60 us, then 10 % of the time) and for reading
+// the other arguments by query number, and the batch is large enough.
+// Measured, ms as they come / sorted, 2^28 symbols: 20 levels, access of 2^18.5
+// queries 0.206 / 0.167, 2^20 0.651 / 0.230, rank 0.155 / 0.167, 0.438 / 0.241;
+// 12 levels, access of 2^18.5 0.112 / 0.119, 2^19 0.164 / 0.127, rank 0.111 /
+// 0.130; 8 levels, access of 2^19 0.098 / 0.101, 2^19.5 0.141 / 0.110; 3
+// levels, 2^24 queries 0.61 / 1.23.  Just above L2 (45 M x 20, 112 MB) access
+// of 2^19 0.110 / 0.108, 2^19.5 0.160 / 0.130, rank 0.107 / 0.111, 0.150 /
+// 0.134.  Trees that L2 holds gain only by the sectors that neighbours share,
+// over many levels: 2^24 x 20, 2^22 queries 0.60 / 0.45, 2^20 queries 0.16 /
+// 0.16; 2^25 x 12 0.35 / 0.39.
+// Two positions a query (lex_count, range_count) gain from fewer on.
+inline bool order_pays(const TreeImpl& t, uint64_t nq, bool two = false) {
   const uint64_t bytes = t.n * (uint64_t)t.levels / 8;
-  if (bytes >= (100ull << 20)) return t.levels >= 6 && nq >= (1ull << 20);
+  if (bytes >= (256ull << 20)) return t.levels >= 6 && nq * t.levels >= (two ? 5ull : 7ull) << 20;
+  if (larger_than_l2(t)) return t.levels >= 6 && nq >= (5ull << 17);
   return bytes >= (20ull << 20) && t.levels >= 16 && nq >= (1ull << 21);
 }
 
@@ -93,8 +101,8 @@ int sorted_batches(uint64_t nq, int lo, int passes, uint32_t* d_err, cudaStream_
 // Calls launch(sorted, order, first query, queries) over the batch: sorted by
 // position where that pays, otherwise once over all queries as they come.
 template <typename F>
-int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch) {
-  if (!order_pays(t, nq)) return launch(false, QueryOrder{}, 0, nq);
+int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch, bool two = false) {
+  if (!order_pays(t, nq, two)) return launch(false, QueryOrder{}, 0, nq);
   constexpr int passes = 2;
   const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
   return sorted_batches(
@@ -105,12 +113,12 @@ int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F la
       launch);
 }
 
-// Patterns by length (one sort pass), from 2^16 of them on: a warp runs as
-// long as its longest pattern, and lengths of 8 to 32 left 48 % of the lanes
+// Patterns by length (one sort pass), in batches that are worth it: a warp runs
+// as long as its longest pattern, and lengths of 8 to 32 left 48 % of the lanes
 // without work.
 template <typename F>
-int by_length(const uint64_t* off, uint64_t npat, uint32_t* d_err, cudaStream_t s, F launch) {
-  if (npat < (1ull << 16)) return launch(false, QueryOrder{}, 0, npat);
+int by_length(bool pays, const uint64_t* off, uint64_t npat, uint32_t* d_err, cudaStream_t s, F launch) {
+  if (!pays) return launch(false, QueryOrder{}, 0, npat);
   return sorted_batches(
       npat, 0, 1, d_err, s,
       [&](uint64_t at, uint64_t m, uint32_t* key) {

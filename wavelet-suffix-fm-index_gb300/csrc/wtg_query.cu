@@ -25,6 +25,7 @@ __device__ __forceinline__ int bit_at(const uint64_t* __restrict__ w, uint64_t p
 //          (rank1 of the concatenated bits), bit 0 goes on at step.x + x - R
 //          and bit 1 at step.y + R, positions inside the next level; after
 //          the last level the position inside the leaf.  All modulo 2^32.
+//          Node h at step[h + 1], so that the children lie in one 16 bytes.
 // With step, a query level costs one rank entry, one word and 8 bytes of a
 // table that is read beside them; tab took two 16-byte entries a level.
 __global__ void node_table_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
@@ -38,16 +39,7 @@ __global__ void node_table_kernel(const uint64_t* __restrict__ tree, const uint6
   const uint64_t y = rank1_dev(rt, tree, off);
   tab[h] = make_ulonglong2(off, y);
   const uint32_t Y = (uint32_t)y;
-  step[h] = (int)l + 1 < L ? make_uint2(Y, c + Z[h] - Y) : make_uint2(Y - c, 0u - Y);
-}
-
-// ones before bit pos (mod 2^32), and the word holding pos
-__device__ __forceinline__ uint32_t rank_step(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                                              uint64_t pos, uint64_t& word) {
-  const ulonglong2 e = __ldg(reinterpret_cast<const ulonglong2*>(rt) + (pos >> 9));
-  word = __ldg(tree + (pos >> 6));
-  const uint32_t in = (uint32_t)(e.y >> (63 - 9 * ((uint32_t)(pos >> 6) & 7))) & 0x1FFu;
-  return (uint32_t)e.x + in + __popcll(word & ((1ull << (pos & 63)) - 1));
+  step[h + 1] = (int)l + 1 < L ? make_uint2(Y, c + Z[h] - Y) : make_uint2(Y - c, 0u - Y);
 }
 
 // What the descents probe: the rank table and the bitvector, or for large
@@ -68,10 +60,10 @@ struct LevelBits {
       bit = r.bit;
       return r.ones;
     } else {
-      uint64_t word;
-      const uint32_t R = rank_step(tree, rt, pos, word);
+      const ulonglong2 e = load_entry(rt, pos);
+      const uint64_t word = load_word(tree, pos);
       bit = (uint32_t)(word >> (pos & 63)) & 1u;
-      return R;
+      return entry_rank(e, word, pos);
     }
   }
 };
@@ -94,12 +86,15 @@ __global__ void wt_descend_kernel(LevelBits<BLOCKS> bits, const uint2* __restric
   }
   uint32_t x = (uint32_t)i, h = 1;  // h: heap id + 1, the path with a leading 1
   uint64_t lbase = 0;
+  uint2 st = __ldg(step + 1);
   for (int lv = 0; lv < L; ++lv, lbase += n) {
-    uint2 st = make_uint2(0u, 0u);
-    if (INV || lv + 1 < L) st = __ldg(step + (h - 1));
+    // the children's constants come with this level's reads, not after them
+    uint4 next = make_uint4(0u, 0u, 0u, 0u);
+    if (lv + 1 < L) next = __ldg(reinterpret_cast<const uint4*>(step + 2 * h));
     uint32_t bit;
     const uint32_t R = bits.rank(lbase + x, bit);
     x = bit ? st.y + R : st.x + x - R;
+    st = bit ? make_uint2(next.z, next.w) : make_uint2(next.x, next.y);
     h = 2 * h + bit;
   }
   const uint64_t c = h - (1u << L);
@@ -132,13 +127,103 @@ __global__ void wt_rank_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__
   const uint32_t path = (uint32_t)c | (1u << L);
   uint32_t x = (uint32_t)i;
   uint64_t lbase = 0;
+  uint2 st = __ldg(step + 1);
   for (int lv = 0; lv < L; ++lv, lbase += n) {
-    const uint2 st = __ldg(step + ((path >> (L - lv)) - 1));
+    const uint2 next = __ldg(step + (path >> (lv + 1 < L ? L - 1 - lv : L)));  // one level ahead
     uint32_t bit;
     const uint32_t R = bits.rank(lbase + x, bit);
     x = (path >> (L - 1 - lv)) & 1u ? st.y + R : st.x + x - R;
+    st = next;
   }
   out[k] = x;
+}
+
+// Descents of batches that are not sorted, over trees larger than L2: node
+// entries and positions inside the node, 64-bit.  They read the same lines as
+// the kernels above and are slower by 10 % where L2 holds the tree, but their
+// queries stay together level by level (the levels of all queries in flight
+// must meet in L2: 0.72 GB from DRAM where the other rank read 1.01 GB, at 80 %
+// of its bandwidth both): 2^28 x 12 levels, rank of 2^19 queries 0.11 ms
+// against 0.15, access of 2^18 66 us against 70.
+__device__ __forceinline__ uint64_t entry_rank64(const ulonglong2& e, uint64_t word, uint64_t pos) {
+  return e.x + ((e.y >> (63 - 9 * ((pos >> 6) & 7))) & 0x1FF) + __popcll(word & ((1ull << (pos & 63)) - 1));
+}
+
+template <bool INV>
+__global__ void wt_descend_far_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                  const ulonglong2* __restrict__ tab, uint64_t n, int L,
+                                  const uint64_t* __restrict__ q, uint64_t nq, uint64_t* __restrict__ out,
+                                  uint64_t* __restrict__ sym_out) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nq) return;
+  uint64_t i = q[k];
+  if (i >= n) {
+    out[k] = NONE64;
+    if (INV) sym_out[k] = NONE64;
+    return;
+  }
+  uint64_t h = 0, c = 0;
+  ulonglong2 nd = __ldg(tab);
+  for (int lv = 0; lv < L; ++lv) {
+    const uint64_t pos = nd.x + i;
+    ulonglong2 c0 = nd, c1 = nd;
+    if (lv + 1 < L) {
+      c0 = __ldg(tab + 2 * h + 1);
+      c1 = __ldg(tab + 2 * h + 2);
+    }
+    const uint64_t word = load_word(tree, pos);
+    const uint64_t r = entry_rank64(load_entry(rt, pos), word, pos) - nd.y;
+    const uint64_t bit = (word >> (pos & 63)) & 1;
+    c = (c << 1) | bit;
+    if (bit) {
+      i = r;
+      h = 2 * h + 2;
+      nd = c1;
+    } else {
+      i -= r;
+      h = 2 * h + 1;
+      nd = c0;
+    }
+  }
+  if (INV) {
+    out[k] = i;
+    sym_out[k] = c;
+  } else {
+    out[k] = c;
+  }
+}
+
+__global__ void wt_rank_far_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                   const ulonglong2* __restrict__ tab, uint64_t n, int L,
+                                   const uint64_t* __restrict__ q, const uint64_t* __restrict__ sym, uint64_t nq,
+                                   uint64_t* __restrict__ out) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nq) return;
+  uint64_t i = q[k];
+  const uint64_t c = sym[k];
+  if (i > n) {
+    out[k] = NONE64;
+    return;
+  }
+  if (L < 64 && (1ull << L) <= c) {
+    out[k] = 0;
+    return;
+  }
+  uint64_t h = 0;
+  ulonglong2 nd = __ldg(tab);
+  for (int lv = 0; lv < L && i; ++lv) {
+    const uint64_t bit = (c >> (L - 1 - lv)) & 1;
+    const uint64_t child = 2 * h + 1 + bit;
+    ulonglong2 next = nd;
+    if (lv + 1 < L) next = __ldg(tab + child);
+    const uint64_t pos = nd.x + i;
+    const uint64_t word = load_word(tree, pos);
+    const uint64_t r = entry_rank64(load_entry(rt, pos), word, pos) - nd.y;
+    i = bit ? r : i - r;
+    h = child;
+    nd = next;
+  }
+  out[k] = i;
 }
 
 // wt_int::select (wt_int_par.hpp:622-660)
@@ -213,7 +298,7 @@ int tree_node_table(TreeImpl& t, cudaStream_t s) {
   if (t.node_tab_ok) return WTG_OK;
   const uint64_t nodes = (1ull << t.levels) - 1;
   if ((rc = t.node_tab.ensure(nodes * sizeof(ulonglong2), s))) return rc;
-  if ((rc = t.node_step.ensure(nodes * sizeof(uint2), s))) return rc;
+  if ((rc = t.node_step.ensure((nodes + 1) * sizeof(uint2), s))) return rc;
   const uint64_t heap = 1ull << t.levels;
   node_table_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(
       t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>(), t.zeros.as<uint32_t>() + heap, t.n,
@@ -233,6 +318,9 @@ int tree_node_table(TreeImpl& t, cudaStream_t s) {
 static bool blocks_pay(const TreeImpl& t, uint64_t nq) {
   return order_pays(t, nq) && t.levels >= 12 && nq >= block_count(t.n * (uint64_t)t.levels) / 3;
 }
+
+// (below 2^17 queries the tree's lines that they read stay in L2)
+static bool far_descent(const TreeImpl& t, uint64_t nq) { return larger_than_l2(t) && nq >= (1ull << 17); }
 
 // in_order, with the blocks where they pay and there is room for them:
 // launch(bits, ordered, order, first query, queries), ordered a bool constant
@@ -259,7 +347,12 @@ static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t 
 int launch_wt_access(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* out, cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "access")) return rc;
   return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
-    wt_descend_kernel<false, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
+    if (!ord() && far_descent(t, m))
+      wt_descend_far_kernel<false><<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
+                                                            t.node_tab.as<ulonglong2>(), t.n, t.levels, idx + at, m,
+                                                            out + at, nullptr);
+    else
+      wt_descend_kernel<false, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
                                                              m, out + at, nullptr);
   });
 }
@@ -268,8 +361,13 @@ int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64
                    cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "rank")) return rc;
   return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
-    wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o, sym + at,
-                                                   m, out + at);
+    if (!ord() && far_descent(t, m))
+      wt_rank_far_kernel<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
+                                                  t.node_tab.as<ulonglong2>(), t.n, t.levels, idx + at, sym + at, m,
+                                                  out + at);
+    else
+      wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
+                                                     sym + at, m, out + at);
   });
 }
 
@@ -277,7 +375,12 @@ int launch_wt_inverse_select(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint
                              uint64_t* sym_out, cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "inverse_select")) return rc;
   return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
-    wt_descend_kernel<true, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
+    if (!ord() && far_descent(t, m))
+      wt_descend_far_kernel<true><<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
+                                                           t.node_tab.as<ulonglong2>(), t.n, t.levels, idx + at, m,
+                                                           rank_out + at, sym_out + at);
+    else
+      wt_descend_kernel<true, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
                                                             m, rank_out + at, sym_out + at);
   });
 }

@@ -51,10 +51,15 @@ __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t*
   const uint32_t path = (uint32_t)c | (1u << L);
   uint32_t x = (uint32_t)i, y = (uint32_t)j, smaller = 0, greater = 0;  // counts below 2^32
   uint64_t lbase = 0;
+  uint2 st = __ldg(step + 1);
   for (int lv = 0; lv < L; ++lv, lbase += n) {
-    const uint2 st = __ldg(step + ((path >> (L - lv)) - 1));
-    const uint32_t rx = (uint32_t)rank1_dev(rt, tree, lbase + x);
-    const uint32_t ry = (uint32_t)rank1_dev(rt, tree, lbase + y);
+    const uint2 next = __ldg(step + (path >> (lv + 1 < L ? L - 1 - lv : L)));  // one level ahead
+    const uint64_t px = lbase + x, py = lbase + y;
+    const ulonglong2 ex = load_entry(rt, px);
+    const uint64_t wx = load_word(tree, px);
+    const ulonglong2 ey = load_entry(rt, py);
+    const uint64_t wy = load_word(tree, py);
+    const uint32_t rx = entry_rank(ex, wx, px), ry = entry_rank(ey, wy, py);
     if ((path >> (L - 1 - lv)) & 1u) {
       smaller += (y - x) - (ry - rx);
       x = st.y + rx;
@@ -64,6 +69,7 @@ __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t*
       x = st.x + x - rx;
       y = st.x + y - ry;
     }
+    st = next;
   }
   out_rank[k] = x;
   out_smaller[k] = smaller;
@@ -384,7 +390,7 @@ int launch_wt_lex_count(TreeImpl& t, const uint64_t* i, const uint64_t* j, const
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
-  });
+  }, true);
 }
 
 int launch_wt_lex_smaller_count(TreeImpl& t, const uint64_t* i, const uint64_t* c, uint64_t nq, uint64_t* rank_out,
@@ -414,7 +420,7 @@ int launch_wt_range_count(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, c
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
-  });
+  }, true);
 }
 
 int launch_wt_range_report(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, const uint64_t* vlb,

@@ -14,6 +14,19 @@ __device__ __forceinline__ uint64_t rank1_dev(const uint64_t* __restrict__ tbl, 
   return r;
 }
 
+// a rank entry and a word of the bits
+__device__ __forceinline__ ulonglong2 load_entry(const uint64_t* __restrict__ rt, uint64_t pos) {
+  return __ldg(reinterpret_cast<const ulonglong2*>(rt) + (pos >> 9));
+}
+__device__ __forceinline__ uint64_t load_word(const uint64_t* __restrict__ words, uint64_t pos) {
+  return __ldg(words + (pos >> 6));
+}
+// ones before pos (mod 2^32) from its rank entry and word
+__device__ __forceinline__ uint32_t entry_rank(const ulonglong2& e, uint64_t word, uint64_t pos) {
+  const uint32_t in = (uint32_t)(e.y >> (63 - 9 * ((uint32_t)(pos >> 6) & 7))) & 0x1FFu;
+  return (uint32_t)e.x + in + __popcll(word & ((1ull << (pos & 63)) - 1));
+}
+
 struct SelView {
   const uint64_t* words;
   uint64_t nwords;  // data words at `words`
