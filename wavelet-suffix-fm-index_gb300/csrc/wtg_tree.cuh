@@ -73,7 +73,7 @@ int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64
                    cudaStream_t s);
 int launch_wt_inverse_select(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* rank_out,
                              uint64_t* sym_out, cudaStream_t s);
-int launch_wt_select(const TreeImpl& t, const uint64_t* i, const uint64_t* sym, uint64_t nq, uint64_t* out,
+int launch_wt_select(TreeImpl& t, const uint64_t* i, const uint64_t* sym, uint64_t nq, uint64_t* out,
                      cudaStream_t s);
 int launch_bv_rank(const BvSupport& bv, const uint64_t* idx, uint64_t nq, uint64_t* out, cudaStream_t s);
 int launch_bv_select(const BvSupport& bv, int t_b, const uint64_t* i, uint64_t nq, uint64_t* out,
