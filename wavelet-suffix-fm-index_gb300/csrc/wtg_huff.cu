@@ -45,6 +45,7 @@
 
 #include "wtg_blocks.cuh"
 #include "wtg_fm_table.cuh"
+#include "wtg_hist.cuh"
 #include "wtg_order.cuh"
 #include "wtg_pass.cuh"
 #include "wtg_select.cuh"
@@ -88,36 +89,6 @@ struct HuffImpl {
 };
 
 namespace {
-
-// Byte counts.  Sixteen copies of a byte's counter, a lane's by its number,
-// lie side by side, so that the lanes of a warp that read the same byte meet on
-// few words: the shared atomics bound it, not the read.
-constexpr int HIST_COPIES = 16;
-__global__ void __launch_bounds__(512)
-    huff_hist_kernel(const uint8_t* __restrict__ s, uint64_t n, unsigned long long* __restrict__ hist) {
-  __shared__ uint32_t h[256 * HIST_COPIES];
-  for (uint32_t i = threadIdx.x; i < 256 * HIST_COPIES; i += blockDim.x) h[i] = 0;
-  __syncthreads();
-  uint32_t* const mine = h + (threadIdx.x & (HIST_COPIES - 1));
-  const uint64_t head = min(n, (uint64_t)((16 - ((uintptr_t)s & 15)) & 15)), quads = (n - head) / 16;
-  const uint4* __restrict__ q = reinterpret_cast<const uint4*>(s + head);
-  const uint64_t me = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t i = me; i < quads; i += stride) {
-    const uint4 v = __ldg(q + i);
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int k = 0; k < 16; ++k) atomicAdd(mine + ((w[k / 4] >> (8 * (k % 4))) & 0xFFu) * HIST_COPIES, 1u);
-  }
-  const uint64_t rest = n - 16 * quads;  // below 32: the bytes before and after the 16-byte words
-  if (me < rest) atomicAdd(mine + s[me < head ? me : 16 * quads + me] * HIST_COPIES, 1u);
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) {
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < HIST_COPIES; ++k) sum += h[i * HIST_COPIES + ((k + i) & (HIST_COPIES - 1))];
-    if (sum) atomicAdd(&hist[i], (unsigned long long)sum);
-  }
-}
 
 // the depth-d bits of a warp's 512-symbol chunk: bit of symbol i at global
 // position D + i (ORed, as runs need not start on a word); its zero count
@@ -725,7 +696,7 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
   if ((rc = h.hist.ensure(256 * sizeof(uint64_t), s))) return rc;
   WTG_CK(cudaMemsetAsync(h.hist.p, 0, 256 * sizeof(uint64_t), s));
   if (n) {
-    huff_hist_kernel<<<hgrid(n, 512 * 16, 152 * 4), 512, 0, s>>>(d_text, n, h.hist.as<unsigned long long>());
+    byte_hist_kernel<unsigned long long><<<hgrid(n, 512 * 16, 152 * 4), 512, 0, s>>>(d_text, n, h.hist.as<unsigned long long>());
     count_launch();
     WTG_CK(cudaGetLastError());
   }
