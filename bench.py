@@ -53,18 +53,26 @@ def algorithmic_bytes(n, L, w, sel_words=0):
     return (L * n * w + (L - 1) * n * w + bits + (bits + 16 * ((nb >> 9) + 1)) + 2 * bits + 8 * sel_words)
 
 
-# DRAM bytes (read + write) per symbol of one uint32 partitioning level pass,
-# from ncu's dram__bytes_read.sum + dram__bytes_write.sum over three level
-# launches (levels 9-11) of an n=2^28 build: 2137.7 MB per launch (1079.0 MB
-# read, 1058.7 MB written) against 2181.0 MB algorithmic; traffic grows
-# linearly with n, so a full launch's traffic is this figure times n.
-LEVEL_DRAM_BYTES_PER_SYMBOL_U32 = 2137.7e6 / 2 ** 28
+# DRAM bytes (read + write) per symbol of the scattering passes of a uint32
+# build with 20 levels (four levels each, 4 -> 2, 2 -> 2, 2 -> 1 and 1 -> 1
+# bytes a symbol), averaged over the four, from ncu's dram__bytes_read.sum +
+# dram__bytes_write.sum at n = 2^28: 1193.1 MB a pass against 1140.9 MB
+# algorithmic; traffic grows linearly with n, so a full
+# launch's traffic is this figure times n.
+LEVEL_DRAM_BYTES_PER_SYMBOL_U32 = 1193.1e6 / 2 ** 28
 
 
-def level_launch_bytes(n, w):
-    """Algorithmic bytes of one partitioning level pass: read n symbols,
-    write n symbols, write n bits."""
-    return 2 * n * w + n / 8
+def level_launch_bytes(n, w, L=LEVELS):
+    """Algorithmic bytes of one scattering pass over four levels, averaged over
+    a build's: read n symbols, write n narrowed ones, write 4 n bits.  The
+    symbols between the groups have the narrowest of 4, 2 and 1 bytes that
+    holds the bits left."""
+    total, passes, width = 0.0, 0, min(w, 4)
+    for done in range(4, L, 4):
+        out = min(width, 4 if L - done > 16 else 2 if L - done > 8 else 1)
+        total += n * (width + out) + 4 * n / 8
+        width, passes = out, passes + 1
+    return total / max(passes, 1)
 
 
 def init_ranks(dist, backend, timeout_s):
@@ -794,7 +802,7 @@ def run_wtg(args, rank, world, local_rank):
     lv_bytes = level_launch_bytes(n, 4)
     traffic = args.traffic if args.traffic is not None else LEVEL_DRAM_BYTES_PER_SYMBOL_U32 * n
     roofline = {
-        "bound": "hbm", "kernel": "level_kernel<uint32,partition>", "achieved": lv_bytes / (lv_avg / 1e3) / 1e9,
+        "bound": "hbm", "kernel": "level_pass_kernel<scatter>", "achieved": lv_bytes / (lv_avg / 1e3) / 1e9,
         "peak": peak, "unit": "GB/s", "peak_kind": peak_kind, "traffic": traffic,
         "launch_ms": lv_avg, "launches": lv_n, "bytes_per_launch": lv_bytes,
     }

@@ -84,12 +84,11 @@ int wtg_tree_build(const void* seq, uint64_t n, int elem_bytes, int levels, uint
 
 /* Same as wtg_tree_build, and copies the level bitvector (bit words) and the
  * rank table (rank words, see wtg_tree_info) to host memory while the build
- * runs: the bits of each level leave as soon as its pass is done, and the
- * rank entries of each level as soon as the rank/select pass has covered it
- * (n % 512 == 0 and a page-locked rank_dst; otherwise the whole rank table
- * beside the select finishing kernels).  A page-locked input of at least
- * 2^22 symbols is copied in eight pieces, and the build's first pass counts
- * each piece as it lands.  Either destination may be
+ * runs: the bits of each group of four levels leave as soon as its pass is
+ * done, and with a page-locked rank_dst the rank entries whose bits are final
+ * right after it (otherwise the whole rank table beside the select finishing
+ * kernels).  A page-locked input of at least 2^22 symbols is copied in up to
+ * eight pieces, and the build's first pass counts each piece as it lands.  Either destination may be
  * NULL; levels must be given (not 0).  With page-locked destinations the
  * copies overlap the kernels; pageable ones work but wait for each copy.
  * Returns once the build and the copies are complete.  No counterpart in the
@@ -294,7 +293,8 @@ int wtg_suffix_array(const uint8_t* text, uint64_t n, int32_t* sa_out);
 int wtg_bwt(const uint8_t* text, uint64_t n, uint8_t* bwt_out, int32_t* sa_out);
 /* device text / outputs on a stream (d_sa or d_bwt may be NULL); returns
  * once the stream has finished; rounds (may be NULL) gets the number of
- * doubling rounds.  Allocates its scratch (about 33 bytes per symbol). */
+ * doubling rounds.  Allocates its scratch (about 40 bytes per symbol,
+ * 44 without d_sa). */
 int wtg_suffix_array_device(const uint8_t* d_text, uint64_t n, int32_t* d_sa, uint8_t* d_bwt, void* stream,
                             int* rounds);
 
@@ -363,8 +363,9 @@ int wtg_lsel_query_device(wtg_lsel* m, int t_b, const uint64_t* d_level, const u
  * When enabled, every build records a CUDA event pair around each kernel it
  * launches, on the launching stream.  wtg_profile_read waits for those events
  * and returns, per kernel class, the number of launches and their summed
- * device time in ms, then clears the record.  Classes: 0 level pass with
- * partition, 1 last level pass, 2 key histogram, 3 node tables and scans,
+ * device time in ms, then clears the record.  Classes: 0 pass over a
+ * group of levels with partition, 1 the last group's pass, 2 digit counts, 3
+ * node tables and scans,
  * 4 bitvector pass (rank + select samples), 5 select finishing kernels. */
 #define WTG_PROF_CLASSES 6
 int wtg_profile_enable(int on);
