@@ -793,7 +793,12 @@ struct LevelPass {
   }
 
   // A chunk over many small nodes: symbol per lane, row by row, every bit by
-  // its own position (counts per string run in shared memory).
+  // its own position (counts per string run in shared memory).  Bound by one
+  // read after another: the starts of the chunk's nodes are searched in shared
+  // memory, and what does not depend on the counts (symbols, nodes, bases) is
+  // fetched for four rows at once (10^7 symbols, 20 levels: the passes of levels
+  // 12-15 and 16-19 take 69 and 87 us, 87 and 103 row by row).  Bits collected
+  // in shared memory before they are set gained nothing.
   static __device__ __noinline__ void scattered_chunk(const PassArgs& a, uint32_t c, uint32_t zc, uint32_t base) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
@@ -817,51 +822,85 @@ struct LevelPass {
       sts32(base + 4 * lane, in ? zb - za : 0u);
     }
     __syncwarp();
-    const uint32_t p_lo = a.cnode[c], p_hi = a.cnode[c + 1];
-    bool bad = false;
-    for (int r = 0; r < 32; ++r) {
-      const uint64_t i = ((uint64_t)c << LOG_CHUNK) + 32 * r + lane;
-      const bool valid = i < a.n;
-      uint32_t x = valid ? (uint32_t)src[i] : 0u;
-      if constexpr (HUFF) x = __ldg(a.huff.lut + x);
-      const uint32_t dg = (x >> a.ds) & ((1u << TAU) - 1);  // TAU bits
-      const uint32_t p = valid ? find_node(a.Cl, p_lo, p_hi, (uint32_t)i) : p_lo;
-      const uint32_t* __restrict__ rp = a.rec + (uint64_t)p * REC;
-      uint32_t m = __ballot_sync(0xffffffffu, valid);
-      const uint32_t inner = HUFF ? __ldg(rp + 15) : 0u;
-#pragma unroll
-      for (int j = 0; j < TAU; ++j) {
-        const bool bit = (dg >> (TAU - 1 - j)) & 1u;
-        const uint32_t q = dg >> (TAU - j);  // the j bits above
-        if (j >= 1 && valid && (!HUFF || (inner >> ((1 << j) - 1 + q) & 1u))) {
-          const uint32_t pos = __ldg(rp + (1 << j) - 1 + q) + lds32(base + 4 * ((1 << j) - 1 + q)) + __popc(m & lt);
-          if (pos >= level_size<HUFF>(a, j)) bad = true;
-          else if (bit) {
-            const uint64_t g = level_begin<HUFF>(a, j) + pos;
-            atomicOr(a.bits + (g >> 5), 1u << (g & 31));
-          }
-        }
-        __syncwarp();
-        if (j >= 1 && valid && !(m & ~lt & ~(1u << lane))) {  // the last lane of the string adds its count
-          const uint32_t ad = base + 4 * ((1 << j) - 1 + q);
-          sts32(ad, lds32(ad) + __popc(m));
-        }
-        __syncwarp();
-        const uint32_t bm = __ballot_sync(0xffffffffu, bit);
-        m &= bit ? bm : ~bm;
+    constexpr int BATCH = 4;
+    constexpr uint32_t ROOM = (4096 - 256) / 4;  // node starts that the warp's region holds beside the counts
+    const uint32_t p_lo = a.cnode[c], nn = a.cnode[c + 1] - p_lo + 1;
+    const bool staged = nn <= ROOM;
+    if (staged) {
+      for (uint32_t k = lane; k < nn; k += 32) sts32(base + 256 + 4 * k, __ldg(a.Cl + p_lo + k));
+      __syncwarp();
+    }
+    auto node_of = [&](uint32_t pos) -> uint32_t {
+      if (!staged) return find_node(a.Cl, p_lo, p_lo + nn - 1, pos);
+      uint32_t lo = 0, hi = nn - 1;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (lds32(base + 256 + 4 * mid) <= pos) lo = mid;
+        else hi = mid - 1;
       }
-      if constexpr (SCATTER) {
-        if (valid && (!HUFF || (inner >> (16 + dg) & 1u))) {
-          const uint32_t pos = __ldg(rp + 16 + dg) + lds32(base + 4 * (15 + dg)) + __popc(m & lt);
-          if (pos >= (HUFF ? __ldg(a.huff.lv + 8) : a.n)) bad = true;
-          else static_cast<Tout*>(a.dst)[pos] = (Tout)x;
+      return p_lo + lo;
+    };
+    bool bad = false;
+    const uint64_t cbase = (uint64_t)c << LOG_CHUNK;
+    for (int r0 = 0; r0 < 32 && cbase + 32 * r0 < a.n; r0 += BATCH) {
+      uint32_t xs[BATCH], bases[BATCH][TAU], inner[BATCH];  // bases[.][0]: of the scatter
+#pragma unroll
+      for (int b = 0; b < BATCH; ++b) {
+        const uint64_t i = cbase + 32 * (r0 + b) + lane;
+        xs[b] = i < a.n ? (uint32_t)src[i] : 0u;
+      }
+#pragma unroll
+      for (int b = 0; b < BATCH; ++b) {
+        const uint64_t i = cbase + 32 * (r0 + b) + lane;
+        if constexpr (HUFF) xs[b] = __ldg(a.huff.lut + xs[b]);
+        const uint32_t dg = (xs[b] >> a.ds) & ((1u << TAU) - 1);
+        const uint32_t* __restrict__ rp = a.rec + (uint64_t)(i < a.n ? node_of((uint32_t)i) : p_lo) * REC;
+#pragma unroll
+        for (int j = 1; j < TAU; ++j) bases[b][j] = __ldg(rp + (1 << j) - 1 + (dg >> (TAU - j)));
+        bases[b][0] = SCATTER ? __ldg(rp + 16 + dg) : 0u;
+        inner[b] = HUFF ? __ldg(rp + 15) : 0u;
+      }
+#pragma unroll
+      for (int b = 0; b < BATCH; ++b) {
+        const uint64_t i = cbase + 32 * (r0 + b) + lane;
+        const bool valid = i < a.n;
+        const uint32_t x = xs[b];
+        const uint32_t dg = (x >> a.ds) & ((1u << TAU) - 1);  // TAU bits
+        uint32_t m = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+        for (int j = 0; j < TAU; ++j) {
+          const bool bit = (dg >> (TAU - 1 - j)) & 1u;
+          const uint32_t q = dg >> (TAU - j);  // the j bits above
+          if (j >= 1 && valid && (!HUFF || (inner[b] >> ((1 << j) - 1 + q) & 1u))) {
+            const uint32_t pos = bases[b][j] + lds32(base + 4 * ((1 << j) - 1 + q)) + __popc(m & lt);
+            if (pos >= level_size<HUFF>(a, j)) bad = true;
+            else if (bit) {
+              const uint64_t g = level_begin<HUFF>(a, j) + pos;
+              atomicOr(a.bits + (g >> 5), 1u << (g & 31));
+            }
+          }
+          __syncwarp();
+          if (j >= 1 && valid && !(m & ~lt & ~(1u << lane))) {  // the last lane of the string adds its count
+            const uint32_t ad = base + 4 * ((1 << j) - 1 + q);
+            sts32(ad, lds32(ad) + __popc(m));
+          }
+          __syncwarp();
+          const uint32_t bm = __ballot_sync(0xffffffffu, bit);
+          m &= bit ? bm : ~bm;
         }
-        __syncwarp();
-        if (valid && !(m & ~lt & ~(1u << lane))) {
-          const uint32_t ad = base + 4 * (15 + dg);
-          sts32(ad, lds32(ad) + __popc(m));
+        if constexpr (SCATTER) {
+          if (valid && (!HUFF || (inner[b] >> (16 + dg) & 1u))) {
+            const uint32_t pos = bases[b][0] + lds32(base + 4 * (15 + dg)) + __popc(m & lt);
+            if (pos >= (HUFF ? __ldg(a.huff.lv + 8) : a.n)) bad = true;
+            else static_cast<Tout*>(a.dst)[pos] = (Tout)x;
+          }
+          __syncwarp();
+          if (valid && !(m & ~lt & ~(1u << lane))) {
+            const uint32_t ad = base + 4 * (15 + dg);
+            sts32(ad, lds32(ad) + __popc(m));
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicCAS(a.err, 0u, (uint32_t)DERR_BAD_INDEX);
