@@ -59,9 +59,11 @@ int check_seq_args(uint64_t n, int eb, int levels, uint32_t flags) {
 // waits for the stream; an error that a kernel reported stays until the next build
 int sync_and_check(cudaStream_t s, ErrWord& err) {
   uint32_t e = 0;
-  const bool read = err.p && (err.pending || err.elsewhere);
-  if (read) WTG_CK(cudaMemcpyAsync(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost, s));
+  if (err.p && err.pending && !err.elsewhere)
+    WTG_CK(cudaMemcpyAsync(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost, s));
   WTG_CK(cudaStreamSynchronize(s));
+  // (a plain copy also waits for the work of the default stream)
+  if (err.p && err.elsewhere) WTG_CK(cudaMemcpy(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost));
   if (!e) err.pending = false;
   if (e == DERR_LOOKBACK_TIMEOUT) return fail(WTG_ERR_TIMEOUT, "a device-side wait timed out; results are invalid");
   if (e == DERR_BAD_INDEX) return fail(WTG_ERR_CUDA, "a computed index fell outside its buffer (inconsistent tables)");
