@@ -32,7 +32,7 @@ def build(ref=True):
     import shutil
     if shutil.which("make"):
         subprocess.run(["make", "-s", "-C", HERE, "all"], check=True)
-        if ref and os.path.isdir(REF_SRC):
+        if ref and os.path.isdir(os.path.join(REF_SRC, "wavelet")):  # (an empty directory is no checkout)
             subprocess.run(["make", "-s", "-C", HERE, "ref", "ref-src", "REF=" + REF_SRC], check=True)
         if ref and os.path.isdir(os.path.join(REF_DIR, "src")):
             subprocess.run(["make", "-s", "-C", HERE, "bench-ref"], check=True)
