@@ -77,9 +77,11 @@ __global__ void node_kernel(const uint32_t* __restrict__ C, const uint32_t* __re
   }
 }
 
-// The sequence on a 32-byte boundary in at most 4 bytes a symbol: 8-byte
-// symbols keep their low half (levels <= 24), and a sequence that does not
-// start on a 32-byte boundary is moved, so that the passes' row loads apply.
+// The sequence as the passes read it, on a 32-byte boundary in at most 4 bytes
+// a symbol: 8-byte symbols keep their low half (levels <= 24), a sequence that
+// does not start on a 32-byte boundary is moved, so that the row loads apply,
+// and symbols of fewer bits than there are levels are widened: a digit is
+// taken from several packed symbols at once and has to lie inside its own.
 template <typename T, typename U>
 __global__ void repack_kernel(const T* __restrict__ s, uint64_t n, U* __restrict__ out) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -104,6 +106,12 @@ static void launch_max(const void* s, uint64_t n, unsigned long long* out, cudaS
   unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 8);
   if (grid == 0) grid = 1;
   max_kernel<T><<<grid, 256, 0, st>>>((const T*)s, n, out);
+}
+
+template <typename T, typename U>
+static void launch_repack(const void* s, uint64_t n, void* out, cudaStream_t st) {
+  const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16);
+  repack_kernel<T, U><<<grid, 256, 0, st>>>((const T*)s, n, (U*)out);
 }
 
 #define WTG_DISPATCH(eb, fn, ...)                       \
@@ -202,9 +210,10 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   if (n) {
     // sequence buffers: what the groups after the first read
     auto bytes_of = [&](int bits_left) { return bits_left > 16 ? 4 : bits_left > 8 ? 2 : 1; };
-    const bool repack = eb == 8 || (uintptr_t)d_seq % 32;
-    size_t lvl_bytes[2] = {0, repack ? n * std::min(eb, 4) : 0};
-    for (int g = 0, sb = std::min(eb, 4); g + 1 < groups; ++g) {
+    const int width = L > 8 * eb ? bytes_of(L) : std::min(eb, 4);
+    const bool repack = eb != width || (uintptr_t)d_seq % 32;
+    size_t lvl_bytes[2] = {0, repack ? n * width : 0};
+    for (int g = 0, sb = width; g + 1 < groups; ++g) {
       sb = std::min(sb, bytes_of(L - 4 * g - 4));
       lvl_bytes[g & 1] = std::max<size_t>(lvl_bytes[g & 1], n * sb);
     }
@@ -228,11 +237,13 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
       return WTG_OK;
     };
     if (repack) {
-      sb = std::min(eb, 4);
+      sb = width;
       if ((rc = wait_pieces())) return rc;
-      const unsigned grid = (unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count() * 16);
-      if (eb == 8) {
-        repack_kernel<uint64_t, uint32_t><<<grid, 256, 0, s>>>((const uint64_t*)d_seq, n, (uint32_t*)lvl[1]);
+      if (eb != width) {
+        if (eb == 8) launch_repack<uint64_t, uint32_t>(d_seq, n, lvl[1], s);
+        else if (eb == 2) launch_repack<uint16_t, uint32_t>(d_seq, n, lvl[1], s);
+        else if (width == 2) launch_repack<uint8_t, uint16_t>(d_seq, n, lvl[1], s);
+        else launch_repack<uint8_t, uint32_t>(d_seq, n, lvl[1], s);
         count_launch();
         WTG_CK(cudaGetLastError());
       } else {
