@@ -386,6 +386,8 @@ void tree_release(TreeImpl& t) {
   t.node_tab.release(s);
   t.node_step.release(s);
   t.node_tab_ok = false;
+  if (t.node_made) cudaEventDestroy(t.node_made);
+  t.node_made = nullptr;
   t.scratch.release(s);
   t.nodes.release(s);
   t.qbuf.release(s);

@@ -69,6 +69,12 @@ bool test_take_lookback_stall() {
   return g_lookback_stall.compare_exchange_strong(armed, 0);
 }
 
+bool stream_captures(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) cudaGetLastError();  // (the legacy stream beside a capture)
+  return st != cudaStreamCaptureStatusNone;
+}
+
 int DevBuf::ensure(size_t need, cudaStream_t s) {
   if (need <= bytes && p) return WTG_OK;
   int rc = ensure_pool_setup();

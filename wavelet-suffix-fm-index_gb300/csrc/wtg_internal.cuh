@@ -343,6 +343,9 @@ enum {
 
 // ------------------------------------------------------- host-side pieces
 
+// whether the stream's work goes into a graph instead of running
+bool stream_captures(cudaStream_t s);
+
 // Stream-ordered device buffer that keeps its allocation across rebuilds.
 struct DevBuf {
   void* p = nullptr;

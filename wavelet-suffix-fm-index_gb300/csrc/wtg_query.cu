@@ -320,20 +320,52 @@ static int need(const TreeImpl& t, uint32_t f, const char* what) {
 
 WTG_WAIT_LIMIT_SETTER(query)
 
-int tree_node_table(TreeImpl& t, cudaStream_t s) {
+static int make_node_tables(const TreeImpl& t, DevBuf& tab, DevBuf& step, cudaStream_t s) {
   int rc;
-  if (t.node_tab_ok) return WTG_OK;
-  const uint64_t nodes = (1ull << t.levels) - 1;
-  if ((rc = t.node_tab.ensure(nodes * sizeof(ulonglong2), s))) return rc;
-  if ((rc = t.node_step.ensure((nodes + 1) * sizeof(uint2), s))) return rc;
-  const uint64_t heap = 1ull << t.levels;
+  const uint64_t heap = 1ull << t.levels, nodes = heap - 1;
+  if ((rc = tab.ensure(nodes * sizeof(ulonglong2), s))) return rc;
+  if ((rc = step.ensure((nodes + 1) * sizeof(uint2), s))) return rc;
   node_table_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(
       t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>(), t.zeros.as<uint32_t>() + heap, t.n,
-      t.levels, nodes, t.node_tab.as<ulonglong2>(), t.node_step.as<uint2>());
+      t.levels, nodes, tab.as<ulonglong2>(), step.as<uint2>());
   count_launch();
   WTG_CK(cudaGetLastError());
+  return WTG_OK;
+}
+
+// the tree's own tables, made or waited for
+static int shared_node_tables(TreeImpl& t, cudaStream_t s, bool make) {
+  if (t.node_tab_ok) {
+    if (!t.node_on_own || s != t.stream) WTG_CK(cudaStreamWaitEvent(s, t.node_made, 0));
+    return WTG_OK;
+  }
+  if (!make) return WTG_OK;
+  int rc;
+  if (!t.node_made) WTG_CK(cudaEventCreateWithFlags(&t.node_made, cudaEventDisableTiming));
+  if ((rc = make_node_tables(t, t.node_tab, t.node_step, s))) return rc;
+  WTG_CK(cudaEventRecord(t.node_made, s));
+  t.node_on_own = s == t.stream;
   t.node_tab_ok = true;
   return WTG_OK;
+}
+
+NodeTables::NodeTables(TreeImpl& t, cudaStream_t s, bool make) : stream(s) {
+  const bool captured = stream_captures(s);
+  std::lock_guard<std::mutex> lk(t.node_mu);
+  if (!captured) rc = shared_node_tables(t, s, make);
+  if (rc == WTG_OK && t.node_tab_ok) {
+    tab = t.node_tab.as<ulonglong2>();
+    step = t.node_step.as<uint2>();
+  } else if (rc == WTG_OK && captured && make) {
+    if ((rc = make_node_tables(t, own_tab, own_step, s))) return;
+    tab = own_tab.as<ulonglong2>();
+    step = own_step.as<uint2>();
+  }
+}
+
+NodeTables::~NodeTables() {
+  own_tab.release(stream);
+  own_step.release(stream);
 }
 
 // Blocks (built from the bitvector for the call: 1.1 ms for 2^30 x 20 levels,
@@ -350,19 +382,19 @@ static bool blocks_pay(const TreeImpl& t, uint64_t nq) {
 static bool far_descent(const TreeImpl& t, uint64_t nq) { return larger_than_l2(t) && nq >= (1ull << 17); }
 
 // in_order, with the blocks where they pay and there is room for them:
-// launch(bits, ordered, order, first query, queries), ordered a bool constant
+// launch(nodes, bits, ordered, order, first query, queries), ordered a bool constant
 template <typename F>
 static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t s, F launch) {
-  int rc;
   if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
+  const NodeTables nodes(t, s);
+  if (nodes.rc) return nodes.rc;
   const uint64_t* const words = t.bits.as<uint64_t>();
   const uint64_t* const rt = t.bv.rank.as<uint64_t>();
   uint4* const blocks = blocks_pay(t, nq) ? make_blocks(words, rt, t.n * (uint64_t)t.levels, s) : nullptr;
-  rc = in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
-    if (sorted && blocks) launch(LevelBits<true>{words, rt, blocks}, std::true_type{}, o, at, m);
-    else if (sorted) launch(LevelBits<false>{words, rt, nullptr}, std::true_type{}, o, at, m);
-    else launch(LevelBits<false>{words, rt, nullptr}, std::false_type{}, o, at, m);
+  const int rc = in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    if (sorted && blocks) launch(nodes, LevelBits<true>{words, rt, blocks}, std::true_type{}, o, at, m);
+    else if (sorted) launch(nodes, LevelBits<false>{words, rt, nullptr}, std::true_type{}, o, at, m);
+    else launch(nodes, LevelBits<false>{words, rt, nullptr}, std::false_type{}, o, at, m);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
@@ -373,42 +405,42 @@ static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t 
 
 int launch_wt_access(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* out, cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "access")) return rc;
-  return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
+  return descents(t, idx, nq, s, [&](const NodeTables& nodes, auto bits, auto ord, const QueryOrder& o, uint64_t at,
+                                     uint64_t m) {
     if (!ord() && far_descent(t, m))
-      wt_descend_far_kernel<false><<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                            t.node_tab.as<ulonglong2>(), t.n, t.levels, idx + at, m,
-                                                            out + at, nullptr);
+      wt_descend_far_kernel<false><<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab,
+                                                            t.n, t.levels, idx + at, m, out + at, nullptr);
     else
-      wt_descend_kernel<false, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
-                                                             m, out + at, nullptr);
+      wt_descend_kernel<false, ord()><<<qgrid(m), 256, 0, s>>>(bits, nodes.step, t.n, t.levels, idx + at, o, m,
+                                                               out + at, nullptr);
   });
 }
 
 int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64_t nq, uint64_t* out,
                    cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "rank")) return rc;
-  return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
+  return descents(t, idx, nq, s, [&](const NodeTables& nodes, auto bits, auto ord, const QueryOrder& o, uint64_t at,
+                                     uint64_t m) {
     if (!ord() && far_descent(t, m))
-      wt_rank_far_kernel<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                  t.node_tab.as<ulonglong2>(), t.n, t.levels, idx + at, sym + at, m,
-                                                  out + at);
+      wt_rank_far_kernel<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab, t.n,
+                                                  t.levels, idx + at, sym + at, m, out + at);
     else
-      wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
-                                                     sym + at, m, out + at);
+      wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, nodes.step, t.n, t.levels, idx + at, o, sym + at, m,
+                                                       out + at);
   });
 }
 
 int launch_wt_inverse_select(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* rank_out,
                              uint64_t* sym_out, cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "inverse_select")) return rc;
-  return descents(t, idx, nq, s, [&](auto bits, auto ord, const QueryOrder& o, uint64_t at, uint64_t m) {
+  return descents(t, idx, nq, s, [&](const NodeTables& nodes, auto bits, auto ord, const QueryOrder& o, uint64_t at,
+                                     uint64_t m) {
     if (!ord() && far_descent(t, m))
-      wt_descend_far_kernel<true><<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                           t.node_tab.as<ulonglong2>(), t.n, t.levels, idx + at, m,
-                                                           rank_out + at, sym_out + at);
+      wt_descend_far_kernel<true><<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab,
+                                                           t.n, t.levels, idx + at, m, rank_out + at, sym_out + at);
     else
-      wt_descend_kernel<true, ord()><<<qgrid(m), 256, 0, s>>>(bits, t.node_step.as<uint2>(), t.n, t.levels, idx + at, o,
-                                                            m, rank_out + at, sym_out + at);
+      wt_descend_kernel<true, ord()><<<qgrid(m), 256, 0, s>>>(bits, nodes.step, t.n, t.levels, idx + at, o, m,
+                                                              rank_out + at, sym_out + at);
   });
 }
 
@@ -419,11 +451,12 @@ int launch_wt_select(TreeImpl& t, const uint64_t* i, const uint64_t* sym, uint64
   // the node table where there is one, or the batch is worth making it (24
   // bytes and a rank per node) and there is room
   const uint64_t heap = 1ull << t.levels;
-  const bool tab = t.n && (t.node_tab_ok || (heap <= 8 * nq && tree_node_table(t, s) == WTG_OK));
-  if (!tab) cudaGetLastError();
+  const NodeTables nodes(t, s, heap <= 8 * nq);
+  if (nodes.rc) cudaGetLastError();
+  const bool tab = t.n && nodes.rc == WTG_OK && nodes.tab;
   auto* const f = tab ? wt_select_kernel<true> : wt_select_kernel<false>;
   f<<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), sel_view(t.bv, 1), sel_view(t.bv, 0),
-                              t.node_tab.as<ulonglong2>(), t.zeros.as<uint32_t>() + heap, t.n, t.levels, i, sym, nq, out);
+                              nodes.tab, t.zeros.as<uint32_t>() + heap, t.n, t.levels, i, sym, nq, out);
   count_launch();
   WTG_CK(cudaGetLastError());
   return WTG_OK;

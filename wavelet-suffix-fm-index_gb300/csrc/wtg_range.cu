@@ -382,10 +382,11 @@ int launch_wt_lex_count(TreeImpl& t, const uint64_t* i, const uint64_t* j, const
   int rc;
   if ((rc = need_rank(t, "lex_count"))) return rc;
   if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
+  const NodeTables nodes(t, s);
+  if ((rc = nodes.rc)) return rc;
   return in_order(t, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_lex_kernel<true> : wt_lex_kernel<false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_step.as<uint2>(), t.n, t.levels,
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.step, t.n, t.levels,
                                o, i + at, j + at, c + at, m, rank_out + at, smaller_out + at, greater_out + at);
     count_launch();
     WTG_CK(cudaGetLastError());
@@ -398,9 +399,10 @@ int launch_wt_lex_smaller_count(TreeImpl& t, const uint64_t* i, const uint64_t* 
   int rc;
   if ((rc = need_rank(t, "lex_smaller_count"))) return rc;
   if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
+  const NodeTables nodes(t, s);
+  if ((rc = nodes.rc)) return rc;
   wt_lex_smaller_kernel<<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(),
-                                                  t.node_tab.as<ulonglong2>(), t.n, t.levels, i, c, nq, rank_out,
+                                                  nodes.tab, t.n, t.levels, i, c, nq, rank_out,
                                                   smaller_out);
   count_launch();
   WTG_CK(cudaGetLastError());
@@ -412,10 +414,11 @@ int launch_wt_range_count(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, c
   int rc;
   if ((rc = need_rank(t, "range_search_2d"))) return rc;
   if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
+  const NodeTables nodes(t, s);
+  if ((rc = nodes.rc)) return rc;
   return in_order(t, lb, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_range_count_kernel<true> : wt_range_count_kernel<false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_tab.as<ulonglong2>(), t.n,
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab, t.n,
                                t.levels, o, lb + at, rb + at, vlb + at, vrb + at, m, count_out + at);
     count_launch();
     WTG_CK(cudaGetLastError());
@@ -430,9 +433,10 @@ int launch_wt_range_report(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, 
   if ((t.flags & WTG_ALL) != WTG_ALL)
     return fail(WTG_ERR_INVALID, "range_search_2d with report needs rank and both selects");
   if (!nq || !cap) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
+  const NodeTables nodes(t, s);
+  if ((rc = nodes.rc)) return rc;
   wt_range_report_kernel<<<qgrid(nq * 32), 256, 0, s>>>(
-      t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.node_tab.as<ulonglong2>(), sel_view(t.bv, 1),
+      t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab, sel_view(t.bv, 1),
       sel_view(t.bv, 0), t.n, t.levels, lb, rb, vlb, vrb, nq, off, cap, pos, val);
   count_launch();
   WTG_CK(cudaGetLastError());
@@ -445,10 +449,11 @@ int launch_wt_interval_symbols(TreeImpl& t, const uint64_t* i, const uint64_t* j
   int rc;
   if ((rc = need_rank(t, "interval_symbols"))) return rc;
   if (!nq) return WTG_OK;
-  if ((rc = tree_node_table(t, s))) return rc;
+  const NodeTables nodes(t, s);
+  if ((rc = nodes.rc)) return rc;
   const uint64_t* tree = t.bits.as<uint64_t>();
   const uint64_t* rt = t.bv.rank.as<uint64_t>();
-  const ulonglong2* tab = t.node_tab.as<ulonglong2>();
+  const ulonglong2* tab = nodes.tab;
   if (k_out) {
     wt_interval_symbols_kernel<false><<<qgrid(nq), 256, 0, s>>>(tree, rt, tab, t.n, t.levels, i, j, nq, k_out,
                                                                 nullptr, 0, nullptr, nullptr, nullptr);
