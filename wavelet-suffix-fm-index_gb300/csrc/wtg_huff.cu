@@ -341,6 +341,7 @@ struct HuffFmInfo {
   uint64_t depth[HF_MAX_DEPTH];  // first bit of each depth's run
 };
 
+// Made by the build, so that counts on any stream only read them.
 // steps[first + d]: x = position of the node's bits in its depth's run, y =
 // ones before them (mod 2^32).  With r the ones before (depth + x + i), bit 1
 // goes on at i' = r - y, bit 0 at i' = i - (r - y).
@@ -825,6 +826,13 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
                                                              h.bv.rank.as<uint64_t>(), h.bits.as<uint64_t>());
       count_launch();
       WTG_CK(cudaGetLastError());
+      if (h.n < (1ull << 32)) {
+        if ((rc = h.fmsteps.ensure(std::max<uint32_t>(h.fm_steps, 1) * sizeof(uint2), s))) return rc;
+        huff_steps_kernel<<<1, 256, 0, s>>>(h.dnodes.as<HuffNodeDev>(), h.fminfo.as<HuffFmInfo>(),
+                                            h.fmsteps.as<uint2>());
+        count_launch();
+        WTG_CK(cudaGetLastError());
+      }
     }
   }
   return WTG_OK;
@@ -945,17 +953,12 @@ int launch_huff_fm_count(HuffImpl& h, const uint64_t* C, const uint8_t* pat, con
     WTG_CK(cudaGetLastError());
     return WTG_OK;
   }
-  int rc;
-  if ((rc = h.fmsteps.ensure(std::max<uint32_t>(h.fm_steps, 1) * sizeof(uint2), s))) return rc;
-  huff_steps_kernel<<<1, 256, 0, s>>>(h.dnodes.as<HuffNodeDev>(), h.fminfo.as<HuffFmInfo>(), h.fmsteps.as<uint2>());
-  count_launch();
-  WTG_CK(cudaGetLastError());
   // as for the balanced tree: blocks once the batch probes a good part of them
   uint4* blocks = h.size && huff_batch_pays(h, npat) && npat >= block_count(h.size) / 8
                       ? make_blocks(h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), h.size, s)
                       : nullptr;
-  rc = blocks ? huff_fm_run<true>(h, blocks, C, pat, off, npat, out, s)
-              : huff_fm_run<false>(h, blocks, C, pat, off, npat, out, s);
+  const int rc = blocks ? huff_fm_run<true>(h, blocks, C, pat, off, npat, out, s)
+                        : huff_fm_run<false>(h, blocks, C, pat, off, npat, out, s);
   if (blocks) cudaFreeAsync(blocks, s);
   return rc;
 }
