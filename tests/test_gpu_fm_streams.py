@@ -30,11 +30,16 @@ def _huff(wtg, bwt, st):
     return h, h.fm_count_device
 
 
+def _balanced(wtg, bwt, st):
+    f = wtg.FMIndex.from_device(bwt.data_ptr(), N, 6, st)
+    return f.tree, f.count_device
+
+
 def _device(torch, arrays):
     return [torch.from_numpy(a.view(np.int64) if a.dtype == np.uint64 else a.copy()).cuda() for a in arrays]
 
 
-@pytest.mark.parametrize("make", [_huff])
+@pytest.mark.parametrize("make", [_huff, _balanced])
 def test_counts_on_two_streams(wtg, text, make):
     torch, bwt, C, pat, off, exp = text
     d_bwt, d_C, d_pat, d_off = _device(torch, (bwt, C, pat, off))
@@ -55,7 +60,35 @@ def test_counts_on_two_streams(wtg, text, make):
     h.free()
 
 
-@pytest.mark.parametrize("make", [_huff])
+def test_counts_with_different_C_on_two_streams(wtg, text):
+    """The balanced tree's steps hold the call's own C and number of symbols."""
+    torch, bwt, C, pat, off, exp = text
+    d_bwt, d_C, d_pat, d_off = _device(torch, (bwt, C, pat, off))
+    d_zero = torch.zeros_like(d_C)
+    slow, st = torch.cuda.Stream(), torch.cuda.current_stream()
+    t = wtg.FMIndex.from_device(d_bwt.data_ptr(), N, 6, st.cuda_stream).tree
+
+    def count(d_c, sigma, stream, out):
+        wtg._ck(wtg.lib().wtg_fm_count_device(t.h, d_c.data_ptr(), sigma, d_pat.data_ptr(), d_off.data_ptr(), NPAT,
+                                              out.data_ptr(), stream.cuda_stream))
+
+    calls = [(d_C, 4), (d_zero, 6), (d_C, 6), (d_zero, 4)]
+    alone = [torch.zeros(NPAT, dtype=torch.int64, device="cuda") for _ in calls]
+    got = [torch.zeros(NPAT, dtype=torch.int64, device="cuda") for _ in calls]
+    for (c, sigma), out in zip(calls, alone):
+        count(c, sigma, st, out)
+        torch.cuda.synchronize()
+    with torch.cuda.stream(slow):
+        torch.cuda._sleep(400_000_000)
+    for k, ((c, sigma), out) in enumerate(zip(calls, got)):
+        count(c, sigma, (slow, st)[k % 2], out)
+    torch.cuda.synchronize()
+    for a, b in zip(got, alone):
+        assert torch.equal(a, b)
+    assert np.array_equal(got[2].cpu().numpy()[:20], exp)
+
+
+@pytest.mark.parametrize("make", [_huff, _balanced])
 def test_captured_count(wtg, text, make):
     torch, bwt, C, pat, off, exp = text
     d_bwt, d_C, d_pat, d_off = _device(torch, (bwt, C, pat, off))

@@ -382,7 +382,6 @@ void tree_release(TreeImpl& t) {
   t.err.release(s);
   t.lvl_args.release(s);
   t.lvl_args_ok = false;
-  t.fm_paths.release(s);
   t.node_tab.release(s);
   t.node_step.release(s);
   t.node_tab_ok = false;

@@ -10,10 +10,10 @@
 // and C[c] counts the symbols below c.
 //
 // The path of a symbol through the tree does not depend on the position, so
-// each symbol's step constants are tabulated once per call (fm_steps_kernel)
-// and kept in shared memory; a rank then costs one rank_support_v probe per
-// level, and sp and ep share the path -- and, once the interval is short, the
-// rank entry and the word.  The last K symbols of a pattern come from a table
+// each symbol's step constants are tabulated once per call (fm_steps_kernel; in
+// scratch of the call, as they hold its C) and kept in shared memory; a rank
+// then costs one rank_support_v probe per level, and sp and ep share the path
+// -- and, once the interval is short, the rank entry and the word.  The last K symbols of a pattern come from a table
 // of the intervals of all strings of K symbols, made once per call where the
 // batch is much larger than the table (wtg_fm_table.cuh).
 #include "wtg_blocks.cuh"
@@ -182,10 +182,9 @@ __global__ void __launch_bounds__(256, 6)
 }
 
 template <bool BLOCKS>
-int fm_run(TreeImpl& t, const uint4* blocks, uint64_t sigma, const uint8_t* pat, const uint64_t* off, uint64_t npat,
+int fm_run(TreeImpl& t, const uint4* blocks, const uint2* steps, uint64_t sigma, const uint8_t* pat, const uint64_t* off, uint64_t npat,
            uint64_t* out, cudaStream_t s) {
-  const FmTree<BLOCKS> v{t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), blocks, t.fm_paths.as<uint2>(), t.n, sigma,
-                         t.levels};
+  const FmTree<BLOCKS> v{t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), blocks, steps, t.n, sigma, t.levels};
   const bool pays = fm_batch_pays(npat, t.levels);
   return with_fm_table<uint2>(
       pays, sigma, npat, s,
@@ -217,9 +216,14 @@ int launch_fm_count(TreeImpl& t, const uint64_t* C, uint64_t sigma, const uint8_
   if (sigma == 0 || sigma > 256 || (t.levels < 63 && sigma > (1ull << t.levels)))
     return fail(WTG_ERR_INVALID, "sigma must be 1..256 and at most 2^levels");
   if (npat == 0) return WTG_OK;
-  if ((rc = t.fm_paths.ensure(sigma * t.levels * sizeof(uint2), s))) return rc;
+  struct Steps : DevBuf {
+    cudaStream_t s;
+    explicit Steps(cudaStream_t st) : s(st) {}
+    ~Steps() { release(s); }
+  } steps(s);
+  if ((rc = steps.ensure(sigma * t.levels * sizeof(uint2), s))) return rc;
   fm_steps_kernel<<<(unsigned)((sigma + 127) / 128), 128, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.n,
-                                                                  t.levels, sigma, C, t.fm_paths.as<uint2>());
+                                                                  t.levels, sigma, C, steps.as<uint2>());
   count_launch();
   WTG_CK(cudaGetLastError());
   // blocks pay once the batch probes a good part of them: making them is a
@@ -228,8 +232,8 @@ int launch_fm_count(TreeImpl& t, const uint64_t* C, uint64_t sigma, const uint8_
   uint4* blocks = fm_batch_pays(npat, t.levels) && npat >= block_count(size) / 8
                       ? make_blocks(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), size, s)
                       : nullptr;
-  rc = blocks ? fm_run<true>(t, blocks, sigma, pat, off, npat, out, s)
-              : fm_run<false>(t, blocks, sigma, pat, off, npat, out, s);
+  rc = blocks ? fm_run<true>(t, blocks, steps.as<uint2>(), sigma, pat, off, npat, out, s)
+              : fm_run<false>(t, blocks, steps.as<uint2>(), sigma, pat, off, npat, out, s);
   if (blocks) cudaFreeAsync(blocks, s);
   return rc;
 }

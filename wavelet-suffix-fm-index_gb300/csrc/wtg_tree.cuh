@@ -35,7 +35,6 @@ struct TreeImpl {
   BvSupport bv;
   DevBuf lvl_args;
   bool lvl_args_ok = false;
-  DevBuf fm_paths;  // per-symbol node paths for FM-index counting
   // node tables (see NodeTables): made by the first query after a build that
   // uses them, on its stream; queries on other streams wait for node_made
   DevBuf node_tab;   // per heap node: bit offset of its start, ones before it
