@@ -50,3 +50,27 @@ def test_balanced_and_huffman(wtg, sigma, n, shift):
         res[name] = whole
     assert torch.equal(res["balanced"], res["huff"])
     assert int(res["huff"][0]) == n
+
+
+@pytest.mark.parametrize("npat", [1000, 1 << 19])  # without and with the interval table
+def test_offsets_that_decrease_are_empty_patterns(wtg, npat):
+    """A device batch's offsets are not checked; nothing outside the patterns is read."""
+    torch = pytest.importorskip("torch")
+    n, st = 1 << 16, torch.cuda.current_stream().cuda_stream
+    rng = np.random.default_rng(npat)
+    text = rng.integers(1, 6, n).astype(np.uint8)
+    text[-1] = 0
+    C = np.zeros(256, dtype=np.uint64)
+    C[1:] = np.cumsum(np.bincount(text, minlength=256))[:-1]
+    off = np.zeros(npat + 1, dtype=np.uint64)
+    off[1::2] = 12  # 0, 12, 0, 12, ..: every second pattern's offsets decrease to 0
+    d_b, d_C, d_off = (torch.from_numpy(x).cuda() for x in (wtg.bwt(text), C.view(np.int64), off.view(np.int64)))
+    d_pat = torch.from_numpy(text[:12].copy()).cuda()
+    torch.cuda.synchronize()
+    fm = wtg.FMIndex.from_device(d_b.data_ptr(), n, 6, st)
+    hf = wtg.HuffmanTree.from_device(d_b.data_ptr(), n, wtg.ALL, st)
+    for f in (fm.count_device, hf.fm_count_device):
+        out = torch.empty(npat, dtype=torch.int64, device="cuda")
+        f(d_C.data_ptr(), d_pat.data_ptr(), d_off.data_ptr(), npat, out.data_ptr(), st)
+        torch.cuda.synchronize()
+        assert bool((out[1::2] == n).all()) and bool((out[::2] >= 1).all()) and bool((out[::2] < n).all())

@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(256, 6)
   uint32_t x = 0, y = (uint32_t)t.n;
   uint64_t i = b;
   bool known = true;  // every symbol read so far is one of the tree's
-  if (K && b - a >= (uint64_t)K) {
+  if (K && b >= a + K) {  // (offsets that decrease: an empty pattern)
     uint32_t at = 0, scale = 1;
     for (int k = 0; k < K; ++k) {
       const uint32_t c = rd.at(--i);

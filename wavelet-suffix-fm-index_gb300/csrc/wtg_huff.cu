@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(256, 5)
   uint32_t x = 0, y = t.n;
   uint64_t i = b;
   bool known = true;  // every symbol read so far is one of the text's
-  if (K && b - a >= (uint64_t)K) {
+  if (K && b >= a + K) {  // (offsets that decrease: an empty pattern)
     uint32_t at = 0, scale = 1;
     for (int k = 0; k < K; ++k) {
       const uint32_t d = s_sym[rd.at(--i)].dense;

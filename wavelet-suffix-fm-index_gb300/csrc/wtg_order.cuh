@@ -26,7 +26,7 @@ static __global__ void __launch_bounds__(256)
     pattern_keys_kernel(const uint64_t* __restrict__ off, uint64_t npat, uint32_t* __restrict__ len) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < npat; k += stride) {
-    const uint64_t m = off[k + 1] - off[k];
+    const uint64_t a = off[k], b = off[k + 1], m = b > a ? b - a : 0;
     len[k] = (uint32_t)(m < 255 ? m : 255);
   }
 }
