@@ -439,16 +439,17 @@ int wtg_bv_serialize(wtg_bv* b, uint32_t part, void* dst, uint64_t cap, uint64_t
  * spins at most `lookback_spins` times (with a backoff of up to 1 us each,
  * default 2^22: seconds), an mbarrier wait tries at most `mbarrier_tries`
  * times (default 2^24).  On expiry the kernel records the failure and
- * returns, and the build's sync reports WTG_ERR_TIMEOUT; the context stays
- * usable.  wtg_set_wait_limits changes both limits for later launches on the
+ * returns, and the sync of the build or query batch reports WTG_ERR_TIMEOUT;
+ * the answers are then incomplete, nothing is written outside the caller's
+ * arrays, and the context stays usable.  wtg_set_wait_limits changes both limits for later launches on the
  * current device (0 restores a default).
  *
  * Test hooks, host side only (they never make a device fault):
  * wtg_test_fail_alloc(k), k >= 1, makes the k-th next device allocation of
  * the library fail with WTG_ERR_OOM (0 disarms); wtg_test_stall_lookback(1)
- * makes the next rank/select pass over a caller bitvector start its tile
- * counter at 1, so tile 0 never publishes its count and the other tiles'
- * look-back waits run out (WTG_ERR_TIMEOUT). */
+ * makes the next rank/select pass, or the next sort of a query batch or of
+ * suffixes, start its tile counter at 1, so tile 0 never publishes its count
+ * and the other tiles' look-back waits run out (WTG_ERR_TIMEOUT). */
 int wtg_set_wait_limits(uint32_t lookback_spins, uint32_t mbarrier_tries);
 int wtg_test_fail_alloc(int64_t nth);
 int wtg_test_stall_lookback(int on);

@@ -205,8 +205,8 @@ int set_wait_limits_range(const uint32_t lim[2]);
 // test_take_alloc_failure() is true for the one device allocation the armed
 // countdown selects (DevBuf::ensure then reports WTG_ERR_OOM);
 // test_take_lookback_stall() is true once after arming, and the rank/select
-// pass then starts its tile counter at 1, so tile 0 never publishes and the
-// other tiles' bounded look-back waits run out.
+// pass or the first pass of a radix sort then starts its tile counter at 1, so
+// tile 0 never publishes and the other tiles' bounded look-back waits run out.
 bool test_take_alloc_failure();
 bool test_take_lookback_stall();
 void test_arm_alloc_failure(int64_t nth);

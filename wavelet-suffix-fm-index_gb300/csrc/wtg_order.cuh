@@ -13,6 +13,8 @@
 
 namespace wtg {
 
+// After a look-back wait that ran out some places of both hold whatever the
+// memory held; a kernel leaves out the ids that are no query of its batch.
 struct QueryOrder {
   const uint32_t* pos;  // positions, sorted by their top bits (n: outside the sequence)
   const uint32_t* id;   // the query each belongs to

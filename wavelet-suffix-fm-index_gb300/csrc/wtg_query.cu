@@ -78,7 +78,7 @@ __global__ void wt_descend_kernel(LevelBits<BLOCKS> bits, const uint2* __restric
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
   const uint64_t i = ORD ? ord.pos[k] : q[k];
-  if (ORD) k = ord.id[k];
+  if (ORD && (k = ord.id[k]) >= nq) return;
   if (i >= n) {
     out[k] = NONE64;
     if (INV) sym_out[k] = NONE64;
@@ -113,7 +113,7 @@ __global__ void wt_rank_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__
                                uint64_t* __restrict__ out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  if (ORD) k = ord.id[k];
+  if (ORD && (k = ord.id[k]) >= nq) return;
   const uint64_t i = q[k];
   const uint64_t c = sym[k];
   if (i > n) {

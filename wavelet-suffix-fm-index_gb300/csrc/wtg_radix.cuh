@@ -260,11 +260,16 @@ int radix_passes(K* const key[2], uint32_t* const val[2], uint64_t n, int lo, in
     uint8_t* st = status + p * per;
     uint32_t* counter = reinterpret_cast<uint32_t*>(st);
     S* words = reinterpret_cast<S*>(st + 16);
+    uint32_t grid = tiles;
+    if (p == 0 && tiles > 1 && test_take_lookback_stall()) {  // tile 0 is never taken, as in bv_prepare
+      WTG_CK(cudaMemsetAsync(counter, 1, 1, s));
+      --grid;
+    }
     if (iota && p == 0)
-      radix_pass_kernel<K, S, true><<<tiles, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo, hist, words, counter,
+      radix_pass_kernel<K, S, true><<<grid, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo, hist, words, counter,
                                                                  key[cur ^ 1], val[cur ^ 1], d_err);
     else
-      radix_pass_kernel<K, S, false><<<tiles, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo + 8 * p,
+      radix_pass_kernel<K, S, false><<<grid, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo + 8 * p,
                                                                   hist + p * RS_RADIX, words, counter, key[cur ^ 1],
                                                                   val[cur ^ 1], d_err);
     count_launch();

@@ -34,7 +34,7 @@ __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t*
                               uint64_t* __restrict__ out_smaller, uint64_t* __restrict__ out_greater) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  if (ORD) k = ord.id[k];
+  if (ORD && (k = ord.id[k]) >= nq) return;
   const uint64_t i = qi[k], j = qj[k], c = qc[k];
   if (i > j || j > n) {
     out_rank[k] = NONE64;
@@ -144,7 +144,7 @@ __global__ void wt_range_count_kernel(const uint64_t* __restrict__ tree, const u
                                       uint64_t nq, uint64_t* __restrict__ out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  if (ORD) k = ord.id[k];
+  if (ORD && (k = ord.id[k]) >= nq) return;
   const uint64_t lb0 = qlb[k], rb0 = qrb[k];
   uint64_t vlb = qvlb[k], vrb = qvrb[k];
   if (lb0 <= rb0 && rb0 >= n) {
