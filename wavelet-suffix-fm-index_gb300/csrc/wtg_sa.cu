@@ -105,7 +105,8 @@ __global__ void active_keys_kernel(const uint32_t* __restrict__ act, const uint3
 // another are compacted into act_next, their ranks beside them.  In round 0
 // (FIRST) every suffix is active, act is the identity and val the suffix
 // array; with rank_of the rank goes beside the suffix for the binned scatter,
-// otherwise to its place.
+// otherwise to its place.  After a wait that ran out (here, or in the sort
+// before) the values are no suffixes in places; those are left out.
 // A warp takes 16 rows of 32 keys; run starts are one ballot a row.
 constexpr int ST_ROWS = 16;
 constexpr int ST_TILE = SA_WARPS * ST_ROWS * 32;
@@ -113,7 +114,7 @@ constexpr int ST_TILE = SA_WARPS * ST_ROWS * 32;
 template <bool FIRST>
 __global__ void __launch_bounds__(SA_THREADS)
     settle_kernel(const uint64_t* __restrict__ key, const uint32_t* __restrict__ val, const uint32_t* __restrict__ act,
-                  uint64_t m, uint32_t* __restrict__ sa, uint32_t* __restrict__ rank, uint32_t* __restrict__ rank_of,
+                  uint64_t m, uint64_t n, uint32_t* __restrict__ sa, uint32_t* __restrict__ rank, uint32_t* __restrict__ rank_of,
                   uint32_t* __restrict__ act_next, uint32_t* __restrict__ act_rank_next,
                   uint32_t* __restrict__ shared_total, uint64_t* status_cnt, uint64_t* status_head, uint32_t* counter,
                   uint32_t* err) {
@@ -190,7 +191,7 @@ __global__ void __launch_bounds__(SA_THREADS)
           while (((v = lb_load(status_head, (uint64_t)p)) >> 62) == 0) {
             if (++spins > c_wait_limit[0]) {
               atomicCAS(err, 0u, (uint32_t)DERR_LOOKBACK_TIMEOUT);
-              v = LB_FLAG_INC;
+              v = LB_FLAG_INC | 1;  // (position 0 is a start)
               break;
             }
             __nanosleep(ns);
@@ -229,7 +230,7 @@ __global__ void __launch_bounds__(SA_THREADS)
       } else {
         const uint32_t i = val[k];
         if (!FIRST) sa[pos] = i;
-        rank[i] = r;
+        if (i < n) rank[i] = r;
       }
       if ((shared >> lane) & 1u) {
         act_next[c + __popc(shared & lt)] = pos;
@@ -252,7 +253,10 @@ __global__ void __launch_bounds__(256) rank_scatter_kernel(const uint32_t* __res
 #pragma unroll
   for (int j = 0; j < RSC_PAIRS; ++j) {
     const uint64_t k = k0 + 256 * j;
-    if (k < n) rank[i[k]] = r[k];
+    if (k < n) {
+      const uint32_t at = i[k];
+      if (at < n) rank[at] = r[k];  // (always, but after a failed look-back of the binning)
+    }
   }
 }
 
@@ -357,7 +361,7 @@ constexpr uint64_t RANK_BIN_MIN = 1ull << 24;
 // after a sort of the m active pairs (in key[cur] / val[cur]): place them,
 // refresh their ranks and compact the still-shared ones into act[ac ^ 1];
 // first: round 0, all suffixes
-static int settle_round(SaScratch& x, uint64_t m, bool first, const uint32_t* val, int cur, int& ac,
+static int settle_round(SaScratch& x, uint64_t m, uint64_t n, bool first, const uint32_t* val, int cur, int& ac,
                         uint64_t* m_next) {
   int rc;
   const uint64_t tiles = (m + ST_TILE - 1) / ST_TILE;
@@ -370,7 +374,7 @@ static int settle_round(SaScratch& x, uint64_t m, bool first, const uint32_t* va
   uint32_t* rank_of = binned ? x.key[cur ^ 1].as<uint32_t>() : nullptr;
   auto* const f = first ? settle_kernel<true> : settle_kernel<false>;
   f<<<(unsigned)tiles, SA_THREADS, 0, x.s>>>(
-      x.key[cur].as<uint64_t>(), val, first ? nullptr : x.act[ac].as<uint32_t>(), m, x.sa, x.rank.as<uint32_t>(),
+      x.key[cur].as<uint64_t>(), val, first ? nullptr : x.act[ac].as<uint32_t>(), m, n, x.sa, x.rank.as<uint32_t>(),
       rank_of, x.act[ac ^ 1].as<uint32_t>(), x.act_rank.as<uint32_t>(), total, st + 1, st + 1 + tiles,
       reinterpret_cast<uint32_t*>(st), x.err.as<uint32_t>());
   count_launch();
@@ -482,7 +486,7 @@ int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8
   uint32_t* const val[2] = {x.val[0].as<uint32_t>(), x.val[1].as<uint32_t>()};
   if ((rc = sort_pairs(x, n, 8 * passes, true, val0, cur))) return rc;
   uint64_t m = 0;
-  if ((rc = settle_round(x, n, true, x.sa, cur, ac, &m))) return rc;
+  if ((rc = settle_round(x, n, n, true, x.sa, cur, ac, &m))) return rc;
   uint64_t h = (uint64_t)K;
   int r = 0;
   const int B = bit_width64(n);               // rank[i + h] + 1 <= n
@@ -494,7 +498,7 @@ int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8
     count_launch();
     WTG_CK(cudaGetLastError());
     if ((rc = sort_pairs(x, m, hi, false, val, cur))) return rc;
-    if ((rc = settle_round(x, m, false, val[cur], cur, ac, &m))) return rc;
+    if ((rc = settle_round(x, m, n, false, val[cur], cur, ac, &m))) return rc;
     h *= 2;
     ++r;
   }
