@@ -825,7 +825,7 @@ struct LevelPass {
     constexpr int BATCH = 4;
     constexpr uint32_t ROOM = (4096 - 256) / 4;  // node starts that the warp's region holds beside the counts
     const uint32_t p_lo = a.cnode[c], nn = a.cnode[c + 1] - p_lo + 1;
-    const bool staged = nn <= ROOM;
+    const bool staged = nn - 1 < ROOM;  // (0 after a count pass's wait that ran out: nodes not in order)
     if (staged) {
       for (uint32_t k = lane; k < nn; k += 32) sts32(base + 256 + 4 * k, __ldg(a.Cl + p_lo + k));
       __syncwarp();
