@@ -415,7 +415,9 @@ __global__ void __launch_bounds__(SD_THREADS)
 // and 64-bit shifts a word and was bound by issue: 0.98 ms of the 2^30 x 20
 // build's 5.2 M superblocks, against 0.3 ms of traffic.)  Wider entries go
 // word by word through shared memory.  The blocks after them: m_superblock,
-// entry i = position of arg 4096*i, width logn.
+// entry i = position of arg 4096*i, width logn.  These kernels and those of the
+// long blocks do nothing after an error: the starts and pool offsets of a pass
+// whose wait ran out lead out of range.
 template <int T_B>
 __device__ __forceinline__ void mini_blocks_warp(const SelBuild& sb, uint64_t i0, const uint32_t* __restrict__ samples,
                                                  uint64_t samp_last, uint32_t (*ent)[64]) {
@@ -487,11 +489,12 @@ __device__ __forceinline__ void mini_blocks_warp(const SelBuild& sb, uint64_t i0
 }
 
 __global__ void __launch_bounds__(256)
-    select_mini_kernel(SelBuild2 sb2, const uint32_t* __restrict__ samples, uint64_t samp_last, uint32_t logn) {
+    select_mini_kernel(SelBuild2 sb2, const uint32_t* __restrict__ samples, uint64_t samp_last, uint32_t logn,
+                       const uint32_t* __restrict__ err) {
   __shared__ uint32_t ent[256 / 32][2][64];
   const int t_b = blockIdx.y;
   const SelBuild& sb = sb2.t[t_b];
-  if (!sb.on) return;
+  if (!sb.on || *err) return;
   const uint64_t mini_blocks = (sb.nsb + 15) / 16;
   if (blockIdx.x >= mini_blocks) {
     const uint64_t q = (blockIdx.x - mini_blocks) * 256 + threadIdx.x;
@@ -515,6 +518,8 @@ __global__ void __launch_bounds__(256)
                             const uint64_t* __restrict__ rank, const uint64_t* __restrict__ starts,
                             const uint64_t* __restrict__ ends, const unsigned long long* info,
                             const uint64_t* __restrict__ long_list, uint64_t* __restrict__ ent, uint32_t* err) {
+  // (uniform over the launch but for an inconsistency that a thread of it reports)
+  if (*(volatile const uint32_t*)err) return;
   const uint64_t gt = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t m = info[t_b ? INF_M1 : INF_M0];
   const uint64_t last = info[t_b ? INF_LAST1 : INF_LAST0];  // last arg position + 1
@@ -553,7 +558,9 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     select_long_pack_kernel(int t_b, const unsigned long long* info, const uint64_t* __restrict__ long_list,
                             const uint64_t* __restrict__ descw, const uint64_t* __restrict__ offs,
-                            const uint64_t* __restrict__ ent, uint64_t* __restrict__ pool) {
+                            const uint64_t* __restrict__ ent, uint64_t* __restrict__ pool,
+                            const uint32_t* __restrict__ err) {
+  if (*err) return;
   const uint64_t nlong = info[t_b ? INF_NLONG1 : INF_NLONG0];
   for (uint64_t li = blockIdx.x; li < nlong; li += gridDim.x) {
     const uint64_t i = long_list[li];
@@ -764,7 +771,7 @@ int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
   }
   if (blocks) {
     prof_begin(PROF_SELECT, s);
-    select_mini_kernel<<<dim3((unsigned)blocks, 2), 256, 0, s>>>(sb, samples, samp_n - 1, logn);
+    select_mini_kernel<<<dim3((unsigned)blocks, 2), 256, 0, s>>>(sb, samples, samp_n - 1, logn, d_err);
     prof_end(PROF_SELECT, s);
     count_launch();
     WTG_CK(cudaGetLastError());
@@ -785,7 +792,7 @@ int bv_finish(BvSupport& bv, uint32_t* d_err, cudaStream_t s) {
     unsigned grid = (unsigned)std::min<uint64_t>(nlong, 8 * 152);
     prof_begin(PROF_SELECT, s);
     select_long_pack_kernel<<<grid, 256, 0, s>>>(t_b, info, sd.long_list.as<uint64_t>(), sb.t[t_b].descw,
-                                                 sb.t[t_b].offs, sd.long_ent.as<uint64_t>(), sd.pool.as<uint64_t>());
+                                                 sb.t[t_b].offs, sd.long_ent.as<uint64_t>(), sd.pool.as<uint64_t>(), d_err);
     prof_end(PROF_SELECT, s);
     count_launch();
     WTG_CK(cudaGetLastError());
