@@ -59,12 +59,18 @@ int check_seq_args(uint64_t n, int eb, int levels, uint32_t flags) {
 // waits for the stream; an error that a kernel reported stays until the next build
 int sync_and_check(cudaStream_t s, ErrWord& err) {
   uint32_t e = 0;
-  if (err.p && err.pending && !err.elsewhere)
-    WTG_CK(cudaMemcpyAsync(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost, s));
-  WTG_CK(cudaStreamSynchronize(s));
+  // (the mark goes before the read: a launch that sets it meanwhile is read next time)
+  const bool read = err.p && err.pending.exchange(false) && !err.elsewhere;
+  cudaError_t ce = cudaSuccess;
+  if (read) ce = cudaMemcpyAsync(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost, s);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
   // (a plain copy also waits for the work of the default stream)
-  if (err.p && err.elsewhere) WTG_CK(cudaMemcpy(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost));
-  if (!e) err.pending = false;
+  if (ce == cudaSuccess && err.p && err.elsewhere) ce = cudaMemcpy(&e, err.p, sizeof(e), cudaMemcpyDeviceToHost);
+  if (ce != cudaSuccess) {
+    err.pending = true;
+    return cuda_fail(ce, "wait for the stream");
+  }
+  if (e) err.pending = true;
   if (e == DERR_LOOKBACK_TIMEOUT) return fail(WTG_ERR_TIMEOUT, "a device-side wait timed out; results are invalid");
   if (e == DERR_BAD_INDEX) return fail(WTG_ERR_CUDA, "a computed index fell outside its buffer (inconsistent tables)");
   if (e) return fail(WTG_ERR_CUDA, "device reported error code " + std::to_string(e));

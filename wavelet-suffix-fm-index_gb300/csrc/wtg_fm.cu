@@ -195,7 +195,7 @@ int fm_run(TreeImpl& t, const uint4* blocks, const uint2* steps, uint64_t sigma,
         return WTG_OK;
       },
       [&](int K, const uint2* table) -> int {
-        return by_length(pays, off, npat, pays ? t.err.arm(s, t.stream) : nullptr, s,
+        return by_length(pays, off, npat, t.err, t.stream, s,
                          [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
                            auto* const f = sorted ? fm_count_kernel<BLOCKS, true> : fm_count_kernel<BLOCKS, false>;
                            f<<<(unsigned)((m + 255) / 256), 256, 0, s>>>(v, K, table, pat, off + at, off + npat, o, m,

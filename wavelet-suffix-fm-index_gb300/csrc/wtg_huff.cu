@@ -931,7 +931,7 @@ static int huff_fm_run(HuffImpl& h, const uint4* blocks, const uint64_t* C, cons
         return WTG_OK;
       },
       [&](int K, const uint2* table) -> int {
-        return by_length(pays, off, npat, pays ? h.err.arm(s, h.stream) : nullptr, s,
+        return by_length(pays, off, npat, h.err, h.stream, s,
                          [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
                            auto* const f = sorted ? huff_count_kernel<BLOCKS, true> : huff_count_kernel<BLOCKS, false>;
                            f<<<(unsigned)((m + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(

@@ -378,14 +378,31 @@ struct DevLayout {
 // A handle's device error word.  Reading it costs 13 us, so it is read only
 // when a kernel that can set it was launched since it was last found clear: on
 // the handle's own stream, the check after the next wait covers the launch;
-// on another stream nothing does, and every later check reads it.
+// on another stream, or from a graph (which may be launched again at any time),
+// nothing does, and every later check reads it.
 struct ErrWord : DevBuf {
-  bool pending = false, elsewhere = false;
+  std::atomic<bool> pending{false}, elsewhere{false};
   uint32_t* arm(cudaStream_t s, cudaStream_t own) {
+    if (s != own || stream_captures(s)) elsewhere = true;
     pending = true;
-    if (s != own) elsewhere = true;
     return as<uint32_t>();
   }
+};
+
+// The error word for the launches of a query call.  Armed once they are
+// enqueued: a check on another thread between the two would clear the mark
+// without having waited for them.
+class ErrUse {
+ public:
+  ErrUse(ErrWord& err, cudaStream_t s, cudaStream_t own) : err_(err), s_(s), own_(own) {}
+  ~ErrUse() { err_.arm(s_, own_); }
+  ErrUse(const ErrUse&) = delete;
+  ErrUse& operator=(const ErrUse&) = delete;
+  uint32_t* word() const { return err_.as<uint32_t>(); }
+
+ private:
+  ErrWord& err_;
+  const cudaStream_t s_, own_;
 };
 
 int scan_exclusive_u32(const uint32_t* in, uint32_t* out, uint64_t n, DevBuf& scratch, uint32_t* d_err,

@@ -107,8 +107,9 @@ int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F la
   if (!order_pays(t, nq, two)) return launch(false, QueryOrder{}, 0, nq);
   constexpr int passes = 2;
   const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
+  const ErrUse err(t.err, s, t.stream);
   return sorted_batches(
-      nq, bits > 8 * passes ? bits - 8 * passes : 0, passes, t.err.arm(s, t.stream), s,
+      nq, bits > 8 * passes ? bits - 8 * passes : 0, passes, err.word(), s,
       [&](uint64_t at, uint64_t m, uint32_t* key) {
         order_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(pos + at, m, t.n, key);
       },
@@ -119,10 +120,12 @@ int in_order(TreeImpl& t, const uint64_t* pos, uint64_t nq, cudaStream_t s, F la
 // as long as its longest pattern, and lengths of 8 to 32 left 48 % of the lanes
 // without work.
 template <typename F>
-int by_length(bool pays, const uint64_t* off, uint64_t npat, uint32_t* d_err, cudaStream_t s, F launch) {
+int by_length(bool pays, const uint64_t* off, uint64_t npat, ErrWord& err_word, cudaStream_t own, cudaStream_t s,
+              F launch) {
   if (!pays) return launch(false, QueryOrder{}, 0, npat);
+  const ErrUse err(err_word, s, own);
   return sorted_batches(
-      npat, 0, 1, d_err, s,
+      npat, 0, 1, err.word(), s,
       [&](uint64_t at, uint64_t m, uint32_t* key) {
         pattern_keys_kernel<<<(unsigned)((m + 2047) / 2048), 256, 0, s>>>(off + at, m, key);
       },
