@@ -294,7 +294,8 @@ int wtg_bwt(const uint8_t* text, uint64_t n, uint8_t* bwt_out, int32_t* sa_out);
 /* device text / outputs on a stream (d_sa or d_bwt may be NULL); returns
  * once the stream has finished; rounds (may be NULL) gets the number of
  * doubling rounds.  Allocates its scratch (about 40 bytes per symbol,
- * 44 without d_sa). */
+ * 44 without d_sa or where it is not device memory on a 4-byte boundary, or
+ * overlaps d_bwt). */
 int wtg_suffix_array_device(const uint8_t* d_text, uint64_t n, int32_t* d_sa, uint8_t* d_bwt, void* stream,
                             int* rounds);
 

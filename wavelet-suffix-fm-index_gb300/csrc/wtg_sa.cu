@@ -331,7 +331,7 @@ unsigned grid_for(uint64_t n) {
 // Scratch of one suffix-array run, released when it ends.
 struct SaScratch {
   DevBuf key[2], val[2], rank, sa_own, act[2], act_rank, hist, status, err, small;
-  uint32_t* sa = nullptr;  // the suffix array: the caller's, or sa_own
+  uint32_t* sa = nullptr;  // the suffix array: in the caller's array, or sa_own
   cudaStream_t s;
   explicit SaScratch(cudaStream_t st) : s(st) {}
   ~SaScratch() {
@@ -403,6 +403,21 @@ static int settle_round(SaScratch& x, uint64_t m, uint64_t n, bool first, const 
   return WTG_OK;
 }
 
+// Whether the suffix array can be made in the caller's array: device memory on
+// 4 bytes, apart from the BWT (which is written while it is read).  Others get a
+// copy at the end.
+static bool usable_in_place(const uint32_t* d_sa, const uint8_t* d_bwt, uint64_t n) {
+  if ((uintptr_t)d_sa % 4) return false;
+  const uintptr_t a = (uintptr_t)d_sa, b = (uintptr_t)d_bwt;
+  if (d_bwt && a < b + n && b < a + 4 * n) return false;
+  cudaPointerAttributes pa{};
+  if (cudaPointerGetAttributes(&pa, d_sa) != cudaSuccess) {
+    cudaGetLastError();  // clear the query's error
+    return false;
+  }
+  return pa.type == cudaMemoryTypeDevice;
+}
+
 int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8_t* d_bwt, int* rounds,
                         cudaStream_t s) {
   int rc;
@@ -410,9 +425,10 @@ int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8
   if (n == 0) return WTG_OK;
   if (n >= (1ull << 31)) return fail(WTG_ERR_INVALID, "suffix array: n must be below 2^31 (32-bit entries)");
   SaScratch x(s);
+  const bool in_place = d_sa && usable_in_place(d_sa, d_bwt, n);
   if ((rc = x.key[0].ensure(n * 8 + 8, s)) || (rc = x.key[1].ensure(n * 8 + 8, s)) ||
       (rc = x.val[0].ensure(n * 4, s)) || (rc = x.val[1].ensure(n * 4, s)) || (rc = x.rank.ensure(n * 4, s)) ||
-      (!d_sa && (rc = x.sa_own.ensure(n * 4, s))) || (rc = x.act[0].ensure(n * 4, s)) || (rc = x.act[1].ensure(n * 4, s)) ||
+      (!in_place && (rc = x.sa_own.ensure(n * 4, s))) || (rc = x.act[0].ensure(n * 4, s)) || (rc = x.act[1].ensure(n * 4, s)) ||
       (rc = x.act_rank.ensure(n * 4, s)) ||
       (rc = x.hist.ensure(RS_MAX_PASSES * RS_RADIX * 4, s)) || (rc = x.err.ensure(4, s)) ||
       (rc = x.small.ensure(2048 + PAIR_SIGMA * PAIR_SIGMA * 4, s)))
@@ -481,7 +497,7 @@ int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8
   // the values of the last pass are the suffix array: it is one of the two
   // value buffers, the one that the number of passes ends in
   int cur = 0, ac = 0;
-  x.sa = d_sa ? d_sa : x.sa_own.as<uint32_t>();
+  x.sa = in_place ? d_sa : x.sa_own.as<uint32_t>();
   uint32_t* const val0[2] = {passes & 1 ? x.val[0].as<uint32_t>() : x.sa, passes & 1 ? x.sa : x.val[0].as<uint32_t>()};
   uint32_t* const val[2] = {x.val[0].as<uint32_t>(), x.val[1].as<uint32_t>()};
   if ((rc = sort_pairs(x, n, 8 * passes, true, val0, cur))) return rc;
@@ -503,6 +519,7 @@ int suffix_array_device(const uint8_t* d_text, uint64_t n, uint32_t* d_sa, uint8
     ++r;
   }
   if (rounds) *rounds = r;
+  if (d_sa && !in_place) WTG_CK(cudaMemcpyAsync(d_sa, x.sa, n * 4, cudaMemcpyDeviceToDevice, s));
   if (d_bwt) {
     if (sigma <= 16 && n >= PACK_MIN) {  // (the keys' buffers are free by now)
       pack_codes_kernel<<<grid_for((n + 7) / 8), 256, 0, s>>>(d_text, n, d_code, x.key[0].as<uint32_t>());
