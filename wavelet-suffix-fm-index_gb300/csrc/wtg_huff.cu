@@ -25,7 +25,8 @@
 // whose code has ended.  On 2^26 zipf bytes (13 depths) the bits took 1.88 ms
 // in a pass per depth, 0.55 ms in groups.
 //
-// Texts above HUFF_OUT bytes (positions beyond 32 bits) take one pass per depth:
+// Texts above HUFF_OUT bytes (positions beyond 32 bits) take one pass per
+// depth, with positions and zero counts in 64 bits:
 //   huff_bits_kernel    the run's bits (one ballot per 32 symbols) and the
 //                       zero count of every 512-symbol chunk;
 //   (scan of the chunk counts)
@@ -94,7 +95,7 @@ namespace {
 // position D + i (ORed, as runs need not start on a word); its zero count
 __global__ void __launch_bounds__(HUFF_THREADS)
     huff_bits_kernel(const uint8_t* __restrict__ src, uint64_t cnt, int d, const uint64_t* __restrict__ path,
-                     uint64_t D, uint64_t* __restrict__ bits, uint32_t* __restrict__ chunkz) {
+                     uint64_t D, uint64_t* __restrict__ bits, uint64_t* __restrict__ chunkz) {
   __shared__ uint64_t s_path[256];
   for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) s_path[i] = path[i];
   __syncthreads();
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(HUFF_THREADS)
 // child the 1s at base1 + (ones before them), modulo 2^64 (unused for a leaf
 // child)
 __global__ void huff_node_kernel(const HuffNodeDev* __restrict__ nodes, const uint16_t* __restrict__ ids, int count,
-                                 uint64_t D, uint64_t Dnext, const uint32_t* __restrict__ chunkpre,
+                                 uint64_t D, uint64_t Dnext, const uint64_t* __restrict__ chunkpre,
                                  const uint64_t* __restrict__ bits, uint64_t* __restrict__ nbase) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= count) return;
@@ -149,7 +150,7 @@ __global__ void huff_node_kernel(const HuffNodeDev* __restrict__ nodes, const ui
 
 __global__ void __launch_bounds__(HUFF_THREADS)
     huff_scatter_kernel(const uint8_t* __restrict__ src, uint64_t cnt, int d, const uint64_t* __restrict__ path,
-                        const uint16_t* __restrict__ node_at, const uint32_t* __restrict__ chunkpre,
+                        const uint16_t* __restrict__ node_at, const uint64_t* __restrict__ chunkpre,
                         const uint64_t* __restrict__ nbase, uint8_t* __restrict__ dst, uint64_t cnt_next,
                         uint32_t* __restrict__ err) {
   __shared__ uint64_t s_path[256];
@@ -786,30 +787,30 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
     if ((rc = h.seq[0].ensure(n, s))) return rc;
     if ((rc = h.seq[1].ensure(n, s))) return rc;
     const uint64_t nch = (n + HUFF_CHUNK - 1) / HUFF_CHUNK;
-    if ((rc = h.chunkz.ensure((nch + 1) * sizeof(uint32_t), s))) return rc;
-    if ((rc = h.chunkpre.ensure((nch + 1) * sizeof(uint32_t), s))) return rc;
+    if ((rc = h.chunkz.ensure((nch + 1) * sizeof(uint64_t), s))) return rc;
+    if ((rc = h.chunkpre.ensure((nch + 1) * sizeof(uint64_t), s))) return rc;
     const uint8_t* src = d_text;
     size_t idoff = 0;
     for (int d = 0; d < depths && cntd[d]; ++d) {
       const uint64_t cnt = cntd[d], chunks = (cnt + HUFF_CHUNK - 1) / HUFF_CHUNK;
       const unsigned grid = hgrid(chunks, HUFF_THREADS / 32, 152 * 16);
       huff_bits_kernel<<<grid, HUFF_THREADS, 0, s>>>(src, cnt, d, h.dpath.as<uint64_t>(), D[d],
-                                                     h.bits.as<uint64_t>(), h.chunkz.as<uint32_t>());
+                                                     h.bits.as<uint64_t>(), h.chunkz.as<uint64_t>());
       count_launch();
       WTG_CK(cudaGetLastError());
-      if ((rc = scan_exclusive_u32(h.chunkz.as<uint32_t>(), h.chunkpre.as<uint32_t>(), chunks, h.scan_tmp, d_err,
+      if ((rc = scan_exclusive_u64(h.chunkz.as<uint64_t>(), h.chunkpre.as<uint64_t>(), chunks, h.scan_tmp, d_err,
                                    s)))
         return rc;
       const int cnt_nodes = (int)inner[d].size();
       if (d + 1 < depths && cntd[d + 1]) {
         huff_node_kernel<<<(cnt_nodes + 127) / 128, 128, 0, s>>>(
             h.dnodes.as<HuffNodeDev>(), dids.as<uint16_t>() + idoff, cnt_nodes, D[d], D[d + 1],
-            h.chunkpre.as<uint32_t>(), h.bits.as<uint64_t>(), h.nbase.as<uint64_t>());
+            h.chunkpre.as<uint64_t>(), h.bits.as<uint64_t>(), h.nbase.as<uint64_t>());
         count_launch();
         WTG_CK(cudaGetLastError());
         uint8_t* dst = h.seq[d & 1].as<uint8_t>();
         huff_scatter_kernel<<<grid, HUFF_THREADS, 0, s>>>(src, cnt, d, h.dpath.as<uint64_t>(),
-                                                          h.dnode_at.as<uint16_t>(), h.chunkpre.as<uint32_t>(),
+                                                          h.dnode_at.as<uint16_t>(), h.chunkpre.as<uint64_t>(),
                                                           h.nbase.as<uint64_t>(), dst, cntd[d + 1], d_err);
         count_launch();
         WTG_CK(cudaGetLastError());
