@@ -682,6 +682,66 @@ static int huff_group_passes(HuffImpl& h, const uint8_t* d_text, const std::vect
   return WTG_OK;
 }
 
+// the same in a pass per depth, for texts that the group passes do not take
+static int huff_depth_passes(HuffImpl& h, const uint8_t* d_text, const std::vector<std::vector<uint16_t>>& inner,
+                             const std::vector<uint64_t>& D, const std::vector<uint64_t>& cntd, uint32_t* d_err,
+                             cudaStream_t s) {
+  int rc;
+  const uint64_t n = h.n;
+  const int depths = h.maxlen;
+  // per depth the node on each byte's path, and the inner nodes breadth first
+  std::vector<uint16_t> node_at((size_t)depths * 256, HUFF_NONE), ids;
+  for (int c = 0; c < 256; ++c) {
+    if (h.leaf[c] < 0) continue;
+    int u = 0;
+    for (int d = 0; d < h.len[c]; ++d) {
+      node_at[(size_t)d * 256 + c] = (uint16_t)u;
+      u = h.nodes[u].child[(h.path[c] >> d) & 1];
+    }
+  }
+  for (const std::vector<uint16_t>& v : inner) ids.insert(ids.end(), v.begin(), v.end());
+  if ((rc = h.dnode_at.ensure(node_at.size() * sizeof(uint16_t), s))) return rc;
+  if ((rc = h.nbase.ensure(2 * h.nodes.size() * sizeof(uint64_t), s))) return rc;
+  if ((rc = h.ids.ensure(ids.size() * sizeof(uint16_t), s))) return rc;
+  WTG_CK(cudaMemcpyAsync(h.dnode_at.p, node_at.data(), node_at.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
+  WTG_CK(cudaMemcpyAsync(h.ids.p, ids.data(), ids.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
+  if ((rc = h.seq[0].ensure(n, s))) return rc;
+  if ((rc = h.seq[1].ensure(n, s))) return rc;
+  const uint64_t nch = (n + HUFF_CHUNK - 1) / HUFF_CHUNK;
+  if ((rc = h.chunkz.ensure((nch + 1) * sizeof(uint64_t), s))) return rc;
+  if ((rc = h.chunkpre.ensure((nch + 1) * sizeof(uint64_t), s))) return rc;
+  const uint8_t* src = d_text;
+  size_t idoff = 0;
+  for (int d = 0; d < depths && cntd[d]; ++d) {
+    const uint64_t cnt = cntd[d], chunks = (cnt + HUFF_CHUNK - 1) / HUFF_CHUNK;
+    const unsigned grid = hgrid(chunks, HUFF_THREADS / 32, 152 * 16);
+    huff_bits_kernel<<<grid, HUFF_THREADS, 0, s>>>(src, cnt, d, h.dpath.as<uint64_t>(), D[d],
+                                                   h.bits.as<uint64_t>(), h.chunkz.as<uint64_t>());
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    if ((rc = scan_exclusive_u64(h.chunkz.as<uint64_t>(), h.chunkpre.as<uint64_t>(), chunks, h.scan_tmp, d_err,
+                                 s)))
+      return rc;
+    const int cnt_nodes = (int)inner[d].size();
+    if (d + 1 < depths && cntd[d + 1]) {
+      huff_node_kernel<<<(cnt_nodes + 127) / 128, 128, 0, s>>>(
+          h.dnodes.as<HuffNodeDev>(), h.ids.as<uint16_t>() + idoff, cnt_nodes, D[d], D[d + 1],
+          h.chunkpre.as<uint64_t>(), h.bits.as<uint64_t>(), h.nbase.as<uint64_t>());
+      count_launch();
+      WTG_CK(cudaGetLastError());
+      uint8_t* dst = h.seq[d & 1].as<uint8_t>();
+      huff_scatter_kernel<<<grid, HUFF_THREADS, 0, s>>>(src, cnt, d, h.dpath.as<uint64_t>(),
+                                                        h.dnode_at.as<uint16_t>(), h.chunkpre.as<uint64_t>(),
+                                                        h.nbase.as<uint64_t>(), dst, cntd[d + 1], d_err);
+      count_launch();
+      WTG_CK(cudaGetLastError());
+      src = dst;
+    }
+    idoff += cnt_nodes;
+  }
+  return WTG_OK;
+}
+
 int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
   int rc;
   cudaStream_t s = h.stream;
@@ -711,7 +771,7 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
   const uint64_t W = (h.size + 63) / 64;
   if ((rc = h.bits.ensure((W + 2) * sizeof(uint64_t), s))) return rc;
   WTG_CK(cudaMemsetAsync(h.bits.p, 0, (W + 2) * sizeof(uint64_t), s));
-  // node table, codes, and per depth the node on each byte's path
+  // node table and codes
   std::vector<HuffNodeDev> hn(std::max(nn, 1));
   for (int v = 0; v < nn; ++v) {
     const HuffImpl::Node& u = h.nodes[v];
@@ -729,24 +789,11 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
     lf[c] = h.leaf[c] < 0 ? HUFF_NONE : (uint16_t)h.leaf[c];
   }
   const int depths = std::max(h.maxlen, 1);
-  std::vector<uint16_t> node_at((size_t)depths * 256, HUFF_NONE);
-  for (int c = 0; c < 256; ++c) {
-    if (h.leaf[c] < 0) continue;
-    int u = 0;
-    for (int d = 0; d < h.len[c]; ++d) {
-      node_at[(size_t)d * 256 + c] = (uint16_t)u;
-      u = h.nodes[u].child[(h.path[c] >> d) & 1];
-    }
-  }
   if ((rc = h.dnodes.ensure(hn.size() * sizeof(HuffNodeDev), s))) return rc;
   if ((rc = h.dpath.ensure(256 * (sizeof(uint64_t) + sizeof(uint16_t)), s))) return rc;
-  if ((rc = h.dnode_at.ensure(node_at.size() * sizeof(uint16_t), s))) return rc;
-  if ((rc = h.nbase.ensure(2 * std::max(nn, 1) * sizeof(uint64_t), s))) return rc;
   WTG_CK(cudaMemcpyAsync(h.dnodes.p, hn.data(), hn.size() * sizeof(HuffNodeDev), cudaMemcpyHostToDevice, s));
   WTG_CK(cudaMemcpyAsync(h.dpath.p, pl, sizeof(pl), cudaMemcpyHostToDevice, s));
   WTG_CK(cudaMemcpyAsync((uint8_t*)h.dpath.p + sizeof(pl), lf, sizeof(lf), cudaMemcpyHostToDevice, s));
-  WTG_CK(cudaMemcpyAsync(h.dnode_at.p, node_at.data(), node_at.size() * sizeof(uint16_t), cudaMemcpyHostToDevice,
-                         s));
   // per depth: its inner nodes (breadth-first order), the run start D and the sequence length
   std::vector<std::vector<uint16_t>> inner(depths + 1);
   for (int v = 0; v < nn; ++v)
@@ -757,8 +804,6 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
       D[d] = h.nodes[inner[d][0]].bv_pos;
       for (uint16_t v : inner[d]) cntd[d] += h.nodes[v].freq;
     }
-  std::vector<uint16_t> ids;
-  for (int d = 0; d <= depths; ++d) ids.insert(ids.end(), inner[d].begin(), inner[d].end());
   {
     static_assert(HF_MAX_DEPTH >= 64, "");
     HuffFmInfo fi;
@@ -777,47 +822,10 @@ int huff_build(HuffImpl& h, const uint8_t* d_text, uint64_t n, uint32_t flags) {
     if ((rc = h.fminfo.ensure(sizeof(HuffFmInfo), s))) return rc;
     WTG_CK(cudaMemcpyAsync(h.fminfo.p, &fi, sizeof(fi), cudaMemcpyHostToDevice, s));
   }
-  DevBuf& dids = h.ids;
-  if ((rc = dids.ensure(std::max<size_t>(ids.size(), 1) * sizeof(uint16_t), s))) return rc;
-  if (!ids.empty())
-    WTG_CK(cudaMemcpyAsync(dids.p, ids.data(), ids.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, s));
   if (n && h.size && n <= HUFF_OUT) {
     if ((rc = huff_group_passes(h, d_text, inner, D, cntd, d_err, s))) return rc;
   } else if (n && h.size) {
-    if ((rc = h.seq[0].ensure(n, s))) return rc;
-    if ((rc = h.seq[1].ensure(n, s))) return rc;
-    const uint64_t nch = (n + HUFF_CHUNK - 1) / HUFF_CHUNK;
-    if ((rc = h.chunkz.ensure((nch + 1) * sizeof(uint64_t), s))) return rc;
-    if ((rc = h.chunkpre.ensure((nch + 1) * sizeof(uint64_t), s))) return rc;
-    const uint8_t* src = d_text;
-    size_t idoff = 0;
-    for (int d = 0; d < depths && cntd[d]; ++d) {
-      const uint64_t cnt = cntd[d], chunks = (cnt + HUFF_CHUNK - 1) / HUFF_CHUNK;
-      const unsigned grid = hgrid(chunks, HUFF_THREADS / 32, 152 * 16);
-      huff_bits_kernel<<<grid, HUFF_THREADS, 0, s>>>(src, cnt, d, h.dpath.as<uint64_t>(), D[d],
-                                                     h.bits.as<uint64_t>(), h.chunkz.as<uint64_t>());
-      count_launch();
-      WTG_CK(cudaGetLastError());
-      if ((rc = scan_exclusive_u64(h.chunkz.as<uint64_t>(), h.chunkpre.as<uint64_t>(), chunks, h.scan_tmp, d_err,
-                                   s)))
-        return rc;
-      const int cnt_nodes = (int)inner[d].size();
-      if (d + 1 < depths && cntd[d + 1]) {
-        huff_node_kernel<<<(cnt_nodes + 127) / 128, 128, 0, s>>>(
-            h.dnodes.as<HuffNodeDev>(), dids.as<uint16_t>() + idoff, cnt_nodes, D[d], D[d + 1],
-            h.chunkpre.as<uint64_t>(), h.bits.as<uint64_t>(), h.nbase.as<uint64_t>());
-        count_launch();
-        WTG_CK(cudaGetLastError());
-        uint8_t* dst = h.seq[d & 1].as<uint8_t>();
-        huff_scatter_kernel<<<grid, HUFF_THREADS, 0, s>>>(src, cnt, d, h.dpath.as<uint64_t>(),
-                                                          h.dnode_at.as<uint16_t>(), h.chunkpre.as<uint64_t>(),
-                                                          h.nbase.as<uint64_t>(), dst, cntd[d + 1], d_err);
-        count_launch();
-        WTG_CK(cudaGetLastError());
-        src = dst;
-      }
-      idoff += cnt_nodes;
-    }
+    if ((rc = huff_depth_passes(h, d_text, inner, D, cntd, d_err, s))) return rc;
   }
   // rank / select supports and the node ranks
   if (flags) {
