@@ -56,11 +56,6 @@ __global__ void fm_steps_kernel(const uint64_t* __restrict__ tree, const uint64_
   }
 }
 
-__device__ __forceinline__ uint32_t fm_rank(const ulonglong2& e, uint64_t word, uint64_t pos) {
-  const uint32_t in = (uint32_t)(e.y >> (63 - 9 * ((uint32_t)(pos >> 6) & 7))) & 0x1FFu;
-  return (uint32_t)e.x + in + __popcll(word & ((1ull << (pos & 63)) - 1));
-}
-
 // the tree with its rank table (BLOCKS false) or as 192-bit blocks
 template <bool BLOCKS>
 struct FmTree {
@@ -98,8 +93,8 @@ struct FmTree {
         ey = __ldg(re + (py >> 9));
         wy = __ldg(tree + (py >> 6));
       }
-      rx = fm_rank(ex, wx, px);
-      ry = fm_rank(ey, wy, py);
+      rx = entry_rank(ex, wx, px);
+      ry = entry_rank(ey, wy, py);
     }
   }
   // prepends symbol c (< sigma) to the interval [x, y)

@@ -80,10 +80,6 @@ __global__ void __launch_bounds__(SA_THREADS)
 // suffixes by (rank, rank of the suffix h on) lays the groups out in
 // position order again, so the k-th sorted suffix goes to position act[k].
 
-__device__ __forceinline__ bool run_start(const uint64_t* __restrict__ key, uint64_t k) {
-  return k == 0 || key[k] != key[k - 1];
-}
-
 // key of active suffix k: (its rank, rank[i + h] + 1, or 0 past the end) for
 // i = sa[act[k]]
 __global__ void active_keys_kernel(const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_rank,
