@@ -72,11 +72,8 @@ static __global__ void __launch_bounds__(256)
 // stream; null when there is no room for them.
 inline uint4* make_blocks(const uint64_t* words, const uint64_t* rt, uint64_t size, cudaStream_t s) {
   const uint64_t count = block_count(size);
-  uint4* blocks = nullptr;
-  if (cudaMallocAsync(&blocks, count * 32, s) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
+  uint4* const blocks = (uint4*)try_scratch(count * 32, s);
+  if (!blocks) return nullptr;
   blocks_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(words, rt, (size + 63) / 64, count, blocks);
   count_launch();
   if (cudaGetLastError() != cudaSuccess) {

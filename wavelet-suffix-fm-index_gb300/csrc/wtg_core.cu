@@ -96,6 +96,15 @@ int DevBuf::ensure(size_t need, cudaStream_t s) {
   return WTG_OK;
 }
 
+void* try_scratch(size_t bytes, cudaStream_t s) {
+  void* p = nullptr;
+  if (test_take_alloc_failure() || cudaMallocAsync(&p, bytes, s) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
 void DevBuf::release(cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
   p = nullptr;

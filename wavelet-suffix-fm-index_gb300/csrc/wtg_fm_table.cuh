@@ -51,11 +51,8 @@ int with_fm_table(bool pays, uint64_t sigma, uint64_t npat, cudaStream_t s, Make
   if (!K) return count(0, (const V*)nullptr);
   uint64_t entries = 1;
   for (int k = 0; k < K; ++k) entries *= sigma;
-  V* buf = nullptr;
-  if (cudaMallocAsync(&buf, 2 * entries * sizeof(V), s) != cudaSuccess) {
-    cudaGetLastError();
-    return count(0, (const V*)nullptr);
-  }
+  V* const buf = (V*)try_scratch(2 * entries * sizeof(V), s);
+  if (!buf) return count(0, (const V*)nullptr);
   // strings of k symbols alternate between the halves and end in the first
   int rc = WTG_OK;
   const V* prev = nullptr;

@@ -356,6 +356,10 @@ struct DevBuf {
   T* as() const { return (T*)p; }
 };
 
+// Scratch of one call that can also do without it (cudaFreeAsync gives it
+// back); null, and no error, where there is no room.
+void* try_scratch(size_t bytes, cudaStream_t s);
+
 // A part of a DevBuf, which owns it.
 struct DevPart {
   void* p = nullptr;

@@ -74,11 +74,8 @@ int sorted_batches(uint64_t nq, int lo, int passes, uint32_t* d_err, cudaStream_
   const uint64_t most = nq < ORDER_BATCH ? nq : ORDER_BATCH;
   const uint64_t pairs = (most + 63) / 64 * 64;
   const uint64_t bytes = 16 * pairs + passes * RS_RADIX * 4 + radix_status_bytes(most, passes);
-  uint8_t* scratch = nullptr;
-  if (cudaMallocAsync(&scratch, bytes, s) != cudaSuccess) {
-    cudaGetLastError();  // no room: the queries as they come
-    return launch(false, QueryOrder{}, 0, nq);
-  }
+  uint8_t* const scratch = (uint8_t*)try_scratch(bytes, s);
+  if (!scratch) return launch(false, QueryOrder{}, 0, nq);  // no room: the queries as they come
   uint32_t* const key[2] = {(uint32_t*)scratch, (uint32_t*)scratch + pairs};
   uint32_t* const val[2] = {(uint32_t*)scratch + 2 * pairs, (uint32_t*)scratch + 3 * pairs};
   uint32_t* hist = (uint32_t*)scratch + 4 * pairs;

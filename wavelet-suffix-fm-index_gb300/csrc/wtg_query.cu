@@ -390,8 +390,10 @@ static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t 
   if (nodes.rc) return nodes.rc;
   const uint64_t* const words = t.bits.as<uint64_t>();
   const uint64_t* const rt = t.bv.rank.as<uint64_t>();
-  uint4* const blocks = blocks_pay(t, nq) ? make_blocks(words, rt, t.n * (uint64_t)t.levels, s) : nullptr;
+  uint4* blocks = nullptr;
   const int rc = in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+    // (once the sort has its scratch, which comes first)
+    if (sorted && !at && blocks_pay(t, nq)) blocks = make_blocks(words, rt, t.n * (uint64_t)t.levels, s);
     if (sorted && blocks) launch(nodes, LevelBits<true>{words, rt, blocks}, std::true_type{}, o, at, m);
     else if (sorted) launch(nodes, LevelBits<false>{words, rt, nullptr}, std::true_type{}, o, at, m);
     else launch(nodes, LevelBits<false>{words, rt, nullptr}, std::false_type{}, o, at, m);
