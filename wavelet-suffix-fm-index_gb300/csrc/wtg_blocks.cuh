@@ -51,32 +51,40 @@ __device__ __forceinline__ uint64_t block_of(uint64_t pos, uint32_t& off) {
 
 static __global__ void __launch_bounds__(256)
     blocks_kernel(const uint64_t* __restrict__ words, const uint64_t* __restrict__ rt, uint64_t nwords, uint64_t count,
-                  uint4* __restrict__ blocks) {
-  const uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= count) return;
-  uint64_t w[3];
+                  uint4* __restrict__ blocks, const uint32_t* __restrict__ wanted) {
+  if (wanted && !*wanted) return;
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < count; b += stride) {
+    uint64_t w[3];
 #pragma unroll
-  for (int k = 0; k < 3; ++k) w[k] = 3 * b + k < nwords ? __ldg(words + 3 * b + k) : 0ull;
-  const uint64_t first = 3 * b;
-  const uint64_t* e = rt + 2 * (first >> 3);
-  const uint32_t k = (uint32_t)first & 7;
-  const uint32_t ones = (uint32_t)__ldg(e) + (k ? (uint32_t)(__ldg(e + 1) >> (63 - 9 * k)) & 0x1FFu : 0u);
-  const uint32_t c1 = __popcll(w[0]), c2 = c1 + __popcll(w[1]);
-  uint64_t* o = reinterpret_cast<uint64_t*>(blocks + 2 * b);
-  const uint64_t head = (uint64_t)ones | ((uint64_t)c1 << 32) | ((uint64_t)c2 << 40);
-  *reinterpret_cast<ulonglong2*>(o) = make_ulonglong2(head, w[0]);
-  *reinterpret_cast<ulonglong2*>(o + 2) = make_ulonglong2(w[1], w[2]);
+    for (int k = 0; k < 3; ++k) w[k] = 3 * b + k < nwords ? __ldg(words + 3 * b + k) : 0ull;
+    const uint64_t first = 3 * b;
+    const uint64_t* e = rt + 2 * (first >> 3);
+    const uint32_t k = (uint32_t)first & 7;
+    const uint32_t ones = (uint32_t)__ldg(e) + (k ? (uint32_t)(__ldg(e + 1) >> (63 - 9 * k)) & 0x1FFu : 0u);
+    const uint32_t c1 = __popcll(w[0]), c2 = c1 + __popcll(w[1]);
+    uint64_t* o = reinterpret_cast<uint64_t*>(blocks + 2 * b);
+    const uint64_t head = (uint64_t)ones | ((uint64_t)c1 << 32) | ((uint64_t)c2 << 40);
+    *reinterpret_cast<ulonglong2*>(o) = make_ulonglong2(head, w[0]);
+    *reinterpret_cast<ulonglong2*>(o + 2) = make_ulonglong2(w[1], w[2]);
+  }
 }
 
-// The blocks of a bitvector of `size` bits (nwords words) in scratch of the
-// stream; null when there is no room for them.
-inline uint4* make_blocks(const uint64_t* words, const uint64_t* rt, uint64_t size, cudaStream_t s) {
-  const uint64_t count = block_count(size);
-  uint4* const blocks = (uint4*)try_scratch(count * 32, s);
-  if (!blocks) return nullptr;
-  blocks_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(words, rt, (size + 63) / 64, count, blocks);
+// Fills the blocks of a bitvector of `size` bits; wanted: a device word, and
+// nothing is done where it is 0 (the grid is bounded so that this takes no time).
+inline bool fill_blocks(uint4* blocks, const uint64_t* words, const uint64_t* rt, uint64_t size,
+                        const uint32_t* wanted, cudaStream_t s) {
+  const uint64_t count = block_count(size), ctas = (count + 255) / 256;
+  blocks_kernel<<<(unsigned)(ctas < 152 * 64 ? ctas : 152 * 64), 256, 0, s>>>(words, rt, (size + 63) / 64, count, blocks,
+                                                                            wanted);
   count_launch();
-  if (cudaGetLastError() != cudaSuccess) {
+  return cudaGetLastError() == cudaSuccess;
+}
+
+// The blocks in scratch of the stream; null when there is no room for them.
+inline uint4* make_blocks(const uint64_t* words, const uint64_t* rt, uint64_t size, cudaStream_t s) {
+  uint4* const blocks = (uint4*)try_scratch(block_count(size) * 32, s);
+  if (blocks && !fill_blocks(blocks, words, rt, size, nullptr, s)) {
     cudaFreeAsync(blocks, s);
     return nullptr;
   }

@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(256, 6)
   const uint2* const st = in_smem ? s_steps : t.steps;
   uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m) return;
-  if (ORD && (p = ord.id[p]) >= m) return;
+  if (ORD && !ordered_query(ord, m, p)) return;
   const uint64_t a = off[p], b = off[p + 1];
   PatternReader rd(pat, *total);
   uint32_t x = 0, y = (uint32_t)t.n;

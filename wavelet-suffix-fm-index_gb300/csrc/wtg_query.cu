@@ -71,19 +71,10 @@ struct LevelBits {
 // wt_int::operator[] (wt_int/wt_int_par.hpp:519-541) and inverse_select
 // (:588-611): descend by the bit at i; the symbol is the path, the rank the
 // final position
-template <bool INV, bool ORD, bool BLOCKS>
-__global__ void wt_descend_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
-                                  QueryOrder ord, uint64_t nq, uint64_t* __restrict__ out,
-                                  uint64_t* __restrict__ sym_out) {
-  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nq) return;
-  const uint64_t i = ORD ? ord.pos[k] : q[k];
-  if (ORD && (k = ord.id[k]) >= nq) return;
-  if (i >= n) {
-    out[k] = NONE64;
-    if (INV) sym_out[k] = NONE64;
-    return;
-  }
+template <bool INV, bool BLOCKS>
+__device__ __forceinline__ void descend(const LevelBits<BLOCKS>& bits, const uint2* __restrict__ step, uint64_t n, int L,
+                                        uint64_t i, uint64_t k, uint64_t* __restrict__ out,
+                                        uint64_t* __restrict__ sym_out) {
   uint32_t x = (uint32_t)i, h = 1;  // h: heap id + 1, the path with a leading 1
   uint64_t lbase = 0;
   uint2 st = __ldg(step + 1);
@@ -106,14 +97,77 @@ __global__ void wt_descend_kernel(LevelBits<BLOCKS> bits, const uint2* __restric
   }
 }
 
+// A batch that came in order (see order_check_kernel) is read as it is, without
+// the blocks, which were not made for it.
+template <bool INV, bool ORD, bool BLOCKS>
+__global__ void wt_descend_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__ step, uint64_t n, int L,
+                                  const uint64_t* __restrict__ q, QueryOrder ord, uint64_t nq,
+                                  uint64_t* __restrict__ out, uint64_t* __restrict__ sym_out) {
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nq) return;
+  const bool as_is = !ORD || ord.flags[AS_IS];
+  const uint64_t i = as_is ? q[k] : ord.pos[k];
+  if (ORD && !ordered_query(ord, nq, k)) return;
+  if (i >= n) {
+    out[k] = NONE64;
+    if (INV) sym_out[k] = NONE64;
+    return;
+  }
+  if (BLOCKS && as_is) descend<INV>(LevelBits<false>{bits.tree, bits.rt, nullptr}, step, n, L, i, k, out, sym_out);
+  else descend<INV>(bits, step, n, L, i, k, out, sym_out);
+}
+
 // wt_int::rank (wt_int_par.hpp:553-577): descend along c's path
+template <bool BLOCKS>
+__device__ __forceinline__ uint32_t rank_along(const LevelBits<BLOCKS>& bits, const uint2* __restrict__ step, uint64_t n,
+                                               int L, uint32_t x, uint32_t c) {
+  const uint32_t path = c | (1u << L);
+  uint64_t lbase = 0;
+  uint2 st = __ldg(step + 1);
+  for (int lv = 0; lv < L; ++lv, lbase += n) {
+    const uint2 next = __ldg(step + (path >> (lv + 1 < L ? L - 1 - lv : L)));  // one level ahead
+    uint32_t bit;
+    const uint32_t R = bits.rank(lbase + x, bit);
+    x = (path >> (L - 1 - lv)) & 1u ? st.y + R : st.x + x - R;
+    st = next;
+  }
+  return x;
+}
+
+// the same by node entries (see the far kernels).  (The test of the offset is
+// the compiler's better code: 2^22 consecutive positions, 2^28 symbols x 20
+// levels 363 us, without it 391.)
+__device__ __forceinline__ uint64_t rank_far(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                             const ulonglong2* __restrict__ tab, int L, uint64_t i, uint64_t c) {
+  uint64_t h = 0;
+  ulonglong2 nd = __ldg(tab);
+  for (int lv = 0; lv < L && i; ++lv) {
+    const uint64_t bit = (c >> (L - 1 - lv)) & 1;
+    const uint64_t child = 2 * h + 1 + bit;
+    ulonglong2 next = nd;
+    if (lv + 1 < L) next = __ldg(tab + child);
+    const uint64_t pos = nd.x + i;
+    const uint64_t word = load_word(tree, pos);
+    const ulonglong2 e = load_entry(rt, pos);
+    uint64_t r = e.x + ((e.y >> (63 - 9 * ((pos & 0x1FF) >> 6))) & 0x1FF);
+    if (pos & 63) r += __popcll(word & ((1ull << (pos & 63)) - 1));
+    r -= nd.y;
+    i = bit ? r : i - r;
+    h = child;
+    nd = next;
+  }
+  return i;
+}
+
+// far: a batch that came in order goes by node entries (see launch_wt_rank)
 template <bool ORD, bool BLOCKS>
-__global__ void wt_rank_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__ step, uint64_t n, int L, const uint64_t* __restrict__ q,
-                               QueryOrder ord, const uint64_t* __restrict__ sym, uint64_t nq,
+__global__ void wt_rank_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__ step,
+                               const ulonglong2* __restrict__ tab, uint64_t n, int L, const uint64_t* __restrict__ q,
+                               QueryOrder ord, bool far, const uint64_t* __restrict__ sym, uint64_t nq,
                                uint64_t* __restrict__ out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  if (ORD && (k = ord.id[k]) >= nq) return;
+  if (ORD && !ordered_query(ord, nq, k)) return;
   const uint64_t i = q[k];
   const uint64_t c = sym[k];
   if (i > n) {
@@ -124,18 +178,11 @@ __global__ void wt_rank_kernel(LevelBits<BLOCKS> bits, const uint2* __restrict__
     out[k] = 0;
     return;
   }
-  const uint32_t path = (uint32_t)c | (1u << L);
-  uint32_t x = (uint32_t)i;
-  uint64_t lbase = 0;
-  uint2 st = __ldg(step + 1);
-  for (int lv = 0; lv < L; ++lv, lbase += n) {
-    const uint2 next = __ldg(step + (path >> (lv + 1 < L ? L - 1 - lv : L)));  // one level ahead
-    uint32_t bit;
-    const uint32_t R = bits.rank(lbase + x, bit);
-    x = (path >> (L - 1 - lv)) & 1u ? st.y + R : st.x + x - R;
-    st = next;
-  }
-  out[k] = x;
+  const bool as_is = ORD && ord.flags[AS_IS];
+  if (as_is && far) out[k] = rank_far(bits.tree, bits.rt, tab, L, i, c);
+  else if (as_is)
+    out[k] = rank_along(LevelBits<false>{bits.tree, bits.rt, nullptr}, step, n, L, (uint32_t)i, (uint32_t)c);
+  else out[k] = rank_along(bits, step, n, L, (uint32_t)i, (uint32_t)c);
 }
 
 // Descents of batches that are not sorted, over trees larger than L2: node
@@ -199,7 +246,7 @@ __global__ void wt_rank_far_kernel(const uint64_t* __restrict__ tree, const uint
                                    uint64_t* __restrict__ out) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  uint64_t i = q[k];
+  const uint64_t i = q[k];
   const uint64_t c = sym[k];
   if (i > n) {
     out[k] = NONE64;
@@ -209,21 +256,7 @@ __global__ void wt_rank_far_kernel(const uint64_t* __restrict__ tree, const uint
     out[k] = 0;
     return;
   }
-  uint64_t h = 0;
-  ulonglong2 nd = __ldg(tab);
-  for (int lv = 0; lv < L && i; ++lv) {
-    const uint64_t bit = (c >> (L - 1 - lv)) & 1;
-    const uint64_t child = 2 * h + 1 + bit;
-    ulonglong2 next = nd;
-    if (lv + 1 < L) next = __ldg(tab + child);
-    const uint64_t pos = nd.x + i;
-    const uint64_t word = load_word(tree, pos);
-    const uint64_t r = entry_rank64(load_entry(rt, pos), word, pos) - nd.y;
-    i = bit ? r : i - r;
-    h = child;
-    nd = next;
-  }
-  out[k] = i;
+  out[k] = rank_far(tree, rt, tab, L, i, c);
 }
 
 // wt_int::select (wt_int_par.hpp:622-660): down c's path for the nodes' starts
@@ -392,8 +425,13 @@ static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t 
   const uint64_t* const rt = t.bv.rank.as<uint64_t>();
   uint4* blocks = nullptr;
   const int rc = in_order(t, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
-    // (once the sort has its scratch, which comes first)
-    if (sorted && !at && blocks_pay(t, nq)) blocks = make_blocks(words, rt, t.n * (uint64_t)t.levels, s);
+    if (sorted && blocks_pay(t, nq)) {
+      // (once the sort has its scratch, which comes first; by the first batch that does not come in order)
+      const uint64_t size = t.n * (uint64_t)t.levels;
+      if (!at) blocks = (uint4*)try_scratch(block_count(size) * 32, s);
+      if (blocks && !fill_blocks(blocks, words, rt, size, o.flags + MAKE_BLOCKS, s))
+        return fail(WTG_ERR_CUDA, "query blocks: launch failed");
+    }
     if (sorted && blocks) launch(nodes, LevelBits<true>{words, rt, blocks}, std::true_type{}, o, at, m);
     else if (sorted) launch(nodes, LevelBits<false>{words, rt, nullptr}, std::true_type{}, o, at, m);
     else launch(nodes, LevelBits<false>{words, rt, nullptr}, std::false_type{}, o, at, m);
@@ -421,14 +459,17 @@ int launch_wt_access(TreeImpl& t, const uint64_t* idx, uint64_t nq, uint64_t* ou
 int launch_wt_rank(TreeImpl& t, const uint64_t* idx, const uint64_t* sym, uint64_t nq, uint64_t* out,
                    cudaStream_t s) {
   if (int rc = need(t, WTG_RANK, "rank")) return rc;
+  // 2^22 consecutive positions, us by steps / by node entries: 2^28 symbols x 8
+  // levels 99 / 110, x 12 118 / 135, x 20 385 / 363, 2^29 x 20 503 / 419
+  const bool far = t.levels >= 16;
   return descents(t, idx, nq, s, [&](const NodeTables& nodes, auto bits, auto ord, const QueryOrder& o, uint64_t at,
                                      uint64_t m) {
     if (!ord() && far_descent(t, m))
       wt_rank_far_kernel<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab, t.n,
                                                   t.levels, idx + at, sym + at, m, out + at);
     else
-      wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, nodes.step, t.n, t.levels, idx + at, o, sym + at, m,
-                                                       out + at);
+      wt_rank_kernel<ord()><<<qgrid(m), 256, 0, s>>>(bits, nodes.step, nodes.tab, t.n, t.levels, idx + at, o, far,
+                                                     sym + at, m, out + at);
   });
 }
 

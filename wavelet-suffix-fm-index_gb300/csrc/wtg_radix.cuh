@@ -35,7 +35,9 @@ constexpr int RS_MAX_PASSES = 8;
 // hist[pass][digit] of keys' bits [lo + 8 pass, lo + 8 pass + 8)
 template <typename K>
 __global__ void __launch_bounds__(RS_THREADS)
-    radix_hist_kernel(const K* __restrict__ key, uint64_t n, int lo, int passes, uint32_t* __restrict__ hist) {
+    radix_hist_kernel(const K* __restrict__ key, uint64_t n, int lo, int passes, uint32_t* __restrict__ hist,
+                      const uint32_t* __restrict__ skip) {
+  if (skip && *skip) return;
   __shared__ uint32_t h[RS_MAX_PASSES][RS_RADIX];
   for (uint32_t i = threadIdx.x; i < RS_MAX_PASSES * RS_RADIX; i += RS_THREADS) (&h[0][0])[i] = 0;
   __syncthreads();
@@ -116,7 +118,8 @@ template <typename K, typename S, bool IOTA>
 __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
     radix_pass_kernel(const K* __restrict__ key, const uint32_t* __restrict__ val, uint64_t n, int shift,
                       const uint32_t* __restrict__ bases, S* status, uint32_t* counter, K* __restrict__ key_out,
-                      uint32_t* __restrict__ val_out, uint32_t* err) {
+                      uint32_t* __restrict__ val_out, uint32_t* err, const uint32_t* __restrict__ skip) {
+  if (skip && *skip) return;
   using RS = RadixStatus<S>;
   __shared__ __align__(16) K s_key[RS_TILE];
   __shared__ uint32_t wc[RS_WARPS][RS_RADIX];  // per warp: count, then local base
@@ -245,7 +248,8 @@ __global__ void __launch_bounds__(RS_THREADS, RS_CTAS)
 // Sorts n pairs by key bits [lo, lo + 8 passes), lo a multiple of 8 for 8-byte keys; the pairs are in key[cur] /
 // val[cur] and end there (cur flips once per pass).  iota: the values of the
 // first pass are the indices.  hist: passes * 256 words, status: its bytes
-// from radix_status_bytes; both are scratch.  Asynchronous.
+// from radix_status_bytes; both are scratch.  skip: a device word that, when
+// set, leaves the sort out (nothing of its outputs is written).  Asynchronous.
 inline uint64_t radix_status_bytes(uint64_t n, int passes) {
   const uint64_t tiles = (n + RS_TILE - 1) / RS_TILE;
   return (uint64_t)passes * (tiles * RS_RADIX * (n < (1ull << 30) ? 4 : 8) + 16);
@@ -253,7 +257,7 @@ inline uint64_t radix_status_bytes(uint64_t n, int passes) {
 
 template <typename K, typename S>
 int radix_passes(K* const key[2], uint32_t* const val[2], uint64_t n, int lo, int passes, bool iota, uint32_t* hist,
-                 uint8_t* status, uint32_t* d_err, int& cur, cudaStream_t s) {
+                 uint8_t* status, uint32_t* d_err, int& cur, cudaStream_t s, const uint32_t* skip) {
   const uint32_t tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
   const uint64_t per = (uint64_t)tiles * RS_RADIX * sizeof(S) + 16;
   for (int p = 0; p < passes; ++p) {
@@ -267,11 +271,11 @@ int radix_passes(K* const key[2], uint32_t* const val[2], uint64_t n, int lo, in
     }
     if (iota && p == 0)
       radix_pass_kernel<K, S, true><<<grid, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo, hist, words, counter,
-                                                                 key[cur ^ 1], val[cur ^ 1], d_err);
+                                                                key[cur ^ 1], val[cur ^ 1], d_err, skip);
     else
       radix_pass_kernel<K, S, false><<<grid, RS_THREADS, 0, s>>>(key[cur], val[cur], n, lo + 8 * p,
                                                                   hist + p * RS_RADIX, words, counter, key[cur ^ 1],
-                                                                  val[cur ^ 1], d_err);
+                                                                 val[cur ^ 1], d_err, skip);
     count_launch();
     WTG_CK(cudaGetLastError());
     cur ^= 1;
@@ -281,20 +285,27 @@ int radix_passes(K* const key[2], uint32_t* const val[2], uint64_t n, int lo, in
 
 template <typename K>
 int radix_sort_pairs(K* const key[2], uint32_t* const val[2], uint64_t n, int lo, int passes, bool iota,
-                     uint32_t* hist, uint8_t* status, uint32_t* d_err, int& cur, cudaStream_t s) {
+                     uint32_t* hist, uint8_t* status, uint32_t* d_err, int& cur, cudaStream_t s,
+                     const uint32_t* skip = nullptr) {
   if (n == 0 || passes == 0) return WTG_OK;
-  WTG_CK(cudaMemsetAsync(hist, 0, (uint64_t)passes * RS_RADIX * sizeof(uint32_t), s));
-  WTG_CK(cudaMemsetAsync(status, 0, radix_status_bytes(n, passes), s));
+  const uint64_t hist_bytes = (uint64_t)passes * RS_RADIX * sizeof(uint32_t), status_bytes = radix_status_bytes(n, passes);
+  if ((uint8_t*)hist + hist_bytes == status) {
+    WTG_CK(cudaMemsetAsync(hist, 0, hist_bytes + status_bytes, s));
+  } else {
+    WTG_CK(cudaMemsetAsync(hist, 0, hist_bytes, s));
+    WTG_CK(cudaMemsetAsync(status, 0, status_bytes, s));
+  }
   const uint64_t blocks = (n + 8 * RS_THREADS - 1) / (8 * RS_THREADS);
   radix_hist_kernel<K><<<(unsigned)(blocks < 152 * 8 ? blocks : 152 * 8), RS_THREADS, 0, s>>>(key[cur], n, lo, passes,
-                                                                                             hist);
+                                                                                             hist, skip);
   count_launch();
   WTG_CK(cudaGetLastError());
   radix_bases_kernel<<<passes, RS_RADIX, 0, s>>>(hist);
   count_launch();
   WTG_CK(cudaGetLastError());
-  return n < (1ull << 30) ? radix_passes<K, uint32_t>(key, val, n, lo, passes, iota, hist, status, d_err, cur, s)
-                          : radix_passes<K, uint64_t>(key, val, n, lo, passes, iota, hist, status, d_err, cur, s);
+  return n < (1ull << 30) ? radix_passes<K, uint32_t>(key, val, n, lo, passes, iota, hist, status, d_err, cur, s, skip)
+                          : radix_passes<K, uint64_t>(key, val, n, lo, passes, iota, hist, status, d_err, cur, s,
+                                                      skip);
 }
 
 }  // namespace wtg

@@ -22,34 +22,24 @@ constexpr int RQ_STACK = 32;  // DFS stack entries per query (at most L + 1 <= 2
 
 __device__ __forceinline__ int level_of(uint64_t h) { return 63 - __clzll((long long)(h + 1)); }
 
+// the node tables as a kernel's argument
+struct NodeView {
+  const ulonglong2* tab;
+  const uint2* step;
+};
+
 // lex_count (wt_int_par.hpp:715-745): descend along c's path carrying both
-// bounds (positions inside the level; the node's step constants take them to
-// its child, see node_table_kernel); symbols below / above c are counted
-// where the path turns.
-template <bool ORD>
-__global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
-                              const uint2* __restrict__ step, uint64_t n, int L, QueryOrder ord,
-                              const uint64_t* __restrict__ qi, const uint64_t* __restrict__ qj,
-                              const uint64_t* __restrict__ qc, uint64_t nq, uint64_t* __restrict__ out_rank,
-                              uint64_t* __restrict__ out_smaller, uint64_t* __restrict__ out_greater) {
-  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nq) return;
-  if (ORD && (k = ord.id[k]) >= nq) return;
-  const uint64_t i = qi[k], j = qj[k], c = qc[k];
-  if (i > j || j > n) {
-    out_rank[k] = NONE64;
-    out_smaller[k] = NONE64;
-    out_greater[k] = NONE64;
-    return;
-  }
-  if ((1ull << L) <= c) {  // c above every symbol of the tree
-    out_rank[k] = 0;
-    out_smaller[k] = j - i;
-    out_greater[k] = 0;
-    return;
-  }
-  const uint32_t path = (uint32_t)c | (1u << L);
-  uint32_t x = (uint32_t)i, y = (uint32_t)j, smaller = 0, greater = 0;  // counts below 2^32
+// bounds; symbols below / above c are counted where the path turns.  Positions
+// inside the level, the node's step constants take them to its child (see
+// node_table_kernel):
+struct LexCounts {
+  uint64_t rank, smaller, greater;
+};
+__device__ __forceinline__ LexCounts lex_steps(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                               const uint2* __restrict__ step, uint64_t n, int L, uint32_t x, uint32_t y,
+                                               uint32_t c) {
+  const uint32_t path = c | (1u << L);
+  uint32_t smaller = 0, greater = 0;  // counts below 2^32
   uint64_t lbase = 0;
   uint2 st = __ldg(step + 1);
   for (int lv = 0; lv < L; ++lv, lbase += n) {
@@ -71,9 +61,56 @@ __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t*
     }
     st = next;
   }
-  out_rank[k] = x;
-  out_smaller[k] = smaller;
-  out_greater[k] = greater;
+  return {x, smaller, greater};
+}
+
+// The same by node entries and positions inside the node.
+__device__ __forceinline__ LexCounts lex_far(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt,
+                                             const ulonglong2* __restrict__ tab, int L, uint64_t i, uint64_t j,
+                                             uint64_t c) {
+  uint64_t smaller = 0, greater = 0, h = 0;
+  ulonglong2 nd = __ldg(tab);
+  for (int lv = 0; lv < L; ++lv) {
+    const uint64_t bit = (c >> (L - 1 - lv)) & 1;
+    const uint64_t child = 2 * h + 1 + bit;
+    const ulonglong2 next = lv + 1 < L ? __ldg(tab + child) : nd;
+    const uint64_t oi = rank1_dev(rt, tree, nd.x + i) - nd.y;
+    const uint64_t oj = rank1_dev(rt, tree, nd.x + j) - nd.y;
+    if (bit) {
+      smaller += (j - i) - (oj - oi);
+      i = oi;
+      j = oj;
+    } else {
+      greater += oj - oi;
+      i -= oi;
+      j -= oj;
+    }
+    h = child;
+    nd = next;
+  }
+  return {i, smaller, greater};
+}
+
+// far: a batch that came in order goes by node entries (see launch_wt_lex_count)
+template <bool ORD>
+__global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt, const NodeView nodes,
+                              uint64_t n, int L, QueryOrder ord, bool far, const uint64_t* __restrict__ qi,
+                              const uint64_t* __restrict__ qj, const uint64_t* __restrict__ qc, uint64_t nq,
+                              uint64_t* __restrict__ out_rank, uint64_t* __restrict__ out_smaller,
+                              uint64_t* __restrict__ out_greater) {
+  uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= nq) return;
+  if (ORD && !ordered_query(ord, nq, k)) return;
+  const uint64_t i = qi[k], j = qj[k], c = qc[k];
+  LexCounts r{NONE64, NONE64, NONE64};
+  if (i <= j && j <= n) {
+    if ((1ull << L) <= c) r = {0, j - i, 0};  // c above every symbol of the tree
+    else if (ORD && far && ord.flags[AS_IS]) r = lex_far(tree, rt, nodes.tab, L, i, j, c);
+    else r = lex_steps(tree, rt, nodes.step, n, L, (uint32_t)i, (uint32_t)j, (uint32_t)c);
+  }
+  out_rank[k] = r.rank;
+  out_smaller[k] = r.smaller;
+  out_greater[k] = r.greater;
 }
 
 // lex_smaller_count (wt_int_par.hpp:758-782): the same with one bound
@@ -144,7 +181,7 @@ __global__ void wt_range_count_kernel(const uint64_t* __restrict__ tree, const u
                                       uint64_t nq, uint64_t* __restrict__ out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  if (ORD && (k = ord.id[k]) >= nq) return;
+  if (ORD && !ordered_query(ord, nq, k)) return;
   const uint64_t lb0 = qlb[k], rb0 = qrb[k];
   uint64_t vlb = qvlb[k], vrb = qvrb[k];
   if (lb0 <= rb0 && rb0 >= n) {
@@ -384,10 +421,14 @@ int launch_wt_lex_count(TreeImpl& t, const uint64_t* i, const uint64_t* j, const
   if (!nq) return WTG_OK;
   const NodeTables nodes(t, s);
   if ((rc = nodes.rc)) return rc;
+  const NodeView view{nodes.tab, nodes.step};
+  // 2^22 consecutive positions, 20 levels, us by steps / by node entries: 2^28
+  // symbols 521 / 606, 2^29 611 / 637, 2^30 842 / 762
+  const bool far = t.n * (uint64_t)t.levels / 8 >= (2ull << 30);
   return in_order(t, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_lex_kernel<true> : wt_lex_kernel<false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.step, t.n, t.levels,
-                               o, i + at, j + at, c + at, m, rank_out + at, smaller_out + at, greater_out + at);
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), view, t.n, t.levels, o, far, i + at,
+                               j + at, c + at, m, rank_out + at, smaller_out + at, greater_out + at);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
