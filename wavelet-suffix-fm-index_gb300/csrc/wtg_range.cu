@@ -425,14 +425,14 @@ int launch_wt_lex_count(TreeImpl& t, const uint64_t* i, const uint64_t* j, const
   // 2^22 consecutive positions, 20 levels, us by steps / by node entries: 2^28
   // symbols 521 / 606, 2^29 611 / 637, 2^30 842 / 762
   const bool far = t.n * (uint64_t)t.levels / 8 >= (2ull << 30);
-  return in_order(t, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+  return in_order(t, OrderOp::LEX, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_lex_kernel<true> : wt_lex_kernel<false>;
     f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), view, t.n, t.levels, o, far, i + at,
                                j + at, c + at, m, rank_out + at, smaller_out + at, greater_out + at);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
-  }, true);
+  });
 }
 
 int launch_wt_lex_smaller_count(TreeImpl& t, const uint64_t* i, const uint64_t* c, uint64_t nq, uint64_t* rank_out,
@@ -457,14 +457,14 @@ int launch_wt_range_count(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, c
   if (!nq) return WTG_OK;
   const NodeTables nodes(t, s);
   if ((rc = nodes.rc)) return rc;
-  return in_order(t, lb, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+  return in_order(t, OrderOp::RANGE, lb, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_range_count_kernel<true> : wt_range_count_kernel<false>;
     f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab, t.n,
                                t.levels, o, lb + at, rb + at, vlb + at, vrb + at, m, count_out + at);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
-  }, true);
+  });
 }
 
 int launch_wt_range_report(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, const uint64_t* vlb,
