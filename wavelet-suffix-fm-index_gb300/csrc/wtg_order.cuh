@@ -147,33 +147,28 @@ __global__ void __launch_bounds__(RS_THREADS)
 // what L2 keeps of a tree: its bits from about 100 MB on (with the rank table 125 MB)
 inline bool larger_than_l2(const TreeImpl& t) { return t.n * (uint64_t)t.levels / 8 >= (100ull << 20); }
 
-// Operations that break even at different batch sizes: access, rank and
-// inverse_select read one position, lex_count and range_count two.
-enum class OrderOp { ONE, LEX, RANGE };
-
 // When sorting pays: the tree is larger than what L2 keeps of it, has enough
 // levels to make up for the sort (45 us, then 10 % of the time) and for reading
 // the other arguments by query number, and the batch is large enough.
 // Measured, us as they come / sorted, random positions.  2^28 symbols, 20
 // levels: access of 2^18.25 queries 152 / 148, 2^18.5 192 / 156, rank 124 / 150,
-// 164 / 159, lex_count of 2^18 152 / 159, 2^18.25 180 / 164, range_count 150 / 166,
+// 164 / 159, lex_count of 2^18 141 / 159, 2^18.25 160 / 164, range_count 150 / 166,
 // 173 / 168, 2^18.5 188 / 170.  12 levels: access of 2^18.5 103 / 110, 2^18.75 121
-// / 111, rank of 2^19 113 / 121, 2^19.5 183 / 133, lex_count of 2^18.5 121 / 125,
-// 2^18.75 129 / 133, 2^19 173 / 148, range_count of 2^18.5 140 / 131.  8 levels:
-// access of 2^19 88 / 94, 2^19.5 131 / 106, rank of 2^19.5 112 / 111, lex_count of
-// 2^19 112 / 116, 2^19.5 150 / 137, range_count of 2^19 128 / 124.
+// / 111, rank of 2^19 113 / 121, 2^19.5 183 / 133, lex_count of 2^18.5 122 / 125,
+// 2^18.75 140 / 133, range_count of 2^18.5 140 / 131.  8 levels: access of 2^19 88
+// / 94, 2^19.5 131 / 106, rank of 2^19.5 112 / 111, lex_count of 2^19 106 / 116,
+// 2^19.3 123 / 132, range_count of 2^19 128 / 124.
 // Just above L2 (2^27 x 8, 128 MB): access of 2^19.5 83 / 85, 2^20 117 / 101, rank
-// 80 / 88, 107 / 107, lex_count of 2^19.35 112 / 98; 2^28 x 6, rank of 2^20 119 /
-// 113, lex_count of 2^19.35 105 / 108, 2^19.5 118 / 119; 2^26 x 20, access of
+// 80 / 88, 107 / 107, lex_count of 2^19.5 108 / 110; 2^28 x 6, rank of 2^20 119 /
+// 113, range_count of 2^19.5 135 / 123; 2^26 x 20, access of
 // 2^18.75 114 / 99, 2^19.5 205 / 129, rank of 2^19 109 / 110, 2^19.5 159 / 132.
 // Trees that L2 holds gain only by the sectors that neighbours share, over many
 // levels: 2^24 x 20, 2^21 queries, access 353 / 232, rank 316 / 245.
-inline bool order_pays(const TreeImpl& t, uint64_t nq, OrderOp op) {
+// two: lex_count and range_count, which read two positions a query.
+inline bool order_pays(const TreeImpl& t, uint64_t nq, bool two) {
   const uint64_t bytes = t.n * (uint64_t)t.levels / 8, probes = nq * t.levels;
-  const bool one = op == OrderOp::ONE;
-  if (bytes >= (256ull << 20))
-    return t.levels >= 6 && probes >= (one ? 14ull : op == OrderOp::LEX ? 11ull : 12ull) << 19;
-  if (larger_than_l2(t)) return t.levels >= 6 && nq >= (5ull << 17) && probes >= (one ? 8ull : 4ull) << 20;
+  if (bytes >= (256ull << 20)) return t.levels >= 6 && probes >= (two ? 6ull : 7ull) << 20;
+  if (larger_than_l2(t)) return t.levels >= 6 && nq >= (5ull << 17) && probes >= (two ? 4ull : 8ull) << 20;
   return bytes >= (20ull << 20) && t.levels >= 16 && nq >= (1ull << 21);
 }
 
@@ -220,8 +215,8 @@ static_assert(ORDER_BATCH < (1ull << 30), "32-bit status words");
 // Calls launch(sorted, order, first query, queries) over the batch: sorted by
 // position where that pays, otherwise once over all queries as they come.
 template <typename F>
-int in_order(TreeImpl& t, OrderOp op, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch) {
-  if (!order_pays(t, nq, op)) return launch(false, QueryOrder{}, 0, nq);
+int in_order(TreeImpl& t, bool two, const uint64_t* pos, uint64_t nq, cudaStream_t s, F launch) {
+  if (!order_pays(t, nq, two)) return launch(false, QueryOrder{}, 0, nq);
   constexpr int passes = 2;
   const int bits = 64 - __builtin_clzll(t.n | 1);  // positions 0 .. n
   const int lo = bits > 8 * passes ? bits - 8 * passes : 0;

@@ -408,7 +408,7 @@ NodeTables::~NodeTables() {
 // 2^27 x 20 (14 M blocks), 2^26 6.52 / 5.98, 2^23 0.89 / 0.86, 2^22 0.48 /
 // 0.53; but 2^28 x 8 (11 M), 2^26 4.52 / 4.28, 2^25 2.19 / 2.17, 2^24 1.04 / 1.10.
 static bool blocks_pay(const TreeImpl& t, uint64_t nq) {
-  return order_pays(t, nq, OrderOp::ONE) && t.levels >= 12 && nq >= block_count(t.n * (uint64_t)t.levels) / 3;
+  return order_pays(t, nq, false) && t.levels >= 12 && nq >= block_count(t.n * (uint64_t)t.levels) / 3;
 }
 
 // (below 2^17 queries the tree's lines that they read stay in L2)
@@ -424,7 +424,7 @@ static int descents(TreeImpl& t, const uint64_t* idx, uint64_t nq, cudaStream_t 
   const uint64_t* const words = t.bits.as<uint64_t>();
   const uint64_t* const rt = t.bv.rank.as<uint64_t>();
   uint4* blocks = nullptr;
-  const int rc = in_order(t, OrderOp::ONE, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+  const int rc = in_order(t, false, idx, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     if (sorted && blocks_pay(t, nq)) {
       // (once the sort has its scratch, which comes first; by the first batch that does not come in order)
       const uint64_t size = t.n * (uint64_t)t.levels;

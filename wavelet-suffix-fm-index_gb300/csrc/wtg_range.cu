@@ -91,7 +91,12 @@ __device__ __forceinline__ LexCounts lex_far(const uint64_t* __restrict__ tree, 
   return {i, smaller, greater};
 }
 
-// far: a batch that came in order goes by node entries (see launch_wt_lex_count)
+// far: a batch that came in order goes by node entries (see launch_wt_lex_count).
+// A batch that is not sorted goes by steps, with the registers that both loops
+// take: at 40 an SM runs six CTAs, where the steps alone, at 34, ran seven and
+// more queries in flight that meet on fewer lines in L2 (2^18 queries, 2^28
+// symbols x 8, 12 and 20 levels: 59, 94 and 141 us; 70, 105 and 170 at 34
+// registers; by node entries 66, 99 and 155).
 template <bool ORD>
 __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt, const NodeView nodes,
                               uint64_t n, int L, QueryOrder ord, bool far, const uint64_t* __restrict__ qi,
@@ -105,7 +110,7 @@ __global__ void wt_lex_kernel(const uint64_t* __restrict__ tree, const uint64_t*
   LexCounts r{NONE64, NONE64, NONE64};
   if (i <= j && j <= n) {
     if ((1ull << L) <= c) r = {0, j - i, 0};  // c above every symbol of the tree
-    else if (ORD && far && ord.flags[AS_IS]) r = lex_far(tree, rt, nodes.tab, L, i, j, c);
+    else if (far && (!ORD || ord.flags[AS_IS])) r = lex_far(tree, rt, nodes.tab, L, i, j, c);
     else r = lex_steps(tree, rt, nodes.step, n, L, (uint32_t)i, (uint32_t)j, (uint32_t)c);
   }
   out_rank[k] = r.rank;
@@ -425,10 +430,11 @@ int launch_wt_lex_count(TreeImpl& t, const uint64_t* i, const uint64_t* j, const
   // 2^22 consecutive positions, 20 levels, us by steps / by node entries: 2^28
   // symbols 521 / 606, 2^29 611 / 637, 2^30 842 / 762
   const bool far = t.n * (uint64_t)t.levels / 8 >= (2ull << 30);
-  return in_order(t, OrderOp::LEX, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+  return in_order(t, true, i, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_lex_kernel<true> : wt_lex_kernel<false>;
-    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), view, t.n, t.levels, o, far, i + at,
-                               j + at, c + at, m, rank_out + at, smaller_out + at, greater_out + at);
+    f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), view, t.n, t.levels, o,
+                               sorted && far, i + at, j + at, c + at, m, rank_out + at, smaller_out + at,
+                               greater_out + at);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
@@ -457,7 +463,7 @@ int launch_wt_range_count(TreeImpl& t, const uint64_t* lb, const uint64_t* rb, c
   if (!nq) return WTG_OK;
   const NodeTables nodes(t, s);
   if ((rc = nodes.rc)) return rc;
-  return in_order(t, OrderOp::RANGE, lb, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
+  return in_order(t, true, lb, nq, s, [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
     auto* const f = sorted ? wt_range_count_kernel<true> : wt_range_count_kernel<false>;
     f<<<qgrid(m), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), nodes.tab, t.n,
                                t.levels, o, lb + at, rb + at, vlb + at, vrb + at, m, count_out + at);
