@@ -267,6 +267,7 @@ __global__ void huff_rank_kernel(HuffView v, const uint64_t* __restrict__ qi, co
 // select(i, c) (wt_huff/wt_pc_par.hpp:527-552): from c's leaf up, select1 /
 // select0 on the bitvector; n where c does not occur; UINT64_MAX where c
 // occurs fewer than i times (the reference asserts)
+template <bool WORDS>
 __global__ void huff_select_kernel(HuffView v, const uint64_t* __restrict__ qi, const uint64_t* __restrict__ qc,
                                    uint64_t nq, uint64_t* __restrict__ out) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -290,8 +291,8 @@ __global__ void huff_select_kernel(HuffView v, const uint64_t* __restrict__ qi, 
     const uint16_t par = v.nodes[u].parent;
     const uint64_t bp = v.nodes[par].bv_pos, br = v.nodes[par].rank;
     uint64_t s;
-    if (v.nodes[par].child1 == u) s = select_dev(v.s1, br + res + 1);
-    else s = select_dev(v.s0, bp - br + res + 1);
+    if (v.nodes[par].child1 == u) s = select_dev<WORDS>(v.s1, br + res + 1);
+    else s = select_dev<WORDS>(v.s0, bp - br + res + 1);
     if (s == NONE64) {
       res = NONE64;
       break;
@@ -912,7 +913,8 @@ int launch_huff_query(HuffImpl& h, int what, const uint64_t* a, const uint64_t* 
   if (what == 0) huff_access_kernel<false><<<grid, 256, 0, s>>>(v, a, nq, out, nullptr);
   else if (what == 3) huff_access_kernel<true><<<grid, 256, 0, s>>>(v, a, nq, out, out2);
   else if (what == 1) huff_rank_kernel<<<grid, 256, 0, s>>>(v, a, b, nq, out);
-  else huff_select_kernel<<<grid, 256, 0, s>>>(v, a, b, nq, out);
+  else if (nq < SEL_MANY) huff_select_kernel<false><<<grid, 256, 0, s>>>(v, a, b, nq, out);
+  else huff_select_kernel<true><<<grid, 256, 0, s>>>(v, a, b, nq, out);
   count_launch();
   WTG_CK(cudaGetLastError());
   return WTG_OK;

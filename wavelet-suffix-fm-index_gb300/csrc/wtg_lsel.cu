@@ -121,7 +121,7 @@ __global__ void level_args_kernel(const uint64_t* __restrict__ tbl, const uint64
   if (l <= L) out[l] = rank1_dev(tbl, words, (uint64_t)l * n);
 }
 
-template <int T_B>
+template <int T_B, bool WORDS>
 __global__ void level_select_kernel(SelView v, const uint64_t* __restrict__ la, uint64_t n, int L,
                                     const uint64_t* __restrict__ lev, const uint64_t* __restrict__ kq, uint64_t nq,
                                     uint64_t* __restrict__ out) {
@@ -135,7 +135,7 @@ __global__ void level_select_kernel(SelView v, const uint64_t* __restrict__ la, 
     const uint64_t A = T_B ? o0 : off - o0;
     const uint64_t m = T_B ? o1 - o0 : n - (o1 - o0);
     if (k >= 1 && k <= m) {
-      const uint64_t p = select_dev(v, A + k);
+      const uint64_t p = select_dev<WORDS>(v, A + k);
       res = p == NONE64 ? NONE64 : p - off;
     }
   }
@@ -559,13 +559,12 @@ int launch_level_select(TreeImpl& t, int t_b, const uint64_t* level, const uint6
   if ((rc = need_supports(t, WTG_RANK | (t_b ? WTG_SELECT1 : WTG_SELECT0)))) return rc;
   if (nq == 0) return WTG_OK;
   if ((rc = tree_level_args(t, s))) return rc;
-  const SelView v = sel_view(t.bv, t_b);
+  const bool words = select_by_words(t.bv.sel[t_b], t.bv.size, nq);
   const unsigned grid = (unsigned)((nq + 255) / 256);
   count_launch();
-  if (t_b)
-    level_select_kernel<1><<<grid, 256, 0, s>>>(v, t.lvl_args.as<uint64_t>(), t.n, t.levels, level, k, nq, out);
-  else
-    level_select_kernel<0><<<grid, 256, 0, s>>>(v, t.lvl_args.as<uint64_t>(), t.n, t.levels, level, k, nq, out);
+  auto* const f = t_b ? words ? level_select_kernel<1, true> : level_select_kernel<1, false>
+                      : words ? level_select_kernel<0, true> : level_select_kernel<0, false>;
+  f<<<grid, 256, 0, s>>>(sel_view(t.bv, t_b), t.lvl_args.as<uint64_t>(), t.n, t.levels, level, k, nq, out);
   WTG_CK(cudaGetLastError());
   return WTG_OK;
 }

@@ -264,7 +264,7 @@ __global__ void wt_rank_far_kernel(const uint64_t* __restrict__ tree, const uint
 // the node table's and the occurrences of c a leaf's size, so that nothing but
 // the selects waits for one another (a call of 1000 over 2^20 x 8 levels 73 / 70
 // us, over 2^22 x 20 108 / 95, of 2^18 293 / 255).
-template <bool TAB>
+template <bool TAB, bool WORDS>
 __global__ void wt_select_kernel(const uint64_t* __restrict__ tree, const uint64_t* __restrict__ rt, SelView s1,
                                  SelView s0, const ulonglong2* __restrict__ tab, const uint32_t* __restrict__ C, uint64_t n,
                                  int L, const uint64_t* __restrict__ q,
@@ -291,8 +291,8 @@ __global__ void wt_select_kernel(const uint64_t* __restrict__ tree, const uint64
     }
     for (int lv = L; lv > 0; --lv) {
       const ulonglong2 up = __ldg(tab + (lv > 1 ? (path >> (L - lv + 2)) - 1 : 0));
-      if ((path >> (L - lv)) & 1u) i = select_dev(s1, nd.y + i) - nd.x + 1;
-      else i = select_dev(s0, nd.x - nd.y + i) - nd.x + 1;
+      if ((path >> (L - lv)) & 1u) i = select_dev<WORDS>(s1, nd.y + i) - nd.x + 1;
+      else i = select_dev<WORDS>(s0, nd.x - nd.y + i) - nd.x + 1;
       nd = up;
     }
     out[k] = i - 1;
@@ -323,8 +323,8 @@ __global__ void wt_select_kernel(const uint64_t* __restrict__ tree, const uint64
   for (int lv = L; lv > 0; --lv) {
     offset = path_off[lv - 1];
     const uint64_t o = path_rank[lv - 1];
-    if (c & mask) i = select_dev(s1, o + i) - offset + 1;
-    else i = select_dev(s0, offset - o + i) - offset + 1;
+    if (c & mask) i = select_dev<WORDS>(s1, o + i) - offset + 1;
+    else i = select_dev<WORDS>(s0, offset - o + i) - offset + 1;
     mask <<= 1;
   }
   out[k] = i - 1;
@@ -338,10 +338,11 @@ __global__ void bv_rank_kernel(const uint64_t* __restrict__ words, const uint64_
   out[k] = idx <= size ? rank1_dev(rt, words, idx) : NONE64;
 }
 
+template <bool WORDS>
 __global__ void bv_select_kernel(SelView v, const uint64_t* __restrict__ q, uint64_t nq, uint64_t* __restrict__ out) {
   uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= nq) return;
-  out[k] = select_dev(v, q[k]);
+  out[k] = select_dev<WORDS>(v, q[k]);
 }
 
 static unsigned qgrid(uint64_t nq) { return (unsigned)((nq + 255) / 256); }
@@ -497,7 +498,11 @@ int launch_wt_select(TreeImpl& t, const uint64_t* i, const uint64_t* sym, uint64
   const NodeTables nodes(t, s, heap <= 8 * nq);
   if (nodes.rc) cudaGetLastError();
   const bool tab = t.n && nodes.rc == WTG_OK && nodes.tab;
-  auto* const f = tab ? wt_select_kernel<true> : wt_select_kernel<false>;
+  // a call of 2^16 queries, us word by word / by sectors: 2^28 symbols x 20 levels 194
+  // / 172, x 8 116 / 105; 2^18: 283 / 358, 182 / 220, 2^22 x 20 248 / 282
+  const bool many = nq >= SEL_MANY;
+  auto* const f = many ? tab ? wt_select_kernel<true, true> : wt_select_kernel<false, true>
+                       : tab ? wt_select_kernel<true, false> : wt_select_kernel<false, false>;
   f<<<qgrid(nq), 256, 0, s>>>(t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), sel_view(t.bv, 1), sel_view(t.bv, 0),
                               nodes.tab, t.zeros.as<uint32_t>() + heap, t.n, t.levels, i, sym, nq, out);
   count_launch();
@@ -517,7 +522,8 @@ int launch_bv_rank(const BvSupport& bv, const uint64_t* idx, uint64_t nq, uint64
 int launch_bv_select(const BvSupport& bv, int t_b, const uint64_t* i, uint64_t nq, uint64_t* out, cudaStream_t s) {
   if (!(bv.flags & (t_b ? WTG_SELECT1 : WTG_SELECT0))) return fail(WTG_ERR_INVALID, "select needs its support built");
   if (!nq) return WTG_OK;
-  bv_select_kernel<<<qgrid(nq), 256, 0, s>>>(sel_view(bv, t_b), i, nq, out);
+  auto* const f = select_by_words(bv.sel[t_b], bv.size, nq) ? bv_select_kernel<true> : bv_select_kernel<false>;
+  f<<<qgrid(nq), 256, 0, s>>>(sel_view(bv, t_b), i, nq, out);
   count_launch();
   WTG_CK(cudaGetLastError());
   return WTG_OK;

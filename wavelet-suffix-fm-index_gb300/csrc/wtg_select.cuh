@@ -39,51 +39,67 @@ struct SelView {
   int t_b;
 };
 
-// The need-th arg (need >= 1) from bit pos on.  A sector of four words at a
-// time, one load each, where the words start on a sector and the sector lies
-// within them: word by word, every word waited for the one before, up to 64
-// args of a sparse node (a call of 1000 selects over 2^20 x 8 levels 70 / 58
-// us, over 2^22 x 20 95 / 83; of 2^18 over 2^22 x 20 255 / 278).
-__device__ __forceinline__ uint64_t select_scan(const SelView& v, uint64_t pos, uint32_t need) {
+// The need-th arg (need >= 1) from bit pos on, word by word.  (The first two
+// words apart from the rest are the compiler's better code: 2^22 selects over
+// 2^30 bits 64 us, 66 in one loop.)
+__device__ __forceinline__ uint64_t select_words(const SelView& v, uint64_t pos, uint32_t need) {
+  const uint64_t flip = v.t_b ? 0ull : ~0ull;
+  uint64_t wp = pos >> 6;
+  if (wp >= v.nwords) return NONE64;
+  const uint64_t first = (v.words[wp] ^ flip) & (~0ull << (pos & 63));
+  uint32_t args = __popcll(first);
+  if (args >= need) return (wp << 6) + sel64(first, need);
+  uint32_t sum = args;
+  if (++wp >= v.nwords) return NONE64;
+  uint64_t w = v.words[wp] ^ flip;
+  args = __popcll(w);
+  while (sum + args < need) {
+    sum += args;
+    if (++wp >= v.nwords) return NONE64;  // inconsistent tables: never read past the data
+    w = v.words[wp] ^ flip;
+    args = __popcll(w);
+  }
+  return (wp << 6) + sel64(w, need - sum);
+}
+
+// The same, a sector of four words at a time, one load each, where the words
+// start on a sector and the sector lies within them: word by word, every word
+// waits for the one before, up to 64 args of a sparse node.
+__device__ __forceinline__ uint64_t select_sectors(const SelView& v, uint64_t pos, uint32_t need) {
+  if ((uintptr_t)v.words & 31) return select_words(v, pos, need);
   uint64_t wp = pos >> 6;
   const uint64_t flip = v.t_b ? 0ull : ~0ull;
   uint64_t keep = ~0ull << (pos & 63);  // of the first word
-  if (((uintptr_t)v.words & 31) == 0) {
-    for (uint64_t s = wp & ~3ull; s + 4 <= v.nwords; s += 4) {
-      uint64_t w[4];
-      asm volatile("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
-                   : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
-                   : "l"(v.words + s));
-      uint32_t c[4];
+  for (uint64_t s = wp & ~3ull; s + 4 <= v.nwords; s += 4) {
+    uint64_t w[4];
+    asm volatile("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(w[0]), "=l"(w[1]), "=l"(w[2]), "=l"(w[3])
+                 : "l"(v.words + s));
+    uint32_t c[4];
 #pragma unroll
-      for (uint32_t k = 0; k < 4; ++k) {
-        w[k] ^= flip;
-        if (s + k <= wp) w[k] &= s + k < wp ? 0ull : keep;
-        c[k] = __popcll(w[k]);
-      }
-      const uint32_t c2 = c[0] + c[1], c3 = c2 + c[2], c4 = c3 + c[3];
-      if (c4 >= need) {
-        const uint32_t k = (c[0] < need) + (c2 < need) + (c3 < need);
-        const uint64_t x = k == 0 ? w[0] : k == 1 ? w[1] : k == 2 ? w[2] : w[3];
-        const uint32_t before = k == 0 ? 0u : k == 1 ? c[0] : k == 2 ? c2 : c3;
-        return ((s + k) << 6) + sel64(x, need - before);
-      }
-      need -= c4;
-      wp = s + 4;  // whole from here on
-      keep = ~0ull;
+    for (uint32_t k = 0; k < 4; ++k) {
+      w[k] ^= flip;
+      if (s + k <= wp) w[k] &= s + k < wp ? 0ull : keep;
+      c[k] = __popcll(w[k]);
     }
+    const uint32_t c2 = c[0] + c[1], c3 = c2 + c[2], c4 = c3 + c[3];
+    if (c4 >= need) {
+      const uint32_t k = (c[0] < need) + (c2 < need) + (c3 < need);
+      const uint64_t x = k == 0 ? w[0] : k == 1 ? w[1] : k == 2 ? w[2] : w[3];
+      const uint32_t before = k == 0 ? 0u : k == 1 ? c[0] : k == 2 ? c2 : c3;
+      return ((s + k) << 6) + sel64(x, need - before);
+    }
+    need -= c4;
+    wp = s + 4;  // whole from here on
+    keep = ~0ull;
   }
-  for (; wp < v.nwords; ++wp, keep = ~0ull) {
-    const uint64_t w = (v.words[wp] ^ flip) & keep;
-    const uint32_t c = __popcll(w);
-    if (c >= need) return (wp << 6) + sel64(w, need);
-    need -= c;
-  }
-  return NONE64;  // inconsistent tables: never read past the data
+  return select_words(v, (wp << 6) | (keep == ~0ull ? 0 : pos & 63), need);
 }
 
 // select_support_mcl::select(i), 1 <= i <= arg_cnt
-// (select/select_support_mcl_par.hpp:564-611) on the flat layout
+// (select/select_support_mcl_par.hpp:564-611) on the flat layout; WORDS: see
+// select_by_words
+template <bool WORDS = false>
 __device__ __forceinline__ uint64_t select_dev(const SelView& v, uint64_t i) {
   if (i == 0 || i > v.arg_cnt) return NONE64;
   i = i - 1;
@@ -97,7 +113,7 @@ __device__ __forceinline__ uint64_t select_dev(const SelView& v, uint64_t i) {
   if ((off & 0x3F) == 0) return base + mini;
   i = i - (sb << 12) - ((off >> 6) << 6);
   const uint64_t pos = base + mini + 1;
-  return select_scan(v, pos, (uint32_t)i);
+  return WORDS ? select_words(v, pos, (uint32_t)i) : select_sectors(v, pos, (uint32_t)i);
 }
 
 // Select marks of one 64-bit word wi, given K1 = ones before it: for
@@ -157,6 +173,20 @@ __device__ __forceinline__ uint64_t last_arg_end(const uint64_t* __restrict__ wo
   uint64_t x = __ldcg(words + wi);
   if (!t_b) x = ~x & (wi == W - 1 ? tailmask : ~0ull);
   return (wi << 6) + hi64(x) + 1;
+}
+
+// Batches of so many selects hide the latency of reading word by word, and pay
+// for what a sector holds beyond the args' word.  (us word by word / by sectors:
+// level selects of 2^16 queries, 2^28 x 20 levels, 12.4 / 10.3.)
+constexpr uint64_t SEL_MANY = 1ull << 17;
+// A bitvector's selects: by words in such batches where a word or two hold the
+// arg asked for: most of the bits are args, or a third where L2 holds them.  2^22
+// queries over 2^30 bits, 97 % of them args 56 / 67 us, half 64 / 68, 3 % 240 / 170;
+// over the levels of 2^22 x 20, 64 % args, 71 / 76, 36 % 81 / 84; of 2^28 x 20, 163
+// / 154, 131 / 119.
+inline bool select_by_words(const SelectDev& sd, uint64_t size, uint64_t nq) {
+  const bool in_l2 = size / 8 <= (160ull << 20);
+  return nq >= SEL_MANY && sd.arg_cnt >= (in_l2 ? size / 3 : size / 4 * 3);
 }
 
 inline SelView sel_view(const BvSupport& bv, int t_b) {
