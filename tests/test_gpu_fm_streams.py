@@ -61,7 +61,7 @@ def test_counts_on_two_streams(wtg, text, make):
 
 
 def test_counts_with_different_C_on_two_streams(wtg, text):
-    """The balanced tree's steps hold the call's own C and number of symbols."""
+    """A call's C and number of symbols are its own."""
     torch, bwt, C, pat, off, exp = text
     d_bwt, d_C, d_pat, d_off = _device(torch, (bwt, C, pat, off))
     d_zero = torch.zeros_like(d_C)

@@ -23,8 +23,9 @@ class _Setup:
         self.bytes = torch.randint(1, 200, (1 << 18,), device="cuda", generator=g).to(torch.uint8)
         self.C = torch.zeros(256, dtype=torch.int64, device="cuda")
         self.C[1:] = torch.cumsum(torch.bincount(self.bytes.int(), minlength=256), 0)[:-1]
-        self.off = torch.arange(NQ + 1, device="cuda") * 3
-        self.pat = self.bytes[torch.randint(0, 1 << 18, (3 * NQ,), device="cuda", generator=g)].contiguous()
+        self.off = torch.zeros(NQ + 1, dtype=torch.int64, device="cuda")  # lengths that are worth sorting
+        self.off[1:] = torch.cumsum(torch.randint(1, 14, (NQ,), device="cuda", generator=g), 0)
+        self.pat = self.bytes[torch.randint(0, 1 << 18, (int(self.off[-1]),), device="cuda", generator=g)].contiguous()
         torch.cuda.synchronize()
 
 

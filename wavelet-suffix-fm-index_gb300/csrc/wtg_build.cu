@@ -160,7 +160,7 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   t.flags = flags;
   t.bit_words = (n * (uint64_t)L + 63) / 64;
   t.lvl_args_ok = false;
-  t.node_tab_ok = false;
+  t.node_tables.ok = t.fm_steps.ok = false;
   ++t.gen;
   const uint64_t heap = 1ull << L;  // heap ids 0 .. 2^L - 2, plus one pad entry
 
@@ -382,11 +382,8 @@ void tree_release(TreeImpl& t) {
   t.err.release(s);
   t.lvl_args.release(s);
   t.lvl_args_ok = false;
-  t.node_tab.release(s);
-  t.node_step.release(s);
-  t.node_tab_ok = false;
-  if (t.node_made) cudaEventDestroy(t.node_made);
-  t.node_made = nullptr;
+  t.node_tables.release(s);
+  t.fm_steps.release(s);
   t.scratch.release(s);
   t.nodes.release(s);
   t.qbuf.release(s);

@@ -96,6 +96,17 @@ int DevBuf::ensure(size_t need, cudaStream_t s) {
   return WTG_OK;
 }
 
+int Made::wait(MadeOnce& m) {
+  WTG_CK(cudaStreamWaitEvent(stream_, m.made, 0));
+  return WTG_OK;
+}
+
+int Made::record(MadeOnce& m) {
+  if (!m.made) WTG_CK(cudaEventCreateWithFlags(&m.made, cudaEventDisableTiming));
+  WTG_CK(cudaEventRecord(m.made, stream_));
+  return WTG_OK;
+}
+
 void* try_scratch(size_t bytes, cudaStream_t s) {
   void* p = nullptr;
   if (test_take_alloc_failure() || cudaMallocAsync(&p, bytes, s) != cudaSuccess) {

@@ -44,10 +44,8 @@
 #include <queue>
 #include <vector>
 
-#include "wtg_blocks.cuh"
 #include "wtg_fm_table.cuh"
 #include "wtg_hist.cuh"
-#include "wtg_order.cuh"
 #include "wtg_pass.cuh"
 #include "wtg_select.cuh"
 #include "wtg_tree.cuh"
@@ -359,7 +357,6 @@ __global__ void huff_steps_kernel(const HuffNodeDev* __restrict__ nodes, const H
   }
 }
 
-template <bool BLOCKS>
 struct HuffFm {
   const uint64_t* bits;
   const uint64_t* rt;
@@ -368,6 +365,7 @@ struct HuffFm {
   const uint2* steps;
   const uint64_t* C;
   uint32_t n, sigma;
+  template <bool BLOCKS>
   __device__ __forceinline__ void ranks(uint64_t px, uint64_t py, uint32_t& rx, uint32_t& ry) const {
     if constexpr (BLOCKS) {
       uint32_t ox, oy;
@@ -383,13 +381,14 @@ struct HuffFm {
     }
   }
   // prepends a symbol of the text to the interval [x, y)
+  template <bool BLOCKS>
   __device__ __forceinline__ void step(const uint2* __restrict__ st, HuffSymbol s, uint64_t path, uint32_t base,
                                        uint32_t& x, uint32_t& y) const {
     for (uint32_t d = 0; d < s.len; ++d, path >>= 1) {
       const uint2 c = st[s.first + d];
       const uint64_t at = info->depth[d] + c.x;
       uint32_t rx, ry;
-      ranks(at + x, at + y, rx, ry);
+      ranks<BLOCKS>(at + x, at + y, rx, ry);
       rx -= c.y;
       ry -= c.y;
       const bool one = path & 1;
@@ -399,62 +398,82 @@ struct HuffFm {
     x += base;
     y += base;
   }
+  __device__ __forceinline__ void extend(uint32_t k, uint32_t& x, uint32_t& y) const {
+    const uint32_t c = info->byte_of[k];
+    step<false>(steps, info->sym[c], info->path[c], (uint32_t)C[c], x, y);
+  }
 };
 
-template <bool BLOCKS>
-__global__ void huff_table_kernel(HuffFm<BLOCKS> t, uint64_t prev_count, const uint2* __restrict__ prev,
-                                  uint2* __restrict__ out) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= prev_count * t.sigma) return;
-  const uint32_t k = (uint32_t)(i / prev_count), c = t.info->byte_of[k];
-  const uint2 v = prev ? prev[i - k * prev_count] : make_uint2(0u, t.n);
-  uint32_t x = v.x, y = v.y;
-  if (x < y) t.step(t.steps, t.info->sym[c], t.info->path[c], (uint32_t)t.C[c], x, y);
-  out[i] = x < y ? make_uint2(x, y) : make_uint2(0u, 0u);
+struct HuffShared {
+  HuffSymbol sym[256];
+  uint32_t C[256];
+};
+// a CTA's symbols, C and steps in shared memory (256 threads; nsteps 0: the
+// steps stay where they are)
+__device__ __forceinline__ const uint2* huff_load(const HuffFm& t, uint32_t nsteps, uint2* s_steps, HuffShared& sh) {
+  for (uint32_t i = threadIdx.x; i < nsteps; i += blockDim.x) s_steps[i] = t.steps[i];
+  sh.sym[threadIdx.x] = t.info->sym[threadIdx.x];
+  sh.C[threadIdx.x] = (uint32_t)t.C[threadIdx.x];
+  __syncthreads();
+  return nsteps ? s_steps : t.steps;
 }
 
-template <bool BLOCKS, bool ORD>
-__global__ void __launch_bounds__(256, 5)
-    huff_count_kernel(HuffFm<BLOCKS> t, uint32_t nsteps, int K, const uint2* __restrict__ table,
-                      const uint8_t* __restrict__ pat, const uint64_t* __restrict__ off,
-                      const uint64_t* __restrict__ total, QueryOrder ord, uint64_t m, uint64_t* __restrict__ out) {
+template <bool BLOCKS>
+__device__ __forceinline__ uint32_t huff_search(const HuffFm& t, const uint2* __restrict__ st, const HuffShared& sh,
+                                                PatternReader& rd, uint64_t a, uint64_t i, uint32_t x, uint32_t y) {
+  bool known = true;  // every symbol read so far is one of the text's
+  while (known && i > a && x < y) {
+    const uint32_t c = rd.at(--i);
+    const HuffSymbol s = sh.sym[c];
+    known = s.dense != 0xFFFF;
+    if (known) t.template step<BLOCKS>(st, s, __ldg(t.info->path + c), sh.C[c], x, y);
+  }
+  return known && y > x ? y - x : 0;
+}
+
+// a batch that is not prepared
+__global__ void __launch_bounds__(256)
+    huff_count_kernel(HuffFm t, uint32_t nsteps, const uint8_t* __restrict__ pat, const uint64_t* __restrict__ off,
+                      uint64_t m, uint64_t* __restrict__ out) {
   extern __shared__ uint2 s_steps[];  // nsteps, or none
-  __shared__ HuffSymbol s_sym[256];
-  __shared__ uint32_t s_C[256];
-  for (uint32_t i = threadIdx.x; i < nsteps; i += blockDim.x) s_steps[i] = t.steps[i];
-  s_sym[threadIdx.x] = t.info->sym[threadIdx.x];
-  s_C[threadIdx.x] = (uint32_t)t.C[threadIdx.x];
-  __syncthreads();
-  const uint2* const st = nsteps ? s_steps : t.steps;
+  __shared__ HuffShared sh;
+  const uint2* const st = huff_load(t, nsteps, s_steps, sh);
+  const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= m) return;
+  PatternReader rd(pat, off[m]);
+  out[p] = huff_search<false>(t, st, sh, rd, off[p], off[p + 1], 0u, t.n);
+}
+
+__global__ void __launch_bounds__(256, 5)
+    huff_planned_kernel(HuffFm t, uint32_t nsteps, FmTable table, const uint8_t* __restrict__ pat,
+                        const uint64_t* __restrict__ off, const uint64_t* __restrict__ total, QueryOrder ord, uint64_t m,
+                        uint64_t* __restrict__ out) {
+  extern __shared__ uint2 s_steps[];  // nsteps, or none
+  __shared__ HuffShared sh;
+  const uint2* const st = huff_load(t, nsteps, s_steps, sh);
   uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= m) return;
-  if (ORD && !ordered_query(ord, m, p)) return;
+  const int K = table.first ? (int)ord.flags[TABLE_SYMBOLS] : 0;
+  const bool blocks = t.blocks && ord.flags[MAKE_BLOCKS];
+  if (!ordered_query(ord, m, p)) return;
   const uint64_t a = off[p], b = off[p + 1];
   PatternReader rd(pat, *total);
   uint32_t x = 0, y = t.n;
   uint64_t i = b;
-  bool known = true;  // every symbol read so far is one of the text's
   if (K && b >= a + K) {  // (offsets that decrease: an empty pattern)
     uint32_t at = 0, scale = 1;
+    bool known = true;
     for (int k = 0; k < K; ++k) {
-      const uint32_t d = s_sym[rd.at(--i)].dense;
+      const uint32_t d = sh.sym[rd.at(--i)].dense;
       known = known && d != 0xFFFF;
       at += d * scale;
       scale *= t.sigma;
     }
-    if (known) {
-      const uint2 v = __ldg(table + at);
-      x = v.x;
-      y = v.y;
-    }
+    const uint2 v = known ? __ldg(table.of(K) + at) : make_uint2(0u, 0u);
+    x = v.x;
+    y = v.y;
   }
-  while (known && i > a && x < y) {
-    const uint32_t c = rd.at(--i);
-    const HuffSymbol s = s_sym[c];
-    known = s.dense != 0xFFFF;
-    if (known) t.step(st, s, __ldg(t.info->path + c), s_C[c], x, y);
-  }
-  out[p] = known && y > x ? y - x : 0;
+  out[p] = blocks ? huff_search<true>(t, st, sh, rd, a, i, x, y) : huff_search<false>(t, st, sh, rd, a, i, x, y);
 }
 
 unsigned hgrid(uint64_t items, unsigned per, unsigned cap) {
@@ -920,58 +939,45 @@ int launch_huff_query(HuffImpl& h, int what, const uint64_t* a, const uint64_t* 
   return WTG_OK;
 }
 
-// (levels: the bits of a code on average)
-static bool huff_batch_pays(const HuffImpl& h, uint64_t npat) {
-  return fm_batch_pays(npat, (h.size + h.n - 1) / h.n);
-}
-
-template <bool BLOCKS>
-static int huff_fm_run(HuffImpl& h, const uint4* blocks, const uint64_t* C, const uint8_t* pat, const uint64_t* off,
-                       uint64_t npat, uint64_t* out, cudaStream_t s) {
-  const HuffFm<BLOCKS> v{h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), blocks, h.fminfo.as<HuffFmInfo>(),
-                         h.fmsteps.as<uint2>(), C, (uint32_t)h.n, (uint32_t)h.sigma};
-  const uint32_t in_smem = h.fm_steps <= (uint32_t)HF_SMEM_STEPS ? h.fm_steps : 0u;
-  const bool pays = huff_batch_pays(h, npat);
-  return with_fm_table<uint2>(
-      pays, h.sigma, npat, s,
-      [&](uint64_t prev_count, const uint2* prev, uint2* next) -> int {
-        huff_table_kernel<BLOCKS><<<(unsigned)((prev_count * h.sigma + 127) / 128), 128, 0, s>>>(v, prev_count, prev,
-                                                                                                next);
-        count_launch();
-        WTG_CK(cudaGetLastError());
-        return WTG_OK;
-      },
-      [&](int K, const uint2* table) -> int {
-        return by_length(pays, off, npat, h.err, h.stream, s,
-                         [&](bool sorted, const QueryOrder& o, uint64_t at, uint64_t m) -> int {
-                           auto* const f = sorted ? huff_count_kernel<BLOCKS, true> : huff_count_kernel<BLOCKS, false>;
-                           f<<<(unsigned)((m + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(
-                               v, in_smem, K, table, pat, off + at, off + npat, o, m, out + at);
-                           count_launch();
-                           WTG_CK(cudaGetLastError());
-                           return WTG_OK;
-                         });
-      });
-}
-
 int launch_huff_fm_count(HuffImpl& h, const uint64_t* C, const uint8_t* pat, const uint64_t* off, uint64_t npat,
                          uint64_t* out, cudaStream_t s) {
   if (!npat) return WTG_OK;
   if (!(h.flags & WTG_RANK)) return fail(WTG_ERR_INVALID, "counting needs the rank support");
-  if (h.n >= (1ull << 32) || !h.n) {  // positions beyond 32 bits (and the empty text)
+  const uint64_t levels = h.n ? (h.size + h.n - 1) / h.n : 0;  // the bits of a code on average
+  // positions beyond 32 bits, and the empty text; and batches of a CTA or two, or
+  // with short codes, for which the tables of a CTA are not worth their loads (us
+  // without / with them: 16 patterns of 100 symbols, 2^24 symbols of 4 letters, 147 /
+  // 169, of 200 413 / 423; 2^14 of 8 symbols, 4 letters, 17.5 / 19.2, 2^17 31.5 /
+  // 27.4, 200 letters, 2^10 62 / 50)
+  if (h.n >= (1ull << 32) || !h.n || npat <= 512 || (levels <= 3 && npat <= (1u << 16))) {
     huff_fm_count_kernel<<<(unsigned)((npat + 255) / 256), 256, 0, s>>>(huff_view(h), C, pat, off, npat, out);
     count_launch();
     WTG_CK(cudaGetLastError());
     return WTG_OK;
   }
-  // as for the balanced tree: blocks once the batch probes a good part of them
-  uint4* blocks = h.size && huff_batch_pays(h, npat) && npat >= block_count(h.size) / 8
-                      ? make_blocks(h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), h.size, s)
-                      : nullptr;
-  const int rc = blocks ? huff_fm_run<true>(h, blocks, C, pat, off, npat, out, s)
-                        : huff_fm_run<false>(h, blocks, C, pat, off, npat, out, s);
-  if (blocks) cudaFreeAsync(blocks, s);
-  return rc;
+  HuffFm v{h.bits.as<uint64_t>(), h.bv.rank.as<uint64_t>(), nullptr, h.fminfo.as<HuffFmInfo>(),
+           h.fmsteps.as<uint2>(), C, (uint32_t)h.n, (uint32_t)h.sigma};
+  const uint32_t in_smem = h.fm_steps <= (uint32_t)HF_SMEM_STEPS ? h.fm_steps : 0u;
+  auto plain = [&]() -> int {
+    huff_count_kernel<<<(unsigned)((npat + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(v, in_smem, pat, off, npat,
+                                                                                          out);
+    count_launch();
+    WTG_CK(cudaGetLastError());
+    return WTG_OK;
+  };
+  if (!fm_batch_pays(npat, levels)) return plain();
+  return counted_batches(
+      v, off, npat, (uint32_t)(2 * levels), blocks_in_reach(h.size), h.err, h.stream, s,
+      [&](uint4* blocks, const uint32_t* wanted) { return fill_blocks(blocks, v.bits, v.rt, h.size, wanted, s); },
+      [&](const QueryOrder& o, const FmTable& table, const uint4* blocks, uint64_t at, uint64_t m) -> int {
+        v.blocks = blocks;
+        huff_planned_kernel<<<(unsigned)((m + 255) / 256), 256, in_smem * sizeof(uint2), s>>>(
+            v, in_smem, table, pat, off + at, off + npat, o, m, out + at);
+        count_launch();
+        WTG_CK(cudaGetLastError());
+        return WTG_OK;
+      },
+      plain);
 }
 
 }  // namespace wtg

@@ -16,6 +16,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 #include <string>
 
 #include "../../include/wtg.h"
@@ -354,6 +355,71 @@ struct DevBuf {
   void release(cudaStream_t s);
   template <typename T>
   T* as() const { return (T*)p; }
+};
+
+// Up to two tables that follow from a build alone, made by the first query that
+// wants them, on its stream; queries on other streams wait for `made`.
+struct MadeOnce {
+  DevBuf buf[2];
+  bool ok = false;      // enqueued; a build takes it back
+  bool on_own = false;  // on the handle's own stream
+  cudaEvent_t made = nullptr;
+  std::mutex mu;
+  void release(cudaStream_t s) {
+    buf[0].release(s);
+    buf[1].release(s);
+    ok = false;
+    if (made) cudaEventDestroy(made);
+    made = nullptr;
+  }
+};
+
+// Such tables for kernels launched on stream s while this object lives: made by
+// fill(buffers) -> status where no query after the build has made them (make),
+// and otherwise waited for, as another stream may still be filling them.  A
+// call under stream capture can neither wait for that nor leave anything
+// behind that exists before the graph is launched: tables that are there are
+// used as they are (whoever launches the graph orders it after the work
+// before), others are made in the call, for it alone.
+class Made {
+ public:
+  int rc = WTG_OK;
+  template <typename F>
+  Made(MadeOnce& m, cudaStream_t s, cudaStream_t own_stream, bool make, F fill) : stream_(s) {
+    const bool captured = stream_captures(s);
+    std::lock_guard<std::mutex> lk(m.mu);
+    if (m.ok) {
+      if (!captured && (!m.on_own || s != own_stream)) rc = wait(m);
+      if (rc == WTG_OK) use(m.buf);
+    } else if (make && captured) {
+      if ((rc = fill(own_)) == WTG_OK) use(own_);
+    } else if (make) {
+      if ((rc = fill(m.buf)) == WTG_OK && (rc = record(m)) == WTG_OK) {
+        m.on_own = s == own_stream;
+        m.ok = true;
+        use(m.buf);
+      }
+    }
+  }
+  ~Made() {
+    own_[0].release(stream_);
+    own_[1].release(stream_);
+  }
+  Made(const Made&) = delete;
+  Made& operator=(const Made&) = delete;
+  template <typename T>
+  const T* table(int k) const { return (const T*)p_[k]; }
+
+ private:
+  int wait(MadeOnce& m);
+  int record(MadeOnce& m);
+  void use(const DevBuf* b) {
+    p_[0] = b[0].p;
+    p_[1] = b[1].p;
+  }
+  const cudaStream_t stream_;
+  const void* p_[2] = {nullptr, nullptr};
+  DevBuf own_[2];  // of a captured call
 };
 
 // Scratch of one call that can also do without it (cudaFreeAsync gives it

@@ -23,11 +23,13 @@ struct QueryOrder {
   const uint32_t* flags;  // OrderFlags
 };
 
-// Words that order_check_kernel sets: the batch came in the order of its
-// positions, and nothing of the sort has run (pos and id hold nothing); blocks
-// are to be made for it; blocks were made for it or for a batch of the call
-// before it.
-enum OrderFlags { AS_IS = 0, MAKE_BLOCKS, BLOCKS_MADE, KEYS_DONE, ORDER_FLAGS };
+// Words that order_check_kernel or fm_plan_kernel sets: the batch came in the
+// order of its positions, or its patterns are of about one length, and nothing of
+// the sort has run (pos and id hold nothing); blocks are to be made for it; blocks
+// were made for it or for a batch of the call before it; symbols of a pattern
+// that the interval table answers.  (KEYS_DONE: CTAs of order_keys_kernel that
+// have ended.)
+enum OrderFlags { AS_IS = 0, MAKE_BLOCKS, BLOCKS_MADE, KEYS_DONE, TABLE_SYMBOLS, ORDER_FLAGS = 8 };
 
 // the query that thread k takes; false where there is none
 __device__ __forceinline__ bool ordered_query(const QueryOrder& ord, uint64_t nq, uint64_t& k) {
@@ -39,20 +41,13 @@ __device__ __forceinline__ bool ordered_query(const QueryOrder& ord, uint64_t nq
 // the query numbers.
 constexpr uint64_t ORDER_BATCH = 1ull << 26;
 
-// The 32-bit sort keys: a query's position, and a pattern's length.
+// The 32-bit sort key of a query: its position.
 struct PositionKey {
   const uint64_t* q;
   uint64_t n;
   __device__ __forceinline__ uint32_t operator()(uint64_t k) const {
     const uint64_t i = q[k];
     return (uint32_t)(i < n ? i : n);
-  }
-};
-struct LengthKey {
-  const uint64_t* off;
-  __device__ __forceinline__ uint32_t operator()(uint64_t k) const {
-    const uint64_t a = off[k], b = off[k + 1], m = b > a ? b - a : 0;
-    return (uint32_t)(m < 255 ? m : 255);
   }
 };
 
@@ -227,22 +222,6 @@ int in_order(TreeImpl& t, bool two, const uint64_t* pos, uint64_t nq, cudaStream
       [&](uint64_t at, uint64_t m, uint32_t* flags, uint32_t* hist, uint32_t words) {
         order_check_kernel<<<1, CHECK_THREADS, 0, s>>>(key_of(at), m, lo, at == 0, flags, hist, words);
         count_launch();
-      },
-      launch);
-}
-
-// Patterns by length (one sort pass), in batches that are worth it: a warp runs
-// as long as its longest pattern, and lengths of 8 to 32 left 48 % of the lanes
-// without work.
-template <typename F>
-int by_length(bool pays, const uint64_t* off, uint64_t npat, ErrWord& err_word, cudaStream_t own, cudaStream_t s,
-              F launch) {
-  if (!pays) return launch(false, QueryOrder{}, 0, npat);
-  const ErrUse err(err_word, s, own);
-  return sorted_batches(
-      npat, 0, 1, err.word(), s, [&](uint64_t at) { return LengthKey{off + at}; },
-      [&](uint64_t, uint64_t, uint32_t* flags, uint32_t*, uint32_t words) {
-        cudaMemsetAsync(flags, 0, (ORDER_FLAGS + words) * 4, s);  // (the counts follow the flags)
       },
       launch);
 }

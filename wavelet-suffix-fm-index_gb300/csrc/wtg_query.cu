@@ -354,53 +354,22 @@ static int need(const TreeImpl& t, uint32_t f, const char* what) {
 
 WTG_WAIT_LIMIT_SETTER(query)
 
-static int make_node_tables(const TreeImpl& t, DevBuf& tab, DevBuf& step, cudaStream_t s) {
+static int make_node_tables(const TreeImpl& t, DevBuf* buf, cudaStream_t s) {
   int rc;
   const uint64_t heap = 1ull << t.levels, nodes = heap - 1;
-  if ((rc = tab.ensure(nodes * sizeof(ulonglong2), s))) return rc;
-  if ((rc = step.ensure((nodes + 1) * sizeof(uint2), s))) return rc;
+  if ((rc = buf[0].ensure(nodes * sizeof(ulonglong2), s))) return rc;
+  if ((rc = buf[1].ensure((nodes + 1) * sizeof(uint2), s))) return rc;
   node_table_kernel<<<(unsigned)((nodes + 255) / 256), 256, 0, s>>>(
       t.bits.as<uint64_t>(), t.bv.rank.as<uint64_t>(), t.zeros.as<uint32_t>(), t.zeros.as<uint32_t>() + heap, t.n,
-      t.levels, nodes, tab.as<ulonglong2>(), step.as<uint2>());
+      t.levels, nodes, buf[0].as<ulonglong2>(), buf[1].as<uint2>());
   count_launch();
   WTG_CK(cudaGetLastError());
   return WTG_OK;
 }
 
-// the tree's own tables, made or waited for
-static int shared_node_tables(TreeImpl& t, cudaStream_t s, bool make) {
-  if (t.node_tab_ok) {
-    if (!t.node_on_own || s != t.stream) WTG_CK(cudaStreamWaitEvent(s, t.node_made, 0));
-    return WTG_OK;
-  }
-  if (!make) return WTG_OK;
-  int rc;
-  if (!t.node_made) WTG_CK(cudaEventCreateWithFlags(&t.node_made, cudaEventDisableTiming));
-  if ((rc = make_node_tables(t, t.node_tab, t.node_step, s))) return rc;
-  WTG_CK(cudaEventRecord(t.node_made, s));
-  t.node_on_own = s == t.stream;
-  t.node_tab_ok = true;
-  return WTG_OK;
-}
-
-NodeTables::NodeTables(TreeImpl& t, cudaStream_t s, bool make) : stream(s) {
-  const bool captured = stream_captures(s);
-  std::lock_guard<std::mutex> lk(t.node_mu);
-  if (!captured) rc = shared_node_tables(t, s, make);
-  if (rc == WTG_OK && t.node_tab_ok) {
-    tab = t.node_tab.as<ulonglong2>();
-    step = t.node_step.as<uint2>();
-  } else if (rc == WTG_OK && captured && make) {
-    if ((rc = make_node_tables(t, own_tab, own_step, s))) return;
-    tab = own_tab.as<ulonglong2>();
-    step = own_step.as<uint2>();
-  }
-}
-
-NodeTables::~NodeTables() {
-  own_tab.release(stream);
-  own_step.release(stream);
-}
+NodeTables::NodeTables(TreeImpl& t, cudaStream_t s, bool make)
+    : Made(t.node_tables, s, t.stream, make, [&](DevBuf* buf) { return make_node_tables(t, buf, s); }),
+      tab(table<ulonglong2>(0)), step(table<uint2>(1)) {}
 
 // Blocks (built from the bitvector for the call: 1.1 ms for 2^30 x 20 levels,
 // 112 M blocks) pay once the batch probes a good part of them and there are

@@ -1,6 +1,5 @@
 // wtg_tree.cuh -- device-side state of one wavelet tree (internal).
 #pragma once
-#include <mutex>
 #include <vector>
 
 #include "wtg_internal.cuh"
@@ -35,14 +34,10 @@ struct TreeImpl {
   BvSupport bv;
   DevBuf lvl_args;
   bool lvl_args_ok = false;
-  // node tables (see NodeTables): made by the first query after a build that
-  // uses them, on its stream; queries on other streams wait for node_made
-  DevBuf node_tab;   // per heap node: bit offset of its start, ones before it
-  DevBuf node_step;  // per heap node: the constants that take a position to its child
-  bool node_tab_ok = false;
-  bool node_on_own = false;  // made on the tree's own stream
-  cudaEvent_t node_made = nullptr;
-  std::mutex node_mu;
+  // per heap node: bit offset of its start and ones before it; the constants that
+  // take a position to its child (see NodeTables)
+  MadeOnce node_tables;
+  MadeOnce fm_steps;  // per symbol, for FM-index counting
   uint64_t gen = 0;  // builds so far (indexes built on the tree record it)
   // host destinations filled while the build runs (wtg_tree_build_out): the
   // bits of each level are copied on copy_stream as soon as its pass is done
@@ -69,25 +64,11 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
 int tree_nodes(TreeImpl& t, int ib, uint64_t n_entries, void* d_out);
 void tree_release(TreeImpl& t);
 
-// The tree's node tables for kernels launched on stream s while this object
-// lives: made where no query after the build has made them (make), and
-// otherwise waited for, as another stream may still be filling them.  A call
-// under stream capture can neither wait for that nor leave anything behind that
-// exists before the graph is launched: tables that are there are used as they
-// are (whoever launches the graph orders it after the work before), others are
-// made in the call, for it alone.
-struct NodeTables {
-  const ulonglong2* tab = nullptr;
-  const uint2* step = nullptr;
-  int rc = WTG_OK;
+// The tree's node tables for kernels launched on stream s
+struct NodeTables : Made {
+  const ulonglong2* tab;
+  const uint2* step;
   NodeTables(TreeImpl& t, cudaStream_t s, bool make = true);
-  ~NodeTables();
-  NodeTables(const NodeTables&) = delete;
-  NodeTables& operator=(const NodeTables&) = delete;
-
- private:
-  DevBuf own_tab, own_step;  // of a captured call
-  cudaStream_t stream;
 };
 
 // query launchers (wtg_query.cu); all arrays are device arrays
