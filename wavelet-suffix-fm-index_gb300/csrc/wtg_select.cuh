@@ -179,14 +179,15 @@ __device__ __forceinline__ uint64_t last_arg_end(const uint64_t* __restrict__ wo
 // for what a sector holds beyond the args' word.  (us word by word / by sectors:
 // level selects of 2^16 queries, 2^28 x 20 levels, 12.4 / 10.3.)
 constexpr uint64_t SEL_MANY = 1ull << 17;
-// A bitvector's selects: by words in such batches where a word or two hold the
-// arg asked for: most of the bits are args, or a third where L2 holds them.  2^22
-// queries over 2^30 bits, 97 % of them args 56 / 67 us, half 64 / 68, 3 % 240 / 170;
-// over the levels of 2^22 x 20, 64 % args, 71 / 76, 36 % 81 / 84; of 2^28 x 20, 163
+// A bitvector's selects: by words where a word or two hold the arg asked for: in
+// such batches where most of the bits are args, in larger ones where a third are
+// and L2 holds the bits.  2^22 queries over 2^30 bits, 97 % of them args 56 / 67 us
+// (2^18 8.3 / 10.3), half 64 / 68 (2^20 20.9 / 21.0), 3 % 240 / 170; over the levels
+// of 2^22 x 20, 64 % args, 71 / 76, 36 % 81 / 84 (2^18 14.5 / 12.4); of 2^28 x 20, 163
 // / 154, 131 / 119.
 inline bool select_by_words(const SelectDev& sd, uint64_t size, uint64_t nq) {
-  const bool in_l2 = size / 8 <= (160ull << 20);
-  return nq >= SEL_MANY && sd.arg_cnt >= (in_l2 ? size / 3 : size / 4 * 3);
+  if (sd.arg_cnt >= size / 4 * 3) return nq >= SEL_MANY;
+  return nq >= 16 * SEL_MANY && sd.arg_cnt >= size / 3 && size / 8 <= (160ull << 20);
 }
 
 inline SelView sel_view(const BvSupport& bv, int t_b) {
