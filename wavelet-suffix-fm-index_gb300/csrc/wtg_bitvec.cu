@@ -415,12 +415,14 @@ __global__ void __launch_bounds__(SD_THREADS)
 // and 64-bit shifts a word and was bound by issue: 0.98 ms of the 2^30 x 20
 // build's 5.2 M superblocks, against 0.3 ms of traffic.)  Wider entries go
 // word by word through shared memory.  The blocks after them: m_superblock,
-// entry i = position of arg 4096*i, width logn.  These kernels and those of the
-// long blocks do nothing after an error: the starts and pool offsets of a pass
-// whose wait ran out lead out of range.
+// entry i = position of arg 4096*i, width logn.  After an error nothing goes to
+// the pool, and the kernels of the long blocks do nothing: the starts and pool
+// offsets of a pass whose wait ran out lead out of range.  (The error word is
+// tested where the pool is written: before the reads its own read came first in
+// every block, 2 us of the 842 Mbit's.)
 template <int T_B>
 __device__ __forceinline__ void mini_blocks_warp(const SelBuild& sb, uint64_t i0, const uint32_t* __restrict__ samples,
-                                                 uint64_t samp_last, uint32_t (*ent)[64]) {
+                                                 uint64_t samp_last, uint32_t error, uint32_t (*ent)[64]) {
   const uint32_t lane = threadIdx.x & 31, h = lane >> 4, ql = lane & 15;
   const uint64_t i = i0 + h;
   const bool in = i < sb.nsb;
@@ -466,7 +468,7 @@ __device__ __forceinline__ void mini_blocks_warp(const SelBuild& sb, uint64_t i0
         const int32_t sh = (int32_t)(j * wdt) - (int32_t)lo;
         out |= sh >= 0 ? (v << sh) : (v >> (-sh));
       }
-      sb.pool[off + q] = out;
+      if (!error) sb.pool[off + q] = out;
     }
     return;
   }
@@ -485,7 +487,7 @@ __device__ __forceinline__ void mini_blocks_warp(const SelBuild& sb, uint64_t i0
     const uint64_t v = __shfl_sync(0xffffffffu, piece, j & 15, 16);
     if (more) out |= v << sh;
   }
-  if (ql < wdt) sb.pool[off + ql] = out;
+  if (ql < wdt && !error) sb.pool[off + ql] = out;
 }
 
 __global__ void __launch_bounds__(256)
@@ -494,7 +496,8 @@ __global__ void __launch_bounds__(256)
   __shared__ uint32_t ent[256 / 32][2][64];
   const int t_b = blockIdx.y;
   const SelBuild& sb = sb2.t[t_b];
-  if (!sb.on || *err) return;
+  if (!sb.on) return;
+  const uint32_t error = *err;
   const uint64_t mini_blocks = (sb.nsb + 15) / 16;
   if (blockIdx.x >= mini_blocks) {
     const uint64_t q = (blockIdx.x - mini_blocks) * 256 + threadIdx.x;
@@ -503,8 +506,8 @@ __global__ void __launch_bounds__(256)
   }
   const uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2;
   if (i0 >= sb.nsb) return;
-  if (t_b) mini_blocks_warp<1>(sb, i0, samples, samp_last, ent[threadIdx.x >> 5]);
-  else mini_blocks_warp<0>(sb, i0, samples, samp_last, ent[threadIdx.x >> 5]);
+  if (t_b) mini_blocks_warp<1>(sb, i0, samples, samp_last, error, ent[threadIdx.x >> 5]);
+  else mini_blocks_warp<0>(sb, i0, samples, samp_last, error, ent[threadIdx.x >> 5]);
 }
 
 // Long blocks, step 1: the position of every arg of every long superblock,
