@@ -144,10 +144,11 @@ __device__ __forceinline__ uint32_t fm_search(const FmTree& t, const uint2* __re
   return known && y > x ? y - x : 0;
 }
 
-// A batch that is not prepared.  (Bound by the chain of its reads; held to 32
-// registers it spills: 2^16 patterns of 100 symbols, 2^24 symbols of 4 letters,
-// 160 us, 222 so.)
-__global__ void __launch_bounds__(256)
+// A batch that is not prepared.  Bound by the chain of its reads, which the
+// compiler issues ahead where it has 48 registers (5 CTAs an SM): 2^14 patterns of
+// 100 symbols, 2^24 symbols of 4 letters, 81 us, without the bound (40 registers)
+// 117, at 32, which spill, 143.
+__global__ void __launch_bounds__(256, 5)
     fm_count_kernel(FmTree t, const uint8_t* __restrict__ pat, const uint64_t* __restrict__ off, uint64_t m,
                     uint64_t* __restrict__ out) {
   extern __shared__ uint2 s_steps[];

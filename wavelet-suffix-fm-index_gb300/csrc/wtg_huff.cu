@@ -431,8 +431,10 @@ __device__ __forceinline__ uint32_t huff_search(const HuffFm& t, const uint2* __
   return known && y > x ? y - x : 0;
 }
 
-// a batch that is not prepared
-__global__ void __launch_bounds__(256)
+// A batch that is not prepared.  (At 5 CTAs an SM the compiler takes 48 registers,
+// without the bound 40 and half as long again: 60000 patterns over 2^24 zipf bytes
+// 166 us, 222 so.)
+__global__ void __launch_bounds__(256, 5)
     huff_count_kernel(HuffFm t, uint32_t nsteps, const uint8_t* __restrict__ pat, const uint64_t* __restrict__ off,
                       uint64_t m, uint64_t* __restrict__ out) {
   extern __shared__ uint2 s_steps[];  // nsteps, or none
@@ -944,12 +946,7 @@ int launch_huff_fm_count(HuffImpl& h, const uint64_t* C, const uint8_t* pat, con
   if (!npat) return WTG_OK;
   if (!(h.flags & WTG_RANK)) return fail(WTG_ERR_INVALID, "counting needs the rank support");
   const uint64_t levels = h.n ? (h.size + h.n - 1) / h.n : 0;  // the bits of a code on average
-  // positions beyond 32 bits, and the empty text; and batches of a CTA or two, or
-  // with short codes, for which the tables of a CTA are not worth their loads (us
-  // without / with them: 16 patterns of 100 symbols, 2^24 symbols of 4 letters, 147 /
-  // 169, of 200 413 / 423; 2^14 of 8 symbols, 4 letters, 17.5 / 19.2, 2^17 31.5 /
-  // 27.4, 200 letters, 2^10 62 / 50)
-  if (h.n >= (1ull << 32) || !h.n || npat <= 512 || (levels <= 3 && npat <= (1u << 16))) {
+  if (h.n >= (1ull << 32) || !h.n) {  // positions beyond 32 bits (and the empty text)
     huff_fm_count_kernel<<<(unsigned)((npat + 255) / 256), 256, 0, s>>>(huff_view(h), C, pat, off, npat, out);
     count_launch();
     WTG_CK(cudaGetLastError());
