@@ -164,11 +164,11 @@ __global__ void lsel_fit_kernel(SelView v, const LselLevel* __restrict__ lv, int
     const uint64_t len = umin64((uint64_t)1 << d.g, d.m - (j << d.g));
     const uint64_t P = min((uint64_t)samples, len);
     const uint64_t off = (uint64_t)l * n;
-    const uint64_t y0 = select_dev(v, d.A + kS) - off;
+    const uint64_t y0 = select_dev<true>(v, d.A + kS) - off;
     double sx = 0, sy = 0, sxx = 0, sxy = 0;
     for (uint64_t i = lane; i < P; i += 32) {
       const uint64_t x = len > P ? (i * len) / P : i;
-      const double y = (double)(select_dev(v, d.A + kS + x) - off - y0);
+      const double y = (double)(select_dev<true>(v, d.A + kS + x) - off - y0);
       const double xd = (double)x;
       sx += xd;
       sy += y;

@@ -263,8 +263,8 @@ __global__ void wt_range_report_kernel(const uint64_t* __restrict__ tree, const 
         for (int kk = L; kk > 0; --kk) {
           const uint64_t hn = (1ull << (kk - 1)) - 1 + (path >> (L - kk + 1));  // node at level kk - 1
           const ulonglong2 nd = __ldg(tab + hn);
-          if ((path >> (L - kk)) & 1) i = select_dev(s1, nd.y + i) - nd.x + 1;
-          else i = select_dev(s0, nd.x - nd.y + i) - nd.x + 1;
+          if ((path >> (L - kk)) & 1) i = select_dev<true>(s1, nd.y + i) - nd.x + 1;
+          else i = select_dev<true>(s0, nd.x - nd.y + i) - nd.x + 1;
         }
         pos[base + emitted + t] = i - 1;
         val[base + emitted + t] = path;
