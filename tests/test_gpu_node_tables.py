@@ -72,3 +72,20 @@ def test_captured_queries(tree, table_first):
     del g
     torch.cuda.synchronize()
     assert np.array_equal(t.access(idx.astype(np.uint64)), sym)
+
+
+def test_level_selects_on_other_streams_wait_for_the_level_table(tree):
+    torch, t, seq, idx, first = tree
+    level, k = np.full(NQ, L - 1, dtype=np.uint64), np.arange(1, NQ + 1, dtype=np.uint64)
+    d_level, d_k = (torch.from_numpy(x.view(np.int64)).cuda() for x in (level, k))
+    out = torch.zeros(NQ, dtype=torch.int64, device="cuda")
+    slow = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(slow):
+        torch.cuda._sleep(400_000_000)
+    t.level_select_device(1, d_level.data_ptr(), d_k.data_ptr(), NQ, out.data_ptr(), slow.cuda_stream)
+    got = t.level_select(level, k)  # on the tree's own stream
+    order = np.argsort(seq >> 1, kind="stable")  # the last level's order
+    assert np.array_equal(got, np.flatnonzero(seq[order] & 1)[:NQ].astype(np.uint64))
+    torch.cuda.synchronize()
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), got)

@@ -159,8 +159,7 @@ int tree_build(TreeImpl& t, const void* d_seq, uint64_t n, int eb, int L, uint32
   t.elem_bytes = eb;
   t.flags = flags;
   t.bit_words = (n * (uint64_t)L + 63) / 64;
-  t.lvl_args_ok = false;
-  t.node_tables.ok = t.fm_steps.ok = false;
+  t.node_tables.ok = t.level_args.ok = t.fm_steps.ok = false;
   ++t.gen;
   const uint64_t heap = 1ull << L;  // heap ids 0 .. 2^L - 2, plus one pad entry
 
@@ -380,8 +379,7 @@ void tree_release(TreeImpl& t) {
   t.work.release(s);
   t.scan_tmp.release(s);
   t.err.release(s);
-  t.lvl_args.release(s);
-  t.lvl_args_ok = false;
+  t.level_args.release(s);
   t.node_tables.release(s);
   t.fm_steps.release(s);
   t.scratch.release(s);

@@ -540,31 +540,31 @@ int need_supports(const TreeImpl& t, uint32_t f) {
 
 }  // namespace
 
-int tree_level_args(TreeImpl& t, cudaStream_t s) {
-  int rc;
-  if (t.lvl_args_ok) return WTG_OK;
-  if ((rc = need_supports(t, WTG_RANK))) return rc;
-  if ((rc = t.lvl_args.ensure((t.levels + 1) * sizeof(uint64_t), s))) return rc;
-  count_launch();
-  level_args_kernel<<<1, 32, 0, s>>>(t.bv.rank.as<uint64_t>(), t.bits.as<uint64_t>(), t.n, t.levels,
-                                     t.lvl_args.as<uint64_t>());
-  WTG_CK(cudaGetLastError());
-  t.lvl_args_ok = true;
-  return WTG_OK;
-}
+LevelArgs::LevelArgs(TreeImpl& t, cudaStream_t s)
+    : Made(t.level_args, s, t.stream, true, [&](DevBuf* buf) -> int {
+        int rc;
+        if ((rc = need_supports(t, WTG_RANK))) return rc;
+        if ((rc = buf[0].ensure((t.levels + 1) * sizeof(uint64_t), s))) return rc;
+        count_launch();
+        level_args_kernel<<<1, 32, 0, s>>>(t.bv.rank.as<uint64_t>(), t.bits.as<uint64_t>(), t.n, t.levels,
+                                           buf[0].as<uint64_t>());
+        WTG_CK(cudaGetLastError());
+        return WTG_OK;
+      }) {}
 
 int launch_level_select(TreeImpl& t, int t_b, const uint64_t* level, const uint64_t* k, uint64_t nq,
                         uint64_t* out, cudaStream_t s) {
   int rc;
   if ((rc = need_supports(t, WTG_RANK | (t_b ? WTG_SELECT1 : WTG_SELECT0)))) return rc;
   if (nq == 0) return WTG_OK;
-  if ((rc = tree_level_args(t, s))) return rc;
+  const LevelArgs args(t, s);
+  if (args.rc) return args.rc;
   const bool words = select_by_words(t.bv.sel[t_b], t.bv.size, nq);
   const unsigned grid = (unsigned)((nq + 255) / 256);
   count_launch();
   auto* const f = t_b ? words ? level_select_kernel<1, true> : level_select_kernel<1, false>
                       : words ? level_select_kernel<0, true> : level_select_kernel<0, false>;
-  f<<<grid, 256, 0, s>>>(sel_view(t.bv, t_b), t.lvl_args.as<uint64_t>(), t.n, t.levels, level, k, nq, out);
+  f<<<grid, 256, 0, s>>>(sel_view(t.bv, t_b), args.table<uint64_t>(0), t.n, t.levels, level, k, nq, out);
   WTG_CK(cudaGetLastError());
   return WTG_OK;
 }
@@ -626,9 +626,10 @@ int lsel_build(LselImpl& m, TreeImpl& t, uint32_t segments, uint32_t samples, ui
   m.max_window = max_window;
   m.L = L;
   m.n = n;
-  if ((rc = tree_level_args(t, s))) return rc;
+  const LevelArgs args(t, s);
+  if (args.rc) return args.rc;
   std::vector<uint64_t> la(L + 1);
-  WTG_CK(cudaMemcpyAsync(la.data(), t.lvl_args.p, (L + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+  WTG_CK(cudaMemcpyAsync(la.data(), args.table<uint64_t>(0), (L + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   WTG_CK(cudaStreamSynchronize(s));
 
   for (int tb = 0; tb < 2; ++tb) {

@@ -19,8 +19,7 @@ struct LselImpl;
 //   err        the error word, then per group of levels a tile counter and
 //              look-back status words
 //   bv         rank/select supports over `bits`
-//   lvl_args   ones before each level start, L + 1 words (filled on first use
-//              after a build by tree_level_args)
+//   level_args ones before each level start, L + 1 words
 struct TreeImpl {
   uint64_t n = 0;
   int levels = 0;
@@ -32,8 +31,7 @@ struct TreeImpl {
   DevBuf seq, bits, zeros, work, scan_tmp, scratch, nodes, qbuf, qout;
   ErrWord err;  // followed by the status words of the build
   BvSupport bv;
-  DevBuf lvl_args;
-  bool lvl_args_ok = false;
+  MadeOnce level_args;
   // per heap node: bit offset of its start and ones before it; the constants that
   // take a position to its child (see NodeTables)
   MadeOnce node_tables;
@@ -114,7 +112,9 @@ int launch_wt_expand_ranges(TreeImpl& t, uint64_t voff, const uint64_t* ranges, 
 // wt_int_par.hpp:651-656) with the whole level as the node: for each query
 // (level, k) the position, inside the level, of the level's k-th one
 // (t_b = 1) or zero (t_b = 0); UINT64_MAX when the level has fewer than k
-int tree_level_args(TreeImpl& t, cudaStream_t s);
+struct LevelArgs : Made {  // the ones before each level start, for kernels on stream s
+  LevelArgs(TreeImpl& t, cudaStream_t s);
+};
 int launch_level_select(TreeImpl& t, int t_b, const uint64_t* level, const uint64_t* k, uint64_t nq,
                         uint64_t* out, cudaStream_t s);
 
