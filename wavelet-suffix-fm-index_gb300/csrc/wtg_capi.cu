@@ -287,9 +287,11 @@ int wtg_tree_build_out(const void* seq, uint64_t n, int elem_bytes, int levels, 
     if (ce != cudaSuccess) rc = cuda_fail(ce, "copies of the outputs");
   }
   if (rc != WTG_OK) {
-    // a build that stopped before its pre-pass waited for every piece
-    // leaves no copy in flight into the tree's input buffer
+    // a build that stopped leaves no copy in flight, neither into the tree's input
+    // buffer nor into the caller's arrays
     if (pieces) cudaStreamSynchronize(t.in_stream);
+    cudaStreamSynchronize(t.stream);
+    cudaStreamSynchronize(t.copy_stream);
     if (fresh) wtg_tree_free(T);
     return rc;
   }
