@@ -57,6 +57,13 @@ typedef struct wtg_lsel wtg_lsel; /* learned select index over a tree's levels *
 typedef struct wtg_batch wtg_batch; /* batched builds of many short texts */
 typedef struct wtg_huff wtg_huff;   /* Huffman-shaped wavelet tree of a byte text */
 
+/* Streams and threads: a handle's build, getters and host queries run on its
+ * own stream (the one given to the first _device build, or one of its own) and
+ * use its buffers, one call at a time.  _device queries on a built handle may run
+ * on any stream, several at once: what they share follows from the build and is
+ * ordered by the library; what they write beside their outputs is scratch of the
+ * call.  The caller orders them after the build and before a rebuild or free, and
+ * may capture them into CUDA graphs. */
 const char* wtg_last_error(void);
 int wtg_version(void);
 /* Number of kernel launches issued by this process so far (all entry points). */

@@ -33,7 +33,8 @@
 // i = symbol i), and digit counts are popcounts of masks.  A scattering pass
 // takes about 72 warp instructions per 32 symbols for its four levels, where
 // a ballot per level and 32 symbols took 36 for each level; it is bound by the
-// integer ALU pipe (65 %) and shared-memory latency at 21-24 warps per SM.
+// integer ALU pipe (54-66 %) and shared-memory latency at 15-24 warps per SM
+// (two CTAs for 4-byte symbols, three for narrower ones).
 // At 2^30 symbols a pass takes 3.5 ms (4 to 2 bytes), 3.0 ms (2 bytes), 2.9
 // ms (1 byte), the last one 2.1 ms, the count passes 0.32-0.75 ms; a level
 // pass took 1.43 ms before, 19 of them.  Measured and not kept: 32 warps per
